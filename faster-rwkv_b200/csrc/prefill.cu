@@ -1182,7 +1182,7 @@ __global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
 }
 
 // RWKV-4 WKV over rows (WkvForwardOne, att.cu:30-62, with the sigmoid of att.cu:154-159 fused): one thread per
-// (stream, channel).  Seq mode: one stream, T rows in order; batch mode: row b is the one token of stream b.
+// (stream, channel), row b is the one token of stream b (prompts of one stream: wkv4_seq_kernel).
 //   out[row, c] = sigmoid(r) * wkv (fp16, the operand of the output projection); aa, bb, pp updated in place.
 __global__ void __launch_bounds__(256) wkv4_rows_kernel(Wkv4Args a) {
   pdl_trigger();
@@ -1193,8 +1193,8 @@ __global__ void __launch_bounds__(256) wkv4_rows_kernel(Wkv4Args a) {
   float *st = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(a.state) + (size_t)b * a.state_stride);
   float aa = st[c], bb = st[a.C + c], pp = st[2 * a.C + c];
   const float u = a.first[c], w = a.decay[c];
-  const int t0 = a.batch_mode ? b : 0, t1 = a.batch_mode ? b + 1 : a.T;
-  for (int t = t0; t < t1; ++t) {
+  {
+    const int t = b;
     const size_t o = (size_t)t * a.C + c;
     float k, v, rp;
     if (a.split > 1) {
@@ -1225,6 +1225,109 @@ __global__ void __launch_bounds__(256) wkv4_rows_kernel(Wkv4Args a) {
     pp = pm;
   }
   st[c] = aa; st[a.C + c] = bb; st[2 * a.C + c] = pp;
+}
+
+// RWKV-4 WKV over the tokens of ONE stream (prompts).  The recurrence is associative -- a run of tokens acts on the
+// state as (aa, bb, pp) -> decay by exp(len * w), plus the run's own sums -- so the prompt is cut into 64 chunks that
+// are reduced side by side, combined by a prefix scan, and walked again from their start states.  One CTA holds 16
+// channels x 64 chunks (a 64-byte piece of each row per half warp) and does all three steps: no scratch in global
+// memory, one launch.  Up to 1024 tokens a thread keeps its chunk's k and v in registers between the two walks (LEN
+// tokens; 0: read again).  What bounds it: the serial walk it replaces was one dependent expf chain of T steps on C
+// threads, 700 us a layer at T = 1000, C = 2048; this form is 2 x ceil(T / 64) steps on 64 C threads.
+constexpr int W4_CH = 16, W4_CHUNKS = 64, W4_THREADS = W4_CH * W4_CHUNKS;
+// state (a1, b1, p1) followed by a run of decay d = len * w with sums (a2, b2, p2)
+__device__ __forceinline__ void wkv4_join(float &a, float &b, float &p, float d, float a2, float b2, float p2) {
+  const float pd = p + d, pm = fmaxf(pd, p2);
+  const float e1 = expf(pd - pm), e2 = expf(p2 - pm);
+  a = e1 * a + e2 * a2;
+  b = e1 * b + e2 * b2;
+  p = pm;
+}
+template <int LEN>
+__global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
+  pdl_trigger();
+  pdl_wait();
+  // [value][channel][chunk], rows padded by one word
+  __shared__ float sh[3][W4_CH][W4_CHUNKS + 1];
+  __shared__ float half_tot[3][W4_CH];
+  const int cl = threadIdx.x & (W4_CH - 1), ck = threadIdx.x >> 4;
+  const int c = blockIdx.x * W4_CH + cl;
+  const int len = (a.T + W4_CHUNKS - 1) / W4_CHUNKS;           // LEN == 0 or len <= LEN
+  const int t0 = min(a.T, ck * len), t1 = min(a.T, t0 + len);
+  float *st = reinterpret_cast<float *>(a.state);
+  const float u = a.first[c], w = a.decay[c];
+  const float *kp = a.k + c, *vp = a.v + c, *rp = a.r + c;
+  constexpr int NR = LEN > 0 ? LEN : 1;
+  float kr[NR], vr[NR];
+  float aa = 0.f, bb = 0.f, pp = -1e30f;
+  auto absorb = [&](float k, float v) {
+    const float ww = w + pp, pm = fmaxf(ww, k);
+    const float e1 = expf(ww - pm), e2 = expf(k - pm);
+    aa = e1 * aa + e2 * v;
+    bb = e1 * bb + e2;
+    pp = pm;
+  };
+  if (LEN > 0) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+      if (t0 + i < t1) { kr[i] = kp[(size_t)(t0 + i) * a.C]; vr[i] = vp[(size_t)(t0 + i) * a.C]; }
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+      if (t0 + i < t1) absorb(kr[i], vr[i]);
+  } else {
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) absorb(kp[(size_t)t * a.C], vp[(size_t)t * a.C]);
+  }
+  sh[0][cl][ck] = aa; sh[1][cl][ck] = bb; sh[2][cl][ck] = pp;
+  __syncthreads();
+  {
+    // inclusive scan over the chunks: warp pair (2 ch, 2 ch + 1) takes channel ch, lanes along the chunks.  The decay
+    // of a joined run is the distance between the runs' ends (the last chunks of a ragged prompt are short or empty).
+    const int ch = threadIdx.x >> 6, j = threadIdx.x & 63, lane = threadIdx.x & 31;
+    const float wc = a.decay[blockIdx.x * W4_CH + ch];
+    float xa = sh[0][ch][j], xb = sh[1][ch][j], xp = sh[2][ch][j];
+    const int end_j = min(a.T, (j + 1) * len);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      float ya = __shfl_up_sync(0xffffffffu, xa, o), yb = __shfl_up_sync(0xffffffffu, xb, o), yp = __shfl_up_sync(0xffffffffu, xp, o);
+      if (lane >= o) {
+        wkv4_join(ya, yb, yp, wc * (float)(end_j - min(a.T, (j - o + 1) * len)), xa, xb, xp);
+        xa = ya; xb = yb; xp = yp;
+      }
+    }
+    if (j == 31) { half_tot[0][ch] = xa; half_tot[1][ch] = xb; half_tot[2][ch] = xp; }
+    __syncthreads();
+    if (j >= 32) {
+      float ya = half_tot[0][ch], yb = half_tot[1][ch], yp = half_tot[2][ch];
+      wkv4_join(ya, yb, yp, wc * (float)(end_j - min(a.T, 32 * len)), xa, xb, xp);
+      xa = ya; xb = yb; xp = yp;
+    }
+    sh[0][ch][j] = xa; sh[1][ch][j] = xb; sh[2][ch][j] = xp;
+  }
+  __syncthreads();
+  // this chunk's start state: the stream's state followed by all chunks before
+  aa = st[c]; bb = st[a.C + c]; pp = st[2 * a.C + c];
+  __syncthreads();                       // every thread has read the state the last chunk overwrites
+  if (ck > 0) wkv4_join(aa, bb, pp, w * (float)t0, sh[0][cl][ck - 1], sh[1][cl][ck - 1], sh[2][cl][ck - 1]);
+  auto step = [&](int t, float k, float v, float r_pre) {
+    const float r = 1.f / (1.f + expf(-r_pre));
+    const float ww = u + k, pm = fmaxf(pp, ww);
+    const float e1 = expf(pp - pm), e2 = expf(ww - pm);
+    const float y = r * ((e1 * aa + e2 * v) / (e1 * bb + e2));
+    const __half oh = __float2half_rn(y);
+    a.out[(size_t)t * a.C + c] = oh;
+    if (a.out_lo) a.out_lo[(size_t)t * a.C + c] = __float2half_rn(y - __half2float(oh));
+    absorb(k, v);
+  };
+  if (LEN > 0) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+      if (t0 + i < t1) step(t0 + i, kr[i], vr[i], rp[(size_t)(t0 + i) * a.C]);
+  } else {
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) step(t, kp[(size_t)t * a.C], vp[(size_t)t * a.C], rp[(size_t)t * a.C]);
+  }
+  if (ck == W4_CHUNKS - 1) { st[c] = aa; st[a.C + c] = bb; st[2 * a.C + c] = pp; }
 }
 
 // greedy sample of every row: index of the largest logit (lowest index on ties).  ctl (optional): the id also goes
@@ -1528,7 +1631,17 @@ cudaError_t launch_wkv5_seq(const SeqWkvArgs &a, int H, cudaStream_t st) {
   return cudaGetLastError();
 }
 cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
-  dim3 grid((a.C + 255) / 256, a.batch_mode ? a.T : 1);
+  if (!a.batch_mode) {
+    const dim3 grid(a.C / W4_CH), block(W4_THREADS);
+    const int len = (a.T + W4_CHUNKS - 1) / W4_CHUNKS;
+    if (len <= 1) launch_k(wkv4_seq_kernel<1>, grid, block, 0, st, a);
+    else if (len <= 4) launch_k(wkv4_seq_kernel<4>, grid, block, 0, st, a);
+    else if (len <= 12) launch_k(wkv4_seq_kernel<12>, grid, block, 0, st, a);
+    else if (len <= 16) launch_k(wkv4_seq_kernel<16>, grid, block, 0, st, a);
+    else launch_k(wkv4_seq_kernel<0>, grid, block, 0, st, a);
+    return cudaGetLastError();
+  }
+  dim3 grid((a.C + 255) / 256, a.T);
   launch_k(wkv4_rows_kernel, dim3(grid), dim3(256), 0, st, a);
   return cudaGetLastError();
 }

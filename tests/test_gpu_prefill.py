@@ -179,3 +179,23 @@ def test_long_prompts_in_pipelined_pieces(pkg, orc, synth, monkeypatch, name, st
     ids2 = [int(t) for t in synth.token_ids(shape, 2048 + 300, seed=3)]
     _close(m.run(ids2), ref.run_seq(ids2), "second long prompt")
     m.close()
+
+
+@pytest.mark.parametrize("T", [2, 64, 65, 257, 769, 1023, 1090])
+def test_rwkv4_prompt_scan(pkg, orc, synth, T):
+    """RWKV-4 prompts are scanned in 64 chunks (of 1, 2, 5, 13, 16 and 18 tokens here; the last ones short or empty):
+    logits, the WKV state after the prompt and the token after it against the oracle's token loop."""
+    shape = synth.SHAPES["tiny4b"]
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), "fp32")
+    ref = orc.OracleModel(shape, tensors, synth.param_names(shape), rescale_every=0, weight_format="int8", state_fp16=False)
+    ids = [int(t) for t in synth.token_ids(shape, 5 + T, seed=2)]
+    m = pkg.Model(tensors, "cuda int8", shape=shape)
+    m.run(ids[:5]), ref.run_seq(ids[:5])                     # a state to start from
+    _close(m.run(ids[5:]), ref.run_seq(ids[5:]), f"T={T}")
+    C, st = shape.n_embd, m.states()
+    for l in range(shape.n_layer):
+        blk = ref.state[l * 5 * C:(l + 1) * 5 * C].reshape(5, C)
+        for i in (1, 2, 3):
+            _close(st[l][i], blk[i], f"T={T} state {i} of layer {l}", scale_aware=True)
+    _close(m.run(7), ref.run(7), "token after the prompt")
+    m.close()
