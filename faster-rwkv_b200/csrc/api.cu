@@ -88,7 +88,7 @@ struct fr_b200_model {
   PhaseDev *d_head_phase = nullptr;   // the head as a stand-alone matvec phase
   // greedy runs of many streams: two decode steps captured as a CUDA graph and replayed (the step is ~170 launches)
   GreedyCtl *d_ctl = nullptr;
-  uint8_t *d_sample = nullptr; size_t sample_bytes = 0;   // scratch of fr_b200_sample
+  uint8_t *d_sample = nullptr; size_t sample_bytes = 0;   // draws of fr_b200_sample, when they do not travel with the launch
   uint8_t *d_adj = nullptr; size_t adj_bytes = 0;         // staging of fr_b200_logits_add
   cudaStream_t gstream = nullptr;
   cudaEvent_t gev = nullptr;
@@ -911,23 +911,29 @@ int fr_b200_sample(fr_b200_model *m, int batch, float temperature, int top_k, fl
   if (batch < 1 || batch > m->cfg.max_batch) return fail(FR_B200_E_ARG, "batch must be 1..max_batch");
   CU(cudaSetDevice(m->device));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const size_t need = sample_scratch_bytes(batch, m->V) + align256((size_t)batch * 4) * 2;
-  if (m->sample_bytes < need) {
-    CU(cudaStreamSynchronize(st));
-    if (m->d_sample) cudaFree(m->d_sample);
-    m->d_sample = nullptr; m->sample_bytes = 0;
-    CU(cudaMalloc((void **)&m->d_sample, need));
-    m->sample_bytes = need;
+  // up to SAMPLE_INLINE_U draws travel with the launch, and ids for the host are written by the kernel into the pinned
+  // mirror: no copies around the kernel
+  const bool ids_to_host = is_host_ptr(ids), u_inline = batch <= SAMPLE_INLINE_U && is_host_ptr(uniform);
+  int32_t *out = ids_to_host ? reinterpret_cast<int32_t *>(m->h_out + (size_t)m->cfg.max_batch * m->Vpad * 4) : ids;
+  const float *u = uniform;
+  if (!u_inline) {
+    const size_t need = (size_t)batch * 4;
+    if (m->sample_bytes < need) {
+      CU(cudaStreamSynchronize(st));
+      if (m->d_sample) cudaFree(m->d_sample);
+      m->d_sample = nullptr; m->sample_bytes = 0;
+      CU(cudaMalloc((void **)&m->d_sample, need));
+      m->sample_bytes = need;
+    }
+    CU(cudaMemcpyAsync(m->d_sample, uniform, need, cudaMemcpyDefault, st));
+    u = reinterpret_cast<const float *>(m->d_sample);
   }
-  float *d_u = reinterpret_cast<float *>(m->d_sample);
-  int32_t *d_ids = reinterpret_cast<int32_t *>(m->d_sample + align256((size_t)batch * 4));
-  uint8_t *scratch = m->d_sample + 2 * align256((size_t)batch * 4);
-  CU(cudaMemcpyAsync(d_u, uniform, (size_t)batch * 4, cudaMemcpyDefault, st));
-  CU(launch_sample_rows(m->d_out, batch, m->V, m->Vpad, temperature, top_k, top_p, d_u, d_ids, scratch,
-                        need - 2 * align256((size_t)batch * 4), st));
-  m->launches += 4;
-  CU(cudaMemcpyAsync(ids, d_ids, (size_t)batch * 4, cudaMemcpyDefault, st));
-  if (is_host_ptr(ids)) CU(cudaStreamSynchronize(st));
+  CU(launch_sample_rows(m->d_out, batch, m->V, m->Vpad, temperature, top_k, top_p, u, u_inline, out, st));
+  m->launches += 1;
+  if (ids_to_host) {
+    CU(cudaStreamSynchronize(st));
+    memcpy(ids, out, (size_t)batch * 4);
+  }
   return FR_B200_OK;
 }
 

@@ -99,3 +99,31 @@ def test_sample_matches_the_reference_sampler_binary_at_full_vocab(pkg, synth, t
     flat = top_k == 0 and top_p >= 1.0 and temperature > 1.0
     assert flat or checked >= B * draws // 2
     m.close()
+
+
+@pytest.mark.parametrize("vocab", [65536, 50277])
+@pytest.mark.parametrize("gain", [0.0, 0.002, 1.0, 8.0])
+def test_sample_finds_its_entry_at_any_spread_of_the_logits(pkg, synth, vocab, gain):
+    """All logits equal (the entry is found by its index), packed within a few thousandths (several narrowings), spread
+    like untrained and like trained logits; with and without the two cuts.  Every pick lies within rounding of where the
+    reference's walk over the sorted probabilities stops."""
+    shape = synth.Shape("4", 1, 64, 64, vocab)
+    master = synth.generate(shape, seed=3, ln_random=True)
+    master["head.weight"] = master["head.weight"] * np.float32(gain)
+    B = 5
+    m = pkg.Model(synth.to_file_dtypes(shape, master, "fp32"), "cuda int8", shape=shape, max_batch=B)
+    logits = m.decode(synth.token_ids(shape, B, seed=1)).copy()
+    tol = 1e-4 if gain > 0.5 else 5e-4        # of the fp32 running sum of tens of thousands of equal probabilities
+    rng = np.random.default_rng(5)
+    for temperature, top_k, top_p in ((1.0, 0, 0.9), (0.7, 3000, 0.95), (2.0, 0, 0.99), (1.0, 0, 1.0), (0.3, 40, 0.999), (5.0, 1, 1.0)):
+        u = rng.uniform(0, 1, B).astype(np.float32)
+        u[0] = 0.0
+        got = m.sample(B, temperature, top_k, top_p, u)
+        assert np.array_equal(got, m.sample(B, temperature, top_k, top_p, u))
+        for b in range(B):
+            want, margin = ref_sample(logits[b], temperature, top_k, top_p, u[b])
+            if margin > tol:
+                assert got[b] == want, (temperature, top_k, top_p, b, int(got[b]), want, margin)
+            else:
+                assert pick_distance(logits[b], temperature, top_k, top_p, u[b], int(got[b])) <= tol
+    m.close()
