@@ -61,7 +61,6 @@ struct fr_b200_model {
   uint8_t *d_weights = nullptr;  size_t weights_bytes = 0;
   __half *d_rscale = nullptr;    size_t rscale_n = 0;
   float *d_vecs = nullptr;       size_t vecs_n = 0;
-  __half *d_vecs16 = nullptr;    // fp16 image of d_vecs, kept when LayerNorm / mix vectors are all exact in fp16
   uint8_t *d_emb = nullptr;      int emb_dtype = -1;   // rows kept in the dtype they arrive in
   uint8_t *d_state = nullptr;    size_t state_stride = 0, layer_stride = 0;
   exch_t *d_x = nullptr, *d_xa = nullptr, *d_rwkv = nullptr, *d_kk = nullptr, *d_rr = nullptr;   // tagged exchange vectors
@@ -70,8 +69,6 @@ struct fr_b200_model {
   unsigned seq = 0;              // phases launched so far (tags continue across launches)
   std::vector<unsigned> par;     // per stream slot: which copy of the token-shift states it reads next
   float *d_out = nullptr;        // [B][Vpad] logits, then [B] argmax ints, then status int
-  LayerDev *d_layers = nullptr;
-  PhaseDev *d_phases = nullptr;
   uint8_t *h_out = nullptr;      // pinned mirror of d_out
   unsigned long long *d_hist = nullptr; size_t hist_n = 0;   // packed arg-max words of decode_greedy, [tokens][batch]
   unsigned long long *d_amax = nullptr;   // packed arg-max words of a single decode, [max_batch]
@@ -107,8 +104,9 @@ struct fr_b200_model {
   bool emb_set = false;
   std::vector<PhaseDev> phases;
   bool finalized = false;
-  int n_stages[3] = {0, 0, 0}, grid = 0;   // per decode mode (1, <=4, <=8 streams)
-  size_t smem[3] = {0, 0, 0};
+  int n_stages[STEP_MODES] = {0}, grid = 0;   // per instance of the step kernel (0 stages: does not fit)
+  size_t smem[STEP_MODES] = {0};
+  StepParams step;               // what does not change from token to token
   long long launches = 0;
   int l2_prefetch = 384 * 1024;  // bytes per CTA the producer keeps requested from L2 ahead of the ring
   long long stream_bytes = 0;
@@ -226,8 +224,8 @@ void plan(fr_b200_model *m) {
   if (!big) {
     int optin = 0;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) == cudaSuccess)
-      for (int mode = 1; mode <= decode_mode(m->cfg.max_batch); ++mode)
-        if (decode_smem_bytes(fmt, mode, C, F, m->v5 ? 5 : 4, 2, 1) > (size_t)optin) big = true;
+      for (int mode = 1; mode <= step_mode(m->cfg.max_batch); ++mode)
+        if (step_smem_bytes(fmt, mode, C, F, m->gate ? 4 : 3, 2) > (size_t)optin) big = true;
   }
   m->rows_planned = big;
   for (auto &kv : m->mats) {
@@ -431,8 +429,6 @@ int fr_b200_create(const fr_b200_config *cfg, fr_b200_model **out) {
   if (!rc) rc = alloc((void **)&m->d_head_phase, sizeof(PhaseDev));
   if (!rc) rc = alloc((void **)&m->d_ctl, sizeof(GreedyCtl));
   if (!rc) rc = alloc((void **)&m->d_lnvec, (size_t)m->C * 4);
-  if (!rc) rc = alloc((void **)&m->d_layers, sizeof(LayerDev) * m->L);
-  if (!rc) rc = alloc((void **)&m->d_phases, sizeof(PhaseDev) * m->phases.size());
   if (!rc && cudaMallocHost((void **)&m->h_out, m->out_bytes()) != cudaSuccess) rc = fail(FR_B200_E_NOMEM, "cudaMallocHost failed");
   if (rc) { fr_b200_destroy(m); return rc; }
   cudaMemset(m->d_weights, 0, m->weights_bytes);
@@ -449,8 +445,8 @@ void fr_b200_destroy(fr_b200_model *m) {
   if (!m) return;
   cudaSetDevice(m->device);
   free_scratch(m);
-  void *ptrs[] = {m->d_weights, m->d_rscale, m->d_vecs, m->d_vecs16, m->d_emb, m->d_state, m->d_x, m->d_xa, m->d_rwkv, m->d_kk, m->d_rr,
-                  m->d_v5buf, m->d_out, m->d_layers, m->d_phases, m->d_amax, m->d_plain, m->d_pscale, m->d_qcopy, m->d_qscale, m->d_seq, m->d_head_phase, m->d_lnvec};
+  void *ptrs[] = {m->d_weights, m->d_rscale, m->d_vecs, m->d_emb, m->d_state, m->d_x, m->d_xa, m->d_rwkv, m->d_kk, m->d_rr,
+                  m->d_v5buf, m->d_out, m->d_amax, m->d_plain, m->d_pscale, m->d_qcopy, m->d_qscale, m->d_seq, m->d_head_phase, m->d_lnvec};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (m->h_out) cudaFreeHost(m->h_out);
@@ -534,45 +530,6 @@ int fr_b200_finalize(fr_b200_model *m) {
   for (auto &kv : m->vecs) if (!kv.second.set) return fail(FR_B200_E_MISSING, "missing tensor " + kv.first);
   for (int r = 0; r < m->V; ++r) if (!m->emb_rows_set[r]) return fail(FR_B200_E_MISSING, "missing embedding row " + std::to_string(r));
   free_scratch(m);
-  // layer table
-  std::vector<LayerDev> layers(m->L);
-  auto vp = [&](const std::string &n) -> const float * { return m->d_vecs + m->vecs[n].off; };
-  for (int l = 0; l < m->L; ++l) {
-    const std::string b = "blocks." + std::to_string(l) + ".", a = b + "att.", f = b + "ffn.";
-    LayerDev &d = layers[l];
-    memset(&d, 0, sizeof(d));
-    d.ln1_w = vp(b + "ln1.weight"); d.ln1_b = vp(b + "ln1.bias"); d.ln2_w = vp(b + "ln2.weight"); d.ln2_b = vp(b + "ln2.bias");
-    d.att_mix[0] = vp(a + "time_mix_k"); d.att_mix[1] = vp(a + "time_mix_v"); d.att_mix[2] = vp(a + "time_mix_r");
-    d.att_mix[3] = m->gate ? vp(a + "time_mix_g") : nullptr;
-    d.ffn_mix[0] = vp(f + "time_mix_k"); d.ffn_mix[1] = vp(f + "time_mix_r");
-    d.decay = vp(a + "time_decay"); d.first = vp(a + "time_first");
-    if (m->v5) { d.lnx_w = vp(a + "ln_x.weight"); d.lnx_b = vp(a + "ln_x.bias"); }
-  }
-  CU(cudaMemcpy(m->d_layers, layers.data(), sizeof(LayerDev) * m->L, cudaMemcpyHostToDevice));
-  // LayerNorm weights / biases and the mix vectors as fp16, when that loses nothing (files of the fp16 strategy):
-  // the one-stream kernel stages them in half the shared memory
-  bool par16 = m->cfg.act_fp16 != 0;
-  if (const char *e = getenv("FR_B200_PAR16")) par16 = par16 && atoi(e) != 0;
-  if (par16) {
-    std::vector<float> hv(m->vecs_n);
-    CU(cudaMemcpy(hv.data(), m->d_vecs, m->vecs_n * 4, cudaMemcpyDeviceToHost));
-    std::vector<__half> h16(m->vecs_n);
-    for (auto &kv : m->vecs) {
-      const std::string &n = kv.first;
-      const bool staged = n.find("ln1.") != std::string::npos || n.find("ln2.") != std::string::npos ||
-                          n.find("time_mix_") != std::string::npos || n.rfind("ln_out.", 0) == 0;
-      for (int i = 0; i < kv.second.n; ++i) {
-        const float f = hv[kv.second.off + i];
-        const __half h = __float2half_rn(f);
-        h16[kv.second.off + i] = h;
-        if (staged && __half2float(h) != f) par16 = false;
-      }
-    }
-    if (par16) {
-      CU(cudaMalloc((void **)&m->d_vecs16, m->vecs_n * 2));
-      CU(cudaMemcpy(m->d_vecs16, h16.data(), m->vecs_n * 2, cudaMemcpyHostToDevice));
-    }
-  }
   // kernel geometry: as many ring stages as shared memory allows (capped), one CTA per SM
   int optin = 0;
   CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device));
@@ -581,38 +538,68 @@ int fr_b200_finalize(fr_b200_model *m) {
   if (const char *e = getenv("FR_B200_L2_PREFETCH_KB")) m->l2_prefetch = atoi(e) * 1024;
   if (want < 2) want = 2;
   if (want > MAX_STAGES) want = MAX_STAGES;
-  const int ver = m->v5 ? 5 : 4;
-  const int max_mode = decode_mode(std::min(m->cfg.max_batch, MAX_B));
+  const int nvec = m->gate ? 4 : 3;
+  const int max_mode = step_mode(std::min(m->cfg.max_batch, MAX_B));
   for (int mode = 0; mode <= max_mode; ++mode) {
     int st = 0;
     for (int s = want; s >= 2; --s)
-      if (decode_smem_bytes(m->fmt, mode, m->C, m->F, ver, s, m->d_vecs16 != nullptr) <= (size_t)optin) { st = s; break; }
+      if (step_smem_bytes(m->fmt, mode, m->C, m->F, nvec, s) <= (size_t)optin) { st = s; break; }
     if (st == 0) {
       if (m->rows_planned && mode > 0) { m->n_stages[mode] = 0; continue; }   // such batches take the GEMM path
       return fail(FR_B200_E_UNSUPPORTED, "model too wide for shared memory at this batch size (max_batch " +
                                              std::to_string(m->cfg.max_batch) + ")");
     }
     m->n_stages[mode] = st;
-    m->smem[mode] = decode_smem_bytes(m->fmt, mode, m->C, m->F, ver, st, m->d_vecs16 != nullptr);
+    m->smem[mode] = step_smem_bytes(m->fmt, mode, m->C, m->F, nvec, st);
     int g = 0;
-    CU(decode_max_grid(m->fmt, mode, m->smem[mode], m->device, &g));
+    CU(step_prepare(m->fmt, mode, m->cfg.version, nvec, m->smem[mode], m->device, &g));
     if (g == 0) return fail(FR_B200_E_UNSUPPORTED, "decode kernel does not fit on an SM");
     m->grid = g;
   }
-  // stash capacity: ceil(C / grid) channels per CTA
-  if ((m->C + m->grid - 1) / m->grid > 128) return fail(FR_B200_E_UNSUPPORTED, "n_embd too large for the shift-state stash");
-  // phase table with real pointers; rotate item ownership from phase to phase
-  std::vector<PhaseDev> ph = m->phases;
-  for (size_t i = 0; i < ph.size(); ++i) {
-    ph[i].w = m->d_weights + reinterpret_cast<size_t>(ph[i].w);
-    ph[i].rscale = m->fmt == FMT_INT8 ? m->d_rscale + reinterpret_cast<size_t>(ph[i].rscale) : nullptr;
-    ph[i].rot = (int)((i * 37) % (size_t)m->grid);
-    if (ph[i].kind == PH_ATT_KVR || ph[i].kind == PH5_WKV) { ph[i].aux0 = layers[ph[i].layer].first; ph[i].aux1 = layers[ph[i].layer].decay; }
-    if (ph[i].kind == PH_ATT_O && m->v5) { ph[i].aux0 = layers[ph[i].layer].lnx_w; ph[i].aux1 = layers[ph[i].layer].lnx_b; }
-  }
-  CU(cudaMemcpy(m->d_phases, ph.data(), sizeof(PhaseDev) * ph.size(), cudaMemcpyHostToDevice));
+  // what the step kernel is told on every launch: the phases of layer 0 and how far apart the layers are
   {
-    PhaseDev hp = ph.back();   // the head, as the one phase of a stand-alone matvec launch
+    StepParams &p = m->step;
+    memset(&p, 0, sizeof(p));
+    p.version = m->cfg.version;
+    p.L = m->L; p.C = m->C; p.F = m->F; p.V = m->V; p.Vpad = m->Vpad; p.H = m->H;
+    p.act_fp16 = m->cfg.act_fp16; p.rescale_every = m->cfg.act_fp16 ? 6 : 0;
+    p.n_ph = ((int)m->phases.size() - 1) / m->L; p.n_att_vec = nvec;
+    p.rot_step = 37 % m->grid;
+    p.l2_prefetch_bytes = m->l2_prefetch;
+    auto step_phase = [&](const PhaseDev &d) {
+      StepPhase q;
+      memset(&q, 0, sizeof(q));
+      q.kind = d.kind; q.K = d.K; q.n_items = d.n_items; q.n_sub = d.n_sub;
+      q.split = d.kind == PH5_KVRG ? m->C / ROWS : d.split[0];
+      q.w_off = reinterpret_cast<size_t>(d.w); q.rs_off = reinterpret_cast<size_t>(d.rscale);
+      return q;
+    };
+    for (int k = 0; k < p.n_ph; ++k) p.ph[k] = step_phase(m->phases[k]);
+    p.head = step_phase(m->phases.back());
+    p.w = m->d_weights; p.w_stride = p.head.w_off / m->L;       // the head follows the last layer
+    p.rscale = m->d_rscale; p.rs_stride = p.head.rs_off / m->L;
+    auto vo = [&](const std::string &n) { return (uint32_t)m->vecs[n].off; };
+    const std::string b = "blocks.0.", a = b + "att.", f = b + "ffn.";
+    p.vecs32 = m->d_vecs;
+    p.vec_stride = m->L > 1 ? vo("blocks.1.ln1.weight") - vo("blocks.0.ln1.weight") : 0;
+    p.v_ln1_w = vo(b + "ln1.weight"); p.v_ln1_b = vo(b + "ln1.bias"); p.v_ln2_w = vo(b + "ln2.weight"); p.v_ln2_b = vo(b + "ln2.bias");
+    p.v_att_mix[0] = vo(a + "time_mix_k"); p.v_att_mix[1] = vo(a + "time_mix_v"); p.v_att_mix[2] = vo(a + "time_mix_r");
+    if (m->gate) p.v_att_mix[3] = vo(a + "time_mix_g");
+    p.v_ffn_mix[0] = vo(f + "time_mix_k"); p.v_ffn_mix[1] = vo(f + "time_mix_r");
+    p.v_decay = vo(a + "time_decay"); p.v_first = vo(a + "time_first");
+    if (m->v5) { p.v_lnx_w = vo(a + "ln_x.weight"); p.v_lnx_b = vo(a + "ln_x.bias"); }
+    p.v_lnout_w = vo("ln_out.weight"); p.v_lnout_b = vo("ln_out.bias");
+    p.emb = m->d_emb; p.emb_f32 = m->emb_dtype == FR_B200_T_F32;
+    p.x = m->d_x; p.xa = m->d_xa; p.rwkv = m->d_rwkv; p.kk = m->d_kk; p.rr = m->d_rr; p.logits = m->d_out;
+    const size_t bc = (size_t)m->cfg.max_batch * m->C;
+    p.k5 = m->d_v5buf; p.v5 = p.k5 + bc; p.r5 = p.v5 + bc; p.g5 = p.r5 + bc; p.o5 = p.g5 + bc;
+    p.state = m->d_state; p.state_stride = m->state_stride; p.layer_stride = m->layer_stride;
+    p.status = m->out_status();
+  }
+  {
+    PhaseDev hp = m->phases.back();   // the head, as the one phase of a stand-alone matvec launch
+    hp.w = m->d_weights + reinterpret_cast<size_t>(hp.w);
+    hp.rscale = m->fmt == FMT_INT8 ? m->d_rscale + reinterpret_cast<size_t>(hp.rscale) : nullptr;
     hp.kind = PH_MATVEC; hp.rot = 0;
     CU(cudaMemcpy(m->d_head_phase, &hp, sizeof(hp), cudaMemcpyHostToDevice));
   }
@@ -641,7 +628,7 @@ int align_parity(fr_b200_model *m, int batch, cudaStream_t st) {
 }
 int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids, int R, cudaStream_t st);
 // more streams than the persistent kernel carries (or a model too wide for that many): the GEMM path decodes them
-bool decode_by_rows(const fr_b200_model *m, int batch) { return batch > MAX_B || m->n_stages[decode_mode(batch)] == 0; }
+bool decode_by_rows(const fr_b200_model *m, int batch) { return batch > MAX_B || m->n_stages[step_mode(batch)] == 0; }
 // fp16 models that were created without the W^T copies build them from the streaming tiles (exact: the tiles hold
 // the same fp16 values) the first time the GEMM path is asked for
 int ensure_row_copies(fr_b200_model *m) {
@@ -681,15 +668,9 @@ int rows_decode_check(fr_b200_model *m, const int32_t *ids_host, int batch, cuda
 
 static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned long long *ids_packed, int batch,
                        cudaStream_t st, unsigned long long *amax, unsigned long long *prof = nullptr) {
-  DecodeParams p;
-  memset(&p, 0, sizeof(p));
-  p.version = m->cfg.version == FR_B200_V4 ? 4 : m->cfg.version;
-  p.L = m->L; p.C = m->C; p.F = m->F; p.V = m->V; p.Vpad = m->Vpad; p.H = m->H;
-  p.fmt = m->fmt; p.act_fp16 = m->cfg.act_fp16; p.rescale_every = m->cfg.act_fp16 ? 6 : 0;
+  StepParams p = m->step;
   p.B = batch;
-  p.n_phases = (int)m->phases.size();
-  const int mode = decode_mode(batch);
-  const size_t smem = m->smem[mode];
+  const int mode = step_mode(batch);
   p.n_stages = m->n_stages[mode];
   if (ids_host)
     for (int b = 0; b < batch; ++b) {
@@ -698,11 +679,6 @@ static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned
     }
   p.ids_packed = ids_packed;
   p.amax = amax;
-  p.emb = m->d_emb; p.emb_f32 = m->emb_dtype == FR_B200_T_F32; p.layers = m->d_layers; p.phases = m->d_phases;
-  p.lnout_w = m->d_vecs + m->vecs["ln_out.weight"].off;
-  p.lnout_b = m->d_vecs + m->vecs["ln_out.bias"].off;
-  p.vecs16 = m->d_vecs16; p.vecs32 = m->d_vecs;
-  p.x = m->d_x; p.xa = m->d_xa; p.rwkv = m->d_rwkv; p.kk = m->d_kk; p.rr = m->d_rr; p.logits = m->d_out;
   // Exchange words carry 8-bit tags: unambiguous only against the write just before them in the same slot.  Slots of
   // streams the previous launch did not write, or words a failed launch left half written, could alias: start clean.
   if (m->exch_batch != batch) {
@@ -720,15 +696,9 @@ static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned
     int rc = align_parity(m, batch, st);
     if (rc) return rc;
   }
-  p.par_mask = 0;
-  for (int b = 0; b < batch; ++b) p.par_mask |= m->par[b] << b;
-  const size_t bc = (size_t)m->cfg.max_batch * m->C;
-  p.k5 = m->d_v5buf; p.v5 = p.k5 + bc; p.r5 = p.v5 + bc; p.g5 = p.r5 + bc; p.o5 = p.g5 + bc;
-  p.state = m->d_state; p.state_stride = m->state_stride; p.layer_stride = m->layer_stride;
-  p.status = m->out_status();
+  p.par = (int)m->par[0];
   p.prof = prof;
-  p.l2_prefetch_bytes = m->l2_prefetch;
-  CU(launch_decode(p, mode, m->grid, smem, st));
+  CU(launch_step(p, m->fmt, mode, m->grid, m->smem[mode], st));
   m->launches++;
   // a phase count that is a multiple of 255 would give consecutive tokens identical tags: skip one tag per token then
   m->seq = (m->seq + (unsigned)m->phases.size() + (m->phases.size() % 255u == 0 ? 1u : 0u)) % 255u;
@@ -1690,7 +1660,7 @@ int fr_b200_get_config(const fr_b200_model *m, fr_b200_config *cfg) {
 
 int fr_b200_get_info(const fr_b200_model *m, fr_b200_info *info) {
   if (!m || !info) return fail(FR_B200_E_ARG, "null argument");
-  info->n_ctas = m->grid; info->n_threads = NTHREADS; info->smem_bytes = (int)m->smem[0]; info->n_stages = m->n_stages[0];
+  info->n_ctas = m->grid; info->n_threads = step_threads(); info->smem_bytes = (int)m->smem[0]; info->n_stages = m->n_stages[0];
   info->stage_bytes = (int)stage_bytes(m->fmt, kt_max(m->fmt)); info->n_phases = (int)m->phases.size();
   info->weight_stream_bytes = m->stream_bytes; info->launches = m->launches;
   return FR_B200_OK;

@@ -92,6 +92,55 @@ struct DecodeParams {
   unsigned long long *prof;             // optional [n_phases][8] profile of CTA 0
 };
 
+// ---- one token of 1 .. 8 streams (step.cu) -----------------------------------------------------------
+struct StepPhase {
+  int kind, K;
+  int n_items, n_sub;          // row blocks; matrices fused per row block
+  int split;                   // PH_FFN_KR: first receptance row block; PH5_KVRG: row blocks per class
+  size_t w_off, rs_off;        // layer 0: byte offset of the tiles, element offset of the row scales (int8)
+};
+struct StepParams {
+  int version, L, C, F, V, Vpad, H;
+  int act_fp16, rescale_every;
+  int B;
+  int n_ph;                    // phases per layer
+  int n_att_vec;               // mixed vectors of the attention LayerNorm
+  int n_stages;                // ring depth
+  int l2_prefetch_bytes;       // per CTA: how far ahead of the consumers the producer asks L2 for tiles (0 = off)
+  int rot_step;                // row block i of phase pi runs on CTA (i + pi * rot_step) % gridDim.x
+  int par;                     // which copy of the token-shift states is read (the other one is written)
+  unsigned seq_base;           // tag of phase pi of this launch = 1 + (seq_base + pi) % 255; host keeps it >= 255
+  int ids_val[MAX_B];
+  const unsigned long long *ids_packed;  // when non-null: ids are the packed arg-max words of the previous token
+  unsigned long long *amax;    // optional [B]: packed arg-max of this token's logits (zeroed by the host)
+  const void *emb;             // [V][C], fp32 when emb_f32 else fp16 (the file's dtype)
+  int emb_f32;
+  // weights: layer l of a phase at w + w_off + l * w_stride, scales at rscale + rs_off + l * rs_stride
+  const uint8_t *w;
+  const __half *rscale;
+  size_t w_stride, rs_stride;
+  StepPhase ph[5], head;
+  // vector blob: layer l's vectors at element offset + l * vec_stride
+  const float *vecs32;
+  uint32_t vec_stride, v_ln1_w, v_ln1_b, v_ln2_w, v_ln2_b, v_att_mix[4], v_ffn_mix[2], v_decay, v_first, v_lnx_w, v_lnx_b, v_lnout_w, v_lnout_b;
+  // Residual stream, two copies: x as the ffn value phase (or nothing yet, at layer 0) left it, xa as the attention
+  // output phase left it.  A phase never overwrites the copy that CTAs of the phase before it may still be reading.
+  exch_t *x, *xa;
+  exch_t *rwkv, *kk, *rr;               // [B][C], [B][F], [B][C]
+  exch_t *k5, *v5, *r5, *g5, *o5;       // RWKV-5 exchange vectors [B][C]
+  float *logits;                        // [B][Vpad]
+  uint8_t *state;                       // stream slot b at state + b * state_stride
+  size_t state_stride, layer_stride;    // bytes
+  int *status;                          // 0 = ok, else first failure code
+  unsigned long long *prof;             // optional [CTA][n_phases][8] trace
+};
+constexpr int STEP_MODES = 4;           // instances: 1, 2, up to 4, up to 8 streams
+inline int step_mode(int batch) { return batch == 1 ? 0 : batch == 2 ? 1 : batch <= 4 ? 2 : 3; }
+size_t step_smem_bytes(int fmt, int mode, int C, int F, int nvec, int n_stages);
+cudaError_t step_prepare(int fmt, int mode, int version, int nvec, size_t smem, int device, int *grid);   // kernel attributes; CTAs of the launch
+cudaError_t launch_step(const StepParams &p, int fmt, int mode, int grid, size_t smem, cudaStream_t st);
+int step_threads();
+
 // status codes written by the kernel
 constexpr int ST_TIMEOUT_FULL = 101, ST_TIMEOUT_EMPTY = 102, ST_TIMEOUT_DATA = 103;
 
