@@ -144,7 +144,9 @@ void free_scratch(fr_b200_model *m) {
 // of all streams side by side, the step kernel one stream after the other in a quarter of the code.  Measured, 1.5B shape:
 // 3 / 4 int4 streams 1.12 / 1.26 ms against 1.16 / 1.33, 4 fp16 streams 1.51 against 1.25; 8 int8 streams of the 0.1B
 // shape 0.58 against 0.86.
-bool wide_batch(int fmt, int batch) { return batch > 4 || (batch > 2 && fmt != FMT_FP16); }
+// (Quantised RWKV-5 stays there at every batch: its GroupNorm chain amplifies the last bits of the integer multiply to
+// 1e-3 of the logits over 32 layers, where fp16 weights give the same bits in both kernels.)
+bool wide_batch(int fmt, bool v5, int batch) { return batch > 4 || (fmt != FMT_FP16 && (v5 || batch > 2)); }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -235,7 +237,7 @@ void plan(fr_b200_model *m) {
     int optin = 0;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) == cudaSuccess)
       for (int b = 2; b <= m->cfg.max_batch; ++b)
-        if ((wide_batch(fmt, b) ? decode_smem_bytes(fmt, decode_mode(b), C, F, m->v5 ? 5 : 4, 2) : step_smem_bytes(fmt, step_mode(b), C, F, m->gate ? 4 : 3, 2)) > (size_t)optin) big = true;
+        if ((wide_batch(fmt, m->v5, b) ? decode_smem_bytes(fmt, decode_mode(b), C, F, m->v5 ? 5 : 4, 2) : step_smem_bytes(fmt, step_mode(b), C, F, m->gate ? 4 : 3, 2)) > (size_t)optin) big = true;
   }
   m->rows_planned = big;
   for (auto &kv : m->mats) {
@@ -568,7 +570,7 @@ int fr_b200_finalize(fr_b200_model *m) {
   const int nvec = m->gate ? 4 : 3;
   // every batch up to 8 by the kernel that takes it; what does not fit shared memory takes the GEMM path
   for (int batch = 1; batch <= std::min(m->cfg.max_batch, MAX_B); ++batch) {
-    const bool wide = wide_batch(m->fmt, batch);
+    const bool wide = wide_batch(m->fmt, m->v5, batch);
     const int mode = wide ? decode_mode(batch) : step_mode(batch);
     int &stages = wide ? m->wide_stages[mode] : m->n_stages[mode];
     size_t &smem = wide ? m->wide_smem[mode] : m->smem[mode];
@@ -675,7 +677,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
 // more streams than the persistent kernel carries (or a model too wide for that many): the GEMM path decodes them
 bool decode_by_rows(const fr_b200_model *m, int batch) {
   if (batch > MAX_B) return true;
-  return (wide_batch(m->fmt, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) == 0;
+  return (wide_batch(m->fmt, m->v5, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) == 0;
 }
 // fp16 models that were created without the W^T copies build them from the streaming tiles (exact: the tiles hold
 // the same fp16 values) the first time the GEMM path is asked for
@@ -718,7 +720,7 @@ static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned
                        cudaStream_t st, unsigned long long *amax, unsigned long long *prof = nullptr) {
   StepParams p = m->step;
   p.B = batch;
-  const bool wide = wide_batch(m->fmt, batch);
+  const bool wide = wide_batch(m->fmt, m->v5, batch);
   const int mode = wide ? decode_mode(batch) : step_mode(batch);
   p.n_stages = m->n_stages[wide ? 0 : mode];
   if (ids_host)
@@ -804,8 +806,10 @@ int fr_b200_decode(fr_b200_model *m, const int32_t *ids, int batch, float *logit
   if (lh || ah) {
     // one D2H of [logits rows used][argmax][status] into the pinned mirror, then hand out
     const size_t tail_off = (size_t)m->cfg.max_batch * m->Vpad * 4;
-    if (lh) CU(cudaMemcpyAsync(m->h_out, m->d_out, (size_t)batch * m->Vpad * 4, cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(m->h_out + tail_off, reinterpret_cast<uint8_t *>(m->d_out) + tail_off, (size_t)(m->cfg.max_batch + 1) * 4,
+    // (one copy where the rows in use end at the tail: every model of one stream)
+    const bool joined = lh && batch == m->cfg.max_batch;
+    if (lh) CU(cudaMemcpyAsync(m->h_out, m->d_out, joined ? m->out_bytes() : (size_t)batch * m->Vpad * 4, cudaMemcpyDeviceToHost, st));
+    if (!joined) CU(cudaMemcpyAsync(m->h_out + tail_off, reinterpret_cast<uint8_t *>(m->d_out) + tail_off, (size_t)(m->cfg.max_batch + 1) * 4,
                        cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
     const int status = *reinterpret_cast<int *>(m->h_out + tail_off + (size_t)m->cfg.max_batch * 4);
@@ -1310,9 +1314,11 @@ int fr_b200_run_seq(fr_b200_model *m, int slot, const int32_t *ids, int n, float
         CU(cudaMemcpyAsync(last_logits, m->d_out + (size_t)slot * m->Vpad, (size_t)m->V * 4, cudaMemcpyDeviceToDevice, st));
       }
     }
+    // the status word rides along into the pinned mirror
+    const size_t st_off = (size_t)m->cfg.max_batch * (m->Vpad + 1) * 4;
+    CU(cudaMemcpyAsync(m->h_out + st_off, m->out_status(), 4, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
-    int status = 0;
-    CU(cudaMemcpy(&status, m->out_status(), 4, cudaMemcpyDeviceToHost));
+    const int status = *reinterpret_cast<int *>(m->h_out + st_off);
     if ((rc = check_status(m, status))) return rc;
     if (last_logits && is_host_ptr(last_logits)) memcpy(last_logits, m->h_out, (size_t)m->V * 4);
     return FR_B200_OK;

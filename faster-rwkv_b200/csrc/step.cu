@@ -104,14 +104,13 @@ struct Cx {
   volatile int *abort_flag;
   uint32_t ln, part, xs, ring, queue;   // shared-space addresses
   size_t ring_off;
-  uint32_t xw;                     // this warp's operand area
+  uint32_t xw, xo;                 // this warp's operand area; the area of warp (tid / 16) % 8
   int tid, warp, lane, cta, G;
   int n_stages;
   int slot;                        // ring position of the next stage and the parity of its full barrier
   uint32_t parity;
   uint32_t item;                   // row blocks this CTA has started: row block n uses partial-sum buffer n % EW
   uint32_t ln_buf;
-  float pivot;                     // shift of the next LayerNorm's sums, stream lane % NS
 };
 
 // Bounded polling: gives up after WAIT_LIMIT_NS, or as soon as another thread of the CTA gave up.
@@ -331,29 +330,33 @@ __device__ __forceinline__ void make_operand(Cx &cx, const Slots &sl, int K, con
     }
   };
   const unsigned keep = a.layer0 ? 0xffffffffu : 0xffffff00u;   // (without the tags)
-  auto x_of = [&](uint32_t at, int b) {
-    const uint4 w = lds128(at + (uint32_t)b * 256u + (uint32_t)sl.sub * 16u);
+  auto x_of = [&](uint32_t at) {
+    const uint4 w = lds128(at + (uint32_t)sl.sub * 16u);
     return make_float4(__uint_as_float(w.x & keep), __uint_as_float(w.y & keep), __uint_as_float(w.z & keep), __uint_as_float(w.w & keep));
   };
   float mean = 0.f, rstd = 1.f;
   if (a.ln) {
-    // The sums are shifted by the stream's mean in the LayerNorm before: the residual stream moves little from phase to
-    // phase.  Lane l keeps what belongs to stream l % NS.
+    // Thread t sums the float4 t, t + 256, ... of x, which other warps gathered (they lie in the operand areas until these
+    // are written, behind the second barrier), shifted by the first element.  Lane l keeps the result of stream l % NS.
     params(0);
+    bar_sync(SBAR, SCONS);
+    static_assert(SW == 8, "chunk c belongs to warp c % 8: thread t's float4 are all in the area of warp (t / 16) % 8");
     const uint32_t lnb = cx.ln + cx.ln_buf * (SW * NS * 8u);
     cx.ln_buf ^= 1u;
+    const uint32_t x0 = cx.xs + (uint32_t)(cx.lane % NS) * 256u;
+    const float piv = lds_f32(x0), pivot = __uint_as_float(__float_as_uint(piv) & keep);
 #pragma unroll 1
     for (int b = 0; b < B; ++b) {
-      const float pv = NS == 1 ? cx.pivot : __shfl_sync(0xffffffffu, cx.pivot, b);
+      const float pv = NS == 1 ? pivot : __shfl_sync(0xffffffffu, pivot, b);
       float s1 = 0.f, s2 = 0.f;
+      uint32_t at = cx.xo + (uint32_t)(cx.tid >> 7) * CB;
 #pragma unroll 1
-      for (int s = 0; s < sl.n_slot; ++s)
-        if (sl.has(s)) {
-          const float4 v = x_of(cx.xw + (uint32_t)sl.local(s) * CB, b);
-          const float d0 = v.x - pv, d1 = v.y - pv, d2 = v.z - pv, d3 = v.w - pv;
-          s1 += (d0 + d1) + (d2 + d3);
-          s2 += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
-        }
+      for (int i = cx.tid; i < (p.C >> 2); i += SCONS, at += 2u * CB) {
+        const float4 v = x_of(at + (uint32_t)b * 256u);
+        const float d0 = v.x - pv, d1 = v.y - pv, d2 = v.z - pv, d3 = v.w - pv;
+        s1 += (d0 + d1) + (d2 + d3);
+        s2 += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+      }
       __syncwarp();
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -367,12 +370,14 @@ __device__ __forceinline__ void make_operand(Cx &cx, const Slots &sl, int K, con
 #pragma unroll
     for (int w = 0; w < SW; w += 2) {              // two warps' sums per load
       const float4 f = lds_f32x4(lnb + (uint32_t)((NS == 1 ? 0 : cx.lane % NS) * SW + w) * 8u);
-      t1 += f.x + f.z; t2 += f.y + f.w;
+      t1 += f.x; t2 += f.y;
+      t1 += f.z; t2 += f.w;
     }
     const float inv = 1.f / (float)p.C, m = t1 * inv;
-    mean = cx.pivot + m;
-    rstd = rsqrtf(fmaxf(t2 * inv - m * m, 0.f) + 1e-5f);
-    cx.pivot = mean;
+    float var = t2 * inv - m * m;
+    var = var > 0.f ? var : 0.f;
+    mean = pivot + m;
+    rstd = rsqrtf(var + 1e-5f);
   } else if (gn) {
     params(0);
   }
@@ -388,7 +393,7 @@ __device__ __forceinline__ void make_operand(Cx &cx, const Slots &sl, int K, con
     float4 xs[NS];
 #pragma unroll
     for (int b = 0; b < NS; ++b)
-      if (has) xs[b] = x_of(at, b);
+      if (has) xs[b] = x_of(at + (uint32_t)b * 256u);
     __syncwarp();
 #pragma unroll 1
     for (int b = 0; b < B; ++b) {
@@ -430,7 +435,7 @@ __device__ __forceinline__ void make_operand(Cx &cx, const Slots &sl, int K, con
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
           const float4 m = mx[v];
-          y[v] = make_float4(fmaf(xx.x - z.x, m.x, z.x), fmaf(xx.y - z.y, m.y, z.y), fmaf(xx.z - z.z, m.z, z.z), fmaf(xx.w - z.w, m.w, z.w));
+          y[v] = make_float4(xx.x * m.x + z.x * (1.f - m.x), xx.y * m.y + z.y * (1.f - m.y), xx.z * m.z + z.z * (1.f - m.z), xx.w * m.w + z.w * (1.f - m.w));
         }
       } else {
 #pragma unroll
@@ -446,10 +451,11 @@ __device__ __forceinline__ void make_operand(Cx &cx, const Slots &sl, int K, con
 }
 
 // ---- multiply ---------------------------------------------------------------------------------------
-// One chunk: 16 output rows x 64 inputs of the streamed tile, and the operand.  acc[t][0], acc[t][1]: this lane's share
-// of rows g and g + 8 (sum_lanes() turns it into the sums of a stream).
-//   fp16:  four m16n8k16 MMAs; lane q holds stream q (hi + lo columns)
-//   int:   two m16n8k32 int8 MMAs, exact; lane q holds digits 0, 1 (q even: low) or 2 (q odd: high) of stream q / 2.
+// One chunk: 16 output rows x 64 inputs of the streamed tile, and the operand.  acc[t]: this lane's share of rows g and
+// g + 8, which sum_lanes() turns into the sums of a stream:
+//   fp16:  four m16n8k16 MMAs into two accumulator sets (no MMA waits for the one before it); lane q holds stream q (hi +
+//          lo columns).  Sums are taken in the order of the batched-prologue kernel, the results are the same bit by bit
+//   int:   [0][0], [1][0]; two m16n8k32 int8 MMAs, exact; lane q holds digits 0, 1 (q even: low) or 2 (q odd: high) of stream q / 2.
 //          int4 keeps the codes times 16 (the nibble stays in the upper half of its byte); one MMA is one scale group.
 template <int FMT, int NS> __host__ __device__ constexpr int acc_tiles() { return FMT == FMT_FP16 ? n_tiles<NS>() : (NS + 1) / 2; }
 
@@ -487,17 +493,15 @@ __device__ __forceinline__ void fetch_chunk(Frag<FMT, NS> &f, uint32_t A, uint32
   if constexpr (FMT == FMT_INT4) f.sc = lds64(scales);
 }
 template <int FMT, int NS>
-__device__ __forceinline__ void mul_chunk(const Frag<FMT, NS> &f, int lane, float (&acc)[acc_tiles<FMT, NS>()][2][2]) {
+__device__ __forceinline__ void mul_chunk(const Frag<FMT, NS> &f, int lane, float (&acc)[acc_tiles<FMT, NS>()][2][4]) {
   constexpr int NT = acc_tiles<FMT, NS>();
   if constexpr (FMT == FMT_FP16) {
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      float u[4] = {acc[t][0][0], acc[t][0][1], acc[t][1][0], acc[t][1][1]}, v[4] = {0.f, 0.f, 0.f, 0.f};
-      mma16816(u, f.a[0].x, f.a[0].y, f.a[0].z, f.a[0].w, f.b[t][0].x, f.b[t][0].y);
-      mma16816(v, f.a[1].x, f.a[1].y, f.a[1].z, f.a[1].w, f.b[t][0].z, f.b[t][0].w);
-      mma16816(u, f.a[2].x, f.a[2].y, f.a[2].z, f.a[2].w, f.b[t][1].x, f.b[t][1].y);
-      mma16816(v, f.a[3].x, f.a[3].y, f.a[3].z, f.a[3].w, f.b[t][1].z, f.b[t][1].w);
-      acc[t][0][0] = u[0] + v[0]; acc[t][0][1] = u[1] + v[1]; acc[t][1][0] = u[2] + v[2]; acc[t][1][1] = u[3] + v[3];
+      mma16816(acc[t][0], f.a[0].x, f.a[0].y, f.a[0].z, f.a[0].w, f.b[t][0].x, f.b[t][0].y);
+      mma16816(acc[t][1], f.a[1].x, f.a[1].y, f.a[1].z, f.a[1].w, f.b[t][0].z, f.b[t][0].w);
+      mma16816(acc[t][0], f.a[2].x, f.a[2].y, f.a[2].z, f.a[2].w, f.b[t][1].x, f.b[t][1].y);
+      mma16816(acc[t][1], f.a[3].x, f.a[3].y, f.a[3].z, f.a[3].w, f.b[t][1].z, f.b[t][1].w);
     }
   } else {
     const float m256 = lane & 1 ? 0.f : 256.f;       // column 3 of a stream is not a digit
@@ -537,12 +541,12 @@ __device__ __forceinline__ void mul_chunk(const Frag<FMT, NS> &f, int lane, floa
   }
 }
 
-// sums of a stream over this warp's K share from a lane's accumulators
-template <int FMT, int NS>
-__device__ __forceinline__ float sum_lanes(int lane, const float (&a)[2]) {
-  if constexpr (FMT == FMT_FP16) return a[0] + a[1];
+// sum of row g + 8 r of a stream over this warp's K share
+template <int FMT>
+__device__ __forceinline__ float sum_lanes(int lane, const float (&a)[2][4], int r) {
+  if constexpr (FMT == FMT_FP16) return (a[0][2 * r] + a[1][2 * r]) + (a[0][2 * r + 1] + a[1][2 * r + 1]);
   // low digits + 2^16 x high digit; int4 codes are 16 times too large
-  float v = a[0] * (lane & 1 ? 65536.f : 1.f) * (FMT == FMT_INT4 ? 0.0625f : 1.f);
+  const float v = a[r][0] * (lane & 1 ? 65536.f : 1.f) * (FMT == FMT_INT4 ? 0.0625f : 1.f);
   return v + __shfl_xor_sync(0xffffffffu, v, 1);
 }
 
@@ -566,9 +570,11 @@ __device__ __forceinline__ void multiply_items(Cx &cx, int K, int n_items, int n
     for (int u = 0; u < n_sub; ++u) {
       const uint32_t vec = n_sub > 1 ? (uint32_t)u : split == 0 || it < split ? 0u : min(it < 2 * split ? 1u : it < 3 * split ? 2u : 3u, last_vec);
       uint32_t bop = cx.xw + vec * vb;
-      float acc[NT][2][2];
+      float acc[NT][2][4];
 #pragma unroll
-      for (int t = 0; t < NT; ++t) { acc[t][0][0] = acc[t][0][1] = acc[t][1][0] = acc[t][1][1] = 0.f; }
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { acc[t][0][i] = 0.f; acc[t][1][i] = 0.f; }
       int left = n_ch;                               // chunks from this stage on
 #pragma unroll 1
       for (int s = 0; s < nst; ++s, left -= CH) {
@@ -601,7 +607,7 @@ __device__ __forceinline__ void multiply_items(Cx &cx, int K, int n_items, int n
       const int sq = FMT == FMT_FP16 ? q : q >> 1;
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        const float r0 = sum_lanes<FMT, NS>(cx.lane, acc[t][0]), r1 = sum_lanes<FMT, NS>(cx.lane, acc[t][1]);
+        const float r0 = sum_lanes<FMT>(cx.lane, acc[t], 0), r1 = sum_lanes<FMT>(cx.lane, acc[t], 1);
         if (FMT == FMT_FP16 ? q < TS : (q & 1) == 0 && sq < TS) {
           const uint32_t d = dst + (uint32_t)u * (ROWS * NS * 4u) + (uint32_t)(g * NS + t * TS + sq) * 4u;
           sts_f32(d, r0);
@@ -750,17 +756,10 @@ __device__ __forceinline__ void epilogue_items(Cx &cx, const StepPhase &ph, int 
       const int b = idx % NS, o = o0 + idx / NS;
       const size_t bo = (size_t)b * C + o;
       auto sum = [&](uint32_t u) {
+        const uint32_t a = cx.part + (uint32_t)e * SW * 3u * MB + u * MB + (uint32_t)idx * 4u;
         float s = 0.f;
-        if (NS == 1) {
-          const uint32_t a = cx.part + ((uint32_t)e * SW + (uint32_t)(cx.lane >> 4) * (SW / 2)) * 3u * MB + u * MB + (uint32_t)(cx.lane & 15) * 4u;
 #pragma unroll
-          for (int w = 0; w < SW / 2; ++w) s += lds_f32(a + (uint32_t)w * 3u * MB);
-          s += __shfl_xor_sync(0xffffffffu, s, 16);
-        } else {
-          const uint32_t a = cx.part + (uint32_t)e * SW * 3u * MB + u * MB + (uint32_t)(cx.lane + 32 * k) * 4u;
-#pragma unroll
-          for (int w = 0; w < SW; ++w) s += lds_f32(a + (uint32_t)w * 3u * MB);
-        }
+        for (int w = 0; w < SW; ++w) s += lds_f32(a + (uint32_t)w * 3u * MB);
         return s;
       };
       float v0 = sum(0) * r0[k], v1 = 0.f, v2 = v0;
@@ -780,17 +779,14 @@ __device__ __forceinline__ void epilogue_items(Cx &cx, const StepPhase &ph, int 
         }
         continue;
       }
-      // one division serves the WKV quotient, the receptance row's sigmoid and the gate row's SiLU
-      float num = 1.f, den = 1.f + expf(-v2);
-      float pm = 0.f;
+      const float sg = 1.f / (1.f + expf(-v2));  // of r, the receptance row or the gate row, whichever this is
+      float pm = 0.f, quo = sg;
       if (kind == PH_ATT_KVR) {
         const float2 e1 = exp_pair(f2[k], f3[k] + v0, pm);
-        num = e1.x * f0[k] + e1.y * v1;
-        den *= e1.x * f1[k] + e1.y;
+        quo = sg * ((e1.x * f0[k] + e1.y * v1) / (e1.x * f1[k] + e1.y));
       } else if (kind == PH5_KVRG) {
-        num = v0;
+        quo = v0 * sg;
       }
-      const float quo = num / den;
       exch_t *dst = p.x + bo;
       float out = f0[k] + f1[k] * v0;
       if (kind == PH_ATT_KVR) {
@@ -942,7 +938,6 @@ __device__ __forceinline__ void consume(Cx &cx) {
     if (a.own < 0) a.own += cx.G;
     if (a.layer0) {
       // embedding rows: plain memory, always there
-      cx.pivot = emb4(p, NS == 1 ? 0 : min(cx.lane % NS, p.B - 1), 0).x;
 #pragma unroll 1
       for (int s = 0; s < sl.n_slot; ++s)
 #pragma unroll 1
@@ -1015,13 +1010,17 @@ __global__ void __launch_bounds__(STHREADS, 1) step_kernel(const __grid_constant
   cx.tid = threadIdx.x; cx.warp = threadIdx.x >> 5; cx.lane = threadIdx.x & 31;
   cx.cta = blockIdx.x; cx.G = gridDim.x;
   cx.n_stages = p.n_stages;
-  cx.slot = 0; cx.parity = 0; cx.item = 0; cx.ln_buf = 0; cx.pivot = 0.f;
+  cx.slot = 0; cx.parity = 0; cx.item = 0; cx.ln_buf = 0;
   const uint32_t base = smem_u32(step_smem);
   cx.ln = base + LN_OFF; cx.queue = base + QUEUE_OFF;
   cx.part = base + (uint32_t)o.part; cx.xs = base + (uint32_t)o.xs; cx.ring = base + (uint32_t)o.ring;
   cx.ring_off = o.ring;
-  cx.xw = cx.xs;
-  for (int w = 0; w < cx.warp && w < SW; ++w) cx.xw += (uint32_t)operand_chunks(p.C, p.F, p.n_att_vec, w) * chunk_operand_bytes<NS>();
+  cx.xw = cx.xo = cx.xs;
+  for (int w = 0; w < SW; ++w) {
+    const uint32_t n = (uint32_t)operand_chunks(p.C, p.F, p.n_att_vec, w) * chunk_operand_bytes<NS>();
+    if (w < cx.warp) cx.xw += n;
+    if (w < ((cx.tid >> 4) & 7)) cx.xo += n;
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.n_stages; ++s) { mbar_init(&cx.full[s], 1); mbar_init(&cx.empty[s], SW); }
     for (int e = 0; e < EW; ++e) { mbar_init(&cx.part_full[e], SW); mbar_init(&cx.part_empty[e], 1); }
