@@ -62,6 +62,24 @@ def test_eight_streams_of_a_wide_model_take_the_gemm_path(pkg, orc, synth, fmt):
     m.close()
 
 
+@pytest.mark.parametrize("name,fmt", [("tiny4b", "fp16"), ("tiny4b", "int8"), ("tiny4b", "int4"), ("mid52", "fp16"),
+                                      ("tiny50", "fp16"), ("tiny52", "int8"), ("wide4", "fp16"), ("wide4", "int4")])
+def test_every_few_stream_batch_of_one_model(pkg, orc, synth, name, fmt):
+    """Batches of 1 .. 5 and 8 streams of the same slots, alternating between the two persistent kernels and their
+    instances, down to one stream: input widths that are not a multiple of eight 64-input chunks (some warps own none),
+    and one that takes several weight tiles per row block."""
+    shape, m, ref = _pair(pkg, orc, synth, name, fmt, 8)
+    sizes = [8, 4, 1, 3, 2, 5, 1, 2]
+    ids = synth.token_ids(shape, len(sizes) * 8, seed=5).reshape(len(sizes), 8)
+    got = [m.decode(ids[t][:n]) for t, n in enumerate(sizes)]
+    for b in (0, 1, 2, 4, 7):
+        ref.reset()
+        for t, n in enumerate(sizes):
+            if b < n:
+                _close(got[t][b], ref.run(int(ids[t, b])), f"{name} {fmt} stream {b} step {t} of {n} streams")
+    m.close()
+
+
 def test_small_and_large_batches_share_state(pkg, orc, synth):
     """The persistent kernel (<= 8 streams) and the GEMM path (> 8) read and write the same state slots, and streams
     that are decoded together need not have seen the same number of tokens (continuous batching: a stream joins a
