@@ -759,7 +759,7 @@ static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned
     memcpy(d.ids_val, p.ids_val, sizeof(d.ids_val));
     d.ids_packed = ids_packed; d.amax = amax;
     d.emb = p.emb; d.emb_f32 = p.emb_f32; d.layers = m->d_layers; d.phases = m->d_phases;
-    d.lnout_w = m->d_vecs + p.v_lnout_w; d.lnout_b = m->d_vecs + p.v_lnout_b; d.vecs32 = m->d_vecs;
+    d.lnout_w = m->d_vecs + p.v_lnout_w; d.lnout_b = m->d_vecs + p.v_lnout_b;
     d.x = p.x; d.xa = p.xa; d.rwkv = p.rwkv; d.kk = p.kk; d.rr = p.rr; d.logits = p.logits;
     d.k5 = p.k5; d.v5 = p.v5; d.r5 = p.r5; d.g5 = p.g5; d.o5 = p.o5;
     d.seq_base = p.seq_base; d.par_mask = m->par[0] ? (1u << batch) - 1u : 0u;
@@ -1734,7 +1734,9 @@ int fr_b200_get_config(const fr_b200_model *m, fr_b200_config *cfg) {
 
 int fr_b200_get_info(const fr_b200_model *m, fr_b200_info *info) {
   if (!m || !info) return fail(FR_B200_E_ARG, "null argument");
-  info->n_ctas = m->grid; info->n_threads = step_threads(); info->smem_bytes = (int)m->smem[0]; info->n_stages = m->n_stages[0];
+  const bool wide = wide_batch(m->fmt, m->v5, 1);   // of the kernel that takes one stream
+  info->n_ctas = m->grid; info->n_threads = wide ? NTHREADS : step_threads();
+  info->smem_bytes = (int)(wide ? m->wide_smem[0] : m->smem[0]); info->n_stages = wide ? m->wide_stages[0] : m->n_stages[0];
   info->stage_bytes = (int)stage_bytes(m->fmt, kt_max(m->fmt)); info->n_phases = (int)m->phases.size();
   info->weight_stream_bytes = m->stream_bytes; info->launches = m->launches;
   return FR_B200_OK;

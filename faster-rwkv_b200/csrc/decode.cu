@@ -1,4 +1,6 @@
-// Persistent whole-token decode kernel for sm_100a.
+// Persistent whole-token decode kernel with batched prologues, for sm_100a: the operands of all streams are made side
+// by side, with more code per phase than step.cu, which is the faster kernel for few streams.  It takes the batches the
+// other is slower at (5 - 8 streams, 3 - 4 quantised ones), quantised RWKV-5, and the stand-alone matrix-vector products.
 //
 // One cooperative launch (all CTAs co-resident, one per SM) runs a whole token — all layers and the
 // head — for up to 8 independent streams.  Each CTA has one producer warp and NW consumer warps:
@@ -55,20 +57,18 @@ __host__ __device__ inline size_t xs_halfs_needed(int C, int F, int version, int
   size_t b = F;
   return (a > b ? a : b) * NB * NT;
 }
-// one stream and a model narrow enough for the register-resident LayerNorm: parameters are staged in shared memory,
-// as fp16 when every LayerNorm / mix vector of the model is exact in fp16 (a "cuda fp16" file): half the space, which
-// buys another ring slot for the weight stream
-template <int NB, int NT> __host__ __device__ inline size_t par_bytes(int C, int par16) {
-  return (NB == 2 && (C >> 2) <= XR * NCONS) ? (size_t)PAR_VECS * C * (par16 ? 2 : 4) : 0;
+// one stream and a model narrow enough for the register-resident LayerNorm: parameters are staged in shared memory
+template <int NB, int NT> __host__ __device__ inline size_t par_bytes(int C) {
+  return (NB == 2 && (C >> 2) <= XR * NCONS) ? (size_t)PAR_VECS * C * 4 : 0;
 }
 
 template <int NB, int NT>
-__host__ __device__ inline size_t smem_layout(int fmt, int C, int F, int version, int n_stages, int par16, size_t *off_red,
-                                              size_t *off_par, size_t *off_xs, size_t *off_ring) {
+__host__ __device__ inline size_t smem_layout(int fmt, int C, int F, int version, int n_stages, size_t *off_red, size_t *off_par,
+                                              size_t *off_xs, size_t *off_ring) {
   size_t o = 1024;  // barriers + flags + LN scratch
   *off_red = o;   o += sizeof(float) * 3 * NW * red_n<NB, NT>() * (NB == 2 ? 2 : 1);
   o = align_up(o, 128);
-  *off_par = o;   o += par_bytes<NB, NT>(C, par16);
+  *off_par = o;   o += par_bytes<NB, NT>(C);
   *off_xs = o;    o += xs_halfs_needed(C, F, version, NB, NT) * 2;
   o = align_up(o, 1024);
   *off_ring = o;  o += (size_t)n_stages * slot_bytes(fmt);
@@ -453,16 +453,12 @@ __device__ __forceinline__ LnArgs ln_args(const DecodeParams &p, const PhaseDev 
 __device__ __forceinline__ void ln_stage_params(Ctx &cx, const LnArgs &a) {
   const DecodeParams &p = *cx.p;
   uint8_t *par = reinterpret_cast<uint8_t *>(cx.sm.par);
-  const uint32_t vb = (uint32_t)p.C * (p.vecs16 ? 2u : 4u);   // bytes per staged vector
+  const uint32_t vb = (uint32_t)p.C * 4u;   // bytes per staged vector
   const uint32_t sxb = a.nvec > 0 ? (uint32_t)p.C * (p.act_fp16 ? 2u : 4u) : 0u;
-  // the fp16 image of a vector sits at the same element offset in the fp16 copy of the vector blob
-  auto src = [&](const float *v) -> const void * {
-    return p.vecs16 ? static_cast<const void *>(p.vecs16 + (v - p.vecs32)) : static_cast<const void *>(v);
-  };
   mbar_expect_tx(cx.sm.par_bar, vb * (2u + (uint32_t)a.nvec) + sxb);
-  bulk_g2s(par, src(a.ln_w), vb, cx.sm.par_bar);
-  bulk_g2s(par + vb, src(a.ln_b), vb, cx.sm.par_bar);
-  for (int v = 0; v < a.nvec; ++v) bulk_g2s(par + (2 + v) * vb, src(a.mix[v]), vb, cx.sm.par_bar);
+  bulk_g2s(par, a.ln_w, vb, cx.sm.par_bar);
+  bulk_g2s(par + vb, a.ln_b, vb, cx.sm.par_bar);
+  for (int v = 0; v < a.nvec; ++v) bulk_g2s(par + (2 + v) * vb, a.mix[v], vb, cx.sm.par_bar);
   if (a.nvec > 0) bulk_g2s(par + 6 * vb, a.sx_rd, sxb, cx.sm.par_bar);
 }
 
@@ -518,17 +514,14 @@ __device__ __forceinline__ void prologue_ln_one(Ctx &cx, const PhaseDev &ph, con
   const float mean = piv + m, rstd = rsqrtf(var + 1e-5f);
   if (p.prof && cx.tid == 0) cx.pc[3] = clock64();  // trace
   const uint8_t *par = reinterpret_cast<const uint8_t *>(cx.sm.par);
-  const bool par16 = p.vecs16 != nullptr;
-  const uint32_t vb = (uint32_t)p.C * (par16 ? 2u : 4u);
+  const uint32_t vb = (uint32_t)p.C * 4u;
   auto half4 = [](const uint8_t *base, int i4) {
     const uint2 u = *reinterpret_cast<const uint2 *>(base + (size_t)i4 * 8);
     const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
     const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
     return make_float4(lo.x, lo.y, hi.x, hi.y);
   };
-  auto par4 = [&](int v, int i4) {
-    return par16 ? half4(par + v * vb, i4) : *reinterpret_cast<const float4 *>(par + v * vb + (size_t)i4 * 16);
-  };
+  auto par4 = [&](int v, int i4) { return *reinterpret_cast<const float4 *>(par + v * vb + (size_t)i4 * 16); };
 #pragma unroll
   for (int r = 0; r < XR; ++r) {
     const bool valid = cx.tid + r * NCONS < n4;
@@ -1313,8 +1306,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_kernel(const __grid_consta
   cx.slot = 0; cx.parity = 0; cx.wait_ns = 0; cx.prof_phase = 0; cx.red_buf = 0; cx.ready = false;
   cx.slot_b = slot_bytes(FMT);
   size_t o_red, o_par, o_xs, o_ring;
-  smem_layout<NB, NT>(FMT, p.C, p.F, p.version, p.n_stages, p.vecs16 != nullptr, &o_red, &o_par, &o_xs, &o_ring);
-  cx.sm.par = par_bytes<NB, NT>(p.C, p.vecs16 != nullptr) ? reinterpret_cast<float *>(smem + o_par) : nullptr;
+  smem_layout<NB, NT>(FMT, p.C, p.F, p.version, p.n_stages, &o_red, &o_par, &o_xs, &o_ring);
+  cx.sm.par = par_bytes<NB, NT>(p.C) ? reinterpret_cast<float *>(smem + o_par) : nullptr;
   cx.par_parity = 0;
   cx.sm.par_bar = reinterpret_cast<uint64_t *>(smem + 200);
   cx.sm.par_free = reinterpret_cast<uint64_t *>(smem + 208);
@@ -1379,12 +1372,12 @@ cudaError_t max_grid_t(size_t smem, int device, int *grid) {
 }  // namespace
 
 // mode: 0 = one stream, 1 = up to 4 streams, 2 = up to 8 streams
-size_t decode_smem_bytes(int fmt, int mode, int C, int F, int version, int n_stages, int par16) {
+size_t decode_smem_bytes(int fmt, int mode, int C, int F, int version, int n_stages) {
   size_t a, b, c, d;
   switch (mode) {
-    case 0: return smem_layout<2, 1>(fmt, C, F, version, n_stages, par16, &a, &b, &c, &d);
-    case 1: return smem_layout<8, 1>(fmt, C, F, version, n_stages, par16, &a, &b, &c, &d);
-    default: return smem_layout<8, 2>(fmt, C, F, version, n_stages, par16, &a, &b, &c, &d);
+    case 0: return smem_layout<2, 1>(fmt, C, F, version, n_stages, &a, &b, &c, &d);
+    case 1: return smem_layout<8, 1>(fmt, C, F, version, n_stages, &a, &b, &c, &d);
+    default: return smem_layout<8, 2>(fmt, C, F, version, n_stages, &a, &b, &c, &d);
   }
 }
 

@@ -274,7 +274,8 @@ int fr_b200_get_info(const fr_b200_model *m, fr_b200_info *info);
 /* One decode step with a per-CTA, per-phase trace: stamps[cta][phase][8] = {phase start, inputs staged, row
  * blocks done (ns of the GPU's global timer), then SM cycles: waiting for weight tiles, phase descriptor ->
  * phase start, phase start -> inputs arrived, inputs arrived -> statistics / conversion done, -> operands staged};
- * zero where the CTA had no work in the phase.
+ * zero where the CTA had no work in the phase, and in the entries 3, 4 and 6 of batches that the step kernel takes
+ * (1 and 2 streams, fp16 RWKV up to 4, not quantised RWKV-5), which does not stage a phase in those steps.
  * A tracing aid (the reference has only wall-clock FR_SHOW_SPEED prints, chat.cpp:98-111).
  * stamps: host, n_ctas * n_phases * 8 entries (fr_b200_get_info gives both counts). */
 int fr_b200_decode_profile(fr_b200_model *m, const int32_t *ids, int batch, uint64_t *stamps, int n_stamps);
