@@ -859,22 +859,22 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 // blockIdx.y picks the problem of the group (grid.x covers the largest one).
 __global__ void __launch_bounds__(256) gemm_finish_kernel(const __grid_constant__ GemmGroup grp) {
   pdl_trigger();
-  pdl_wait();
   const GemmArgs &g = grp.p[blockIdx.y];
   const int split = grp.split;
   const int n4 = g.N >> 2;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= g.M * n4) return;
   const int row = idx / n4, col = (idx - row * n4) * 4;
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), cs = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (g.col_scale)
+    cs = make_float4(__half2float(g.col_scale[col]), __half2float(g.col_scale[col + 1]), __half2float(g.col_scale[col + 2]),
+                     __half2float(g.col_scale[col + 3]));
+  pdl_wait();
   for (int z = 0; z < split; ++z) {
     const float4 p = *reinterpret_cast<const float4 *>(g.raw + ((size_t)z * g.M + row) * g.N + col);
     v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
   }
-  if (g.col_scale) {
-    v.x *= __half2float(g.col_scale[col]); v.y *= __half2float(g.col_scale[col + 1]);
-    v.z *= __half2float(g.col_scale[col + 2]); v.w *= __half2float(g.col_scale[col + 3]);
-  }
+  if (g.col_scale) { v.x *= cs.x; v.y *= cs.y; v.z *= cs.z; v.w *= cs.w; }
   const size_t o = (size_t)row * g.ldo + col;
   float a[4] = {v.x, v.y, v.z, v.w};
   if (g.epi == GEMM_EPI_F32) {
@@ -1025,18 +1025,42 @@ __global__ void gather_emb_kernel(const void *emb, int emb_f32, const int32_t *i
 // row writes its new one.  nvec == 0: plain LayerNorm into op[0] (ln_out before the head).
 // Each thread keeps its float4 pieces of the row (and of the row before) in registers: x is read once.
 constexpr int LN_MAX4 = 8;   // float4 per thread: n_embd <= 8192
-template <int NJ>
+constexpr int LN_FEW_ROWS = 512;   // two resident CTAs of 512 threads per SM carry 296 rows at once
+template <int NT, int NJ>
 __device__ __forceinline__ float2 stats_from_regs(const float4 *v, int n4, float piv, int C, float *red) {
   float s1 = 0.f, s2 = 0.f;
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    if ((int)threadIdx.x + j * 256 < n4) {
+    if ((int)threadIdx.x + j * NT < n4) {
       const float d0 = v[j].x - piv, d1 = v[j].y - piv, d2 = v[j].z - piv, d3 = v[j].w - piv;
       s1 += (d0 + d1) + (d2 + d3);
       s2 += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
     }
   }
-  const float2 s = block_sum2(s1, s2, red);
+  float2 s;
+  if (NT == 256) {
+    s = block_sum2(s1, s2, red);
+  } else {
+    // the order of 256 threads with NT / 256 pieces each: the same bits for every launch shape
+    float2 *fold = reinterpret_cast<float2 *>(red + 16);
+    const int tid = threadIdx.x;
+    if (tid >= 256) fold[tid - 256] = make_float2(s1, s2);
+    __syncthreads();
+    if (tid < 256) {
+#pragma unroll
+      for (int i = 0; i < NT / 256 - 1; ++i) { const float2 f = fold[tid + i * 256]; s1 += f.x; s2 += f.y; }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      }
+      if ((tid & 31) == 0) { red[(tid >> 5) * 2] = s1; red[(tid >> 5) * 2 + 1] = s2; }
+    }
+    __syncthreads();
+    s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { s.x += red[w * 2]; s.y += red[w * 2 + 1]; }
+  }
   const float m = s.x / (float)C;
   float var = s.y / (float)C - m * m;
   var = var > 0.f ? var : 0.f;
@@ -1064,22 +1088,42 @@ __device__ __forceinline__ float4 load_act_f4(const void *p, int i4, int act_fp1
 }
 __device__ __forceinline__ float round_h(float v) { return __half2float(__float2half_rn(v)); }
 
-// NJ = float4 pieces of a row per thread (2, 4 or 8: n_embd up to 2048, 4096, 8192)
-template <int NJ>
-__global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
+__device__ __forceinline__ float4 half4_value(const uint2 &u) {
+  const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// NT threads, NJ float4 pieces of a row per thread
+template <int NT, int NJ>
+__global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
+  constexpr bool EARLY = NJ == 1;
   pdl_trigger();
-  pdl_wait();
-  __shared__ float red[16];
+  __shared__ __align__(8) float red[16 + 2 * (NT - 256)];
   const int t = blockIdx.x, C = a.C, n4 = C >> 2;
+  // the parameters are constants: one round trip of them is over before the kernel ahead of this one has finished
+  float4 ew = make_float4(0.f, 0.f, 0.f, 0.f), eb = ew, em[4], esx = ew;
+  uint2 ecs = make_uint2(0u, 0u);
+  if (EARLY && (int)threadIdx.x < n4) {
+    ew = reinterpret_cast<const float4 *>(a.ln_w)[threadIdx.x];
+    eb = reinterpret_cast<const float4 *>(a.ln_b)[threadIdx.x];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (v < a.nvec) em[v] = reinterpret_cast<const float4 *>(a.mix[v])[threadIdx.x];
+    if (a.pend_split > 1 && a.pend_cscale) ecs = reinterpret_cast<const uint2 *>(a.pend_cscale)[threadIdx.x];
+  }
+  pdl_wait();
+  const uint8_t *srd = reinterpret_cast<const uint8_t *>(a.sx_rd) + (a.batch_mode ? (size_t)t * a.state_stride : 0);
+  uint8_t *swr = reinterpret_cast<uint8_t *>(a.sx_wr) + (a.batch_mode ? (size_t)t * a.state_stride : 0);
   const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * C);
   const bool from_row = !a.batch_mode && t > 0 && a.nvec > 0;
   float4 xv[NJ], pv[NJ];
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const int i4 = threadIdx.x + j * 256;
+    const int i4 = threadIdx.x + j * NT;
     if (i4 < n4) {
       xv[j] = xr[i4];
       if (from_row) pv[j] = xr[i4 - n4];
+      else if (EARLY && a.nvec > 0) esx = load_act_f4(srd, i4, a.act_fp16);
     }
   }
   float piv = a.x[(size_t)t * C];
@@ -1091,12 +1135,17 @@ __global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
 #pragma unroll
     for (int j = 0; j < NJ; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     const size_t zs = (size_t)a.T * C;
-    constexpr int ZB = NJ <= 2 ? 8 : 4;   // slabs per batch: NJ x ZB 16-byte loads in flight per thread
+    uint2 erh = make_uint2(0u, 0u), erl = erh;   // the factor, asked for together with the slabs
+    if (EARLY && a.pend_r && (int)threadIdx.x < n4) {
+      erh = reinterpret_cast<const uint2 *>(a.pend_r + (size_t)t * C)[threadIdx.x];
+      if (a.pend_r_lo) erl = reinterpret_cast<const uint2 *>(a.pend_r_lo + (size_t)t * C)[threadIdx.x];
+    }
+    constexpr int ZB = NJ == 1 && NT <= 512 ? 16 : 4;   // slabs per batch: NJ x ZB 16-byte loads in flight per thread
     for (int z0 = 0; z0 < a.pend_split; z0 += ZB) {
       float4 p[NJ][ZB];
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
-        const int i4 = threadIdx.x + j * 256;
+        const int i4 = threadIdx.x + j * NT;
         const float *slab = a.pend_raw + (size_t)t * C + (size_t)i4 * 4;
 #pragma unroll
         for (int i = 0; i < ZB; ++i)
@@ -1110,20 +1159,20 @@ __global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
     }
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-      const int i4 = threadIdx.x + j * 256;
+      const int i4 = threadIdx.x + j * NT;
       if (i4 >= n4) continue;
       float4 v = acc[j];
       if (a.pend_cscale) {
-        const __half *cs = a.pend_cscale + (size_t)i4 * 4;
-        v.x *= __half2float(cs[0]); v.y *= __half2float(cs[1]); v.z *= __half2float(cs[2]); v.w *= __half2float(cs[3]);
+        const float4 cs = half4_value(EARLY ? ecs : reinterpret_cast<const uint2 *>(a.pend_cscale)[i4]);
+        v.x *= cs.x; v.y *= cs.y; v.z *= cs.z; v.w *= cs.w;
       }
       float r[4] = {1.f, 1.f, 1.f, 1.f};
       if (a.pend_r) {
-        const size_t o = (size_t)t * C + (size_t)i4 * 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          r[i] = __half2float(a.pend_r[o + i]);
-          if (a.pend_r_lo) r[i] += __half2float(a.pend_r_lo[o + i]);
+        const float4 rh = half4_value(EARLY ? erh : reinterpret_cast<const uint2 *>(a.pend_r + (size_t)t * C)[i4]);
+        r[0] = rh.x; r[1] = rh.y; r[2] = rh.z; r[3] = rh.w;
+        if (a.pend_r_lo) {
+          const float4 rl = half4_value(EARLY ? erl : reinterpret_cast<const uint2 *>(a.pend_r_lo + (size_t)t * C)[i4]);
+          r[0] += rl.x; r[1] += rl.y; r[2] += rl.z; r[3] += rl.w;
         }
       }
       xv[j] = make_float4((xv[j].x + r[0] * v.x) * a.pend_scale, (xv[j].y + r[1] * v.y) * a.pend_scale,
@@ -1134,16 +1183,14 @@ __global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
     __syncthreads();
     piv = piv_s;
   }
-  const float2 st = stats_from_regs<NJ>(xv, n4, piv, C, red);
+  const float2 st = stats_from_regs<NT, NJ>(xv, n4, piv, C, red);
   float2 sp = make_float2(0.f, 0.f);
-  if (from_row) sp = stats_from_regs<NJ>(pv, n4, a.x[(size_t)(t - 1) * C], C, red);
-  const uint8_t *srd = reinterpret_cast<const uint8_t *>(a.sx_rd) + (a.batch_mode ? (size_t)t * a.state_stride : 0);
-  uint8_t *swr = reinterpret_cast<uint8_t *>(a.sx_wr) + (a.batch_mode ? (size_t)t * a.state_stride : 0);
+  if (from_row) sp = stats_from_regs<NT, NJ>(pv, n4, a.x[(size_t)(t - 1) * C], C, red);
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    const int i4 = threadIdx.x + j * 256;
+    const int i4 = threadIdx.x + j * NT;
     if (i4 >= n4) continue;
-    const float4 w = reinterpret_cast<const float4 *>(a.ln_w)[i4], b = reinterpret_cast<const float4 *>(a.ln_b)[i4];
+    const float4 w = EARLY ? ew : reinterpret_cast<const float4 *>(a.ln_w)[i4], b = EARLY ? eb : reinterpret_cast<const float4 *>(a.ln_b)[i4];
     const float4 xx = make_float4((xv[j].x - st.x) * st.y * w.x + b.x, (xv[j].y - st.x) * st.y * w.y + b.y,
                                   (xv[j].z - st.x) * st.y * w.z + b.z, (xv[j].w - st.x) * st.y * w.w + b.w);
     const size_t o = (size_t)t * C + (size_t)i4 * 4;
@@ -1158,12 +1205,12 @@ __global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
       // what the token loop would have stored as shift state
       if (a.act_fp16) prev = make_float4(round_h(prev.x), round_h(prev.y), round_h(prev.z), round_h(prev.w));
     } else {
-      prev = load_act_f4(srd, i4, a.act_fp16);
+      prev = EARLY ? esx : load_act_f4(srd, i4, a.act_fp16);
     }
 #pragma unroll
     for (int v = 0; v < 4; ++v)
       if (v < a.nvec) {
-        const float4 m = reinterpret_cast<const float4 *>(a.mix[v])[i4];
+        const float4 m = EARLY ? em[v] : reinterpret_cast<const float4 *>(a.mix[v])[i4];
         store_hl4(a.op[v], a.op_lo[v], o,
                   make_float4(xx.x * m.x + prev.x * (1.f - m.x), xx.y * m.y + prev.y * (1.f - m.y),
                               xx.z * m.z + prev.z * (1.f - m.z), xx.w * m.w + prev.w * (1.f - m.w)));
@@ -1184,15 +1231,20 @@ __global__ void __launch_bounds__(256) ln_mix_seq_kernel(SeqLnArgs a) {
 // RWKV-4 WKV over rows (WkvForwardOne, att.cu:30-62, with the sigmoid of att.cu:154-159 fused): one thread per
 // (stream, channel), row b is the one token of stream b (prompts of one stream: wkv4_seq_kernel).
 //   out[row, c] = sigmoid(r) * wkv (fp16, the operand of the output projection); aa, bb, pp updated in place.
+// The loads are all asked for at once: the constants before the kernel ahead has finished, then the state and the slabs.
+// ZB: slabs per batch of loads.
+template <int ZB>
 __global__ void __launch_bounds__(256) wkv4_rows_kernel(Wkv4Args a) {
   pdl_trigger();
-  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (c >= a.C) return;
+  const float u = a.first[c], w = a.decay[c];
+  float ck = 1.f, cv = 1.f, cr = 1.f;
+  if (a.split > 1 && a.cs_k) { ck = __half2float(a.cs_k[c]); cv = __half2float(a.cs_v[c]); cr = __half2float(a.cs_r[c]); }
+  pdl_wait();
   float *st = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(a.state) + (size_t)b * a.state_stride);
   float aa = st[c], bb = st[a.C + c], pp = st[2 * a.C + c];
-  const float u = a.first[c], w = a.decay[c];
   {
     const int t = b;
     const size_t o = (size_t)t * a.C + c;
@@ -1200,11 +1252,19 @@ __global__ void __launch_bounds__(256) wkv4_rows_kernel(Wkv4Args a) {
     if (a.split > 1) {
       // the projections left their split-K slabs: sum them here, in slab order like gemm_finish_kernel
       k = 0.f; v = 0.f; rp = 0.f;
-      for (int z = 0; z < a.split; ++z) {
-        const size_t zo = ((size_t)z * a.T + t) * a.C + c;
-        k += a.raw_k[zo]; v += a.raw_v[zo]; rp += a.raw_r[zo];
+      for (int z0 = 0; z0 < a.split; z0 += ZB) {
+        float pk[ZB], pv[ZB], pr[ZB];
+#pragma unroll
+        for (int i = 0; i < ZB; ++i)
+          if (z0 + i < a.split) {
+            const size_t zo = ((size_t)(z0 + i) * a.T + t) * a.C + c;
+            pk[i] = a.raw_k[zo]; pv[i] = a.raw_v[zo]; pr[i] = a.raw_r[zo];
+          }
+#pragma unroll
+        for (int i = 0; i < ZB; ++i)
+          if (z0 + i < a.split) { k += pk[i]; v += pv[i]; rp += pr[i]; }
       }
-      if (a.cs_k) { k *= __half2float(a.cs_k[c]); v *= __half2float(a.cs_v[c]); rp *= __half2float(a.cs_r[c]); }
+      k *= ck; v *= cv; rp *= cr;
     } else {
       k = a.k[o]; v = a.v[o]; rp = a.r[o];
     }
@@ -1599,9 +1659,19 @@ cudaError_t launch_gather_emb(const void *emb, int emb_f32, const int32_t *ids, 
 }
 cudaError_t launch_ln_mix_seq(const SeqLnArgs &a, cudaStream_t st) {
   const int n4 = a.C >> 2;
-  if (n4 <= 2 * 256) launch_k(ln_mix_seq_kernel<2>, dim3(a.T), dim3(256), 0, st, a);
-  else if (n4 <= 4 * 256) launch_k(ln_mix_seq_kernel<4>, dim3(a.T), dim3(256), 0, st, a);
-  else launch_k(ln_mix_seq_kernel<LN_MAX4>, dim3(a.T), dim3(256), 0, st, a);
+  // Few rows: one piece of the row per thread, everything the row needs asked for at once (16 streams of the 1.5B shape:
+  // 1.46 ms a step against 1.63; 100: 1.69 against 1.85; a 29 token prompt: 1.68 against 1.80).  Many rows hide the round trips
+  // behind one another, and small CTAs with several pieces per thread pack better (a
+  // prompt of 1,000: 6.56 ms against 6.67).
+  if (a.T > LN_FEW_ROWS) {
+    if (n4 <= 2 * 256) launch_k(ln_mix_seq_kernel<256, 2>, dim3(a.T), dim3(256), 0, st, a);
+    else if (n4 <= 4 * 256) launch_k(ln_mix_seq_kernel<256, 4>, dim3(a.T), dim3(256), 0, st, a);
+    else launch_k(ln_mix_seq_kernel<256, LN_MAX4>, dim3(a.T), dim3(256), 0, st, a);
+  } else if (n4 <= 256) launch_k(ln_mix_seq_kernel<256, 1>, dim3(a.T), dim3(256), 0, st, a);
+  else if (n4 <= 512) launch_k(ln_mix_seq_kernel<512, 1>, dim3(a.T), dim3(512), 0, st, a);
+  else if (n4 <= 768) launch_k(ln_mix_seq_kernel<768, 1>, dim3(a.T), dim3(768), 0, st, a);
+  else if (n4 <= 4 * 256) launch_k(ln_mix_seq_kernel<256, 4>, dim3(a.T), dim3(256), 0, st, a);
+  else launch_k(ln_mix_seq_kernel<256, LN_MAX4>, dim3(a.T), dim3(256), 0, st, a);
   return cudaGetLastError();
 }
 // CTAs of the readout pass of the scan that are resident at once on the device: one wave of (head, chunk) pairs is what
@@ -1642,7 +1712,10 @@ cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
     return cudaGetLastError();
   }
   dim3 grid((a.C + 255) / 256, a.T);
-  launch_k(wkv4_rows_kernel, dim3(grid), dim3(256), 0, st, a);
+  // up to 64 rows of a 2,048 channel model a CTA per SM or two has to cover the whole round trip by itself (16 streams: 1.41 ms
+  // a step against 1.42); beyond, fewer registers and more CTAs are better (100: 1.68 against 1.70, 256: 2 % of the step)
+  if ((long long)a.T * a.C <= 64 * 2048) launch_k(wkv4_rows_kernel<8>, dim3(grid), dim3(256), 0, st, a);
+  else launch_k(wkv4_rows_kernel<4>, dim3(grid), dim3(256), 0, st, a);
   return cudaGetLastError();
 }
 cudaError_t launch_argmax_rows(const float *logits, int rows, int V, int ld, int32_t *out, GreedyCtl *ctl, cudaStream_t st) {

@@ -80,6 +80,25 @@ def test_every_few_stream_batch_of_one_model(pkg, orc, synth, name, fmt):
     m.close()
 
 
+@pytest.mark.parametrize("C", [1024, 1088, 2112, 3136])
+def test_layernorm_rows_of_every_width(pkg, orc, synth, C):
+    """The LayerNorm launch shapes of few rows (256, 512 or 768 threads with one piece of the row each, 256 with several)
+    at widths that leave their last warps partly idle, behind a projection that left its partial sums."""
+    shape = synth.Shape("4", 2, C, 1152, 96)
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), "fp16")
+    ref = orc.OracleModel(shape, tensors, synth.param_names(shape), rescale_every=6, weight_format="fp16", state_fp16=True)
+    m = pkg.Model(tensors, "cuda fp16", shape=shape, max_batch=12)
+    ids = synth.token_ids(shape, 2 * 12 + 7, seed=4)
+    got = [m.decode(ids[:12]), m.decode(ids[12:24])]
+    prompt = m.run([int(t) for t in ids[24:]])
+    for b in (11, 0):
+        ref.reset()
+        for t in range(2):
+            _close(got[t][b], ref.run(int(ids[t * 12 + b])), f"C={C} stream {b} step {t}")
+    _close(prompt, ref.run_seq([int(t) for t in ids[24:]]), f"C={C} prompt after the steps of stream 0")
+    m.close()
+
+
 def test_small_and_large_batches_share_state(pkg, orc, synth):
     """The persistent kernel (<= 8 streams) and the GEMM path (> 8) read and write the same state slots, and streams
     that are decoded together need not have seen the same number of tokens (continuous batching: a stream joins a
