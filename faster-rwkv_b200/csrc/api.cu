@@ -1015,6 +1015,12 @@ int fr_b200_vocab_padded(const fr_b200_model *m) { return m ? m->Vpad : FR_B200_
 
 namespace {
 
+// Prompts of up to this many rows and channels have no finishing pass: 29 int4 tokens of the 1.5B shape take 1.61 ms
+// instead of 1.67, 60 fp16 ones 1.39 instead of 1.49, 100 1.61 instead of 1.64; 200 int8 ones would take 2.56 instead of 2.51,
+// and at 2,560 channels a CTA has no registers left for the slabs of two rows (29 tokens: 2.73 instead of 2.40).
+// Key / value / receptance: as long as a thread of the scan has one token.
+constexpr int PROMPT_DEFER_ROWS = 128, PROMPT_DEFER_C = 2048, PROMPT_DEFER_KVR = 64;
+
 // The forward pass over R rows through [R, K] x [K, N] tensor-core GEMMs and row kernels.
 //   seq mode   (batch_mode = false): the rows are the tokens of one prompt of stream `slot`
 //              (def::ModelForwardSeq, kernels/default/model_forward_seq.cpp:48-184); logits of the last row only.
@@ -1025,6 +1031,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   const int C = m->C, F = m->F, H = m->H, af = m->cfg.act_fp16, T = R;
   if (C > 8192) return fail(FR_B200_E_UNSUPPORTED, "the row kernels of the GEMM path hold at most n_embd = 8192");
   const size_t TC = (size_t)T * C, TF = (size_t)T * F;
+  const bool defer_x = batch_mode || (T <= PROMPT_DEFER_ROWS && C <= PROMPT_DEFER_C);
   // activation buffers: one blob, 256-byte aligned pieces
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += align256(bytes); return o; };
@@ -1033,6 +1040,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
                o_g = take(TC * 2), o_yn = take(TC * 2), o_kk = take(TF * 2), o_lo0 = take(TC * 2), o_lo1 = take(TC * 2),
                o_lo2 = take(batch_mode ? TC * 2 : 0), o_lo3 = take(batch_mode ? TC * 2 : 0), o_ynlo = take(batch_mode ? TC * 2 : 0),
                o_kklo = take(batch_mode ? TF * 2 : 0), o_glo = take(batch_mode ? TC * 2 : 0),
+               o_x2 = take(!batch_mode && defer_x ? TC * 4 : 0),   // the residual rows of a short prompt alternate between two buffers
                o_raw = take(T <= GEMM_SMALL_M ? (size_t)GEMM_SPLIT_MAX * T * std::max(4 * C, F + C) * 4 : 0);   // split-K slabs
   // Long prompts are cut into pieces of rows that run on streams of their own, a layer apart: piece p's layer l needs
   // piece p's layer l - 1 (its stream order) and the recurrent state piece p - 1 left after layer l (an event), nothing
@@ -1117,15 +1125,17 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     CU(cudaEventRecord(start, st));
     for (int pc = 0; pc < n_pieces; ++pc) CU(cudaStreamWaitEvent(m->seq_streams[pc], start, 0));
   }
-  float *const x_all = x;
-  // Batch mode: a projection that was split over K leaves its slabs to the row kernel that follows it (the WKV step
-  // after key / value / receptance, the LayerNorm after the two projections that add to x) instead of a finishing
-  // pass of its own: three launches fewer per layer.
+  float *x_all = x, *x_other = (float *)(B + o_x2);
+  // Batch mode and short prompts: a projection that was split over K leaves its slabs to the row kernel that follows it
+  // (the WKV step after key / value / receptance, the LayerNorm after the two projections that add to x) instead of a
+  // finishing pass of its own: three launches fewer per layer.  A prompt's LayerNorm finishes the row before its own, too,
+  // and therefore writes the finished rows to a second buffer.
   struct Pending { const float *raw; const __half *cscale, *r, *r_lo; float scale; int split; } pend_x = {nullptr, nullptr, nullptr, nullptr, 1.f, 1};
   auto take_pending = [&](SeqLnArgs &la, float *xrows) {
     if (pend_x.split > 1) {
       la.pend_raw = pend_x.raw; la.pend_cscale = pend_x.cscale; la.pend_r = pend_x.r; la.pend_r_lo = pend_x.r_lo;
       la.pend_scale = pend_x.scale; la.pend_split = pend_x.split; la.x_wr = xrows;
+      if (!batch_mode) { la.x_wr = x_other; std::swap(x_all, x_other); }   // (one piece: row 0 is x_all)
     }
     pend_x.split = 1;
   };
@@ -1167,6 +1177,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     // activations as hi + lo fp16 pairs (a second pass over K), like every decode matvec does
     la.op_lo[0] = lo0; la.op_lo[1] = lo1; la.op_lo[2] = lo2; la.op_lo[3] = lo3;
     take_pending(la, x);
+    x = x_all + rc;
     CU(launch_ln_mix_seq(la, st));
     int kvr_split = 1;
     const __half *kvr_cs[3] = {nullptr, nullptr, nullptr};
@@ -1179,7 +1190,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
                          mk(T, op[2], a + "receptance.weight", C, C, GEMM_EPI_F32, r, nullptr, nullptr, 1.f, lo2)};
       if (m->gate) { grp[3] = mk(T, op[3], a + "gate.weight", C, C, GEMM_EPI_SILU_F16, g, nullptr, nullptr, 1.f, lo3); grp[3].out_lo = g_lo; }
       give_raw(grp, m->gate ? 4 : 3);
-      const bool defer = batch_mode && !m->v5;
+      const bool defer = defer_x && !m->v5 && (batch_mode || T <= PROMPT_DEFER_KVR);
       CU(launch_gemm_group(grp, m->gate ? 4 : 3, mt, st, defer ? &kvr_split : nullptr));
       for (int i = 0; i < 3; ++i) { kvr_cs[i] = grp[i].col_scale; kvr_raw[i] = grp[i].raw; }
     }
@@ -1210,7 +1221,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
       give_raw(&go, 1);
       // prompts: few tiles, 128-row tiles fill the SMs better (measured); streams: one pass over the weights for all rows
       int sp = 1;
-      CU(launch_gemm_group(&go, 1, batch_mode ? mt : 1, st, batch_mode ? &sp : nullptr));
+      CU(launch_gemm_group(&go, 1, batch_mode ? mt : 1, st, defer_x ? &sp : nullptr));
       if (sp > 1) pend_x = {go.raw, go.col_scale, nullptr, nullptr, go.scale, sp};
     }
     // ---- channel mix ----
@@ -1223,6 +1234,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     la.T = T; la.C = C; la.nvec = 2; la.act_fp16 = af;
     la.batch_mode = batch_mode; la.state_stride = m->state_stride;
     take_pending(la, x);
+    x = x_all + rc;
     CU(launch_ln_mix_seq(la, st));
     const bool halve = af && (l + 1) % 6 == 0;   // x / 2 every 6 layers under fp16 activations (model_forward_seq.cpp:165-167)
     {
@@ -1235,7 +1247,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
       gv.aux1_lo = rr_lo;
       give_raw(&gv, 1);
       int sp = 1;
-      CU(launch_gemm_group(&gv, 1, batch_mode ? mt : 1, st, batch_mode ? &sp : nullptr));
+      CU(launch_gemm_group(&gv, 1, batch_mode ? mt : 1, st, defer_x && (batch_mode || l + 1 < m->L) ? &sp : nullptr));
       if (sp > 1) pend_x = {gv.raw, gv.col_scale, rr, rr_lo, gv.scale, sp};
     }
     m->launches += m->v5 ? 9 : 7;
@@ -1262,7 +1274,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     return 0;
   }
   // last token -> ln_out -> head, as a stand-alone matvec over the head's streaming tiles
-  CU(launch_ln_row(x + (size_t)(T - 1) * C, vp("ln_out.weight"), vp("ln_out.bias"), C, m->d_lnvec, st));
+  CU(launch_ln_row(x_all + (size_t)(T - 1) * C, vp("ln_out.weight"), vp("ln_out.bias"), C, m->d_lnvec, st));
   DecodeParams p;
   memset(&p, 0, sizeof(p));
   p.version = 4; p.L = 0; p.C = 64; p.F = C; p.V = m->V; p.Vpad = m->Vpad; p.fmt = m->fmt; p.B = 1; p.n_phases = 1;

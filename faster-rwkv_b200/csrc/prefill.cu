@@ -1025,7 +1025,7 @@ __global__ void gather_emb_kernel(const void *emb, int emb_f32, const int32_t *i
 // row writes its new one.  nvec == 0: plain LayerNorm into op[0] (ln_out before the head).
 // Each thread keeps its float4 pieces of the row (and of the row before) in registers: x is read once.
 constexpr int LN_MAX4 = 8;   // float4 per thread: n_embd <= 8192
-constexpr int LN_FEW_ROWS = 512;   // two resident CTAs of 512 threads per SM carry 296 rows at once
+constexpr int LN_FEW_ROWS = 256;   // about two CTAs of 512 threads per SM
 template <int NT, int NJ>
 __device__ __forceinline__ float2 stats_from_regs(const float4 *v, int n4, float piv, int C, float *red) {
   float s1 = 0.f, s2 = 0.f;
@@ -1093,8 +1093,10 @@ __device__ __forceinline__ float4 half4_value(const uint2 &u) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// NT threads, NJ float4 pieces of a row per thread
-template <int NT, int NJ>
+// NT threads, NJ float4 pieces of a row per thread.  LN_PROMPT_PENDING: the tokens of a prompt behind a projection that
+// left its slabs, which two rows of a CTA have to add up (the registers for it would cost the other launches CTAs).
+enum LnKind { LN_ROWS, LN_PROMPT_PENDING };
+template <int NT, int NJ, LnKind KIND>
 __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
   constexpr bool EARLY = NJ == 1;
   pdl_trigger();
@@ -1126,66 +1128,75 @@ __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
       else if (EARLY && a.nvec > 0) esx = load_act_f4(srd, i4, a.act_fp16);
     }
   }
-  float piv = a.x[(size_t)t * C];
+  float piv = a.x[(size_t)t * C], ppiv = from_row ? a.x[(size_t)(t - 1) * C] : 0.f;
   if (a.pend_split > 1) {
     // the projection before this LayerNorm left its split-K slabs: sum them (in slab order, like gemm_finish_kernel),
-    // apply its epilogue x = (x + [r *] sum) * scale, store the finished row and normalise it from the registers
-    __shared__ float piv_s;
-    float4 acc[NJ];
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // apply its epilogue x = (x + [r *] sum) * scale, store the finished row and normalise it from the registers; a
+    // prompt's CTA does the same for the row before (which its own CTA stores: to another buffer than it is read from)
+    __shared__ float piv_s[2];
     const size_t zs = (size_t)a.T * C;
-    uint2 erh = make_uint2(0u, 0u), erl = erh;   // the factor, asked for together with the slabs
-    if (EARLY && a.pend_r && (int)threadIdx.x < n4) {
-      erh = reinterpret_cast<const uint2 *>(a.pend_r + (size_t)t * C)[threadIdx.x];
-      if (a.pend_r_lo) erl = reinterpret_cast<const uint2 *>(a.pend_r_lo + (size_t)t * C)[threadIdx.x];
-    }
     constexpr int ZB = NJ == 1 && NT <= 512 ? 16 : 4;   // slabs per batch: NJ x ZB 16-byte loads in flight per thread
-    for (int z0 = 0; z0 < a.pend_split; z0 += ZB) {
-      float4 p[NJ][ZB];
+    auto finish = [&](float4 *rowv, int row, const uint2 &erh, const uint2 &erl) {
+      float4 acc[NJ];
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int z0 = 0; z0 < a.pend_split; z0 += ZB) {
+        float4 p[NJ][ZB];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const int i4 = threadIdx.x + j * NT;
+          const float *slab = a.pend_raw + (size_t)row * C + (size_t)i4 * 4;
+#pragma unroll
+          for (int i = 0; i < ZB; ++i)
+            if (i4 < n4 && z0 + i < a.pend_split) p[j][i] = *reinterpret_cast<const float4 *>(slab + (size_t)(z0 + i) * zs);
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int i = 0; i < ZB; ++i)   // in slab order
+            if (z0 + i < a.pend_split) { acc[j].x += p[j][i].x; acc[j].y += p[j][i].y; acc[j].z += p[j][i].z; acc[j].w += p[j][i].w; }
+      }
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
         const int i4 = threadIdx.x + j * NT;
-        const float *slab = a.pend_raw + (size_t)t * C + (size_t)i4 * 4;
-#pragma unroll
-        for (int i = 0; i < ZB; ++i)
-          if (i4 < n4 && z0 + i < a.pend_split) p[j][i] = *reinterpret_cast<const float4 *>(slab + (size_t)(z0 + i) * zs);
-      }
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int i = 0; i < ZB; ++i)   // in slab order
-          if (z0 + i < a.pend_split) { acc[j].x += p[j][i].x; acc[j].y += p[j][i].y; acc[j].z += p[j][i].z; acc[j].w += p[j][i].w; }
-    }
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int i4 = threadIdx.x + j * NT;
-      if (i4 >= n4) continue;
-      float4 v = acc[j];
-      if (a.pend_cscale) {
-        const float4 cs = half4_value(EARLY ? ecs : reinterpret_cast<const uint2 *>(a.pend_cscale)[i4]);
-        v.x *= cs.x; v.y *= cs.y; v.z *= cs.z; v.w *= cs.w;
-      }
-      float r[4] = {1.f, 1.f, 1.f, 1.f};
-      if (a.pend_r) {
-        const float4 rh = half4_value(EARLY ? erh : reinterpret_cast<const uint2 *>(a.pend_r + (size_t)t * C)[i4]);
-        r[0] = rh.x; r[1] = rh.y; r[2] = rh.z; r[3] = rh.w;
-        if (a.pend_r_lo) {
-          const float4 rl = half4_value(EARLY ? erl : reinterpret_cast<const uint2 *>(a.pend_r_lo + (size_t)t * C)[i4]);
-          r[0] += rl.x; r[1] += rl.y; r[2] += rl.z; r[3] += rl.w;
+        if (i4 >= n4) continue;
+        float4 v = acc[j];
+        if (a.pend_cscale) {
+          const float4 cs = half4_value(EARLY ? ecs : reinterpret_cast<const uint2 *>(a.pend_cscale)[i4]);
+          v.x *= cs.x; v.y *= cs.y; v.z *= cs.z; v.w *= cs.w;
         }
+        float r[4] = {1.f, 1.f, 1.f, 1.f};
+        if (a.pend_r) {
+          const float4 rh = half4_value(EARLY ? erh : reinterpret_cast<const uint2 *>(a.pend_r + (size_t)row * C)[i4]);
+          r[0] = rh.x; r[1] = rh.y; r[2] = rh.z; r[3] = rh.w;
+          if (a.pend_r_lo) {
+            const float4 rl = half4_value(EARLY ? erl : reinterpret_cast<const uint2 *>(a.pend_r_lo + (size_t)row * C)[i4]);
+            r[0] += rl.x; r[1] += rl.y; r[2] += rl.z; r[3] += rl.w;
+          }
+        }
+        rowv[j] = make_float4((rowv[j].x + r[0] * v.x) * a.pend_scale, (rowv[j].y + r[1] * v.y) * a.pend_scale,
+                              (rowv[j].z + r[2] * v.z) * a.pend_scale, (rowv[j].w + r[3] * v.w) * a.pend_scale);
+        if (row == t) reinterpret_cast<float4 *>(a.x_wr + (size_t)t * C)[i4] = rowv[j];
+        if (i4 == 0) piv_s[t - row] = rowv[j].x;
       }
-      xv[j] = make_float4((xv[j].x + r[0] * v.x) * a.pend_scale, (xv[j].y + r[1] * v.y) * a.pend_scale,
-                          (xv[j].z + r[2] * v.z) * a.pend_scale, (xv[j].w + r[3] * v.w) * a.pend_scale);
-      reinterpret_cast<float4 *>(a.x_wr + (size_t)t * C)[i4] = xv[j];
-      if (i4 == 0) piv_s = xv[j].x;
-    }
+    };
+    // the factor is asked for together with the slabs
+    uint2 eh[2], el[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (EARLY && a.pend_r && (i == 0 || (KIND == LN_PROMPT_PENDING && from_row)) && (int)threadIdx.x < n4) {
+        eh[i] = reinterpret_cast<const uint2 *>(a.pend_r + (size_t)(t - i) * C)[threadIdx.x];
+        if (a.pend_r_lo) el[i] = reinterpret_cast<const uint2 *>(a.pend_r_lo + (size_t)(t - i) * C)[threadIdx.x];
+      }
+    finish(xv, t, eh[0], el[0]);
+    if (KIND == LN_PROMPT_PENDING && from_row) finish(pv, t - 1, eh[1], el[1]);
     __syncthreads();
-    piv = piv_s;
+    piv = piv_s[0];
+    if (KIND == LN_PROMPT_PENDING) ppiv = piv_s[1];
   }
   const float2 st = stats_from_regs<NT, NJ>(xv, n4, piv, C, red);
   float2 sp = make_float2(0.f, 0.f);
-  if (from_row) sp = stats_from_regs<NT, NJ>(pv, n4, a.x[(size_t)(t - 1) * C], C, red);
+  if (from_row) sp = stats_from_regs<NT, NJ>(pv, n4, ppiv, C, red);
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
     const int i4 = threadIdx.x + j * NT;
@@ -1318,7 +1329,7 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
   const float u = a.first[c], w = a.decay[c];
   const float *kp = a.k + c, *vp = a.v + c, *rp = a.r + c;
   constexpr int NR = LEN > 0 ? LEN : 1;
-  float kr[NR], vr[NR];
+  float kr[NR], vr[NR], rsum = 0.f;
   float aa = 0.f, bb = 0.f, pp = -1e30f;
   auto absorb = [&](float k, float v) {
     const float ww = w + pp, pm = fmaxf(ww, k);
@@ -1330,7 +1341,22 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
   if (LEN > 0) {
 #pragma unroll
     for (int i = 0; i < NR; ++i)
-      if (t0 + i < t1) { kr[i] = kp[(size_t)(t0 + i) * a.C]; vr[i] = vp[(size_t)(t0 + i) * a.C]; }
+      if (t0 + i < t1) {
+        if (LEN == 1 && a.split > 1) {
+          // the projections left their split-K slabs: one token per thread sums its own, in slab order
+          float k = 0.f, v = 0.f, r = 0.f;
+#pragma unroll 4
+          for (int z = 0; z < a.split; ++z) {
+            const size_t zo = ((size_t)z * a.T + t0) * a.C + c;
+            k += a.raw_k[zo]; v += a.raw_v[zo]; r += a.raw_r[zo];
+          }
+          if (a.cs_k) { k *= __half2float(a.cs_k[c]); v *= __half2float(a.cs_v[c]); r *= __half2float(a.cs_r[c]); }
+          kr[0] = k; vr[0] = v; rsum = r;
+        } else {
+          kr[i] = kp[(size_t)(t0 + i) * a.C]; vr[i] = vp[(size_t)(t0 + i) * a.C];
+          if (LEN == 1) rsum = rp[(size_t)t0 * a.C];
+        }
+      }
 #pragma unroll
     for (int i = 0; i < NR; ++i)
       if (t0 + i < t1) absorb(kr[i], vr[i]);
@@ -1382,7 +1408,7 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
   if (LEN > 0) {
 #pragma unroll
     for (int i = 0; i < NR; ++i)
-      if (t0 + i < t1) step(t0 + i, kr[i], vr[i], rp[(size_t)(t0 + i) * a.C]);
+      if (t0 + i < t1) step(t0 + i, kr[i], vr[i], LEN == 1 ? rsum : rp[(size_t)(t0 + i) * a.C]);
   } else {
 #pragma unroll 4
     for (int t = t0; t < t1; ++t) step(t, kp[(size_t)t * a.C], vp[(size_t)t * a.C], rp[(size_t)t * a.C]);
@@ -1659,19 +1685,21 @@ cudaError_t launch_gather_emb(const void *emb, int emb_f32, const int32_t *ids, 
 }
 cudaError_t launch_ln_mix_seq(const SeqLnArgs &a, cudaStream_t st) {
   const int n4 = a.C >> 2;
+  const dim3 grid(a.T);
   // Few rows: one piece of the row per thread, everything the row needs asked for at once (16 streams of the 1.5B shape:
   // 1.46 ms a step against 1.63; 100: 1.69 against 1.85; a 29 token prompt: 1.68 against 1.80).  Many rows hide the round trips
-  // behind one another, and small CTAs with several pieces per thread pack better (a
-  // prompt of 1,000: 6.56 ms against 6.67).
-  if (a.T > LN_FEW_ROWS) {
-    if (n4 <= 2 * 256) launch_k(ln_mix_seq_kernel<256, 2>, dim3(a.T), dim3(256), 0, st, a);
-    else if (n4 <= 4 * 256) launch_k(ln_mix_seq_kernel<256, 4>, dim3(a.T), dim3(256), 0, st, a);
-    else launch_k(ln_mix_seq_kernel<256, LN_MAX4>, dim3(a.T), dim3(256), 0, st, a);
-  } else if (n4 <= 256) launch_k(ln_mix_seq_kernel<256, 1>, dim3(a.T), dim3(256), 0, st, a);
-  else if (n4 <= 512) launch_k(ln_mix_seq_kernel<512, 1>, dim3(a.T), dim3(512), 0, st, a);
-  else if (n4 <= 768) launch_k(ln_mix_seq_kernel<768, 1>, dim3(a.T), dim3(768), 0, st, a);
-  else if (n4 <= 4 * 256) launch_k(ln_mix_seq_kernel<256, 4>, dim3(a.T), dim3(256), 0, st, a);
-  else launch_k(ln_mix_seq_kernel<256, LN_MAX4>, dim3(a.T), dim3(256), 0, st, a);
+  // behind one another, and small CTAs with several pieces per thread pack better (a prompt of 1,000: 6.56 ms against 6.67).
+  const bool few = a.T <= LN_FEW_ROWS;
+  if (!a.batch_mode && a.pend_split > 1) {   // (short prompts of models up to 2,048 channels: PROMPT_DEFER_ROWS, _C)
+    if (!few || n4 > 512) return cudaErrorInvalidValue;
+    if (n4 <= 256) launch_k(ln_mix_seq_kernel<256, 1, LN_PROMPT_PENDING>, grid, dim3(256), 0, st, a);
+    else launch_k(ln_mix_seq_kernel<512, 1, LN_PROMPT_PENDING>, grid, dim3(512), 0, st, a);
+  } else if (few && n4 <= 256) launch_k(ln_mix_seq_kernel<256, 1, LN_ROWS>, grid, dim3(256), 0, st, a);
+  else if (few && n4 <= 512) launch_k(ln_mix_seq_kernel<512, 1, LN_ROWS>, grid, dim3(512), 0, st, a);
+  else if (few && n4 <= 768) launch_k(ln_mix_seq_kernel<768, 1, LN_ROWS>, grid, dim3(768), 0, st, a);
+  else if (n4 <= 2 * 256) launch_k(ln_mix_seq_kernel<256, 2, LN_ROWS>, grid, dim3(256), 0, st, a);
+  else if (n4 <= 4 * 256) launch_k(ln_mix_seq_kernel<256, 4, LN_ROWS>, grid, dim3(256), 0, st, a);
+  else launch_k(ln_mix_seq_kernel<256, LN_MAX4, LN_ROWS>, grid, dim3(256), 0, st, a);
   return cudaGetLastError();
 }
 // CTAs of the readout pass of the scan that are resident at once on the device: one wave of (head, chunk) pairs is what

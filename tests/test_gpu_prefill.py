@@ -199,3 +199,18 @@ def test_rwkv4_prompt_scan(pkg, orc, synth, T):
             _close(st[l][i], blk[i], f"T={T} state {i} of layer {l}", scale_aware=True)
     _close(m.run(7), ref.run(7), "token after the prompt")
     m.close()
+
+
+@pytest.mark.parametrize("C,T", [(1024, 2), (1088, 64), (1088, 65), (1088, 128), (1088, 129), (2112, 64)])
+def test_short_prompt_without_finishing_passes(pkg, orc, synth, C, T):
+    """Short prompts whose projections leave their split-K sums to the row kernels behind them: both LayerNorm widths, the
+    edges of the row counts up to which the scan and the LayerNorms take them, and a model too wide for it."""
+    shape = synth.Shape("4", 2, C, 1152, 96)
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), "fp32")
+    ref = orc.OracleModel(shape, tensors, synth.param_names(shape), rescale_every=0, weight_format="int8", state_fp16=False)
+    ids = [int(t) for t in synth.token_ids(shape, 3 + T, seed=2)]
+    m = pkg.Model(tensors, "cuda int8", shape=shape)
+    m.run(ids[:3]), ref.run_seq(ids[:3])
+    _close(m.run(ids[3:]), ref.run_seq(ids[3:]), f"C={C} T={T}")
+    _close(m.run(7), ref.run(7), "token after the prompt")
+    m.close()
