@@ -109,6 +109,10 @@ __device__ __forceinline__ void block_scan(SampleSmem &s, unsigned long long &a,
   if (warp > 0) { a += s.wsum[warp - 1]; c += s.csum[warp - 1]; }
 }
 
+// Distance of a logit below the row's maximum.  What a caller masks (-inf) lies infinitely far below: no weight, and not
+// among the candidates.  +inf is at distance 0 of itself, a row of -inf alone is a row of equals; NaN is no candidate either.
+__device__ __forceinline__ float below(float mx, float v) { return v == mx ? 0.f : mx - v; }
+
 struct Entry { float d; int id; };
 __device__ __forceinline__ bool precedes(float d, int id, const Entry &e) { return d < e.d || (d == e.d && id <= e.id); }
 
@@ -127,12 +131,12 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
     auto inside = [&](float d, int id) {
       for (int q = 0; q < level; ++q)
         if (bin_of(d, s.lo[q], s.scale[q]) != s.bin[q]) return false;
-      return precedes(d, id, last);
+      return d < INFINITY && precedes(d, id, last);
     };
     s.lo32[threadIdx.x] = 0; s.hi32[threadIdx.x] = 0; s.count[threadIdx.x] = 0;
     __syncthreads();
     for_row(row, V, [&](float v, int id) {
-      const float d = mx - v;
+      const float d = below(mx, v);
       if (!inside(d, id)) return;
       const int b = bin_of(d, wlo, wscale);
       const unsigned long long w = fx_weight(d, inv_t);
@@ -149,10 +153,8 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
       const unsigned long long total = s.wsum[31];
       const double t = ceil(frac * (double)total);
       target = t >= (double)total ? total : t > 0.0 ? (unsigned long long)t : 0ull;
-      if (threadIdx.x == 0) s.found = SM_T;
-    } else if (threadIdx.x == 0) {
-      s.found = SM_T;
     }
+    if (threadIdx.x == 0) s.found = SM_T;
     __syncthreads();
     const bool reached = before + a >= target || (k > 0 && cbefore + ca >= k);
     if (reached && (threadIdx.x == 0 || m > 0 || c > 0)) atomicMin(&s.found, (int)threadIdx.x);
@@ -163,7 +165,7 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
     before = s.before; cbefore = s.cbefore;
     // the members of that bin
     for_row(row, V, [&](float v, int id) {
-      const float d = mx - v;
+      const float d = below(mx, v);
       if (!inside(d, id) || bin_of(d, wlo, wscale) != fb) return;
       const unsigned at = atomicAdd(&s.n, 1u);
       if (at < SM_T) { s.d[at] = d; s.count[at] = (unsigned)id; }
@@ -172,6 +174,7 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
     __syncthreads();
     const unsigned n = s.n;
     const float dmin = s.dmin, dmax = s.dmax;
+    if (n == 0) return Entry{0.f, 0};   // a row without candidates (nothing but NaN)
     if (n <= SM_T) {
       // rank the members: running weight and count up to and including each one
       const bool mine = threadIdx.x < n;
@@ -206,7 +209,7 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
       if (k > 0) want = min(want, k > cbefore ? k - cbefore : 1u);
       want = max(want, 1u);
       const int S = (V + SM_T - 1) / SM_T, i0 = min(V, (int)threadIdx.x * S), i1 = min(V, i0 + S);
-      auto member = [&](int i) { const float d = mx - row[i]; return inside(d, i) && bin_of(d, wlo, wscale) == fb; };
+      auto member = [&](int i) { const float d = below(mx, row[i]); return inside(d, i) && bin_of(d, wlo, wscale) == fb; };
       unsigned here = 0;
       for (int i = i0; i < i1; ++i) here += member(i);
       unsigned long long dummy = 0;
@@ -215,7 +218,7 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
       if (upto - here < want && upto >= want) {
         unsigned q = upto - here;
         for (int i = i0; i < i1; ++i)
-          if (member(i) && ++q == want) { s.found = i; s.dmax = mx - row[i]; }
+          if (member(i) && ++q == want) { s.found = i; s.dmax = below(mx, row[i]); }
       }
       __syncthreads();
       Entry r{s.dmax, s.found};

@@ -127,3 +127,34 @@ def test_sample_finds_its_entry_at_any_spread_of_the_logits(pkg, synth, vocab, g
             else:
                 assert pick_distance(logits[b], temperature, top_k, top_p, u[b], int(got[b])) <= tol
     m.close()
+
+
+def _given_logits(pkg, synth, rows):
+    """A model whose device logits are exactly `rows` [B, V]: a zero head, then the values as adjustments (0 + x)."""
+    B, V = rows.shape
+    shape = synth.Shape("4", 1, 64, 64, V)
+    master = synth.generate(shape, seed=3, ln_random=True)
+    master["head.weight"] = master["head.weight"] * np.float32(0)
+    m = pkg.Model(synth.to_file_dtypes(shape, master, "fp16"), "cuda fp16", shape=shape, max_batch=B)
+    m.decode(np.zeros(B, np.int32), want_logits=False, want_argmax=True)
+    m.logits_add(np.repeat(np.arange(B), V), np.tile(np.arange(V), B), rows.reshape(-1))
+    return m
+
+
+def test_sample_of_rows_without_an_ordinary_maximum(pkg, synth):
+    """+inf entries are the maximum, a row of -inf alone is a row of equals, NaN is never picked next to a number."""
+    V = 4096
+    rows = np.zeros((4, V), np.float32)
+    rows[0, [5, 99]] = np.inf
+    rows[1] = -np.inf
+    rows[2, ::2] = np.nan
+    rows[3] = np.nan
+    m = _given_logits(pkg, synth, rows)
+    for top_k, top_p in ((0, 1.0), (10, 0.9), (3, 1.0)):
+        for u in (0.0, 0.4, 1.0):
+            got = m.sample(4, 1.0, top_k, top_p, [u] * 4)
+            assert got[0] in (5, 99)
+            assert 0 <= got[1] < V and (top_k == 0 or got[1] < top_k)
+            assert got[2] % 2 == 1
+            assert got[3] == 0
+    m.close()
