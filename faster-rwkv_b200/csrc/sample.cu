@@ -28,6 +28,7 @@ constexpr int SM_T = 1024;                    // threads = histogram bins = most
 constexpr int SM_LEVELS = 6;                  // narrowings, 1024 times finer each; a bin of equal values ends it
 constexpr float SM_SPAN = 32.f;               // first histogram: the row's spread, at most this far in the exponent (e^-32 has no weight)
 constexpr float SM_ONE = 1099511627776.f;     // 2^40
+constexpr unsigned long long SM_NEVER = 1ull << 62;   // more than any sum of weights
 
 constexpr int SM_RD = 4;
 
@@ -117,7 +118,8 @@ struct Entry { float d; int id; };
 __device__ __forceinline__ bool precedes(float d, int id, const Entry &e) { return d < e.d || (d == e.d && id <= e.id); }
 
 // First entry, in order of (d, index), at which the running weight reaches frac * (total weight) or the running count
-// reaches k (k > 0), among the entries that do not come after `last`; the last entry with weight if neither is reached.
+// reaches k (k > 0), among the entries that do not come after `last`; the last of them if there are fewer than k.
+// frac > 1 is a target that no sum reaches (the count alone decides).
 __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int V, float mx, float span, float inv_t, double frac,
                                               unsigned k, const Entry &last) {
   unsigned long long target = 0, before = 0;   // weight and entries ahead of the interval
@@ -152,7 +154,8 @@ __device__ __noinline__ Entry select_entry(SampleSmem &s, const float *row, int 
     if (level == 0) {
       const unsigned long long total = s.wsum[31];
       const double t = ceil(frac * (double)total);
-      target = t >= (double)total ? total : t > 0.0 ? (unsigned long long)t : 0ull;
+      target = !(frac <= 1.0) ? SM_NEVER : t >= (double)total ? total : t > 0.0 ? (unsigned long long)t : 0ull;
+      k = min(k, s.csum[31]);            // (candidates in all)
     }
     if (threadIdx.x == 0) s.found = SM_T;
     __syncthreads();
@@ -264,6 +267,7 @@ __global__ void __launch_bounds__(SM_T) sample_rows_kernel(const __grid_constant
   if (a.top_p < 1.f || (k > 0 && k < (unsigned)a.V)) cut = select_entry(s, row, a.V, mx, mx - mn, 1.f, (double)a.top_p, k, all);
   const float inv_t = 1.f / fminf(fmaxf(a.temperature, 0.1f), 5.f);
   float u = a.u_dev ? a.u_dev[blockIdx.x] : a.u[blockIdx.x];
+  u = u <= 1.f ? u : 1.f;
   if (inv_t > 1.f) {
     // the reference raises the probabilities themselves: where even the largest one's power underflows, all weights are
     // zero and its walk stops at the first entry

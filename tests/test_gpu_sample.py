@@ -141,6 +141,31 @@ def _given_logits(pkg, synth, rows):
     return m
 
 
+@pytest.mark.parametrize("masked", [0, 1, 40000])
+@pytest.mark.parametrize("top_k,top_p", [(3000, 1.5), (3000, 0.0), (0, 0.5), (0, 1.5), (60000, 2.0)])
+def test_sample_with_masked_logits(pkg, synth, masked, top_k, top_p):
+    """Logits of -inf are never picked and take no part in a cut, and top_p > 1 is no cut at all (the running sum does not
+    reach it, sampler.cpp:59-66).  The rows have a peak far above a bulk that only a temperature above 1 gives weight to, so
+    that the top-k cut falls far behind the last entry with a noticeable probability."""
+    V, B = 65536, 3
+    rng = np.random.default_rng(8)
+    rows = (-33 - 20 * rng.random((B, V))).astype(np.float32)
+    for b in range(B):
+        rows[b, rng.permutation(V)[:masked]] = -np.inf
+        rows[b, 17 + b] = 0.0
+    m = _given_logits(pkg, synth, rows)
+    for temperature in (5.0, 1.0):
+        for u in ([0.0, 0.5, 0.9], [0.97, 0.7, 1.0]):
+            u = np.float32(u)
+            got = m.sample(B, temperature, top_k, top_p, u)
+            for b in range(B):
+                assert np.isfinite(rows[b, got[b]])
+                # the fp32 running sum over tens of thousands of entries: 1e-3 of the total bounds its error
+                dist = pick_distance(rows[b], temperature, top_k, top_p, u[b], int(got[b]))
+                assert dist <= 1e-3, (temperature, top_k, top_p, b, float(u[b]), int(got[b]), dist)
+    m.close()
+
+
 def test_sample_of_rows_without_an_ordinary_maximum(pkg, synth):
     """+inf entries are the maximum, a row of -inf alone is a row of equals, NaN is never picked next to a number."""
     V = 4096
@@ -150,7 +175,7 @@ def test_sample_of_rows_without_an_ordinary_maximum(pkg, synth):
     rows[2, ::2] = np.nan
     rows[3] = np.nan
     m = _given_logits(pkg, synth, rows)
-    for top_k, top_p in ((0, 1.0), (10, 0.9), (3, 1.0)):
+    for top_k, top_p in ((0, 1.0), (10, 0.9), (3, 2.0)):
         for u in (0.0, 0.4, 1.0):
             got = m.sample(4, 1.0, top_k, top_p, [u] * 4)
             assert got[0] in (5, 99)
