@@ -183,3 +183,39 @@ def test_sample_of_rows_without_an_ordinary_maximum(pkg, synth):
             assert got[2] % 2 == 1
             assert got[3] == 0
     m.close()
+
+
+@pytest.mark.parametrize("rows", [1, 512, 513, 700])
+def test_sample_from_and_to_host_and_device_memory(pkg, synth, rows):
+    """Draws as kernel parameters (up to 512 rows on the host) and through device memory (more rows, or given there), ids to
+    the host and to the device: the same picks, and the reference's."""
+    import ctypes
+    import torch
+    shape = synth.Shape("4", 1, 64, 64, 1000)
+    master = synth.generate(shape, seed=3, ln_random=True)
+    master["head.weight"] = master["head.weight"] * np.float32(4)
+    m = pkg.Model(synth.to_file_dtypes(shape, master, "fp16"), "cuda fp16", shape=shape, max_batch=rows)
+    logits = m.decode(np.arange(rows) % shape.vocab)
+    u = np.random.default_rng(2).random(rows).astype(np.float32)
+    want = m.sample(rows, 1.0, 0, 0.8, u)
+    checked = 0
+    for b in range(rows):
+        ref, margin = ref_sample(logits[b], 1.0, 0, 0.8, u[b])
+        if margin > 1e-5:
+            assert want[b] == ref
+            checked += 1
+    assert checked >= rows * 3 // 4
+    ud, out = torch.from_numpy(u).cuda(), np.empty(rows, np.int32)
+    od = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    f = ctypes.c_float
+    for up in (u.ctypes.data, ud.data_ptr()):
+        for op in (out.ctypes.data, od.data_ptr()):
+            out[:] = -1
+            od.fill_(-1)
+            torch.cuda.synchronize()
+            pkg.check(pkg.lib().fr_b200_sample(m.handle, rows, f(1.0), 0, f(0.8), up, op, None), "fr_b200_sample")
+            torch.cuda.synchronize()
+            got = out if op == out.ctypes.data else od.cpu().numpy()
+            assert np.array_equal(got, want)
+    m.close()
