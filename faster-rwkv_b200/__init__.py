@@ -11,7 +11,6 @@ from __future__ import annotations
 
 import ctypes
 import os
-import sys
 from typing import Dict, Iterable, List, Optional, Sequence, Union
 
 import numpy as np
@@ -199,28 +198,13 @@ class Model:
         check(lib().fr_b200_set_tensor(self._h, name.encode(), ptr, dt, sh, len(shp)), f"fr_b200_set_tensor({name})")
 
     # -- forward -----------------------------------------------------------------------------
-    _POOL = 4   # result arrays kept per model
-
-    def _result(self, shape) -> np.ndarray:
-        """An uninitialised fp32 array for logits.  Arrays of earlier results that nobody holds any more (views count) are
-        used again: a fresh 256 KB array costs 64 page faults, a tenth of a small model's token."""
-        pool = self.__dict__.setdefault("_pool", [])
-        for i in range(len(pool)):
-            if pool[i].shape == shape and sys.getrefcount(pool[i]) == 2:   # the pool's reference and the argument's
-                return pool[i]
-        a = np.empty(shape, np.float32)
-        if len(pool) >= self._POOL:
-            pool.pop(0)
-        pool.append(a)
-        return a
-
     def run(self, ids: Union[int, Sequence[int]], slot: int = 0) -> np.ndarray:
         """Model::Run (model.cpp:188-208): one id, or a list processed in order; logits of the last token.
         slot: the stream whose state the prompt advances (prompts on slots > 0 need the seq / GEMM path)."""
         if isinstance(ids, (int, np.integer)):
             ids = [int(ids)]
         ids = np.ascontiguousarray(ids, np.int32)
-        out = self._result((self.vocab,))
+        out = np.empty(self.vocab, np.float32)
         check(lib().fr_b200_run_seq(self._h, slot, _np_ptr(ids), len(ids), _np_ptr(out), None), "fr_b200_run_seq")
         return out
 
@@ -228,7 +212,7 @@ class Model:
         """One token for each of len(ids) independent streams (stream b = state slot b)."""
         ids = np.ascontiguousarray(ids, np.int32)
         B = len(ids)
-        logits = self._result((B, self.vocab)) if want_logits else None
+        logits = np.empty((B, self.vocab), np.float32) if want_logits else None
         amax = np.empty(B, np.int32) if want_argmax else None
         check(lib().fr_b200_decode(self._h, _np_ptr(ids), B, _np_ptr(logits) if want_logits else None,
                                    _np_ptr(amax) if want_argmax else None, None), "fr_b200_decode")

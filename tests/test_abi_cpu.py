@@ -86,3 +86,43 @@ def test_fr_file_roundtrip(synth, tmp_path):
     assert synth.to_file_dtypes(shape, master, "fp16")["blocks.0.att.ln_x.weight"].dtype == np.float32
     names = synth.param_names(shape)
     assert len(names) == shape.n_layer * 22 + 3 and names[-1] == "head.weight"
+
+
+def test_results_belong_to_the_caller(pkg, monkeypatch):
+    """What run and decode return is the caller's alone: held results keep their values and the model keeps no storage of
+    released ones (a weak reference to a result dies with it)."""
+    import weakref
+
+    class Lib:
+        calls = 0
+
+        def _fill(self, ptr, n):
+            self.calls += 1
+            ctypes.memmove(ptr, np.full(n, self.calls, np.float32).ctypes.data, n * 4)
+            return 0
+
+        def fr_b200_run_seq(self, h, slot, ids, n, out, st):
+            return self._fill(out, 6)
+
+        def fr_b200_decode(self, h, ids, B, logits, amax, st):
+            return self._fill(logits, B * 6)
+
+        def fr_b200_destroy(self, h):
+            pass
+
+    fake = Lib()
+    monkeypatch.setattr(pkg, "lib", lambda: fake)
+    m = pkg.Model.__new__(pkg.Model)
+    m._h, m.vocab = ctypes.c_void_p(), 6
+    for call, shape in ((lambda: m.run(1), (6,)), (lambda: m.decode([1, 2]), (2, 6))):
+        held = [call() for _ in range(6)]
+        tail = held[0][1:]
+        assert all(r.shape == shape and r.dtype == np.float32 for r in held)
+        assert [float(r.flat[0]) for r in held] == [fake.calls - 5 + i for i in range(6)]
+        gone = weakref.ref(held.pop(0))
+        want = tail.copy()
+        for _ in range(6):
+            call()
+        assert np.array_equal(tail, want)
+        del tail
+        assert gone() is None
