@@ -119,10 +119,11 @@ def test_results_belong_to_the_caller(pkg, monkeypatch):
         tail = held[0][1:]
         assert all(r.shape == shape and r.dtype == np.float32 for r in held)
         assert [float(r.flat[0]) for r in held] == [fake.calls - 5 + i for i in range(6)]
-        gone = weakref.ref(held.pop(0))
+        gone = [weakref.ref(r) for r in held]
+        held.clear()
         want = tail.copy()
         for _ in range(6):
             call()
         assert np.array_equal(tail, want)
         del tail
-        assert gone() is None
+        assert all(r() is None for r in gone)
