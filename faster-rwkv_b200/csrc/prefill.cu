@@ -1024,6 +1024,24 @@ __global__ void gather_emb_kernel(const void *emb, int emb_f32, const int32_t *i
 // Batch mode (rows = independent streams, one token each): prev of row b is stream b's stored shift state and every
 // row writes its new one.  nvec == 0: plain LayerNorm into op[0] (ln_out before the head).
 // Each thread keeps its float4 pieces of the row (and of the row before) in registers: x is read once.
+// Sums and products are written as the operations they round to: left to the compiler, which product of a sum becomes a
+// fused multiply-add depends on what else an instance contains, and RWKV-5 amplifies the last bit of a row over 32 layers to
+// 1.2 - 2 % of quantised logits.  So every instance gives the same bits.
+__device__ __forceinline__ float ln_squares(float d0, float d1, float d2, float d3) {
+  return __fadd_rn(__fmaf_rn(d0, d0, __fmul_rn(d1, d1)), __fmaf_rn(d2, d2, __fmul_rn(d3, d3)));
+}
+__device__ __forceinline__ float ln_value(float x, const float2 &stats, float w, float b) {
+  return __fmaf_rn(__fmul_rn(__fsub_rn(x, stats.x), stats.y), w, b);
+}
+__device__ __forceinline__ float4 ln_value4(const float4 &x, const float2 &s, const float4 &w, const float4 &b) {
+  return make_float4(ln_value(x.x, s, w.x, b.x), ln_value(x.y, s, w.y, b.y), ln_value(x.z, s, w.z, b.z), ln_value(x.w, s, w.w, b.w));
+}
+__device__ __forceinline__ float mix_value(float x, float prev, float m) { return __fmaf_rn(x, m, __fmul_rn(prev, __fsub_rn(1.f, m))); }
+__device__ __forceinline__ float2 ln_stats(const float2 &sums, float piv, int C) {
+  const float m = sums.x / (float)C;
+  const float var = __fmaf_rn(-m, m, sums.y / (float)C);
+  return make_float2(piv + m, rsqrtf((var > 0.f ? var : 0.f) + 1e-5f));
+}
 constexpr int LN_MAX4 = 8;   // float4 per thread: n_embd <= 8192
 constexpr int LN_FEW_ROWS = 256;   // about two CTAs of 512 threads per SM
 template <int NT, int NJ>
@@ -1034,7 +1052,7 @@ __device__ __forceinline__ float2 stats_from_regs(const float4 *v, int n4, float
     if ((int)threadIdx.x + j * NT < n4) {
       const float d0 = v[j].x - piv, d1 = v[j].y - piv, d2 = v[j].z - piv, d3 = v[j].w - piv;
       s1 += (d0 + d1) + (d2 + d3);
-      s2 += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+      s2 += ln_squares(d0, d1, d2, d3);
     }
   }
   float2 s;
@@ -1061,10 +1079,7 @@ __device__ __forceinline__ float2 stats_from_regs(const float4 *v, int n4, float
 #pragma unroll
     for (int w = 0; w < 8; ++w) { s.x += red[w * 2]; s.y += red[w * 2 + 1]; }
   }
-  const float m = s.x / (float)C;
-  float var = s.y / (float)C - m * m;
-  var = var > 0.f ? var : 0.f;
-  return make_float2(piv + m, rsqrtf(var + 1e-5f));
+  return ln_stats(s, piv, C);
 }
 __device__ __forceinline__ void store_hl4(__half *hi, __half *lo, size_t o, const float4 &v) {
   const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
@@ -1094,9 +1109,9 @@ __device__ __forceinline__ float4 half4_value(const uint2 &u) {
 }
 
 // NT threads, NJ float4 pieces of a row per thread.  What a launch does not need costs it registers, and those cost CTAs, so
-// there are three kinds: LN_ROWS (streams), LN_PROMPT (the tokens of a prompt, nothing pending: 60 registers instead of 152 at
-// 2,560 channels, a prompt of 4,096 tokens in 44.3 ms instead of 46.7), LN_PROMPT_PENDING (behind a projection that left its
-// slabs: two rows of a CTA to add up).
+// there are three kinds: LN_ROWS (streams: one row, its slabs pending or not), LN_PROMPT (the tokens of a prompt, two rows,
+// nothing pending: 60 registers instead of 120 at 2,560 channels), LN_PROMPT_PENDING (behind a projection that left its slabs:
+// two rows of a CTA to add up).
 enum LnKind { LN_ROWS, LN_PROMPT, LN_PROMPT_PENDING };
 template <int NT, int NJ, LnKind KIND>
 __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
@@ -1119,7 +1134,7 @@ __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
   const uint8_t *srd = reinterpret_cast<const uint8_t *>(a.sx_rd) + (a.batch_mode ? (size_t)t * a.state_stride : 0);
   uint8_t *swr = reinterpret_cast<uint8_t *>(a.sx_wr) + (a.batch_mode ? (size_t)t * a.state_stride : 0);
   const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * C);
-  const bool from_row = (KIND != LN_ROWS || (!a.batch_mode && a.nvec > 0)) && t > 0;
+  const bool from_row = KIND != LN_ROWS && t > 0;
   float4 xv[NJ], pv[NJ];
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
@@ -1176,8 +1191,8 @@ __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
             r[0] += rl.x; r[1] += rl.y; r[2] += rl.z; r[3] += rl.w;
           }
         }
-        rowv[j] = make_float4((rowv[j].x + r[0] * v.x) * a.pend_scale, (rowv[j].y + r[1] * v.y) * a.pend_scale,
-                              (rowv[j].z + r[2] * v.z) * a.pend_scale, (rowv[j].w + r[3] * v.w) * a.pend_scale);
+        rowv[j] = make_float4(__fmaf_rn(r[0], v.x, rowv[j].x) * a.pend_scale, __fmaf_rn(r[1], v.y, rowv[j].y) * a.pend_scale,
+                              __fmaf_rn(r[2], v.z, rowv[j].z) * a.pend_scale, __fmaf_rn(r[3], v.w, rowv[j].w) * a.pend_scale);
         if (row == t) reinterpret_cast<float4 *>(a.x_wr + (size_t)t * C)[i4] = rowv[j];
         if (i4 == 0) piv_s[t - row] = rowv[j].x;
       }
@@ -1204,8 +1219,7 @@ __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
     const int i4 = threadIdx.x + j * NT;
     if (i4 >= n4) continue;
     const float4 w = EARLY ? ew : reinterpret_cast<const float4 *>(a.ln_w)[i4], b = EARLY ? eb : reinterpret_cast<const float4 *>(a.ln_b)[i4];
-    const float4 xx = make_float4((xv[j].x - st.x) * st.y * w.x + b.x, (xv[j].y - st.x) * st.y * w.y + b.y,
-                                  (xv[j].z - st.x) * st.y * w.z + b.z, (xv[j].w - st.x) * st.y * w.w + b.w);
+    const float4 xx = ln_value4(xv[j], st, w, b);
     const size_t o = (size_t)t * C + (size_t)i4 * 4;
     if (a.nvec == 0) {
       store_hl4(a.op[0], a.op_lo[0], o, xx);
@@ -1213,8 +1227,7 @@ __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
     }
     float4 prev;
     if (from_row) {
-      prev = make_float4((pv[j].x - sp.x) * sp.y * w.x + b.x, (pv[j].y - sp.x) * sp.y * w.y + b.y,
-                         (pv[j].z - sp.x) * sp.y * w.z + b.z, (pv[j].w - sp.x) * sp.y * w.w + b.w);
+      prev = ln_value4(pv[j], sp, w, b);
       // what the token loop would have stored as shift state
       if (a.act_fp16) prev = make_float4(round_h(prev.x), round_h(prev.y), round_h(prev.z), round_h(prev.w));
     } else {
@@ -1225,8 +1238,8 @@ __global__ void __launch_bounds__(NT) ln_mix_seq_kernel(SeqLnArgs a) {
       if (v < a.nvec) {
         const float4 m = EARLY ? em[v] : reinterpret_cast<const float4 *>(a.mix[v])[i4];
         store_hl4(a.op[v], a.op_lo[v], o,
-                  make_float4(xx.x * m.x + prev.x * (1.f - m.x), xx.y * m.y + prev.y * (1.f - m.y),
-                              xx.z * m.z + prev.z * (1.f - m.z), xx.w * m.w + prev.w * (1.f - m.w)));
+                  make_float4(mix_value(xx.x, prev.x, m.x), mix_value(xx.y, prev.y, m.y), mix_value(xx.z, prev.z, m.z),
+                              mix_value(xx.w, prev.w, m.w)));
       }
     if (a.batch_mode || t == a.T - 1) {
       if (a.act_fp16) {
