@@ -140,12 +140,13 @@ void free_scratch(fr_b200_model *m) {
   }
 }
 
-// Streams of one launch from which on the batched-prologue kernel (decode.cu) is the faster one: it converts the operands
-// of all streams side by side, the step kernel one stream after the other in a quarter of the code.  Measured, 1.5B shape:
+// The batches that the batched-prologue kernel (decode.cu) takes: it converts the operands of all streams side by side, the
+// step kernel one stream after the other in a quarter of the code.  Measured, 1.5B shape, batched against step:
 // 3 / 4 int4 streams 1.12 / 1.26 ms against 1.16 / 1.33, 4 fp16 streams 1.51 against 1.25; 8 int8 streams of the 0.1B
-// shape 0.58 against 0.86.
-// (Quantised RWKV-5 stays there at every batch: its GroupNorm chain amplifies the last bits of the integer multiply to
-// 1e-3 of the logits over 32 layers, where fp16 weights give the same bits in both kernels.)
+// shape 0.58 against 0.86.  (The width is not looked at: these are the shapes that were timed.)
+// Quantised RWKV-5 is there at every batch.  The step kernel multiplies integers in another order; over 32 layers that moved
+// the logits 1e-3 from this kernel's, a distance between two kernels: which of them is nearer to exact was not measured.
+// (fp16 weights give the same bits in both.)
 bool wide_batch(int fmt, bool v5, int batch) { return batch > 4 || (fmt != FMT_FP16 && (v5 || batch > 2)); }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }

@@ -45,6 +45,8 @@ struct Smem {
 
 // NB = operand columns kept per n-tile (2: one stream as hi/lo; 8: four streams as hi/lo), NT = n-tiles.
 template <int NB, int NT> __host__ __device__ constexpr int n_streams() { return NB == 2 ? 1 : 4 * NT; }
+// fp16 tokens of up to 4 streams are the step kernel's: those two instances are left with the stand-alone products
+template <int FMT, int NT> __host__ __device__ constexpr bool carries_tokens() { return FMT != FMT_FP16 || NT > 1; }
 template <int NB, int NT> __host__ __device__ constexpr int red_n() { return ROWS * n_streams<NB, NT>(); }
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1016,7 +1018,7 @@ __device__ __forceinline__ void run_items(Ctx &cx, const PhaseDev &ph, int pi, i
     const int eit = it0 + eslot * cx.G;                       // row block this thread finishes
     const bool epi_thread = eslot < n_in && eb < p.B;
     EpiIn epi_in;
-    if (epi_thread) epilogue_prefetch<FMT>(cx, ph, pi, eit, erow, eb, epi_in);
+    if (carries_tokens<FMT, NT>() && epi_thread) epilogue_prefetch<FMT>(cx, ph, pi, eit, erow, eb, epi_in);
     const uint32_t red_it = red_a + (NB == 2 ? cx.red_buf * RED_BUF : 0u);
     const int n_mat = ph.n_sub == 1 ? n_in : ph.n_sub;        // matrices multiplied before the barrier
     for (int u = 0; u < n_mat; ++u) {
@@ -1087,8 +1089,9 @@ __device__ __forceinline__ void run_items(Ctx &cx, const PhaseDev &ph, int pi, i
           val[u] = s;
         }
       }
-      epilogue(cx, ph, pi, tag, eit, erow, eb, val, epi_in);
-      if (ph.kind == PH_HEAD && p.amax && eit * ROWS + erow < p.V) {
+      if constexpr (carries_tokens<FMT, NT>()) epilogue(cx, ph, pi, tag, eit, erow, eb, val, epi_in);
+      else p.logits[(size_t)eb * p.Vpad + eit * ROWS + erow] = val[0];
+      if (carries_tokens<FMT, NT>() && ph.kind == PH_HEAD && p.amax && eit * ROWS + erow < p.V) {
         unsigned u = __float_as_uint(val[0]);
         u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
         const unsigned long long w = ((unsigned long long)u << 32) | (0xffffffffu - (unsigned)(eit * ROWS + erow));
@@ -1168,7 +1171,7 @@ __device__ __forceinline__ void consumer(Ctx &cx) {
     const PhaseDev ph = nxt;
     if (pi + 1 < p.n_phases) nxt = p.phases[pi + 1];
     const int first = (cx.cta + cx.G - ph.rot) % cx.G;
-    if (ph.kind == PH5_WKV) {
+    if (carries_tokens<FMT, NT>() && ph.kind == PH5_WKV) {
       if (first < p.B * p.H * 4) phase_wkv5(cx, ph, pi);
       continue;
     }
@@ -1176,7 +1179,9 @@ __device__ __forceinline__ void consumer(Ctx &cx) {
     cx.prof_phase = pi;
     if (prof) p.prof[((size_t)cx.cta * p.n_phases + pi) * 8 + 0] = globaltimer_ns();
     cx.pc[1] = cx.pc[2] = cx.pc[3] = cx.pc[4] = prof ? clock64() : 0;  // trace
-    if (is_ln_phase(ph.kind)) {
+    if constexpr (!carries_tokens<FMT, NT>()) {
+      prologue_plain<NB, NT>(cx, reinterpret_cast<const float *>(p.kk), ph.K);
+    } else if (is_ln_phase(ph.kind)) {
       prologue_ln<NB, NT>(cx, ph, pi, phase_tag(p, pi - 1));
     } else if (ph.kind == PH_ATT_O) {
       if (p.version == 4) prologue_vec<NB, NT>(cx, p.rwkv, p.C, phase_tag(p, pi - 1));

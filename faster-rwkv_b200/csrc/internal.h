@@ -87,7 +87,7 @@ struct DecodeParams {
   unsigned long long *prof;             // optional [n_phases][8] profile of CTA 0
 };
 
-// ---- one token of 1 .. 8 streams (step.cu) -----------------------------------------------------------
+// ---- one token of 1 .. 4 streams (step.cu) -----------------------------------------------------------
 struct StepPhase {
   int kind, K;
   int n_items, n_sub;          // row blocks; matrices fused per row block
@@ -129,8 +129,8 @@ struct StepParams {
   int *status;                          // 0 = ok, else first failure code
   unsigned long long *prof;             // optional [CTA][n_phases][8] trace
 };
-constexpr int STEP_MODES = 4;           // instances: 1, 2, up to 4, up to 8 streams
-inline int step_mode(int batch) { return batch == 1 ? 0 : batch == 2 ? 1 : batch <= 4 ? 2 : 3; }
+constexpr int STEP_MODES = 3;           // instances: 1, 2, up to 4 streams (the last with fp16 weights only)
+inline int step_mode(int batch) { return batch == 1 ? 0 : batch == 2 ? 1 : 2; }
 size_t step_smem_bytes(int fmt, int mode, int C, int F, int nvec, int n_stages);
 cudaError_t step_prepare(int fmt, int mode, int version, int nvec, size_t smem, int device, int *grid);   // kernel attributes; CTAs of the launch
 cudaError_t launch_step(const StepParams &p, int fmt, int mode, int grid, size_t smem, cudaStream_t st);

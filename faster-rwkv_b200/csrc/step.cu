@@ -1,5 +1,5 @@
-// Persistent whole-token decode kernel for sm_100a: one token of 1 .. 8 independent streams in one cooperative launch,
-// one CTA per SM, all layers and the head.
+// Persistent whole-token decode kernel for sm_100a: one token of 1 .. 4 independent streams (fp16 weights; quantised RWKV-4:
+// 1 and 2) in one cooperative launch, one CTA per SM, all layers and the head.
 //
 // A token is a chain of 4 L + 1 (RWKV-4) or 5 L + 1 (RWKV-5) matrix-vector phases, each of which needs every output of
 // the one before it.  At batch 1 the chain, not the weight stream, decides the time of all but the widest fp16 models:
@@ -40,9 +40,9 @@ constexpr int STHREADS = SCONS + 128;    // + producer warp + epilogue warps
 constexpr int SBAR = 1;                  // named barrier of the consumer warps
 constexpr int STEP_MAX_STAGES = 12;
 
-// fp16 columns: stream b of an n-tile of 8 is columns 2 b (hi) and 2 b + 1 (lo), so that an accumulator pair is a stream
-template <int NS> __host__ __device__ constexpr int n_tiles() { return NS > 4 ? NS / 4 : 1; }
-template <int NS> __host__ __device__ constexpr int tile_cols() { return NS > 4 ? 8 : 2 * NS; }
+// One tile of 8 MMA columns.  fp16: stream b is columns 2 b (hi) and 2 b + 1 (lo), so that an accumulator pair is a stream;
+// integers: columns 4 b .. 4 b + 2 are the digits of stream b
+template <int FMT, int NS> __host__ __device__ constexpr bool fits_tile() { return FMT == FMT_FP16 ? NS <= 4 : NS <= 2; }
 // operand bytes of one 64-input chunk
 template <int NS> __host__ __device__ constexpr uint32_t chunk_operand_bytes() { return 256u * NS; }
 
@@ -205,9 +205,9 @@ struct Slots {
 };
 
 // Operand of one chunk and nvec <= NV vectors: four inputs of stream b per lane, the 16 lanes of a half warp together.
-//   fp16 weights: columns hi = fp16(x), lo = fp16(x - hi), ~22 mantissa bits:    [n-tile][MMA pair][column][q][16 B]
+//   fp16 weights: columns hi = fp16(x), lo = fp16(x - hi), ~22 mantissa bits:    [MMA pair][column][q][16 B]
 //   int weights:  x as a 23-bit fixed-point number relative to the chunk's largest magnitude, three signed base-256
-//                 digits = three s8 columns, and the scale that undoes it:       [n-tile][column][q][16 B], 4 columns a stream
+//                 digits = three s8 columns, and the scale that undoes it:       [column][q][16 B], 4 columns a stream
 // (In two steps: the chunk's largest magnitude first.)
 template <int FMT, int NV>
 __device__ __forceinline__ unsigned chunk_max(int lane, const float4 (&x)[NV]) {
@@ -225,9 +225,7 @@ template <int FMT, int NS, int NV>
 __device__ __forceinline__ void put_operand(uint32_t at, uint32_t vstride, int sub, int b, int nvec, unsigned m, const float4 (&x)[NV]) {
   const int j = sub >> 2, q = sub & 3;
   if constexpr (FMT == FMT_FP16) {
-    constexpr uint32_t COLS = tile_cols<NS>();
-    const int t = NS > 4 ? b >> 2 : 0, col = NS > 4 ? 2 * (b & 3) : 2 * b;
-    uint32_t a = at + (uint32_t)t * (COLS * 128u) + (uint32_t)(j >> 1) * (COLS * 64u) + (uint32_t)col * 64u + (uint32_t)q * 16u + (uint32_t)(j & 1) * 8u;
+    uint32_t a = at + (uint32_t)(j >> 1) * (2u * NS * 64u) + (uint32_t)(2 * b) * 64u + (uint32_t)q * 16u + (uint32_t)(j & 1) * 8u;
 #pragma unroll
     for (int v = 0; v < NV; ++v, a += vstride) {
       if (v >= nvec) break;
@@ -241,8 +239,7 @@ __device__ __forceinline__ void put_operand(uint32_t at, uint32_t vstride, int s
     // |x| < 2^(e - 126): times 2^(148 - e) it is below 2^22; the last bit of the fixed-point number is 2^(e - 148)
     const unsigned e = min(max(m >> 23, 32u), 254u);
     const float up = __uint_as_float((275u - e) << 23), down = m >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : __uint_as_float((e - 21u) << 23);
-    const int t = b >> 1, col = 4 * (b & 1);
-    uint32_t a = at + (uint32_t)t * 512u + (uint32_t)col * 64u;
+    uint32_t a = at + (uint32_t)(4 * b) * 64u;
     if (sub < nvec) sts_f32(a + (uint32_t)sub * vstride + 192u, down);
     a += (uint32_t)q * 16u + (uint32_t)j * 4u;
 #pragma unroll
@@ -268,7 +265,7 @@ __device__ __forceinline__ void put_operand(uint32_t at, uint32_t vstride, int s
 // again until their tags are there (a word asked for ahead of its time comes back stale and costs another round trip).
 template <int NS>
 __device__ __forceinline__ void gather(const Cx &cx, const Slots &sl, const exch_t *src, int K, unsigned tag4, int phase) {
-  constexpr int R = NS > 4 ? NS : 4, SR = R / NS;   // word r of a round: slot s0 + r / NS, stream r % NS
+  constexpr int R = 4, SR = R / NS;                 // word r of a round: slot s0 + r / NS, stream r % NS
 #pragma unroll 1
   for (int s0 = 0; s0 < sl.n_slot; s0 += SR) {
     uint4 w[R];
@@ -451,58 +448,43 @@ __device__ __forceinline__ void make_operand(Cx &cx, const Slots &sl, int K, con
 }
 
 // ---- multiply ---------------------------------------------------------------------------------------
-// One chunk: 16 output rows x 64 inputs of the streamed tile, and the operand.  acc[t]: this lane's share of rows g and
+// One chunk: 16 output rows x 64 inputs of the streamed tile, and the operand.  acc: this lane's share of rows g and
 // g + 8, which sum_lanes() turns into the sums of a stream:
 //   fp16:  four m16n8k16 MMAs into two accumulator sets (no MMA waits for the one before it); lane q holds stream q (hi +
 //          lo columns).  Sums are taken in the order of the batched-prologue kernel, the results are the same bit by bit
 //   int:   [0][0], [1][0]; two m16n8k32 int8 MMAs, exact; lane q holds digits 0, 1 (q even: low) or 2 (q odd: high) of stream q / 2.
 //          int4 keeps the codes times 16 (the nibble stays in the upper half of its byte); one MMA is one scale group.
-template <int FMT, int NS> __host__ __device__ constexpr int acc_tiles() { return FMT == FMT_FP16 ? n_tiles<NS>() : (NS + 1) / 2; }
 
 // what a chunk's MMAs read from shared memory
 template <int FMT, int NS>
 struct Frag {
   uint4 a[FMT == FMT_FP16 ? 4 : FMT == FMT_INT8 ? 2 : 1];
-  uint4 b[acc_tiles<FMT, NS>()][FMT == FMT_FP16 ? 2 : 1];
+  uint4 b[FMT == FMT_FP16 ? 2 : 1];
   uint2 sc;                                 // int4: group scales of rows g, g + 8
-  float down[acc_tiles<FMT, NS>()];
+  float down;
 };
 template <int FMT, int NS>
 __device__ __forceinline__ void fetch_chunk(Frag<FMT, NS> &f, uint32_t A, uint32_t scales, uint32_t B, int lane) {
-  constexpr int NT = acc_tiles<FMT, NS>();
   // lanes of the columns in use: the others feed zeros and read nothing
   const bool b_lane = FMT == FMT_FP16 ? NS >= 4 || lane < 8 * NS : NS > 1 || lane < 12;
 #pragma unroll
   for (int i = 0; i < (FMT == FMT_FP16 ? 4 : FMT == FMT_INT8 ? 2 : 1); ++i) f.a[i] = lds128(A + 512u * i);
-#pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    if constexpr (FMT == FMT_FP16) {
-      constexpr uint32_t COLS = tile_cols<NS>();
-      f.b[t][0] = make_uint4(0, 0, 0, 0);
-      f.b[t][1] = f.b[t][0];
-      if (b_lane) {
-        f.b[t][0] = lds128(B + (uint32_t)t * (COLS * 128u) + (uint32_t)lane * 16u);
-        f.b[t][1] = lds128(B + (uint32_t)t * (COLS * 128u) + COLS * 64u + (uint32_t)lane * 16u);
-      }
-    } else {
-      f.b[t][0] = make_uint4(0, 0, 0, 0);
-      if (b_lane) f.b[t][0] = lds128(B + (uint32_t)t * 512u + (uint32_t)lane * 16u);
-      f.down[t] = lds_f32(B + (uint32_t)t * 512u + (NS > 1 ? (uint32_t)(lane & 2) * 128u : 0u) + 192u);
-    }
+  f.b[0] = make_uint4(0, 0, 0, 0);
+  if constexpr (FMT == FMT_FP16) f.b[1] = f.b[0];
+  if (b_lane) {
+    f.b[0] = lds128(B + (uint32_t)lane * 16u);
+    if constexpr (FMT == FMT_FP16) f.b[1] = lds128(B + 2u * NS * 64u + (uint32_t)lane * 16u);
   }
+  if constexpr (FMT != FMT_FP16) f.down = lds_f32(B + (NS > 1 ? (uint32_t)(lane & 2) * 128u : 0u) + 192u);
   if constexpr (FMT == FMT_INT4) f.sc = lds64(scales);
 }
 template <int FMT, int NS>
-__device__ __forceinline__ void mul_chunk(const Frag<FMT, NS> &f, int lane, float (&acc)[acc_tiles<FMT, NS>()][2][4]) {
-  constexpr int NT = acc_tiles<FMT, NS>();
+__device__ __forceinline__ void mul_chunk(const Frag<FMT, NS> &f, int lane, float (&acc)[2][4]) {
   if constexpr (FMT == FMT_FP16) {
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      mma16816(acc[t][0], f.a[0].x, f.a[0].y, f.a[0].z, f.a[0].w, f.b[t][0].x, f.b[t][0].y);
-      mma16816(acc[t][1], f.a[1].x, f.a[1].y, f.a[1].z, f.a[1].w, f.b[t][0].z, f.b[t][0].w);
-      mma16816(acc[t][0], f.a[2].x, f.a[2].y, f.a[2].z, f.a[2].w, f.b[t][1].x, f.b[t][1].y);
-      mma16816(acc[t][1], f.a[3].x, f.a[3].y, f.a[3].z, f.a[3].w, f.b[t][1].z, f.b[t][1].w);
-    }
+    mma16816(acc[0], f.a[0].x, f.a[0].y, f.a[0].z, f.a[0].w, f.b[0].x, f.b[0].y);
+    mma16816(acc[1], f.a[1].x, f.a[1].y, f.a[1].z, f.a[1].w, f.b[0].z, f.b[0].w);
+    mma16816(acc[0], f.a[2].x, f.a[2].y, f.a[2].z, f.a[2].w, f.b[1].x, f.b[1].y);
+    mma16816(acc[1], f.a[3].x, f.a[3].y, f.a[3].z, f.a[3].w, f.b[1].z, f.b[1].w);
   } else {
     const float m256 = lane & 1 ? 0.f : 256.f;       // column 3 of a stream is not a digit
     uint32_t a[8];                                   // A fragments of the two MMAs
@@ -522,21 +504,18 @@ __device__ __forceinline__ void mul_chunk(const Frag<FMT, NS> &f, int lane, floa
 #pragma unroll
       for (int i = 0; i < 4; ++i) { a[2 * i] = lop3_and_xor(w[i] << 4, H, S); a[2 * i + 1] = lop3_and_xor(w[i], H, S); }
     }
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      int u[4] = {0, 0, 0, 0}, v[4] = {0, 0, 0, 0};
-      mma16832_s8(u, a[0], a[1], a[2], a[3], f.b[t][0].x, f.b[t][0].y);
-      if constexpr (FMT == FMT_INT8) {
-        mma16832_s8(u, a[4], a[5], a[6], a[7], f.b[t][0].z, f.b[t][0].w);
-        acc[t][0][0] += f.down[t] * fmaf(m256, (float)u[1], (float)u[0]);
-        acc[t][1][0] += f.down[t] * fmaf(m256, (float)u[3], (float)u[2]);
-      } else {
-        mma16832_s8(v, a[4], a[5], a[6], a[7], f.b[t][0].z, f.b[t][0].w);
-        const float r0 = fmaf(s1.x, fmaf(m256, (float)v[1], (float)v[0]), s0.x * fmaf(m256, (float)u[1], (float)u[0]));
-        const float r1 = fmaf(s1.y, fmaf(m256, (float)v[3], (float)v[2]), s0.y * fmaf(m256, (float)u[3], (float)u[2]));
-        acc[t][0][0] += f.down[t] * r0;
-        acc[t][1][0] += f.down[t] * r1;
-      }
+    int u[4] = {0, 0, 0, 0}, v[4] = {0, 0, 0, 0};
+    mma16832_s8(u, a[0], a[1], a[2], a[3], f.b[0].x, f.b[0].y);
+    if constexpr (FMT == FMT_INT8) {
+      mma16832_s8(u, a[4], a[5], a[6], a[7], f.b[0].z, f.b[0].w);
+      acc[0][0] += f.down * fmaf(m256, (float)u[1], (float)u[0]);
+      acc[1][0] += f.down * fmaf(m256, (float)u[3], (float)u[2]);
+    } else {
+      mma16832_s8(v, a[4], a[5], a[6], a[7], f.b[0].z, f.b[0].w);
+      const float r0 = fmaf(s1.x, fmaf(m256, (float)v[1], (float)v[0]), s0.x * fmaf(m256, (float)u[1], (float)u[0]));
+      const float r1 = fmaf(s1.y, fmaf(m256, (float)v[3], (float)v[2]), s0.y * fmaf(m256, (float)u[3], (float)u[2]));
+      acc[0][0] += f.down * r0;
+      acc[1][0] += f.down * r1;
     }
   }
 }
@@ -554,7 +533,7 @@ __device__ __forceinline__ float sum_lanes(int lane, const float (&a)[2][4], int
 // of a fused row block reads operand vector u; else the vector is the row block's class: its index / split, at most last_vec.
 template <int FMT, int NS>
 __device__ __forceinline__ void multiply_items(Cx &cx, int K, int n_items, int n_sub, int split, uint32_t last_vec, int first) {
-  constexpr int NT = acc_tiles<FMT, NS>();
+  static_assert(fits_tile<FMT, NS>(), "the streams' columns fit one MMA tile");
   constexpr int CH = FMT == FMT_FP16 ? 16 : 32;      // chunks of a full stage
   constexpr uint32_t CB = chunk_operand_bytes<NS>(), WB = FMT == FMT_FP16 ? 2048u : FMT == FMT_INT8 ? 1024u : 512u;
   const int n_ch = K >> 6, nst = num_stages(FMT, K);
@@ -570,11 +549,9 @@ __device__ __forceinline__ void multiply_items(Cx &cx, int K, int n_items, int n
     for (int u = 0; u < n_sub; ++u) {
       const uint32_t vec = n_sub > 1 ? (uint32_t)u : split == 0 || it < split ? 0u : min(it < 2 * split ? 1u : it < 3 * split ? 2u : 3u, last_vec);
       uint32_t bop = cx.xw + vec * vb;
-      float acc[NT][2][4];
+      float acc[2][4];
 #pragma unroll
-      for (int t = 0; t < NT; ++t)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { acc[t][0][i] = 0.f; acc[t][1][i] = 0.f; }
+      for (int i = 0; i < 4; ++i) { acc[0][i] = 0.f; acc[1][i] = 0.f; }
       int left = n_ch;                               // chunks from this stage on
 #pragma unroll 1
       for (int s = 0; s < nst; ++s, left -= CH) {
@@ -602,17 +579,13 @@ __device__ __forceinline__ void multiply_items(Cx &cx, int K, int n_items, int n
         if (cx.lane == 0) mbar_arrive(&cx.empty[cur]);
       }
       if (u == 0) bar_wait(cx, &cx.part_empty[buf], (cx.item / EW & 1u) ^ 1u, ST_TIMEOUT_EMPTY);
-      // fp16: lane q of a row holds stream q (of the n-tile); int: lanes 2 s and 2 s + 1 hold stream s
-      constexpr int TS = FMT == FMT_FP16 ? (NS > 4 ? 4 : NS) : (NS > 1 ? 2 : 1);   // streams of a tile
+      // fp16: lane q of a row holds stream q; int: lanes 2 s and 2 s + 1 hold stream s
       const int sq = FMT == FMT_FP16 ? q : q >> 1;
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const float r0 = sum_lanes<FMT>(cx.lane, acc[t], 0), r1 = sum_lanes<FMT>(cx.lane, acc[t], 1);
-        if (FMT == FMT_FP16 ? q < TS : (q & 1) == 0 && sq < TS) {
-          const uint32_t d = dst + (uint32_t)u * (ROWS * NS * 4u) + (uint32_t)(g * NS + t * TS + sq) * 4u;
-          sts_f32(d, r0);
-          sts_f32(d + (uint32_t)(8 * NS) * 4u, r1);
-        }
+      const float r0 = sum_lanes<FMT>(cx.lane, acc, 0), r1 = sum_lanes<FMT>(cx.lane, acc, 1);
+      if (FMT == FMT_FP16 ? q < NS : (q & 1) == 0 && sq < NS) {
+        const uint32_t d = dst + (uint32_t)u * (ROWS * NS * 4u) + (uint32_t)(g * NS + sq) * 4u;
+        sts_f32(d, r0);
+        sts_f32(d + (uint32_t)(8 * NS) * 4u, r1);
       }
     }
     __syncwarp();
@@ -1035,17 +1008,21 @@ __global__ void __launch_bounds__(STHREADS, 1) step_kernel(const __grid_constant
 
 template <int FMT, int NS>
 const void *step_instance(int version, int nvec) {
-  return version == 4 ? (const void *)step_kernel<FMT, NS, 3, false>
+  if constexpr (FMT != FMT_FP16) return version == 4 ? (const void *)step_kernel<FMT, NS, 3, false> : nullptr;
+  else return version == 4 ? (const void *)step_kernel<FMT, NS, 3, false>
          : nvec == 3  ? (const void *)step_kernel<FMT, NS, 3, true> : (const void *)step_kernel<FMT, NS, 4, true>;
 }
 template <int FMT, int NS>
 cudaError_t step_launch_t(const StepParams &p, int grid, size_t smem, cudaStream_t st) {
   void *args[] = {const_cast<StepParams *>(&p)};
-  return cudaLaunchCooperativeKernel(step_instance<FMT, NS>(p.version, p.n_att_vec), dim3(grid), dim3(STHREADS), args, smem, st);
+  const void *kernel = step_instance<FMT, NS>(p.version, p.n_att_vec);
+  if (!kernel) return cudaErrorInvalidValue;
+  return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(STHREADS), args, smem, st);
 }
 template <int FMT, int NS>
 cudaError_t step_prepare_t(int version, int nvec, size_t smem, int device, int *grid) {
   const void *kernel = step_instance<FMT, NS>(version, nvec);
+  if (!kernel) return cudaErrorInvalidValue;
   cudaError_t e;
   int optin = 0;
   // the limit is the kernel's, not the model's: models of different widths share the instance
@@ -1066,8 +1043,7 @@ size_t step_smem_bytes(int fmt, int mode, int C, int F, int nvec, int n_stages) 
   switch (mode) {
     case 0: return step_layout<1>(fmt, C, F, nvec, n_stages).total;
     case 1: return step_layout<2>(fmt, C, F, nvec, n_stages).total;
-    case 2: return step_layout<4>(fmt, C, F, nvec, n_stages).total;
-    default: return step_layout<8>(fmt, C, F, nvec, n_stages).total;
+    default: return step_layout<4>(fmt, C, F, nvec, n_stages).total;
   }
 }
 
@@ -1076,15 +1052,10 @@ size_t step_smem_bytes(int fmt, int mode, int C, int F, int nvec, int n_stages) 
     case 0: return fn<FMT_FP16, 1>(__VA_ARGS__);                \
     case 1: return fn<FMT_FP16, 2>(__VA_ARGS__);                \
     case 2: return fn<FMT_FP16, 4>(__VA_ARGS__);                \
-    case 3: return fn<FMT_FP16, 8>(__VA_ARGS__);                \
-    case 4: return fn<FMT_INT8, 1>(__VA_ARGS__);                \
-    case 5: return fn<FMT_INT8, 2>(__VA_ARGS__);                \
-    case 6: return fn<FMT_INT8, 4>(__VA_ARGS__);                \
-    case 7: return fn<FMT_INT8, 8>(__VA_ARGS__);                \
-    case 8: return fn<FMT_INT4, 1>(__VA_ARGS__);                \
-    case 9: return fn<FMT_INT4, 2>(__VA_ARGS__);                \
-    case 10: return fn<FMT_INT4, 4>(__VA_ARGS__);               \
-    case 11: return fn<FMT_INT4, 8>(__VA_ARGS__);               \
+    case 3: return fn<FMT_INT8, 1>(__VA_ARGS__);                \
+    case 4: return fn<FMT_INT8, 2>(__VA_ARGS__);                \
+    case 6: return fn<FMT_INT4, 1>(__VA_ARGS__);                \
+    case 7: return fn<FMT_INT4, 2>(__VA_ARGS__);                \
     default: return cudaErrorInvalidValue;                      \
   }
 
