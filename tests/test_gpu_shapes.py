@@ -11,12 +11,13 @@ recurrent state within 1e-2 max-abs and 1e-3 relative L2.
       tokens at batch 1, logits of every step and the final state; the same file and ids through the reference's own
       kernels/cuda + cuBLAS path ("cuda fp16", rebuilt for sm_100a) where that binary exists
   c1  RWKV-4 1.5B-shaped (L24 C2048 F8192 V65536), fp16 / int8 / int4: 32 tokens at batch 1, 4 streams in one
-      launch of the persistent kernel, 16 streams through the GEMM path
+      launch of the persistent kernel, 16 streams through the GEMM path; prompts of 29 (int4) and 700 (fp16)
+      tokens: the scan with one and with eleven tokens a chunk, without and with finishing passes
   c3  RWKV-5.2 3B-shaped at full width (C2560 H40 F8960 V65536) with 4 of its 32 layers: one 4096-token prompt
       against the oracle's token loop, then 64 decode steps
   c4  RWKV-4 14B-shaped at full width (C5120 F20480 V50277) with 7 of its 40 layers (one halving of the residual
       stream happens), int8: 32 tokens at batch 1
-The measured distances go to parity_shapes.json in the run's output directory beside the assertions.
+With FR_B200_PARITY_JSON=<file> the measured distances go to that file beside the assertions.
 """
 import dataclasses
 import json
@@ -47,10 +48,10 @@ def _close(got, want, what):
 
 def _note(key, **kw):
     REPORT.setdefault(key, {}).update(kw)
-    out = os.path.join(ROOT, "gpurun_out")
-    os.makedirs(out, exist_ok=True)
-    with open(os.path.join(out, "parity_shapes.json"), "w") as f:
-        json.dump(REPORT, f, indent=1, sort_keys=True)
+    out = os.environ.get("FR_B200_PARITY_JSON")
+    if out:
+        with open(out, "w") as f:
+            json.dump(REPORT, f, indent=1, sort_keys=True)
 
 
 def _build(pkg, orc, shape, fmt, max_batch=1, seed=0):
@@ -179,6 +180,21 @@ def test_c1_batch1_four_streams_and_sixteen_streams(pkg, orc, synth, fmt):
             d = _close(got[t][b], ref.run(int(ids16[t, b])), f"c1 {fmt} 16 streams: stream {b} step {t}")
             w16 = [max(w16[0], d[0]), max(w16[1], d[1])]
     _note(f"c1_{fmt}", b4_logits_max_abs=w4[0], b4_logits_rel_l2=w4[1], b16_logits_max_abs=w16[0], b16_logits_rel_l2=w16[1])
+    m.close()
+
+
+@pytest.mark.parametrize("fmt,T", [("int4", 29), ("fp16", 700)])
+def test_c1_prompts(pkg, orc, synth, fmt, T):
+    """Prompts over all 24 layers, after a token that leaves a state to start from: last logits, recurrent state, next token."""
+    shape = synth.SHAPES["c1"]
+    m, ref, _ = _build(pkg, orc, shape, fmt)
+    ids = [int(t) for t in synth.token_ids(shape, T, seed=30 + T)]
+    m.run(11), ref.run(11)
+    d = _close(m.run(ids), ref.run_seq(ids), f"c1 {fmt} prompt of {T}")
+    sd = _state_check(m, ref, shape, f"c1 {fmt} prompt of {T}")
+    n = _close(m.run(7), ref.run(7), f"c1 {fmt} token after a prompt of {T}")
+    _note(f"c1_{fmt}", prompt_tokens=T, prompt_logits_max_abs=d[0], prompt_logits_rel_l2=d[1], prompt_state_max_abs=sd[0],
+          prompt_state_rel_l2=sd[1], prompt_next_rel_l2=n[1])
     m.close()
 
 
