@@ -1317,9 +1317,10 @@ __global__ void __launch_bounds__(256) wkv4_rows_kernel(Wkv4Args a) {
 // state as (aa, bb, pp) -> decay by exp(len * w), plus the run's own sums -- so the prompt is cut into 64 chunks that
 // are reduced side by side, combined by a prefix scan, and walked again from their start states.  One CTA holds 16
 // channels x 64 chunks (a 64-byte piece of each row per half warp) and does all three steps: no scratch in global
-// memory, one launch.  Up to 1024 tokens a thread keeps its chunk's k and v in registers between the two walks (LEN
-// tokens; 0: read again).  What bounds it: the serial walk it replaces was one dependent expf chain of T steps on C
-// threads, 700 us a layer at T = 1000, C = 2048; this form is 2 x ceil(T / 64) steps on 64 C threads.
+// memory, one launch.  Up to 1024 tokens a thread keeps its chunk's k and v between the two walks (LEN tokens, in
+// registers; of LEN = 16 eight words do not fit the 64 a thread has.  0: read again).  What bounds it: the serial walk
+// it replaces was one dependent expf chain of T steps on C threads, 700 us a layer at T = 1000, C = 2048; this form is
+// 2 x ceil(T / 64) steps on 64 C threads.
 constexpr int W4_CH = 16, W4_CHUNKS = 64, W4_THREADS = W4_CH * W4_CHUNKS;
 // state (a1, b1, p1) followed by a run of decay d = len * w with sums (a2, b2, p2)
 __device__ __forceinline__ void wkv4_join(float &a, float &b, float &p, float d, float a2, float b2, float p2) {
@@ -1759,6 +1760,10 @@ cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
   if (!a.batch_mode) {
     const dim3 grid(a.C / W4_CH), block(W4_THREADS);
     const int len = (a.T + W4_CHUNKS - 1) / W4_CHUNKS;
+    // The fewest tokens kept per thread that cover a chunk: every slot is a pass through the code, taken or not.  This kernel
+    // alone at 2,048 channels, us: 256 tokens <4> 7.1, <0> 11.7; 300 tokens <12> 8.9, <16> 10.2, <0> 13.3; 640 tokens 12.9, 14.1,
+    // 21.4; 1,000 tokens <16> 19.1, <0> 30.6.  (With more CTAs than SMs <0>, of which two fit an SM, is the faster one: 5,120
+    // channels, 640 tokens 31 against 36, 1,000 tokens 49 against 61.)
     if (len <= 1) launch_k(wkv4_seq_kernel<1>, grid, block, 0, st, a);
     else if (len <= 4) launch_k(wkv4_seq_kernel<4>, grid, block, 0, st, a);
     else if (len <= 12) launch_k(wkv4_seq_kernel<12>, grid, block, 0, st, a);
@@ -1767,8 +1772,11 @@ cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
     return cudaGetLastError();
   }
   dim3 grid((a.C + 255) / 256, a.T);
-  // up to 64 rows of a 2,048 channel model a CTA per SM or two has to cover the whole round trip by itself (16 streams: 1.41 ms
-  // a step against 1.42); beyond, fewer registers and more CTAs are better (100: 1.68 against 1.70, 256: 2 % of the step)
+  // Up to 64 rows of a 2,048 channel model a CTA per SM or two has to cover the whole round trip by itself; beyond, fewer
+  // registers and more CTAs are better.  This kernel alone, <8> against <4>, us: 6 slabs, 32 rows 3.0 / 4.0, 64 rows 3.55 /
+  // 4.24, 80 rows 4.12 / 4.24, 100 rows 4.61 / 4.22, 256 rows 9.1 / 8.3; 3 slabs, 32 rows 2.8 / 3.1, 64 rows 3.27 / 3.32, 80 rows
+  // 3.75 / 3.42, 256 rows 8.4 / 6.6.  (768 channels cross at the same T C; up to 16 rows of 2,048 channels the two are within 0.8 us
+  // of one another either way.)
   if ((long long)a.T * a.C <= 64 * 2048) launch_k(wkv4_rows_kernel<8>, dim3(grid), dim3(256), 0, st, a);
   else launch_k(wkv4_rows_kernel<4>, dim3(grid), dim3(256), 0, st, a);
   return cudaGetLastError();
