@@ -73,6 +73,10 @@ def measured_peaks():
         return 6650.0, 1590.0, 1400.0, "fallback"
 
 
+# which of the two takes a batch: wide_batch() in api.cu
+TOKEN_KERNEL = "step_kernel / decode_kernel (persistent, one launch per token)"
+
+
 def hbm_roofline(shape, fmt, ms_per_step, kernel):
     peak, _, _, kind = measured_peaks()
     algo = algorithmic_bytes(shape, fmt)
@@ -333,7 +337,7 @@ def phase_budget(pkg, device_index: int, wl: str = "c1", reps: int = 5):
     """Medians over layers, CTAs and repetitions of the persistent kernel's own trace (fr_b200_decode_profile), per phase
     kind: ns from phase start to inputs staged (hand-over wait + prologue), staged to row blocks done (tile loop +
     reduce + epilogue), of which waiting for weight tiles, and how far the completion front of the whole grid moves
-    per phase (the phase's share of the token)."""
+    per phase (the phase's share of the token).  The step kernel stamps no tile wait and no separate conversion: None."""
     shape = pkg.synth.SHAPES[wl]
     out = {}
     for fmt, B in (("fp16", 1), ("int8", 1), ("int4", 1), ("fp16", 4), ("int4", 4)):
@@ -349,6 +353,7 @@ def phase_budget(pkg, device_index: int, wl: str = "c1", reps: int = 5):
         for _ in range(reps):
             st = m.decode_profile(ids).astype(np.int64)          # [cta][phase][8]
             P = st.shape[1]
+            staged = bool(st[:, :, 6].any())                     # decode_kernel: statistics / conversion and tile wait
             done = np.where(st[:, :, 2] > 0, st[:, :, 2], 0).max(axis=0)       # completion front per phase
             start0 = st[:, 0, 0][st[:, 0, 0] > 0].min()
             tok.append(done[-1] - start0)
@@ -360,9 +365,10 @@ def phase_budget(pkg, device_index: int, wl: str = "c1", reps: int = 5):
                 a = acc[kind]
                 a["prologue_ns"].append(np.median(st[act, pi, 1] - st[act, pi, 0]))
                 a["items_ns"].append(np.median(st[act, pi, 2] - st[act, pi, 1]))
-                a["tile_wait_cycles"].append(np.median(st[act, pi, 3]))
                 a["wait_inputs_cycles"].append(np.median(st[act, pi, 5]))
-                a["convert_cycles"].append(np.median(st[act, pi, 6]))
+                if staged:
+                    a["tile_wait_cycles"].append(np.median(st[act, pi, 3]))
+                    a["convert_cycles"].append(np.median(st[act, pi, 6]))
                 a["stage_cycles"].append(np.median(st[act, pi, 7]))
                 if pi > 0:
                     a["front_ns"].append(done[pi] - done[pi - 1])
@@ -572,7 +578,7 @@ def main():
         clocks = cs.summary()
         ms_max = max_over_ranks(ms)
         value = world * B * K / (ms_max * 1e-3)
-        roofline = hbm_roofline(shape, fmt, ms_max / K, "decode_kernel (persistent, one launch per token)") if B <= 8 else \
+        roofline = hbm_roofline(shape, fmt, ms_max / K, TOKEN_KERNEL) if B <= 8 else \
             batched_roofline(shape, fmt, B, ms_max / K)
         # end to end: host ids in, host logits out, every step, through the public API
         model.reset_states()
@@ -614,7 +620,7 @@ def main():
                 steps_v = 256
                 vms, _, _ = timed_greedy(torch, barrier, mv, synth.token_ids(c1, vb, seed=0), steps_v, W)
                 variants[f"c1_{vf}_b{vb}"] = {"tok_s": vb * steps_v / (vms * 1e-3), "ms_per_step": vms / steps_v,
-                                             "roofline": hbm_roofline(c1, vf, vms / steps_v, "decode_kernel (persistent, one launch per token)")}
+                                             "roofline": hbm_roofline(c1, vf, vms / steps_v, TOKEN_KERNEL)}
                 drop(mv)
                 del mv
             except Exception as ex:  # a variant must not lose the headline
@@ -647,7 +653,7 @@ def main():
                 lat.append(e0.elapsed_time(e1))
             p50 = float(np.median(lat))
             variants["c4_int8_b1"] = {"p50_ms_per_token": p50, "tok_s": 1e3 / p50,
-                                      "roofline": hbm_roofline(c4, "int8", p50, "decode_kernel (persistent, one launch per token)")}
+                                      "roofline": hbm_roofline(c4, "int8", p50, TOKEN_KERNEL)}
             drop(mv)
             del mv
         except Exception as ex:
