@@ -202,7 +202,7 @@ struct SeqLnArgs {
   int T, C, nvec, act_fp16;
   int batch_mode;            // rows are streams: shift states are per row, state_stride bytes apart
   size_t state_stride;
-  // optional (pend_split > 1, batch mode): the projection before this LayerNorm has not been finished -- its
+  // optional (pend_split > 1; streams and short prompts): the projection before this LayerNorm has not been finished -- its
   // split-K slabs [pend_split][T][C] are summed here and x = (x + [r *] sum) * pend_scale is stored to x_wr first
   const float *pend_raw;
   const __half *pend_cscale;          // its per-column scales, or null
