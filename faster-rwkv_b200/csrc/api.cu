@@ -1100,7 +1100,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
       ga.Bt = m->d_plain + ms.plain_off;
     }
     ga.N = N; ga.K = K; ga.epi = epi; ga.out = out; ga.ldo = N; ga.aux0 = aux0; ga.aux1 = aux1;
-    ga.scale = scale; ga.status = m->out_status();
+    ga.scale = scale; ga.status = m->out_status(); ga.fixed_split = m->v5;
     return ga;
   };
   const int mt = Tp > 128 ? 2 : 1;   // 256-row tiles once the rows fill them

@@ -182,6 +182,7 @@ struct GemmArgs {
   float scale;
   int *status;         // device word: set when a bounded wait gives up
   float *raw;          // optional scratch [GEMM_SPLIT_MAX][M][N] f32: allows split-K when M <= GEMM_SMALL_M
+  int fixed_split;     // 1: K is cut the same way whatever kernel serves the product (RWKV-5, see launch_gemm_pair)
 };
 constexpr int GEMM_GROUP_MAX = 4;
 constexpr int GEMM_SMALL_M = 1024;    // up to this many rows the GEMM puts the weights along the MMA rows (and splits K, given scratch)

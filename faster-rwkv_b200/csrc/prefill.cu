@@ -57,12 +57,12 @@ cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
 }
 
 // ------------------------------------------------------------------------------------------------
-// tcgen05 GEMM: out[M, N] = epilogue((A + A2)[M, K] . (Bt + Bt2)[N, K]^T), fp16 operands (both K-major), fp32
-// accumulate.  A2 (optional) holds what rounding the activations to fp16 lost: its tiles travel in the same ring slot
-// and multiply the same B tile.  Bt2 (optional, int4 weights) is a second pass over K.
-// One CTA per 128 x 256 output tile; K is walked in 64-wide slices through a 4-deep TMA ring.
+// tcgen05 GEMMs: out[M, N] = epilogue((A + A2)[M, K] . (Bt + Bt2)[N, K]^T), fp16 operands (both K-major), fp32
+// accumulate.  A2 (optional) holds what rounding the activations to fp16 lost, Bt2 what rounding the weights did.
+// All of them put the weights along the MMA rows, so that an accumulator holds out^T (TMEM lane = output channel, column = row
+// of X) and the epilogue's lanes run along the channels; K is walked in 64-wide slices through a TMA ring.
 //   warp 0 (one lane): TMA producer          warp 1 (one lane): MMA issue; the warp owns the TMEM allocation
-//   warps 2..5: epilogue, one TMEM lane quadrant (32 rows) each
+//   warps 2..5: epilogue, one TMEM lane quadrant (32 channels) each
 constexpr int GBM = 128, GBK = 64;
 constexpr int G_THREADS = 192;
 constexpr uint32_t G_A_BYTES = GBM * GBK * 2;
@@ -115,154 +115,209 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // the result is rounded to fp16: the fast exponential and division are exact enough
 __device__ __forceinline__ float sigmoid_g(float v) { return __fdividef(1.f, 1.f + __expf(-v)); }
 
-// Epilogue of 32 consecutive columns of one output row (16-byte accesses when all 32 columns exist).
+template <int EPI>
+__device__ __forceinline__ float epi_half_op(float a) {
+  if (EPI == GEMM_EPI_SILU_F16) return a * sigmoid_g(a);
+  if (EPI == GEMM_EPI_SIGMOID_F16) return sigmoid_g(a);
+  if (EPI == GEMM_EPI_RELU2_F16) { a = fmaxf(a, 0.f); return a * a; }
+  return a;
+}
 __device__ __forceinline__ float epi_half_op(int epi, float a) {
   if (epi == GEMM_EPI_SILU_F16) return a * sigmoid_g(a);
   if (epi == GEMM_EPI_SIGMOID_F16) return sigmoid_g(a);
   if (epi == GEMM_EPI_RELU2_F16) { a = fmaxf(a, 0.f); return a * a; }
   return a;
 }
-__device__ __forceinline__ void gemm_epilogue_row(const GemmArgs &g, int row, int col0, const uint32_t (&acc)[32]) {
-  const int ncol = min(32, g.N - col0);
-  if (ncol <= 0) return;
-  const size_t o = (size_t)row * g.ldo + col0;
-  const bool full = ncol == 32 && (g.ldo & 7) == 0;
-  if (g.epi == GEMM_EPI_F32) {
-    float *out = reinterpret_cast<float *>(g.out) + o;
-    if (full) {
-#pragma unroll
-      for (int i = 0; i < 32; i += 4)
-        *reinterpret_cast<float4 *>(out + i) = make_float4(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]),
-                                                           __uint_as_float(acc[i + 2]), __uint_as_float(acc[i + 3]));
-    } else {
-      for (int i = 0; i < ncol; ++i) out[i] = __uint_as_float(acc[i]);
-    }
-    return;
-  }
-  if (g.epi == GEMM_EPI_ADD_F32 || g.epi == GEMM_EPI_MULADD_F32) {
-    // residual stream (fp32): x + acc, or x + r * acc (r fp16), optionally scaled
-    float *out = reinterpret_cast<float *>(g.out) + o;
-    const float *x = reinterpret_cast<const float *>(g.aux0) + o;
-    const __half *r = reinterpret_cast<const __half *>(g.aux1) + o;
-    const bool mul = g.epi == GEMM_EPI_MULADD_F32;
-    if (mul && g.aux1_lo) {
-      const __half *rl = reinterpret_cast<const __half *>(g.aux1_lo) + o;
-      for (int i = 0; i < ncol; ++i)
-        out[i] = (x[i] + (__half2float(r[i]) + __half2float(rl[i])) * __uint_as_float(acc[i])) * g.scale;
-      return;
-    }
-    if (full) {
-#pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        const float4 x0 = *reinterpret_cast<const float4 *>(x + i), x1 = *reinterpret_cast<const float4 *>(x + i + 4);
-        float rr[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-        if (mul) {
-          const uint4 rw = *reinterpret_cast<const uint4 *>(r + i);
-          const float2 r0 = __half22float2(*reinterpret_cast<const __half2 *>(&rw.x)), r1 = __half22float2(*reinterpret_cast<const __half2 *>(&rw.y));
-          const float2 r2 = __half22float2(*reinterpret_cast<const __half2 *>(&rw.z)), r3 = __half22float2(*reinterpret_cast<const __half2 *>(&rw.w));
-          rr[0] = r0.x; rr[1] = r0.y; rr[2] = r1.x; rr[3] = r1.y; rr[4] = r2.x; rr[5] = r2.y; rr[6] = r3.x; rr[7] = r3.y;
-        }
-        float4 y0, y1;
-        y0.x = (x0.x + rr[0] * __uint_as_float(acc[i])) * g.scale;     y0.y = (x0.y + rr[1] * __uint_as_float(acc[i + 1])) * g.scale;
-        y0.z = (x0.z + rr[2] * __uint_as_float(acc[i + 2])) * g.scale; y0.w = (x0.w + rr[3] * __uint_as_float(acc[i + 3])) * g.scale;
-        y1.x = (x1.x + rr[4] * __uint_as_float(acc[i + 4])) * g.scale; y1.y = (x1.y + rr[5] * __uint_as_float(acc[i + 5])) * g.scale;
-        y1.z = (x1.z + rr[6] * __uint_as_float(acc[i + 6])) * g.scale; y1.w = (x1.w + rr[7] * __uint_as_float(acc[i + 7])) * g.scale;
-        *reinterpret_cast<float4 *>(out + i) = y0;
-        *reinterpret_cast<float4 *>(out + i + 4) = y1;
-      }
-    } else {
-      for (int i = 0; i < ncol; ++i) {
-        float a = __uint_as_float(acc[i]);
-        if (mul) a *= __half2float(r[i]);
-        out[i] = (x[i] + a) * g.scale;
-      }
-    }
-    return;
-  }
-  __half *out = reinterpret_cast<__half *>(g.out) + o;
-  if (g.out_lo) {
-    // the consumer of this output wants it as a hi + lo pair (batched decode keeps ~22 bits between projections)
-    __half *lo = reinterpret_cast<__half *>(g.out_lo) + o;
-    for (int i = 0; i < ncol; ++i) {
-      const float v = epi_half_op(g.epi, __uint_as_float(acc[i]));
-      const __half h = __float2half_rn(v);
-      out[i] = h;
-      lo[i] = __float2half_rn(v - __half2float(h));
-    }
-    return;
-  }
-  if (full) {
-#pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-      uint4 w;
-      __half2 h;
-      h = __floats2half2_rn(epi_half_op(g.epi, __uint_as_float(acc[i])), epi_half_op(g.epi, __uint_as_float(acc[i + 1])));     w.x = *reinterpret_cast<uint32_t *>(&h);
-      h = __floats2half2_rn(epi_half_op(g.epi, __uint_as_float(acc[i + 2])), epi_half_op(g.epi, __uint_as_float(acc[i + 3]))); w.y = *reinterpret_cast<uint32_t *>(&h);
-      h = __floats2half2_rn(epi_half_op(g.epi, __uint_as_float(acc[i + 4])), epi_half_op(g.epi, __uint_as_float(acc[i + 5]))); w.z = *reinterpret_cast<uint32_t *>(&h);
-      h = __floats2half2_rn(epi_half_op(g.epi, __uint_as_float(acc[i + 6])), epi_half_op(g.epi, __uint_as_float(acc[i + 7]))); w.w = *reinterpret_cast<uint32_t *>(&h);
-      *reinterpret_cast<uint4 *>(out + i) = w;
-    }
-  } else {
-    for (int i = 0; i < ncol; ++i) out[i] = __float2half_rn(epi_half_op(g.epi, __uint_as_float(acc[i])));
-  }
-}
-
 // Up to four GEMMs with the same M in one launch (grid.x walks their N tiles back to back, heaviest first): the
 // attention projections of a layer, or the two channel-mix projections that read the LayerNorm output.
 struct GemmGroup {
   int n;
-  int stages;                           // ring depth (2..4); packed-weight GEMM: weight slots
+  int stages;                           // ring depth; packed-weight GEMM: weight slots
   int estages;                          // packed-weight GEMM: buffers (expanded weights + X; stage_bytes = the X part)
   uint32_t wbox;                        // packed-weight GEMM: bytes per row of a weight slot (64 or 128)
-  uint32_t stage_bytes;                 // bytes per ring slot: [A hi tiles][A lo tiles, if any problem has them][B tile]
+  uint32_t stage_bytes;                 // bytes per ring slot
   int split;                            // split-K factor (grid.z); > 1: CTAs write raw partial sums to GemmArgs::raw
-  int dual;                             // 1: the slot has room for the low halves of A (128-row tiles);
-                                        // 0: low halves of A, if any, are a further pass over K (256-row tiles: a
-                                        //    slot with both would leave a 2-deep ring)
-  int tile_start[GEMM_GROUP_MAX + 1];   // first grid.x index of each problem
+  int dual;                             // few-row GEMM: bit 0, some problem has A2 (the slot holds an X lo tile); bit 1, Bt2
+  int bn, m_tiles;                      // pair GEMM: rows of X per tile, row tiles
+  int lo_each;                          // pair GEMM: the low halves of X follow the high halves slice by slice
+  int tile_start[GEMM_GROUP_MAX + 1];   // first channel tile of each problem
   GemmArgs p[GEMM_GROUP_MAX];
 };
 struct alignas(64) GemmMaps {
   CUtensorMap a[GEMM_GROUP_MAX], a2[GEMM_GROUP_MAX], b[GEMM_GROUP_MAX], b2[GEMM_GROUP_MAX];
 };
 
-// MT = 128-row sub-tiles per CTA (1: 128 x BN output tile; 2: 256 x BN, two accumulators sharing every B tile --
-// half again as many flops per byte fetched from L2).  BN = 256 for prompts; BN = 64 with split-K (grid.z) when
-// there are only a few hundred rows (batched decode): the step is bound by streaming the weights, so the number of
-// CTAs that each stream a distinct slice is what counts; the partial sums go to per-split slabs that
-// gemm_finish_kernel adds up in a fixed order before the epilogue.
-template <int MT, int BN>
-__global__ void __launch_bounds__(G_THREADS, 1)
-gemm_f16_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
-  constexpr int GBN = BN;
-  constexpr uint32_t G_B_BYTES = BN * GBK * 2;
-  constexpr uint32_t G_IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GBM >> 4) << 24);
-  const int STAGES = grp.stages;
-  const uint32_t STAGE_BYTES = grp.stage_bytes;
-  const uint32_t B_OFF = (uint32_t)(grp.dual ? 2 : 1) * MT * G_A_BYTES;   // the B tile follows the A tiles
-  constexpr uint32_t TMEM_COLS = MT * GBN < 32 ? 32 : MT * GBN;
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// the address, in the cluster's shared window, of this CTA's shared address `a` in CTA `rank`
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// tile into this CTA's shared memory, bytes counted on a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier at this offset in both CTAs of the pair
+__device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+               : "memory");
+}
+
+// ------------------------------------------------------------------------------------------------
+// fp16 weights, more than 128 rows: out^T[256 channels, BN rows] per pair of CTAs (BN a multiple of 32 up to 256,
+// chosen at launch).  The pair is one tcgen05.mma.cta_group::2: each CTA holds the weights of its own 128 channels and
+// half of the X tile, so a slice of 64 inputs costs an SM 16 KB of weights and 16 KB of X for 512 clocks of MMA, where a CTA
+// of its own with the same 128 x 256 accumulator would fetch, and read from shared memory at every MMA, all 32 KB of X.
+// Two CTAs per SM (3 slots of 32 KB and 256 TMEM columns each): the start and the end of one hide in part behind the main loop
+// of the other, and tiles are handed out by the hardware, also across the two row pieces of a long prompt.
+// [2048 x 2560] x [2560 x 11520] with the relu^2 epilogue: 107 us (1,130 TFLOP/s); 256 x 256 tiles of single CTAs, whose
+// epilogue nothing hid, 182.  Without its epilogue 82, without its loads 100: the epilogue is what is left.
+//   warp 0: TMA into the own shared memory; the bytes of both CTAs are counted on the even CTA's barrier
+//   warp 1: TMEM, and in the even CTA the MMAs of the pair        warps 2..5: epilogue, a TMEM lane quadrant each
+// Low halves of X (A2) are ring slots of their own that meet the same weights again: after the high halves of the same
+// slice (lo_each) or after all of K.
+// 32 rows of X at one channel per lane, for all 32 lanes of a warp (ok: this lane's channel exists).
+// The kind of epilogue is decided once per 32 rows and not per value, and neighbouring lanes swap every other row, so that fp16
+// results leave two channels at a time: 2-byte stores behind a chain of branches took 12 us a tile, the main loop of K = 2560 takes 11.
+template <int EPI>
+__device__ __forceinline__ void pair_store_half(const GemmArgs &g, int ch, bool ok, int row0, const uint32_t (&acc)[32]) {
+  const int nr = g.M - row0;
+  const size_t ld = (size_t)g.ldo;
+  if (((g.N | g.ldo) & 1) == 0) {
+    const int odd = threadIdx.x & 1;
+    const size_t o = (size_t)(row0 + odd) * ld + (ch - odd);
+    __half *out = reinterpret_cast<__half *>(g.out) + o;
+    __half *lo = g.out_lo ? reinterpret_cast<__half *>(g.out_lo) + o : nullptr;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      const float a = epi_half_op<EPI>(__uint_as_float(acc[i])), b = epi_half_op<EPI>(__uint_as_float(acc[i + 1]));
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+      const float c0 = odd ? other : a, c1 = odd ? b : other;      // channels ch - odd, ch - odd + 1 of row i + odd
+      const __half2 h = __floats2half2_rn(c0, c1);
+      if (ok && i + odd < nr) {
+        *reinterpret_cast<__half2 *>(out + i * ld) = h;
+        if (lo) *reinterpret_cast<__half2 *>(lo + i * ld) = __floats2half2_rn(c0 - __low2float(h), c1 - __high2float(h));
+      }
+    }
+  } else if (ok) {
+    const size_t o = (size_t)row0 * ld + ch;
+    __half *out = reinterpret_cast<__half *>(g.out) + o;
+    __half *lo = g.out_lo ? reinterpret_cast<__half *>(g.out_lo) + o : nullptr;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const float e = epi_half_op<EPI>(__uint_as_float(acc[i]));
+      const __half h = __float2half_rn(e);
+      if (i < nr) {
+        out[i * ld] = h;
+        if (lo) lo[i * ld] = __float2half_rn(e - __half2float(h));
+      }
+    }
+  }
+}
+// residual stream: x + acc, or x + r * acc.  16 rows' inputs are asked for before the first result is stored.
+template <bool MUL>
+__device__ __forceinline__ void pair_store_add(const GemmArgs &g, int ch, int row0, const uint32_t (&acc)[32]) {
+  const int nr = g.M - row0;
+  const size_t o = (size_t)row0 * g.ldo + ch, ld = (size_t)g.ldo;
+  const float *x = reinterpret_cast<const float *>(g.aux0) + o;
+  const __half *r = reinterpret_cast<const __half *>(g.aux1) + o, *rl = g.aux1_lo ? reinterpret_cast<const __half *>(g.aux1_lo) + o : nullptr;
+  float *out = reinterpret_cast<float *>(g.out) + o;
+  const float scale = g.scale;
+#pragma unroll
+  for (int h = 0; h < 32; h += 16) {
+    float xv[16], rv[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      xv[i] = h + i < nr ? x[(h + i) * ld] : 0.f;
+      rv[i] = !MUL ? 1.f : h + i < nr ? __half2float(r[(h + i) * ld]) : 0.f;
+    }
+    if (MUL && rl) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (h + i < nr) rv[i] += __half2float(rl[(h + i) * ld]);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (h + i < nr) out[(h + i) * ld] = (xv[i] + rv[i] * __uint_as_float(acc[h + i])) * scale;
+  }
+}
+__device__ __forceinline__ void pair_store_f32(float *out, size_t ld, int nr, const uint32_t (&acc)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (i < nr) out[i * ld] = __uint_as_float(acc[i]);
+}
+__device__ __forceinline__ void pair_epilogue(const GemmArgs &g, int ch, int row0, const uint32_t (&acc)[32]) {
+  const bool ok = ch < g.N;
+  switch (g.epi) {
+    case GEMM_EPI_F32:
+      if (ok) pair_store_f32(reinterpret_cast<float *>(g.out) + (size_t)row0 * g.ldo + ch, (size_t)g.ldo, g.M - row0, acc);
+      break;
+    case GEMM_EPI_ADD_F32: if (ok) pair_store_add<false>(g, ch, row0, acc); break;
+    case GEMM_EPI_MULADD_F32: if (ok) pair_store_add<true>(g, ch, row0, acc); break;
+    case GEMM_EPI_SILU_F16: pair_store_half<GEMM_EPI_SILU_F16>(g, ch, ok, row0, acc); break;
+    case GEMM_EPI_SIGMOID_F16: pair_store_half<GEMM_EPI_SIGMOID_F16>(g, ch, ok, row0, acc); break;
+    case GEMM_EPI_RELU2_F16: pair_store_half<GEMM_EPI_RELU2_F16>(g, ch, ok, row0, acc); break;
+    default: pair_store_half<GEMM_EPI_PLAIN_F16>(g, ch, ok, row0, acc); break;
+  }
+}
+
+constexpr int PAIR_MAX_STAGES = 8;
+constexpr uint32_t PAIR_TMEM_COLS = 256;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 2)
+gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
+  const int STAGES = grp.stages, BN = grp.bn;
+  const uint32_t X_BYTES = (uint32_t)BN * (GBK * 2 / 2);          // this CTA's half of the X tile
+  const uint32_t STAGE_BYTES = G_A_BYTES + X_BYTES;
+  const uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * GBM >> 4) << 24);
   extern __shared__ uint8_t gsm_raw[];
-  // barriers in the first KB, tiles from the next 1024-byte boundary
+  // the same offsets in both CTAs: barriers in the first KB, tiles from the next 1024-byte boundary
   uint8_t *gsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t *full = reinterpret_cast<uint64_t *>(gsm);
-  uint64_t *empty = full + 4;
-  uint64_t *acc_full = empty + 4;
+  uint64_t *empty = full + PAIR_MAX_STAGES;
+  uint64_t *acc_full = empty + PAIR_MAX_STAGES;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t tiles = smem_u32(gsm + 1024);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  // pairs walk the row tiles of one channel tile before the next channel tile
+  const int pair = blockIdx.x >> 1, ct = pair / grp.m_tiles, m0 = (pair - ct * grp.m_tiles) * BN;
   int pi = 0;
-  while (pi + 1 < grp.n && (int)blockIdx.x >= grp.tile_start[pi + 1]) ++pi;
+  while (pi + 1 < grp.n && ct >= grp.tile_start[pi + 1]) ++pi;
   const GemmArgs &g = grp.p[pi];
-  const int tile_m = blockIdx.y, tile_n = blockIdx.x - grp.tile_start[pi];
+  const int ch0 = (ct - grp.tile_start[pi]) * (2 * GBM) + (int)rank * GBM;
   const int num_k1 = g.K / GBK;
-  // the low halves of A (A2) ride in the same ring slot as the high halves and meet the same B tile; the low
-  // halves of B (Bt2) are a second pass over K into the same accumulator
-  const bool has_lo = g.A2 != nullptr && grp.dual, lo_pass = g.A2 != nullptr && !grp.dual;
-  // split-K: this CTA covers K slices [kz0, kz0 + nkz) of every pass
   const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
-  const int num_k = nkz * (1 + (lo_pass ? 1 : 0) + (g.Bt2 ? 1 : 0));
+  const bool has_lo = g.A2 != nullptr;
+  const int num_e = has_lo ? 2 * nkz : nkz;
+  // ring entry e: slice of K and half of X
+  auto slice_of = [&](int e, bool &lo) {
+    if (!has_lo) { lo = false; return e; }
+    if (grp.lo_each) { lo = (e & 1) != 0; return e >> 1; }
+    lo = e >= nkz;
+    return lo ? e - nkz : e;
+  };
 
+  if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (has_lo) prefetch_tmap(&maps.a2[pi]); }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
@@ -270,108 +325,77 @@ gemm_f16_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ G
     mbar_fence_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(PAIR_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();      // the barriers of both CTAs exist before either one's copies arrive on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
-  pdl_wait();   // operands and epilogue inputs come from the kernels before this one
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int kb = 0; kb < num_k; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t parity = ((kb / STAGES) & 1) ^ 1;   // a fresh barrier reads as "previous phase complete"
-        if (!mbar_wait(&empty[s], parity, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        const int pass = kb / nkz, kk = kz0 + kb - pass * nkz;
-        const bool lo_now = has_lo && pass == 0;   // the (lo A) x (lo B) term is below fp32 resolution: skipped
-        const bool a_is_lo = lo_pass && pass == 1, b_is_lo = pass > 0 && !a_is_lo;
-        mbar_expect_tx(&full[s], (uint32_t)(lo_now ? 2 : 1) * MT * G_A_BYTES + G_B_BYTES);
-        const uint32_t a_dst = tiles + (uint32_t)s * STAGE_BYTES;
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          tma_load_2d(a_dst + (uint32_t)mt * G_A_BYTES, a_is_lo ? &maps.a2[pi] : &maps.a[pi], kk * GBK, (tile_m * MT + mt) * GBM, &full[s]);
-          if (lo_now) tma_load_2d(a_dst + (uint32_t)(MT + mt) * G_A_BYTES, &maps.a2[pi], kk * GBK, (tile_m * MT + mt) * GBM, &full[s]);
+      // the weights do not depend on the kernels before this one: the first round of them is asked for ahead of the wait
+      const int pre = num_e < STAGES ? num_e : STAGES;
+      bool lo;
+      for (int e = 0; e < pre; ++e)
+        tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + slice_of(e, lo)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
+      pdl_wait();
+      for (int e = 0; e < num_e; ++e) {
+        const int s = e % STAGES;
+        const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES, bar = mapa_u32(smem_u32(&full[s]), 0);
+        const int kx = (kz0 + slice_of(e, lo)) * GBK;
+        if (e >= pre) {
+          if (!mbar_wait(&empty[s], ((e / STAGES) & 1) ^ 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+          tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
         }
-        tma_load_2d(a_dst + B_OFF, b_is_lo ? &maps.b2[pi] : &maps.b[pi], kk * GBK, tile_n * GBN, &full[s]);
+        if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);   // (bytes that arrived before are counted, too)
+        tma_load_2d_pair(dst + G_A_BYTES, lo ? &maps.a2[pi] : &maps.a[pi], kx, m0 + (int)rank * (BN / 2), bar);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      for (int kb = 0; kb < num_k; ++kb) {
-        const int s = kb % STAGES;
-        if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+    if (rank == 0 && lane == 0) {
+      for (int e = 0; e < num_e; ++e) {
+        const int s = e % STAGES;
+        if (!mbar_wait(&full[s], (e / STAGES) & 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         tc_fence_after();
-        const uint32_t a_addr = tiles + (uint32_t)s * STAGE_BYTES;
-        const uint64_t bd = umma_desc_k128(a_addr + B_OFF);
-        const bool lo_now = has_lo && kb < nkz;
+        const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
+        const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + G_A_BYTES);
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const uint64_t ad = umma_desc_k128(a_addr + (uint32_t)mt * G_A_BYTES);
-#pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4)   // 16 inputs = 32 bytes further along the swizzled rows
-            umma_f16(tmem_base + (uint32_t)mt * GBN, ad + (uint64_t)(k4 * 2), bd + (uint64_t)(k4 * 2), G_IDESC, (kb | k4) != 0);
-          if (lo_now) {
-            const uint64_t al = umma_desc_k128(a_addr + (uint32_t)(MT + mt) * G_A_BYTES);
-#pragma unroll
-            for (int k4 = 0; k4 < GBK / 16; ++k4)
-              umma_f16(tmem_base + (uint32_t)mt * GBN, al + (uint64_t)(k4 * 2), bd + (uint64_t)(k4 * 2), G_IDESC, 1u);
-          }
-        }
-        umma_commit(&empty[s]);   // the slot is free once these MMAs have read it
+        for (int k4 = 0; k4 < GBK / 16; ++k4)
+          umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, (e | k4) != 0);
+        umma_commit_pair(&empty[s]);
       }
-      umma_commit(acc_full);      // the accumulators are complete once every MMA has retired
+      umma_commit_pair(acc_full);
     }
   } else {
-    // epilogue warps 2..5 -> TMEM lane quadrants 2, 3, 0, 1
     const int quad = warp & 3;
+    const int ch = ch0 + quad * 32 + lane;
+    pdl_wait();
     const bool ok = mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT);
     tc_fence_after();
     if (ok) {
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const int row = (tile_m * MT + mt) * GBM + quad * 32 + lane;
-        if ((tile_m * MT + mt) * GBM >= g.M) break;   // warp-uniform
-        for (int c0 = 0; c0 < GBN; c0 += 32) {
-          if (tile_n * GBN + c0 >= g.N) break;   // warp-uniform
-          uint32_t acc[32];
-          tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(mt * GBN + c0), acc);
-          if (grp.split > 1) {
-            // raw partial sums of this K range: slab blockIdx.z of [split][M][N]
-            if (row < g.M) {
-              float *dst = g.raw + ((size_t)blockIdx.z * g.M + row) * g.N + tile_n * GBN + c0;
-              const int ncol = min(32, g.N - (tile_n * GBN + c0));
-              if (ncol == 32 && (g.N & 3) == 0) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                  *reinterpret_cast<float4 *>(dst + i) = make_float4(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]),
-                                                                     __uint_as_float(acc[i + 2]), __uint_as_float(acc[i + 3]));
-              } else {
-                for (int i = 0; i < ncol; ++i) dst[i] = __uint_as_float(acc[i]);
-              }
-            }
-            continue;
-          }
-          if (g.col_scale) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int col = tile_n * GBN + c0 + i;
-              acc[i] = __float_as_uint(__uint_as_float(acc[i]) * (col < g.N ? __half2float(g.col_scale[col]) : 0.f));
-            }
-          }
-          if (row < g.M) gemm_epilogue_row(g, row, tile_n * GBN + c0, acc);
+      for (int c0 = 0; c0 < BN; c0 += 32) {
+        if (m0 + c0 >= g.M) break;   // warp-uniform
+        uint32_t acc[32];
+        __syncwarp();
+        tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
+        if (grp.split > 1) {
+          if (ch < g.N) pair_store_f32(g.raw + ((size_t)blockIdx.z * g.M + m0 + c0) * g.N + ch, (size_t)g.N, g.M - m0 - c0, acc);
+        } else {
+          pair_epilogue(g, ch, m0 + c0, acc);
         }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();      // neither CTA leaves while the other's MMAs or commits may still reach into it
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PAIR_TMEM_COLS) : "memory");
   }
 }
 
@@ -1797,16 +1821,6 @@ cudaError_t launch_ln_row(const float *x, const float *w, const float *b, int C,
 }
 
 namespace {
-template <int MT, int BN>
-cudaError_t launch_gemm_t(const GemmMaps &maps, const GemmGroup &grp, dim3 grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(gemm_f16_kernel<MT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  launch_k(gemm_f16_kernel<MT, BN>, dim3(grid), dim3(G_THREADS), smem, st, maps, grp);
-  return cudaGetLastError();
-}
-}  // namespace
-
-namespace {
 template <int BN>
 cudaError_t launch_gemm_wt_t(const GemmMaps &maps, const GemmGroup &grp, dim3 grid, size_t smem, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(gemm_wt_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1815,17 +1829,26 @@ cudaError_t launch_gemm_wt_t(const GemmMaps &maps, const GemmGroup &grp, dim3 gr
   return cudaGetLastError();
 }
 
-// FR_B200_GEMM_WT=0 sends few-row GEMMs through the 64-column tiles of gemm_f16_kernel instead (for comparison)
-bool wt_enabled() {
-  static const int on = [] { const char *v = getenv("FR_B200_GEMM_WT"); return !(v && v[0] == '0'); }();
-  return on != 0;
+// In how many pieces K is cut for `ctas` tiles of which a device holds `slots`: the cost of a split, in K slices of one CTA, is
+// waves x (slices per CTA + fill and drain) + the slabs it adds.
+int split_of(int ctas, int slots, int min_k1) {
+  const int max_split = std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 2));
+  int split = 1;
+  float best = 0.f;
+  for (int sp = 1; sp <= max_split; ++sp) {
+    const int waves = (ctas * sp + slots - 1) / slots;
+    const float cost = (float)waves * (float)((min_k1 + sp - 1) / sp + 2) + 0.25f * (float)sp;
+    if (sp == 1 || cost < best) { best = cost; split = sp; }
+  }
+  return split;
 }
+// the cut of a product of RWKV-5 over more than 128 rows: that of one 128 x 256 tile per SM
+int keep_split(int ctas, int min_k1) { return split_of(ctas, device_sm_count(), min_k1); }
 
-// up to GEMM_SMALL_M rows: weights along the MMA rows (gemm_wt_kernel), split-K into slabs when scratch was given
+// up to 128 rows: weights along the MMA rows (gemm_wt_kernel), split-K into slabs when scratch was given
 cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
   const int M = probs[0].M;
-  // (measured at 200 .. 512 rows: 256-row X tiles beat two passes with 128-row tiles by 10 %)
-  const int bn = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  const int bn = M <= 32 ? 32 : M <= 64 ? 64 : 128;
   GemmMaps maps;
   GemmGroup grp;
   memset(&grp, 0, sizeof(grp));
@@ -1858,16 +1881,7 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   grp.split = 1;
   const int sms = device_sm_count();
   const int slots = bn <= 64 ? 2 * sms : sms;
-  if (raw_ok) {
-    // cost of a split, in K slices of one CTA: waves x (slices per CTA + fill and drain) + the slabs it adds
-    const int ctas = tiles * m_tiles, max_split = std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 2));
-    float best = 0.f;
-    for (int sp = 1; sp <= max_split; ++sp) {
-      const int waves = (ctas * sp + slots - 1) / slots;
-      const float cost = (float)waves * (float)((min_k1 + sp - 1) / sp + 2) + 0.25f * (float)sp;
-      if (sp == 1 || cost < best) { best = cost; grp.split = sp; }
-    }
-  }
+  if (raw_ok) grp.split = split_of(tiles * m_tiles, slots, min_k1);
   grp.stage_bytes = ((grp.dual & 2) ? 2u : 1u) * G_A_BYTES + ((grp.dual & 1) ? 2u : 1u) * (uint32_t)bn * GBK * 2;
   // two CTAs per SM with rings of >= 3 slots where they fit (shorter tail when there are more tiles than SMs),
   // else one CTA with as deep a ring as fits
@@ -1878,8 +1892,7 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   dim3 grid(tiles, m_tiles, grp.split);
   cudaError_t e = bn == 32    ? launch_gemm_wt_t<32>(maps, grp, grid, smem, st)
                   : bn == 64  ? launch_gemm_wt_t<64>(maps, grp, grid, smem, st)
-                  : bn == 128 ? launch_gemm_wt_t<128>(maps, grp, grid, smem, st)
-                              : launch_gemm_wt_t<256>(maps, grp, grid, smem, st);
+                              : launch_gemm_wt_t<128>(maps, grp, grid, smem, st);
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
@@ -1966,17 +1979,7 @@ cudaError_t launch_gemm_wq(const GemmArgs *probs, int n, cudaStream_t st, int *d
   }
   for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; maps.b2[i] = maps.b2[0]; }
   const int slots = (two_per_sm ? 2 : 1) * device_sm_count();
-  if (raw_ok) {
-    // split-K: the fewest waves of CTAs, each at least two K slices long; a slice costs 1, a wave's start and end 2,
-    // a slab in the finishing pass a quarter
-    const int ctas = tiles * m_tiles, max_split = std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 2));
-    float best = 0.f;
-    for (int sp = 1; sp <= max_split; ++sp) {
-      const int waves = (ctas * sp + slots - 1) / slots;
-      const float cost = (float)waves * (float)((min_k1 + sp - 1) / sp + 2) + 0.25f * (float)sp;
-      if (sp == 1 || cost < best) { best = cost; grp.split = sp; }
-    }
-  }
+  if (raw_ok) grp.split = split_of(tiles * m_tiles, slots, min_k1);
   grp.stages = pl.nw;
   grp.estages = pl.ne;
   grp.wbox = pl.wbox;
@@ -1995,6 +1998,73 @@ cudaError_t launch_gemm_wq(const GemmArgs *probs, int n, cudaStream_t st, int *d
   }
   return cudaGetLastError();
 }
+
+// more than 128 rows of X, fp16 weights: gemm_pair_kernel
+cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
+  const int M = probs[0].M, num_pairs = device_sm_count() / 2;
+  GemmMaps maps;
+  GemmGroup grp;
+  memset(&grp, 0, sizeof(grp));
+  grp.n = n;
+  int tiles = 0, tiles128 = 0, units = 0, min_k1 = 1 << 30, sum_n = 0;
+  bool raw_ok = M <= GEMM_SMALL_M;
+  for (int i = 0; i < n; ++i) {
+    const GemmArgs &g = probs[i];
+    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M || g.Bt2 || g.col_scale) return cudaErrorInvalidValue;
+    if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
+      return cudaErrorInvalidValue;
+    grp.p[i] = g;
+    grp.tile_start[i] = tiles;
+    const int t = (g.N + 2 * GBM - 1) / (2 * GBM);
+    tiles += t;
+    tiles128 += (g.N + GBM - 1) / GBM;
+    units += t * (g.A2 ? 2 : 1);
+    sum_n += g.N;
+    min_k1 = std::min(min_k1, g.K / GBK);
+    raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
+  }
+  grp.tile_start[n] = tiles;
+  // The sums of a result follow from how K is cut.  RWKV-5 amplifies a changed last bit to percents of its logits, so its
+  // products keep the cut of keep_split(); else a cut and a row tile are chosen together.
+  const int fixed = raw_ok && probs[0].fixed_split ? keep_split(tiles128 * ((M + 255) / 256), min_k1) : 0;
+  const int max_split = raw_ok ? std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 4)) : 1;
+  grp.split = 1;
+  grp.bn = 256;
+  float best = 0.f;
+  for (int rt = (M + 255) / 256; rt <= (M + 127) / 128; ++rt) {
+    const int bn = ((M + rt - 1) / rt + 31) / 32 * 32;
+    for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
+      // in clocks: a slice takes a pair 256 + bn (shared memory: 32 KB of weights and 64 bn bytes of X in, the same out
+      // to the MMAs, at 128 bytes a clock and SM), a wave of tiles about 8 slices more to start and to end, and the slabs are
+      // written and read at about 2,700 bytes a clock
+      const int waves = (units * rt * sp + num_pairs - 1) / num_pairs;
+      float cost = (float)waves * (float)((min_k1 + sp - 1) / sp + 8) * (float)(256 + bn);
+      if (sp > 1) cost += 3000.f + (float)sp * (float)M * (float)sum_n * 8.f / 2700.f;
+      if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
+    }
+  }
+  grp.m_tiles = (M + grp.bn - 1) / grp.bn;
+  grp.lo_each = M <= GEMM_SMALL_M;
+  for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
+    const GemmArgs &g = probs[i < n ? i : 0];
+    if (!make_map(&maps.a[i], g.A, g.M, g.K, grp.bn / 2) || !make_map(&maps.b[i], g.Bt, g.N, g.K, GBM)) return cudaErrorNotSupported;
+    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, grp.bn / 2)) return cudaErrorNotSupported;
+    maps.b2[i] = maps.b[i];
+  }
+  grp.stage_bytes = G_A_BYTES + (uint32_t)grp.bn * GBK;
+  grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((110u << 10) / grp.stage_bytes));
+  const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
+  cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if ((e = launch_k(gemm_pair_kernel, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
+  if (defer_split) *defer_split = grp.split;
+  if (grp.split > 1 && !defer_split) {
+    int max_n = 0;
+    for (int i = 0; i < n; ++i) max_n = std::max(max_n, probs[i].N);
+    launch_k(gemm_finish_kernel, dim3((M * (max_n / 4) + 255) / 256, n), dim3(256), 0, st, grp);
+  }
+  return cudaGetLastError();
+}
 }  // namespace
 
 // defer_split (optional): the caller's next kernel sums the split-K slabs itself (ln_mix_seq_kernel, wkv4_rows_kernel);
@@ -2004,56 +2074,7 @@ cudaError_t launch_gemm_group(const GemmArgs *probs, int n, int mt, cudaStream_t
   const int M = probs[0].M;
   if (defer_split) *defer_split = 1;
   if (probs[0].Wq) return launch_gemm_wq(probs, n, st, defer_split);
-  if (M <= GEMM_SMALL_M && wt_enabled()) return launch_gemm_wt(probs, n, st, defer_split);
-  // few rows (batched decode): narrow N tiles and split-K, so that a few hundred CTAs stream the weights
-  const bool narrow = M <= GEMM_SMALL_M;
-  const int bn = narrow ? 64 : 256;
-  GemmMaps maps;
-  GemmGroup grp;
-  memset(&grp, 0, sizeof(grp));
-  grp.n = n;
-  int tiles = 0, min_k1 = 1 << 30;
-  bool raw_ok = true;
-  for (int i = 0; i < n; ++i) {
-    const GemmArgs &g = probs[i];
-    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
-      return cudaErrorInvalidValue;
-    if (!make_map(&maps.a[i], g.A, g.M, g.K, GBM) || !make_map(&maps.b[i], g.Bt, g.N, g.K, bn)) return cudaErrorNotSupported;
-    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, GBM)) return cudaErrorNotSupported;
-    if (!make_map(&maps.b2[i], g.Bt2 ? g.Bt2 : g.Bt, g.N, g.K, bn)) return cudaErrorNotSupported;
-    grp.p[i] = g;
-    grp.tile_start[i] = tiles;
-    tiles += (g.N + bn - 1) / bn;
-    min_k1 = std::min(min_k1, g.K / GBK);
-    raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
-  }
-  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; maps.b2[i] = maps.b2[0]; }
-  grp.tile_start[n] = tiles;
-  const int m_tiles = (M + mt * GBM - 1) / (mt * GBM);
-  grp.split = 1;
-  if (narrow && raw_ok) {
-    const int want = (2 * device_sm_count() + tiles * m_tiles - 1) / (tiles * m_tiles);    // about two CTAs per SM in total
-    grp.split = std::max(1, std::min(std::min(want, GEMM_SPLIT_MAX), min_k1 / 4));   // at least 4 K slices per CTA
-  }
-  if (mt == 1)
-    for (int i = 0; i < n; ++i) grp.dual |= probs[i].A2 != nullptr;
-  grp.stage_bytes = (uint32_t)(grp.dual ? 2 : 1) * mt * G_A_BYTES + (uint32_t)bn * GBK * 2;
-  grp.stages = (int)std::min<size_t>(4, (192u << 10) / grp.stage_bytes);
-  if (narrow) grp.stages = 2;   // short K ranges per CTA: a 2-deep ring leaves room for two CTAs per SM (measured: 15 % faster steps)
-  const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
-  dim3 grid(tiles, m_tiles, grp.split);
-  cudaError_t e;
-  if (narrow) e = mt == 1 ? launch_gemm_t<1, 64>(maps, grp, grid, smem, st) : launch_gemm_t<2, 64>(maps, grp, grid, smem, st);
-  else e = mt == 1 ? launch_gemm_t<1, 256>(maps, grp, grid, smem, st) : launch_gemm_t<2, 256>(maps, grp, grid, smem, st);
-  if (e != cudaSuccess) return e;
-  if (defer_split) *defer_split = grp.split;
-  if (grp.split > 1 && !defer_split) {
-    int max_n = 0;
-    for (int i = 0; i < n; ++i) max_n = std::max(max_n, probs[i].N);
-    launch_k(gemm_finish_kernel, dim3(dim3((M * (max_n / 4) + 255) / 256, n)), dim3(256), 0, st, grp);
-  }
-  return cudaGetLastError();
+  return M <= 128 ? launch_gemm_wt(probs, n, st, defer_split) : launch_gemm_pair(probs, n, st, defer_split);
 }
 
 cudaError_t launch_gemm_f16(const GemmArgs &g, cudaStream_t st) {

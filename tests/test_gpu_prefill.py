@@ -53,6 +53,22 @@ def _epilogues(pkg, rng, M, N, K):
         assert np.abs(got - w).max() < tol * max(1.0, float(np.abs(w).max())), epi
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 255, 64), (160, 514, 128), (257, 256, 64), (289, 768, 1088), (1025, 33, 128), (1057, 1000, 64)])
+def test_gemm_pair_tiles(pkg, M, N, K):
+    """More than 128 rows: row tiles of 96 to 256 rows with ragged last ones, channel tiles of which the pair's second
+    half is partly or wholly outside, odd N (two-byte stores), one slice of K.  |error| of an fp32 sum of K products: K 2^-24
+    times the sum of their magnitudes (K for these inputs, at most), with fp16 rounding of the result where it is fp16."""
+    rng = np.random.default_rng(M + N + K)
+    A = rng.uniform(-1, 1, (M, K)).astype(np.float32)
+    W = rng.uniform(-1, 1, (K, N)).astype(np.float32)
+    x = rng.standard_normal((M, N), dtype=np.float32)
+    acc = _f16(A).astype(np.float64) @ _f16(W).astype(np.float64)
+    tol = K * K * 2.0 ** -24
+    assert np.abs(pkg.gemm_f16(A, W) - acc).max() < tol
+    assert np.abs(pkg.gemm_f16(A, W, 4, x, None, 0.5) - (x + acc) * 0.5).max() < tol
+    assert (np.abs(pkg.gemm_f16(A, W, 6) - acc) <= tol + 2.0 ** -10 * np.abs(acc)).all()
+
+
 def test_gemm_rejects_bad_arguments(pkg):
     A = np.zeros((4, 100), np.float32)
     W = np.zeros((100, 8), np.float32)
