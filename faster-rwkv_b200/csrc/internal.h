@@ -166,7 +166,6 @@ struct GemmArgs {
   const __half *A;     // [M, K] row-major
   const __half *A2;    // optional [M, K]: low halves of the activations (A + A2 is the fp32 value to ~22 bits)
   const __half *Bt;    // [N, K] row-major (the weight matrix transposed: one row per output channel)
-  const __half *Bt2;   // optional [N, K]: what rounding the weights to fp16 lost (int4: q * scale needs 14 bits); third pass
   const __half *col_scale;   // optional [N]: acc *= col_scale[n] before the epilogue (int8: Bt holds the integer codes)
   // quantised weights in packed form instead of Bt (few-row GEMM that expands them in shared memory):
   const uint8_t *Wq;         // wfmt FMT_INT8: codes [N, K] int8;  FMT_INT4: [N, K/2], nibble = q + 8, even k low
@@ -182,6 +181,7 @@ struct GemmArgs {
   float scale;
   int *status;         // device word: set when a bounded wait gives up
   float *raw;          // optional scratch [GEMM_SPLIT_MAX][M][N] f32: allows split-K when M <= GEMM_SMALL_M
+  int tma_out;         // set by the launcher: out (and out_lo) are written by tensor stores
   int fixed_split;     // 1: K is cut the same way whatever kernel serves the product (RWKV-5, see launch_gemm_pair)
 };
 constexpr int GEMM_GROUP_MAX = 4;

@@ -57,8 +57,8 @@ cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
 }
 
 // ------------------------------------------------------------------------------------------------
-// tcgen05 GEMMs: out[M, N] = epilogue((A + A2)[M, K] . (Bt + Bt2)[N, K]^T), fp16 operands (both K-major), fp32
-// accumulate.  A2 (optional) holds what rounding the activations to fp16 lost, Bt2 what rounding the weights did.
+// tcgen05 GEMMs: out[M, N] = epilogue((A + A2)[M, K] . (Bt)[N, K]^T), fp16 operands (both K-major), fp32
+// accumulate.  A2 (optional) holds what rounding the activations to fp16 lost.
 // All of them put the weights along the MMA rows, so that an accumulator holds out^T (TMEM lane = output channel, column = row
 // of X) and the epilogue's lanes run along the channels; K is walked in 64-wide slices through a TMA ring.
 //   warp 0 (one lane): TMA producer          warp 1 (one lane): MMA issue; the warp owns the TMEM allocation
@@ -112,6 +112,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Place in a ring of barriers.  Its slot and phase are counted: a division by a depth that only the launch knows costs 100
+// to 200 clocks of a chain that takes 300 to 1,000 per slice, and every role had two to four of them.
+struct Ring {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next(int depth) {
+    if (++slot == depth) { slot = 0; phase ^= 1u; }
+  }
+};
+
 // the result is rounded to fp16: the fast exponential and division are exact enough
 __device__ __forceinline__ float sigmoid_g(float v) { return __fdividef(1.f, 1.f + __expf(-v)); }
 
@@ -137,15 +147,174 @@ struct GemmGroup {
   uint32_t wbox;                        // packed-weight GEMM: bytes per row of a weight slot (64 or 128)
   uint32_t stage_bytes;                 // bytes per ring slot
   int split;                            // split-K factor (grid.z); > 1: CTAs write raw partial sums to GemmArgs::raw
-  int dual;                             // few-row GEMM: bit 0, some problem has A2 (the slot holds an X lo tile); bit 1, Bt2
+  int dual;                             // few-row GEMM: some problem has A2 (the slot holds an X lo tile)
   int bn, m_tiles;                      // pair GEMM: rows of X per tile, row tiles
   int lo_each;                          // pair GEMM: the low halves of X follow the high halves slice by slice
   int tile_start[GEMM_GROUP_MAX + 1];   // first channel tile of each problem
   GemmArgs p[GEMM_GROUP_MAX];
 };
 struct alignas(64) GemmMaps {
-  CUtensorMap a[GEMM_GROUP_MAX], a2[GEMM_GROUP_MAX], b[GEMM_GROUP_MAX], b2[GEMM_GROUP_MAX];
+  CUtensorMap a[GEMM_GROUP_MAX], a2[GEMM_GROUP_MAX], b[GEMM_GROUP_MAX];
+  CUtensorMap o[GEMM_GROUP_MAX], o_lo[GEMM_GROUP_MAX];   // results (or slabs) in boxes of 32 channels x 32 rows
 };
+
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ---- epilogue of all of them ----
+// A warp turns 32 rows of X at one channel per lane into 32 x 32 results in shared memory, which a tensor store writes to their
+// rows (4 to 10 KB apart) on its own.  Stored by the lanes themselves, 128 bytes a row, a 128 x 128 accumulator took 4 us
+// behind the last MMA, 2 of them for the address arithmetic alone; staged it takes 1.5.  Outputs whose rows are not multiples of 16 bytes
+// are stored by the lanes.
+constexpr uint32_t EPI_BUF = 4096;      // a warp has two: one is filled while the other is read
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+__device__ __forceinline__ void sts_u16(uint32_t a, uint16_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(v) : "memory"); }
+
+// residual stream: acc <- x + acc, or x + r * acc.  8 rows' inputs are asked for before the first is used.
+template <bool MUL>
+__device__ __forceinline__ void tile_add(const GemmArgs &g, int ch, bool ok, int row0, uint32_t (&acc)[32]) {
+  const int nr = ok ? g.M - row0 : 0;
+  const size_t o = (size_t)row0 * g.ldo + ch, ld = (size_t)g.ldo;
+  const float *x = reinterpret_cast<const float *>(g.aux0) + o;
+  const __half *r = reinterpret_cast<const __half *>(g.aux1) + o, *rl = g.aux1_lo ? reinterpret_cast<const __half *>(g.aux1_lo) + o : nullptr;
+  const float scale = g.scale;
+#pragma unroll
+  for (int h = 0; h < 32; h += 8) {
+    float xv[8], rv[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      xv[i] = h + i < nr ? x[(h + i) * ld] : 0.f;
+      rv[i] = !MUL ? 1.f : h + i < nr ? __half2float(r[(h + i) * ld]) : 0.f;
+    }
+    if (MUL && rl) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (h + i < nr) rv[i] += __half2float(rl[(h + i) * ld]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[h + i] = __float_as_uint((xv[i] + rv[i] * __uint_as_float(acc[h + i])) * scale);
+  }
+}
+template <int EPI>
+__device__ __forceinline__ void tile_half(uint32_t buf, bool lo, const uint32_t (&acc)[32]) {
+  const uint32_t at = buf + (threadIdx.x & 31) * 2;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const float e = epi_half_op<EPI>(__uint_as_float(acc[i]));
+    const __half h = __float2half_rn(e);
+    sts_u16(at + i * 64, __half_as_ushort(h));
+    if (lo) sts_u16(at + 2048 + i * 64, __half_as_ushort(__float2half_rn(e - __half2float(h))));
+  }
+}
+// rows row0 .. row0 + 31, channels ch_w .. ch_w + 31 (lane l: ch_w + l) of one problem; z: its K range, when raw
+__device__ __forceinline__ void tile_out(const GemmArgs &g, const CUtensorMap *om, const CUtensorMap *om_lo, bool raw, int z, int ch_w,
+                                         int row0, uint32_t (&acc)[32], uint32_t buf) {
+  const int lane = threadIdx.x & 31, ch = ch_w + lane;
+  const bool ok = ch < g.N;
+  const int epi = raw ? GEMM_EPI_F32 : g.epi;
+  if (epi == GEMM_EPI_ADD_F32) tile_add<false>(g, ch, ok, row0, acc);
+  else if (epi == GEMM_EPI_MULADD_F32) tile_add<true>(g, ch, ok, row0, acc);
+  const bool f32 = epi == GEMM_EPI_F32 || epi == GEMM_EPI_ADD_F32 || epi == GEMM_EPI_MULADD_F32;
+  if (raw || g.tma_out) {
+    if (f32) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) sts_u32(buf + i * 128 + lane * 4, acc[i]);
+    } else {
+      const bool lo = g.out_lo != nullptr;
+      if (epi == GEMM_EPI_SILU_F16) tile_half<GEMM_EPI_SILU_F16>(buf, lo, acc);
+      else if (epi == GEMM_EPI_SIGMOID_F16) tile_half<GEMM_EPI_SIGMOID_F16>(buf, lo, acc);
+      else if (epi == GEMM_EPI_RELU2_F16) tile_half<GEMM_EPI_RELU2_F16>(buf, lo, acc);
+      else tile_half<GEMM_EPI_PLAIN_F16>(buf, lo, acc);
+    }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) {
+      if (ch_w < g.N) {
+        tma_store_3d(om, buf, ch_w, row0, raw ? z : 0);
+        if (!f32 && g.out_lo) tma_store_3d(om_lo, buf + 2048, ch_w, row0, 0);
+      }
+      asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group.read 1;" ::: "memory");   // the other buffer is free again
+    }
+    __syncwarp();
+    return;
+  }
+  if (!ok) return;
+  const size_t o = (size_t)row0 * g.ldo + ch, ld = (size_t)g.ldo;
+  const int nr = g.M - row0;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    if (i >= nr) continue;
+    if (f32) {
+      reinterpret_cast<float *>(g.out)[o + i * ld] = __uint_as_float(acc[i]);
+    } else {
+      float e = __uint_as_float(acc[i]);
+      e = epi == GEMM_EPI_SILU_F16 ? epi_half_op<GEMM_EPI_SILU_F16>(e) : epi == GEMM_EPI_SIGMOID_F16 ? epi_half_op<GEMM_EPI_SIGMOID_F16>(e)
+          : epi == GEMM_EPI_RELU2_F16 ? epi_half_op<GEMM_EPI_RELU2_F16>(e) : e;
+      const __half h = __float2half_rn(e);
+      reinterpret_cast<__half *>(g.out)[o + i * ld] = h;
+      if (g.out_lo) reinterpret_cast<__half *>(g.out_lo)[o + i * ld] = __float2half_rn(e - __half2float(h));
+    }
+  }
+}
+
+// Slabs of up to 32 rows are stored by the lanes: the way through shared memory and a tensor store takes longer than it saves
+// (29 int4 tokens of the 1.5B shape 1.50 against 1.53 ms, 16 int8 streams 1.33 against 1.35).
+__device__ __forceinline__ void slab_rows(const GemmArgs &g, int z, int ch, int row0, const uint32_t (&acc)[32]) {
+  if (ch >= g.N) return;
+  float *dst = g.raw + ((size_t)z * g.M + row0) * g.N + ch;
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (row0 + i < g.M) dst[(size_t)i * g.N] = __uint_as_float(acc[i]);
+}
+// The same with few registers (72 in gemm_wq_kernel): all kinds of results that are not fp32 as they stand go back through
+// shared memory row by row.
+__device__ __forceinline__ void tile_out_lean(const GemmArgs &g, const CUtensorMap *om, bool raw, int z, int ch_w, int row0,
+                                              const uint32_t (&acc)[32], uint32_t buf) {
+  const int lane = threadIdx.x & 31, ch = ch_w + lane;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) sts_u32(buf + i * 128 + lane * 4, acc[i]);
+  if (raw || (g.tma_out && g.epi == GEMM_EPI_F32)) {
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) {
+      if (ch_w < g.N) tma_store_3d(om, buf, ch_w, row0, raw ? z : 0);
+      asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group.read 1;" ::: "memory");
+    }
+    __syncwarp();
+    return;
+  }
+  if (ch < g.N) {
+    const int nr = min(32, g.M - row0);
+    size_t o = (size_t)row0 * g.ldo + ch;
+#pragma unroll 8
+    for (int i = 0; i < nr; ++i, o += g.ldo) {
+      float e = lds_f32(buf + i * 128 + lane * 4);
+      if (g.epi == GEMM_EPI_F32) {
+        reinterpret_cast<float *>(g.out)[o] = e;
+      } else if (g.epi == GEMM_EPI_ADD_F32) {
+        reinterpret_cast<float *>(g.out)[o] = (reinterpret_cast<const float *>(g.aux0)[o] + e) * g.scale;
+      } else if (g.epi == GEMM_EPI_MULADD_F32) {
+        float r = __half2float(reinterpret_cast<const __half *>(g.aux1)[o]);
+        if (g.aux1_lo) r += __half2float(reinterpret_cast<const __half *>(g.aux1_lo)[o]);
+        reinterpret_cast<float *>(g.out)[o] = (reinterpret_cast<const float *>(g.aux0)[o] + r * e) * g.scale;
+      } else {
+        e = g.epi == GEMM_EPI_SILU_F16 ? epi_half_op<GEMM_EPI_SILU_F16>(e) : g.epi == GEMM_EPI_SIGMOID_F16 ? epi_half_op<GEMM_EPI_SIGMOID_F16>(e)
+            : g.epi == GEMM_EPI_RELU2_F16 ? epi_half_op<GEMM_EPI_RELU2_F16>(e) : e;
+        const __half h = __float2half_rn(e);
+        reinterpret_cast<__half *>(g.out)[o] = h;
+        if (g.out_lo) reinterpret_cast<__half *>(g.out_lo)[o] = __float2half_rn(e - __half2float(h));
+      }
+    }
+  }
+  __syncwarp();   // (the buffer is filled again two turns on)
+}
+// before the CTA may end: its stores have read shared memory
+__device__ __forceinline__ void tile_out_end() {
+  if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
 
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -194,91 +363,6 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 //   warp 1: TMEM, and in the even CTA the MMAs of the pair        warps 2..5: epilogue, a TMEM lane quadrant each
 // Low halves of X (A2) are ring slots of their own that meet the same weights again: after the high halves of the same
 // slice (lo_each) or after all of K.
-// 32 rows of X at one channel per lane, for all 32 lanes of a warp (ok: this lane's channel exists).
-// The kind of epilogue is decided once per 32 rows and not per value, and neighbouring lanes swap every other row, so that fp16
-// results leave two channels at a time: 2-byte stores behind a chain of branches took 12 us a tile, the main loop of K = 2560 takes 11.
-template <int EPI>
-__device__ __forceinline__ void pair_store_half(const GemmArgs &g, int ch, bool ok, int row0, const uint32_t (&acc)[32]) {
-  const int nr = g.M - row0;
-  const size_t ld = (size_t)g.ldo;
-  if (((g.N | g.ldo) & 1) == 0) {
-    const int odd = threadIdx.x & 1;
-    const size_t o = (size_t)(row0 + odd) * ld + (ch - odd);
-    __half *out = reinterpret_cast<__half *>(g.out) + o;
-    __half *lo = g.out_lo ? reinterpret_cast<__half *>(g.out_lo) + o : nullptr;
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      const float a = epi_half_op<EPI>(__uint_as_float(acc[i])), b = epi_half_op<EPI>(__uint_as_float(acc[i + 1]));
-      const float other = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-      const float c0 = odd ? other : a, c1 = odd ? b : other;      // channels ch - odd, ch - odd + 1 of row i + odd
-      const __half2 h = __floats2half2_rn(c0, c1);
-      if (ok && i + odd < nr) {
-        *reinterpret_cast<__half2 *>(out + i * ld) = h;
-        if (lo) *reinterpret_cast<__half2 *>(lo + i * ld) = __floats2half2_rn(c0 - __low2float(h), c1 - __high2float(h));
-      }
-    }
-  } else if (ok) {
-    const size_t o = (size_t)row0 * ld + ch;
-    __half *out = reinterpret_cast<__half *>(g.out) + o;
-    __half *lo = g.out_lo ? reinterpret_cast<__half *>(g.out_lo) + o : nullptr;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float e = epi_half_op<EPI>(__uint_as_float(acc[i]));
-      const __half h = __float2half_rn(e);
-      if (i < nr) {
-        out[i * ld] = h;
-        if (lo) lo[i * ld] = __float2half_rn(e - __half2float(h));
-      }
-    }
-  }
-}
-// residual stream: x + acc, or x + r * acc.  16 rows' inputs are asked for before the first result is stored.
-template <bool MUL>
-__device__ __forceinline__ void pair_store_add(const GemmArgs &g, int ch, int row0, const uint32_t (&acc)[32]) {
-  const int nr = g.M - row0;
-  const size_t o = (size_t)row0 * g.ldo + ch, ld = (size_t)g.ldo;
-  const float *x = reinterpret_cast<const float *>(g.aux0) + o;
-  const __half *r = reinterpret_cast<const __half *>(g.aux1) + o, *rl = g.aux1_lo ? reinterpret_cast<const __half *>(g.aux1_lo) + o : nullptr;
-  float *out = reinterpret_cast<float *>(g.out) + o;
-  const float scale = g.scale;
-#pragma unroll
-  for (int h = 0; h < 32; h += 16) {
-    float xv[16], rv[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      xv[i] = h + i < nr ? x[(h + i) * ld] : 0.f;
-      rv[i] = !MUL ? 1.f : h + i < nr ? __half2float(r[(h + i) * ld]) : 0.f;
-    }
-    if (MUL && rl) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (h + i < nr) rv[i] += __half2float(rl[(h + i) * ld]);
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (h + i < nr) out[(h + i) * ld] = (xv[i] + rv[i] * __uint_as_float(acc[h + i])) * scale;
-  }
-}
-__device__ __forceinline__ void pair_store_f32(float *out, size_t ld, int nr, const uint32_t (&acc)[32]) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i)
-    if (i < nr) out[i * ld] = __uint_as_float(acc[i]);
-}
-__device__ __forceinline__ void pair_epilogue(const GemmArgs &g, int ch, int row0, const uint32_t (&acc)[32]) {
-  const bool ok = ch < g.N;
-  switch (g.epi) {
-    case GEMM_EPI_F32:
-      if (ok) pair_store_f32(reinterpret_cast<float *>(g.out) + (size_t)row0 * g.ldo + ch, (size_t)g.ldo, g.M - row0, acc);
-      break;
-    case GEMM_EPI_ADD_F32: if (ok) pair_store_add<false>(g, ch, row0, acc); break;
-    case GEMM_EPI_MULADD_F32: if (ok) pair_store_add<true>(g, ch, row0, acc); break;
-    case GEMM_EPI_SILU_F16: pair_store_half<GEMM_EPI_SILU_F16>(g, ch, ok, row0, acc); break;
-    case GEMM_EPI_SIGMOID_F16: pair_store_half<GEMM_EPI_SIGMOID_F16>(g, ch, ok, row0, acc); break;
-    case GEMM_EPI_RELU2_F16: pair_store_half<GEMM_EPI_RELU2_F16>(g, ch, ok, row0, acc); break;
-    default: pair_store_half<GEMM_EPI_PLAIN_F16>(g, ch, ok, row0, acc); break;
-  }
-}
-
 constexpr int PAIR_MAX_STAGES = 8;
 constexpr uint32_t PAIR_TMEM_COLS = 256;
 
@@ -286,7 +370,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 2)
 gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   const int STAGES = grp.stages, BN = grp.bn;
   const uint32_t X_BYTES = (uint32_t)BN * (GBK * 2 / 2);          // this CTA's half of the X tile
-  const uint32_t STAGE_BYTES = G_A_BYTES + X_BYTES;
+  const uint32_t STAGE_BYTES = grp.stage_bytes;
   const uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * GBM >> 4) << 24);
   extern __shared__ uint8_t gsm_raw[];
   // the same offsets in both CTAs: barriers in the first KB, tiles from the next 1024-byte boundary
@@ -308,14 +392,8 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   const int num_k1 = g.K / GBK;
   const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
   const bool has_lo = g.A2 != nullptr;
-  const int num_e = has_lo ? 2 * nkz : nkz;
-  // ring entry e: slice of K and half of X
-  auto slice_of = [&](int e, bool &lo) {
-    if (!has_lo) { lo = false; return e; }
-    if (grp.lo_each) { lo = (e & 1) != 0; return e >> 1; }
-    lo = e >= nkz;
-    return lo ? e - nkz : e;
-  };
+  const bool lo_now = has_lo && grp.lo_each, lo_pass = has_lo && !grp.lo_each;
+  const int num_e = lo_pass ? 2 * nkz : nkz;
 
   if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (has_lo) prefetch_tmap(&maps.a2[pi]); }
   if (threadIdx.x == 0) {
@@ -339,55 +417,59 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
     if (lane == 0) {
       // the weights do not depend on the kernels before this one: the first round of them is asked for ahead of the wait
       const int pre = num_e < STAGES ? num_e : STAGES;
-      bool lo;
       for (int e = 0; e < pre; ++e)
-        tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + slice_of(e, lo)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
+        tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + (e < nkz ? e : e - nkz)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
       pdl_wait();
-      for (int e = 0; e < num_e; ++e) {
-        const int s = e % STAGES;
+      Ring at;
+      for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
+        const int s = at.slot;
         const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES, bar = mapa_u32(smem_u32(&full[s]), 0);
-        const int kx = (kz0 + slice_of(e, lo)) * GBK;
+        const int kx = (kz0 + (e < nkz ? e : e - nkz)) * GBK, row = m0 + (int)rank * (BN / 2);
         if (e >= pre) {
-          if (!mbar_wait(&empty[s], ((e / STAGES) & 1) ^ 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+          if (!mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
           tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
         }
-        if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);   // (bytes that arrived before are counted, too)
-        tma_load_2d_pair(dst + G_A_BYTES, lo ? &maps.a2[pi] : &maps.a[pi], kx, m0 + (int)rank * (BN / 2), bar);
+        if (rank == 0) mbar_expect_tx(&full[s], 2 * (G_A_BYTES + (lo_now ? 2u : 1u) * X_BYTES));   // (bytes that arrived before are counted, too)
+        tma_load_2d_pair(dst + G_A_BYTES, e < nkz ? &maps.a[pi] : &maps.a2[pi], kx, row, bar);
+        if (lo_now) tma_load_2d_pair(dst + G_A_BYTES + X_BYTES, &maps.a2[pi], kx, row, bar);
       }
     }
   } else if (warp == 1) {
     if (rank == 0 && lane == 0) {
-      for (int e = 0; e < num_e; ++e) {
-        const int s = e % STAGES;
-        if (!mbar_wait(&full[s], (e / STAGES) & 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+      Ring at;
+      for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
+        const int s = at.slot;
+        if (!mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         tc_fence_after();
         const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
         const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + G_A_BYTES);
 #pragma unroll
         for (int k4 = 0; k4 < GBK / 16; ++k4)
           umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, (e | k4) != 0);
+        if (lo_now) {
+          const uint64_t xl = umma_desc_k128(base + G_A_BYTES + X_BYTES);
+#pragma unroll
+          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
+        }
         umma_commit_pair(&empty[s]);
       }
       umma_commit_pair(acc_full);
     }
   } else {
     const int quad = warp & 3;
-    const int ch = ch0 + quad * 32 + lane;
     pdl_wait();
-    const bool ok = mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT);
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      const uint32_t buf = tiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
+      uint32_t flip = 0;
+      for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
         if (m0 + c0 >= g.M) break;   // warp-uniform
         uint32_t acc[32];
-        __syncwarp();
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
-        if (grp.split > 1) {
-          if (ch < g.N) pair_store_f32(g.raw + ((size_t)blockIdx.z * g.M + m0 + c0) * g.N + ch, (size_t)g.N, g.M - m0 - c0, acc);
-        } else {
-          pair_epilogue(g, ch, m0 + c0, acc);
-        }
+        tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
       }
+      tile_out_end();
     }
   }
   tc_fence_before();
@@ -410,25 +492,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 // lanes along the channels (coalesced), either the finished values or the split-K slabs gemm_finish_kernel sums.
 constexpr int WT_MAX_STAGES = 8;
 
-__device__ __forceinline__ void epi_store_one(const GemmArgs &g, int row, int col, float a) {
-  const size_t o = (size_t)row * g.ldo + col;
-  if (g.epi == GEMM_EPI_F32) {
-    reinterpret_cast<float *>(g.out)[o] = a;
-  } else if (g.epi == GEMM_EPI_ADD_F32) {
-    reinterpret_cast<float *>(g.out)[o] = (reinterpret_cast<const float *>(g.aux0)[o] + a) * g.scale;
-  } else if (g.epi == GEMM_EPI_MULADD_F32) {
-    float r = __half2float(reinterpret_cast<const __half *>(g.aux1)[o]);
-    if (g.aux1_lo) r += __half2float(reinterpret_cast<const __half *>(g.aux1_lo)[o]);
-    reinterpret_cast<float *>(g.out)[o] = (reinterpret_cast<const float *>(g.aux0)[o] + r * a) * g.scale;
-  } else {
-    const float e = epi_half_op(g.epi, a);
-    const __half h = __float2half_rn(e);
-    reinterpret_cast<__half *>(g.out)[o] = h;
-    if (g.out_lo) reinterpret_cast<__half *>(g.out_lo)[o] = __float2half_rn(e - __half2float(h));
-  }
-}
-
-// grp.dual here: bit 0 = some problem has A2 (slot holds an X lo tile), bit 1 = some problem has Bt2 (W lo tile)
+// grp.dual here: some problem has A2 (the slot holds an X lo tile)
 template <int BN>
 __global__ void __launch_bounds__(G_THREADS, 2)
 gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
@@ -441,7 +505,7 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   constexpr uint32_t TMEM_COLS = FUSE_LO ? 2 * BN : BN;
   const int STAGES = grp.stages;
   const uint32_t STAGE_BYTES = grp.stage_bytes;
-  const uint32_t X_OFF = ((grp.dual & 2) ? 2u : 1u) * G_A_BYTES, XLO_OFF = X_OFF + X_BYTES;
+  constexpr uint32_t X_OFF = G_A_BYTES, XLO_OFF = X_OFF + X_BYTES;
   extern __shared__ uint8_t gsm_raw[];
   uint8_t *gsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t *full = reinterpret_cast<uint64_t *>(gsm);
@@ -457,12 +521,11 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   const int tile_n = blockIdx.x - grp.tile_start[pi], m0 = blockIdx.y * BN;
   const int num_k1 = g.K / GBK;
   const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
-  const bool x_lo = g.A2 != nullptr, w_lo = g.Bt2 != nullptr;
+  const bool x_lo = g.A2 != nullptr;
 
   if (threadIdx.x == 64) {
     prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]);
     if (x_lo) prefetch_tmap(&maps.a2[pi]);
-    if (w_lo) prefetch_tmap(&maps.b2[pi]);
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -485,24 +548,23 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 
   if (warp == 0) {
     if (lane == 0) {
-      const uint32_t w_bytes = (w_lo ? 2u : 1u) * G_A_BYTES, x_bytes = (x_lo ? 2u : 1u) * X_BYTES;
+      const uint32_t w_bytes = G_A_BYTES, x_bytes = (x_lo ? 2u : 1u) * X_BYTES;
       const int pre = nkz < STAGES ? nkz : STAGES;
       for (int kb = 0; kb < pre; ++kb) {
         mbar_expect_tx_only(&full[kb], w_bytes);
         const uint32_t dst = tiles + (uint32_t)kb * STAGE_BYTES;
         tma_load_2d(dst, &maps.b[pi], (kz0 + kb) * GBK, tile_n * GBM, &full[kb]);
-        if (w_lo) tma_load_2d(dst + G_A_BYTES, &maps.b2[pi], (kz0 + kb) * GBK, tile_n * GBM, &full[kb]);
       }
       pdl_wait();
-      for (int kb = 0; kb < nkz; ++kb) {
-        const int s = kb % STAGES;
+      Ring at;
+      for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
+        const int s = at.slot;
         const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES;
         const int kx = (kz0 + kb) * GBK;
         if (kb >= pre) {
-          if (!mbar_wait(&empty[s], ((kb / STAGES) & 1) ^ 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+          if (!mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
           mbar_expect_tx(&full[s], w_bytes + x_bytes);
           tma_load_2d(dst, &maps.b[pi], kx, tile_n * GBM, &full[s]);
-          if (w_lo) tma_load_2d(dst + G_A_BYTES, &maps.b2[pi], kx, tile_n * GBM, &full[s]);
         } else {
           mbar_expect_tx(&full[s], x_bytes);
         }
@@ -512,9 +574,10 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      for (int kb = 0; kb < nkz; ++kb) {
-        const int s = kb % STAGES;
-        if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+      Ring at;
+      for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
+        const int s = at.slot;
+        if (!mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         tc_fence_after();
         const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
         const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + X_OFF);
@@ -527,11 +590,6 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 #pragma unroll
           for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
         }
-        if (w_lo) {
-          const uint64_t wl = umma_desc_k128(base + G_A_BYTES);
-#pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16(tmem_base, wl + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
         umma_commit(&empty[s]);
       }
       umma_commit(acc_full);
@@ -540,14 +598,15 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
     const int quad = warp & 3;
     const int ch = tile_n * GBM + quad * 32 + lane;
     pdl_wait();
-    const bool ok = mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT);
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
       const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      const uint32_t buf = tiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
+      uint32_t flip = 0;
+      for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
         if (m0 + c0 >= g.M) break;   // warp-uniform
         uint32_t acc[32];
-        __syncwarp();
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
         if (FUSE_LO && x_lo) {
           uint32_t part[32];
@@ -555,19 +614,14 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
         }
-        if (ch < g.N) {
-          if (grp.split > 1) {
-            float *dst = g.raw + ((size_t)blockIdx.z * g.M + m0 + c0) * g.N + ch;
+        if (g.col_scale && grp.split == 1) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (m0 + c0 + i < g.M) dst[(size_t)i * g.N] = __uint_as_float(acc[i]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (m0 + c0 + i < g.M) epi_store_one(g, m0 + c0 + i, ch, __uint_as_float(acc[i]) * sc);
-          }
+          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
         }
+        if (BN == 32 && grp.split > 1) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
+        else tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, tile_n * GBM + quad * 32, m0 + c0, acc, buf + flip);
       }
+      tile_out_end();
     }
   }
   tc_fence_before();
@@ -600,7 +654,6 @@ constexpr int WQ_MAX_W = 8;        // deepest ring of packed weight slots
 constexpr int WQ_EXP_WARPS = 8;
 constexpr int WQ_THREADS = 192 + 32 * WQ_EXP_WARPS;
 
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -611,6 +664,64 @@ __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
 }
+
+// Expansion of packed weights to fp16 pairs.
+// int4: four bytes (8 consecutive inputs) -> hi = fp16(q s), lo = q s - hi (exact); s2 = {s, s}
+__device__ __forceinline__ void expand_int4(uint32_t word, uint32_t s2, uint32_t *hi, uint32_t *lo) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    // byte j -> {1024 + low nibble, 64 + high nibble} - {1032, 72} = {q_even, q_odd}
+    const uint32_t x = prmt(word, 0u, 0x4040u + (uint32_t)j * 0x0101u);   // bytes [b_j, 0, b_j, 0]
+    const uint32_t qv = hsub2_u32(lop3_and_or(x, 0x00f0000fu, 0x54006400u), 0x54806408u);
+    hi[j] = hmul2_u32(qv, s2);
+    lo[j] = hfma2_u32(qv, s2, hi[j] ^ 0x80008000u);
+  }
+}
+// int8: four codes -> their values, exact
+__device__ __forceinline__ void expand_int8(uint32_t word, uint32_t *out) {
+  const uint32_t M = 0x64646464u, OFF = 0x64806480u, w = word ^ 0x80808080u;    // 1024 + (code + 128) - 1152 = code
+  out[0] = hsub2_u32(prmt(w, M, 0x4140), OFF);
+  out[1] = hsub2_u32(prmt(w, M, 0x4342), OFF);
+}
+// The group scales of one row of int4 weights, slice by slice: straight from global memory, 16 bytes (four slices) at a
+// time and four slices ahead of their use, so that the expansion never waits for them; rows whose scales are not 16-byte
+// aligned (K not a multiple of 256) take them slice by slice, one ahead.
+struct GroupScales {
+  const __half *gs;      // null: a row that does not exist
+  bool quads;
+  int nquads, kz0, kend;
+  uint4 scq, scq_next;
+  uint32_t sc_next;
+  __device__ __forceinline__ void start(const GemmArgs &g, int ch, int k0, int nk) {
+    gs = ch < g.N ? g.wq_scale + (size_t)ch * (g.K / 32) : nullptr;
+    quads = ((g.K / 32) & 7) == 0;
+    nquads = g.K / 256;
+    kz0 = k0; kend = k0 + nk;
+    scq = scq_next = make_uint4(0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u);
+    sc_next = 0x3c003c00u;
+    if (!gs || nk <= 0) return;
+    if (quads) {
+      scq = *reinterpret_cast<const uint4 *>(gs + (size_t)(kz0 >> 2) * 8);
+      if ((kz0 >> 2) + 1 < nquads) scq_next = *reinterpret_cast<const uint4 *>(gs + (size_t)((kz0 >> 2) + 1) * 8);
+    } else {
+      sc_next = *reinterpret_cast<const uint32_t *>(gs + (size_t)kz0 * 2);
+    }
+  }
+  __device__ __forceinline__ uint32_t at(int ks) {   // called with ks = kz0, kz0 + 1, ...: scales of the slice's two groups
+    uint32_t sc = sc_next;
+    if (quads) {
+      if (ks > kz0 && (ks & 3) == 0) {
+        scq = scq_next;
+        if (gs && (ks >> 2) + 1 < nquads) scq_next = *reinterpret_cast<const uint4 *>(gs + (size_t)((ks >> 2) + 1) * 8);
+      }
+      const int qi = ks & 3;
+      sc = qi == 0 ? scq.x : qi == 1 ? scq.y : qi == 2 ? scq.z : scq.w;
+    } else if (gs && ks + 1 < kend) {
+      sc_next = *reinterpret_cast<const uint32_t *>(gs + (size_t)(ks + 1) * 2);
+    }
+    return sc;
+  }
+};
 
 // 72 registers: two CTAs share an SM whenever the launcher's shared-memory plan allows it
 template <int BN, int FMT>
@@ -687,23 +798,27 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         tma_load_2d(wtiles + (uint32_t)kw * WS_BYTES, &maps.b[pi], (g0 + kw) * (int)WB, tile_n * GBM, &wfull[kw]);
       }
       pdl_wait();
+      Ring wat, xat;
+      if (kw == NW) wat.phase = 1; else wat.slot = kw;
       while (kw < ng || kx < nkz) {
         bool moved = false;
-        if (kw < ng && mbar_try(&wempty[kw % NW], ((kw / NW) & 1) ^ 1)) {
-          const int s = kw % NW;
+        if (kw < ng && mbar_try(&wempty[wat.slot], wat.phase ^ 1u)) {
+          const int s = wat.slot;
           mbar_expect_tx(&wfull[s], WS_BYTES);
           tma_load_2d(wtiles + (uint32_t)s * WS_BYTES, &maps.b[pi], (g0 + kw) * (int)WB, tile_n * GBM, &wfull[s]);
           ++kw;
+          wat.next(NW);
           moved = true;
         }
-        if (kx < nkz && mbar_try(&a_empty[kx % NE], ((kx / NE) & 1) ^ 1)) {
-          const int e = kx % NE;
+        if (kx < nkz && mbar_try(&a_empty[xat.slot], xat.phase ^ 1u)) {
+          const int e = xat.slot;
           const uint32_t dst = xtiles + (uint32_t)e * XS_BYTES;
           const int kc = (kz0 + kx) * GBK;
           mbar_expect_tx(&xfull[e], (x_lo ? 2u : 1u) * X_BYTES);
           tma_load_2d(dst, &maps.a[pi], kc, m0, &xfull[e]);
           if (x_lo) tma_load_2d(dst + X_BYTES, &maps.a2[pi], kc, m0, &xfull[e]);
           ++kx;
+          xat.next(NE);
           moved = true;
         }
         if (moved) { idle = 0; continue; }
@@ -716,11 +831,11 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      for (int kb = 0; kb < nkz; ++kb) {
-        const int e = kb % NE;
-        const uint32_t par = (uint32_t)(kb / NE) & 1u;
-        if (!mbar_wait(&xfull[e], par, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        if (!mbar_wait(&a_full[e], par, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+      Ring at;
+      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+        const int e = at.slot;
+        if (!mbar_wait(&xfull[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!mbar_wait(&a_full[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         tc_fence_after();
         const uint32_t xb = xtiles + (uint32_t)e * XS_BYTES, eb = etiles + (uint32_t)e * E_BYTES;
         const uint64_t wd = umma_desc_k128(eb), xd = umma_desc_k128(xb);
@@ -750,42 +865,15 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
     const uint32_t swz = (uint32_t)(row & 7);
     const uint32_t wswz = WB == 128u ? swz : 0u;
     const uint32_t erow = (uint32_t)row * 128u;             // byte offset of the row inside an expanded tile
-    // int4: this row's group scales, two per K slice.  They come straight from global memory, 16 bytes (four slices)
-    // at a time and four slices ahead of their use, so that the expansion never waits for them; rows whose scales
-    // are not 16-byte aligned (K not a multiple of 256) take them slice by slice, one ahead.
-    const __half *gs = nullptr;
-    if (FMT == FMT_INT4 && ch < g.N) gs = g.wq_scale + (size_t)ch * (g.K / 32);
-    const bool quads = FMT == FMT_INT4 && ((g.K / 32) & 7) == 0;
-    const int nquads = g.K / 256;
-    uint4 scq = make_uint4(0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u), scq_next = scq;
-    uint32_t sc_next = 0x3c003c00u;
-    if (FMT == FMT_INT4 && gs && nkz > 0) {
-      if (quads) {
-        scq = *reinterpret_cast<const uint4 *>(gs + (size_t)(kz0 >> 2) * 8);
-        if ((kz0 >> 2) + 1 < nquads) scq_next = *reinterpret_cast<const uint4 *>(gs + (size_t)((kz0 >> 2) + 1) * 8);
-      } else {
-        sc_next = *reinterpret_cast<const uint32_t *>(gs + (size_t)kz0 * 2);
-      }
-    }
-    for (int kb = 0; kb < nkz; ++kb) {
-      const int ks = kz0 + kb;
-      const int wj = (ks >> KSH) - g0, sub = ks & (KSUB - 1);
-      const int s = wj % NW, e = kb % NE;
-      uint32_t sc = sc_next;                                // scales of the two 32-input groups of this slice
-      if (FMT == FMT_INT4) {
-        if (quads) {
-          if (kb > 0 && (ks & 3) == 0) {
-            scq = scq_next;
-            if (gs && (ks >> 2) + 1 < nquads) scq_next = *reinterpret_cast<const uint4 *>(gs + (size_t)((ks >> 2) + 1) * 8);
-          }
-          const int qi = ks & 3;
-          sc = qi == 0 ? scq.x : qi == 1 ? scq.y : qi == 2 ? scq.z : scq.w;
-        } else if (gs && kb + 1 < nkz) {
-          sc_next = *reinterpret_cast<const uint32_t *>(gs + (size_t)(ks + 1) * 2);
-        }
-      }
-      if (!mbar_wait(&wfull[s], (uint32_t)(wj / NW) & 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-      if (!mbar_wait(&a_empty[e], ((uint32_t)(kb / NE) & 1u) ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+    GroupScales scales;
+    if (FMT == FMT_INT4) scales.start(g, ch, kz0, nkz);
+    Ring wat, at;
+    for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+      const int ks = kz0 + kb, sub = ks & (KSUB - 1);
+      const int s = wat.slot, e = at.slot;
+      const uint32_t sc = FMT == FMT_INT4 ? scales.at(ks) : 0u;   // the two 32-input groups of this slice
+      if (!mbar_wait(&wfull[s], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+      if (!mbar_wait(&a_empty[e], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
       // 16-byte chunk c of the row's WB bytes is at (c ^ wswz) << 4
       const uint32_t src = wtiles + (uint32_t)s * WS_BYTES + (uint32_t)row * WB;
       const uint32_t c0 = (uint32_t)sub * (ROW_B / 16u);
@@ -797,12 +885,9 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         for (int pp = 0; pp < 2; ++pp) {
           const uint32_t piece = (uint32_t)part * 2u + ((uint32_t)(pp + row) & 1u);
           const uint4 w = lds128(src + (((c0 + piece) ^ wswz) << 4));
-          const uint32_t M = 0x64646464u, OFF = 0x64806480u;    // 1024 + (code + 128) - 1152 = code
-          const uint32_t wx = w.x ^ 0x80808080u, wy = w.y ^ 0x80808080u, wz = w.z ^ 0x80808080u, ww = w.w ^ 0x80808080u;
-          const uint4 o0 = make_uint4(hsub2_u32(prmt(wx, M, 0x4140), OFF), hsub2_u32(prmt(wx, M, 0x4342), OFF),
-                                      hsub2_u32(prmt(wy, M, 0x4140), OFF), hsub2_u32(prmt(wy, M, 0x4342), OFF));
-          const uint4 o1 = make_uint4(hsub2_u32(prmt(wz, M, 0x4140), OFF), hsub2_u32(prmt(wz, M, 0x4342), OFF),
-                                      hsub2_u32(prmt(ww, M, 0x4140), OFF), hsub2_u32(prmt(ww, M, 0x4342), OFF));
+          uint32_t v[8];
+          expand_int8(w.x, v); expand_int8(w.y, v + 2); expand_int8(w.z, v + 4); expand_int8(w.w, v + 6);
+          const uint4 o0 = make_uint4(v[0], v[1], v[2], v[3]), o1 = make_uint4(v[4], v[5], v[6], v[7]);
           sts128(dst + (((piece * 2u) ^ swz) << 4), o0);        // inputs 16 piece .. +7: 16-byte chunk 2 piece
           sts128(dst + (((piece * 2u + 1u) ^ swz) << 4), o1);
         }
@@ -816,14 +901,7 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         for (int wi = 0; wi < 4; ++wi) {
           // 8 nibbles = 8 consecutive inputs -> one 16-byte chunk of hi and one of lo
           uint32_t hi[4], lo[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            // byte j -> {1024 + low nibble, 64 + high nibble} - {1032, 72} = {q_even, q_odd}
-            const uint32_t x = prmt(words[wi], 0u, 0x4040u + (uint32_t)j * 0x0101u);   // bytes [b_j, 0, b_j, 0]
-            const uint32_t qv = hsub2_u32(lop3_and_or(x, 0x00f0000fu, 0x54006400u), 0x54806408u);
-            hi[j] = hmul2_u32(qv, s2);
-            lo[j] = hfma2_u32(qv, s2, hi[j] ^ 0x80008000u);
-          }
+          expand_int4(words[wi], s2, hi, lo);
           const uint32_t chunk = ((uint32_t)part * 4u + (uint32_t)wi) ^ swz;
           sts128(dst + (chunk << 4), make_uint4(hi[0], hi[1], hi[2], hi[3]));
           sts128(dst + G_A_BYTES + (chunk << 4), make_uint4(lo[0], lo[1], lo[2], lo[3]));
@@ -833,21 +911,23 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&a_full[e]);
-        if (sub == KSUB - 1 || kb == nkz - 1) mbar_arrive(&wempty[s]);   // last slice of the slot this CTA uses
+        if (sub == KSUB - 1) mbar_arrive(&wempty[s]);   // (the last slot of this K range is not asked for again)
       }
+      if (sub == KSUB - 1) wat.next(NW);
     }
   } else {
     const int quad = warp & 3;
     const int ch = tile_n * GBM + quad * 32 + lane;
     pdl_wait();
-    const bool ok = mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT);
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
       const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      const uint32_t buf = etiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
+      uint32_t flip = 0;
+      for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
         if (m0 + c0 >= g.M) break;   // warp-uniform
         uint32_t acc[32];
-        __syncwarp();
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
         if (FUSE_LO && x_lo) {
           uint32_t part[32];
@@ -855,19 +935,14 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
         }
-        if (ch < g.N) {
-          if (grp.split > 1) {
-            float *dst = g.raw + ((size_t)blockIdx.z * g.M + m0 + c0) * g.N + ch;
+        if (g.col_scale && grp.split == 1) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (m0 + c0 + i < g.M) dst[(size_t)i * g.N] = __uint_as_float(acc[i]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (m0 + c0 + i < g.M) epi_store_one(g, m0 + c0 + i, ch, __uint_as_float(acc[i]) * sc);
-          }
+          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
         }
+        if (BN == 32 && grp.split > 1) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
+        else tile_out_lean(g, &maps.o[pi], grp.split > 1, blockIdx.z, tile_n * GBM + quad * 32, m0 + c0, acc, buf + flip);
       }
+      tile_out_end();
     }
   }
   tc_fence_before();
@@ -875,6 +950,230 @@ gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Quantised weights, more than 128 rows: the pair product of gemm_pair_kernel with the weight operand in TMEM.  Eight warps
+// expand a slice of the packed codes straight into the MMA's A operand (TMEM lane = channel, a column = two inputs), so
+// shared memory carries X alone.  Expanded into shared memory instead (one CTA, 128 x 256), a slice of int4 asked it for 163 bytes a
+// clock where it gives 128, with room for two slices only.
+//   warp 0      TMA: this CTA's half of X into slot e, counted on the even CTA's barrier
+//   warp 1      TMEM; in the even CTA the MMAs: acc += W_hi X_hi, W_hi X_lo, and for int4 W_lo X_hi (int8 codes are exact in fp16)
+//   warps 6..13 expanders: warp quadrant = TMEM lane quadrant, two warps share a row's 64 inputs (one scale group each)
+//   warp 14     TMA: packed weights, 128 rows x 128 bytes = 4 (int4) or 2 (int8) slices per slot
+//   warps 2..13 epilogue, three warps per quadrant
+// One commit per slice frees X slot e and A slot e in both CTAs.  The weights do not depend on the kernels before this one.
+__device__ __forceinline__ void umma_f16_pair_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+// arrive on a barrier of either CTA of the cluster (address from mapa_u32)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+constexpr int PQ_THREADS = 32 * 15;
+constexpr int PQ_MAX = 8;                // most slots of any ring
+constexpr uint32_t PQ_ACC_COLS = 256;    // TMEM: accumulator in columns [0, 256), A slots in [256, 512)
+
+template <int FMT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PQ_THREADS, 1)
+gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
+  constexpr uint32_t ROW_B = FMT == FMT_INT8 ? GBK : GBK / 2;          // packed bytes per row and slice
+  constexpr int KSH = FMT == FMT_INT8 ? 1 : 2, KSUB = 1 << KSH;        // slices per weight slot
+  constexpr uint32_t WS_BYTES = GBM * 128;
+  constexpr uint32_t A_COLS = FMT == FMT_INT4 ? 64 : 32;               // expanded slice: hi (+ lo)
+  const int NW = grp.stages, NE = grp.estages, BN = grp.bn;
+  const uint32_t X_BYTES = (uint32_t)BN * (GBK * 2 / 2), XS_BYTES = grp.stage_bytes;
+  const uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * GBM >> 4) << 24);
+  extern __shared__ uint8_t gsm_raw[];
+  uint8_t *gsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t *wfull = reinterpret_cast<uint64_t *>(gsm);
+  uint64_t *wempty = wfull + PQ_MAX;
+  uint64_t *xfull = wempty + PQ_MAX;
+  uint64_t *a_full = xfull + PQ_MAX;
+  uint64_t *a_peer = a_full + PQ_MAX;       // (even CTA) the other CTA's expanded slice
+  uint64_t *empty = a_peer + PQ_MAX;
+  uint64_t *acc_full = empty + PQ_MAX;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const uint32_t xtiles = smem_u32(gsm + 1024), wtiles = xtiles + (uint32_t)NE * XS_BYTES;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int pair = blockIdx.x >> 1, ct = pair / grp.m_tiles, m0 = (pair - ct * grp.m_tiles) * BN;
+  int pi = 0;
+  while (pi + 1 < grp.n && ct >= grp.tile_start[pi + 1]) ++pi;
+  const GemmArgs &g = grp.p[pi];
+  const int ch0 = (ct - grp.tile_start[pi]) * (2 * GBM) + (int)rank * GBM;
+  const int num_k1 = g.K / GBK;
+  const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
+  const bool x_lo = g.A2 != nullptr;
+  const int g0 = kz0 >> KSH, ng = nkz > 0 ? ((kz0 + nkz - 1) >> KSH) - g0 + 1 : 0;   // weight slots of this K range
+
+  if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (x_lo) prefetch_tmap(&maps.a2[pi]); }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 8); }
+    for (int e = 0; e < NE; ++e) { mbar_init(&xfull[e], 1); mbar_init(&a_full[e], 8); mbar_init(&a_peer[e], 1); mbar_init(&empty[e], 1); }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // the barriers of both CTAs exist before anything arrives on them from the other one
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      pdl_wait();
+      Ring at;
+      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+        const int e = at.slot;
+        if (!mbar_wait(&empty[e], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        const uint32_t dst = xtiles + (uint32_t)e * XS_BYTES, bar = mapa_u32(smem_u32(&xfull[e]), 0);
+        const int kx = (kz0 + kb) * GBK, row = m0 + (int)rank * (BN / 2);
+        if (rank == 0) mbar_expect_tx(&xfull[e], (x_lo ? 4u : 2u) * X_BYTES);   // of both CTAs
+        tma_load_2d_pair(dst, &maps.a[pi], kx, row, bar);
+        if (x_lo) tma_load_2d_pair(dst + X_BYTES, &maps.a2[pi], kx, row, bar);
+      }
+    }
+  } else if (warp == 14) {
+    if (lane == 0) {
+      Ring at;
+      for (int kw = 0; kw < ng; ++kw, at.next(NW)) {
+        const int s = at.slot;
+        if (!mbar_wait(&wempty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        mbar_expect_tx(&wfull[s], WS_BYTES);
+        tma_load_2d(wtiles + (uint32_t)s * WS_BYTES, &maps.b[pi], (g0 + kw) * 128, ch0, &wfull[s]);
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {
+      Ring at;
+      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+        const int e = at.slot;
+        if (!mbar_wait(&a_full[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!mbar_wait(&a_peer[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!mbar_wait(&xfull[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        tc_fence_after();
+        const uint32_t xb = xtiles + (uint32_t)e * XS_BYTES, ta = tmem_base + PQ_ACC_COLS + (uint32_t)e * A_COLS;
+        const uint64_t xd = umma_desc_k128(xb), xl = umma_desc_k128(xb + X_BYTES);
+#pragma unroll
+        for (int k4 = 0; k4 < GBK / 16; ++k4)       // 16 inputs = 8 columns of A
+          umma_f16_pair_ta(tmem_base, ta + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, (kb | k4) != 0);
+        if (x_lo) {
+#pragma unroll
+          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair_ta(tmem_base, ta + (uint32_t)k4 * 8, xl + (uint64_t)(k4 * 2), IDESC, 1u);
+        }
+        if (FMT == FMT_INT4) {
+#pragma unroll
+          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair_ta(tmem_base, ta + 32u + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, 1u);
+        }
+        umma_commit_pair(&empty[e]);
+      }
+      umma_commit_pair(acc_full);
+    } else if (rank == 1 && lane == 0) {
+      // A release across the cluster takes 500 to 900 clocks: this thread, which has no MMAs to issue, passes the slices of
+      // its CTA's expanders on.
+      Ring at;
+      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+        if (!mbar_wait(&a_full[at.slot], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        tc_fence_after();
+        tc_fence_before();
+        mbar_arrive_cluster(mapa_u32(smem_u32(&a_peer[at.slot]), 0));
+      }
+    }
+  } else if (warp >= 6) {
+    const int quad = warp & 3, part = (warp - 6) >> 2;
+    const int row = quad * 32 + lane;
+    const uint32_t swz = (uint32_t)(row & 7);
+    GroupScales scales;
+    if (FMT == FMT_INT4) scales.start(g, ch0 + row, kz0, nkz);
+    const uint32_t ta = tmem_base + ((uint32_t)(quad * 32) << 16) + PQ_ACC_COLS + (uint32_t)part * 16;
+    Ring wat, at;
+    for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+      const int ks = kz0 + kb, sub = ks & (KSUB - 1);
+      const int s = wat.slot, e = at.slot;
+      uint32_t s2 = 0;
+      if (FMT == FMT_INT4) {
+        const uint32_t sc = scales.at(ks), s16 = part ? (sc >> 16) : (sc & 0xffffu);
+        s2 = s16 | (s16 << 16);
+      }
+      if (!__all_sync(0xffffffffu, mbar_wait(&wfull[s], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+      // 16-byte chunk c of the row's 128 bytes is at (c ^ swz) << 4
+      const uint32_t src = wtiles + (uint32_t)s * WS_BYTES + (uint32_t)row * 128u, c0 = (uint32_t)sub * (ROW_B / 16u);
+      uint32_t hi[16], lo[16];
+      if (FMT == FMT_INT4) {
+        const uint4 w = lds128(src + (((c0 + (uint32_t)part) ^ swz) << 4));
+        expand_int4(w.x, s2, hi, lo); expand_int4(w.y, s2, hi + 4, lo + 4);
+        expand_int4(w.z, s2, hi + 8, lo + 8); expand_int4(w.w, s2, hi + 12, lo + 12);
+      } else {
+#pragma unroll
+        for (int pp = 0; pp < 2; ++pp) {
+          const uint4 w = lds128(src + (((c0 + (uint32_t)(part * 2 + pp)) ^ swz) << 4));
+          expand_int8(w.x, hi + pp * 8); expand_int8(w.y, hi + pp * 8 + 2);
+          expand_int8(w.z, hi + pp * 8 + 4); expand_int8(w.w, hi + pp * 8 + 6);
+        }
+      }
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty[e], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+      tc_fence_after();
+      tmem_st16(ta + (uint32_t)e * A_COLS, hi);
+      if (FMT == FMT_INT4) tmem_st16(ta + (uint32_t)e * A_COLS + 32u, lo);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&a_full[e]);
+        if (sub == KSUB - 1) mbar_arrive(&wempty[s]);   // (the last slot of this K range is not asked for again)
+      }
+      if (sub == KSUB - 1) wat.next(NW);
+    }
+  }
+  if (warp >= 2 && warp < 14) {
+    const int quad = warp & 3;
+    const int ch = ch0 + quad * 32 + lane;
+    pdl_wait();
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
+    tc_fence_after();
+    if (ok) {
+      const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
+      const uint32_t buf = xtiles + (uint32_t)(warp - 2) * 2 * EPI_BUF;   // the rings have been read
+      uint32_t flip = 0;
+      for (int c0 = ((warp - 2) >> 2) * 32; c0 < BN; c0 += 96, flip ^= EPI_BUF) {
+        if (m0 + c0 >= g.M) break;   // warp-uniform
+        uint32_t acc[32];
+        tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
+        if (g.col_scale && grp.split == 1) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
+        }
+        tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
+      }
+      tile_out_end();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // neither CTA leaves while the other's MMAs or commits may still reach into it
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }
 
@@ -969,6 +1268,40 @@ bool make_map_bytes(CUtensorMap *map, const void *base, int rows, int row_bytes,
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// [planes, rows, cols] of fp16 or fp32 with rows `ld` elements and planes rows x ld elements apart -> tensor map with a
+// (32 cols x 32 rows) box
+bool make_map_out(CUtensorMap *map, void *base, bool f32, int cols, int rows, int planes, int ld) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const size_t elt = f32 ? 4 : 2;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)planes};
+  const cuuint64_t strides[2] = {(cuuint64_t)ld * elt, (cuuint64_t)ld * elt * rows};
+  const cuuint32_t box[3] = {32, 32, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// where a group's results go: slabs when K is split, else the outputs, as tensors when their rows allow it
+bool make_out_maps(GemmMaps &maps, GemmGroup &grp) {
+  for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
+    if (i >= grp.n) { maps.o[i] = maps.o[0]; maps.o_lo[i] = maps.o_lo[0]; continue; }
+    GemmArgs &g = grp.p[i];
+    g.tma_out = 0;
+    maps.o[i] = maps.o_lo[i] = maps.a[0];
+    if (grp.split > 1) {
+      if (!make_map_out(&maps.o[i], g.raw, true, g.N, g.M, grp.split, g.N)) return false;
+      continue;
+    }
+    const bool f32 = g.epi == GEMM_EPI_F32 || g.epi == GEMM_EPI_ADD_F32 || g.epi == GEMM_EPI_MULADD_F32;
+    if (((size_t)g.ldo * (f32 ? 4 : 2)) % 16 || (reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.out_lo)) % 16) continue;
+    g.tma_out = 1;
+    if (!make_map_out(&maps.o[i], g.out, f32, g.N, g.M, 1, g.ldo)) return false;
+    if (!f32 && g.out_lo && !make_map_out(&maps.o_lo[i], g.out_lo, false, g.N, g.M, 1, g.ldo)) return false;
+  }
+  return true;
 }
 
 }  // namespace
@@ -1858,21 +2191,18 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   for (int i = 0; i < n; ++i) {
     const GemmArgs &g = probs[i];
     if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15) ||
-        (reinterpret_cast<uintptr_t>(g.Bt2) & 15))
+    if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
       return cudaErrorInvalidValue;
     if (!make_map(&maps.a[i], g.A, g.M, g.K, bn) || !make_map(&maps.b[i], g.Bt, g.N, g.K, GBM)) return cudaErrorNotSupported;
     if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, bn)) return cudaErrorNotSupported;
-    if (!make_map(&maps.b2[i], g.Bt2 ? g.Bt2 : g.Bt, g.N, g.K, GBM)) return cudaErrorNotSupported;
     grp.p[i] = g;
     grp.tile_start[i] = tiles;
     tiles += (g.N + GBM - 1) / GBM;
     min_k1 = std::min(min_k1, g.K / GBK);
     raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
-    if (g.A2) grp.dual |= 1;
-    if (g.Bt2) grp.dual |= 2;
+    if (g.A2) grp.dual = 1;
   }
-  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; maps.b2[i] = maps.b2[0]; }
+  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; }
   grp.tile_start[n] = tiles;
   const int m_tiles = (M + bn - 1) / bn;
   // one CTA per SM, none waiting for a second wave: split K until the tiles about cover the SMs
@@ -1882,12 +2212,13 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   const int sms = device_sm_count();
   const int slots = bn <= 64 ? 2 * sms : sms;
   if (raw_ok) grp.split = split_of(tiles * m_tiles, slots, min_k1);
-  grp.stage_bytes = ((grp.dual & 2) ? 2u : 1u) * G_A_BYTES + ((grp.dual & 1) ? 2u : 1u) * (uint32_t)bn * GBK * 2;
+  grp.stage_bytes = G_A_BYTES + (grp.dual ? 2u : 1u) * (uint32_t)bn * GBK * 2;
   // two CTAs per SM with rings of >= 3 slots where they fit (shorter tail when there are more tiles than SMs),
   // else one CTA with as deep a ring as fits
   int stages = (int)((100u << 10) / grp.stage_bytes);
   if (stages < 3) stages = (int)((200u << 10) / grp.stage_bytes);
   grp.stages = std::max(2, std::min(stages, WT_MAX_STAGES));
+  if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
   dim3 grid(tiles, m_tiles, grp.split);
   cudaError_t e = bn == 32    ? launch_gemm_wt_t<32>(maps, grp, grid, smem, st)
@@ -1927,11 +2258,11 @@ WqPlan wq_plan(long long avail, long long buf_bytes, uint32_t wbox, int want_ne,
   return p;
 }
 
-// quantised weights in packed form (GemmArgs::Wq): any number of rows, walked in tiles of up to 256 along grid.y
+// quantised weights in packed form (GemmArgs::Wq): up to 128 rows
 cudaError_t launch_gemm_wq(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
   const int M = probs[0].M, fmt = probs[0].wfmt;
   if (fmt != FMT_INT8 && fmt != FMT_INT4) return cudaErrorInvalidValue;
-  const int bn = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  const int bn = M <= 32 ? 32 : M <= 64 ? 64 : 128;
   GemmMaps maps;
   GemmGroup grp;
   memset(&grp, 0, sizeof(grp));
@@ -1975,19 +2306,19 @@ cudaError_t launch_gemm_wq(const GemmArgs *probs, int n, cudaStream_t st, int *d
     if (!make_map(&maps.a[i], g.A, g.M, g.K, bn) || !make_map_bytes(&maps.b[i], g.Wq, g.N, row_bytes, (int)pl.wbox))
       return cudaErrorNotSupported;
     if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, bn)) return cudaErrorNotSupported;
-    maps.b2[i] = maps.b[i];
   }
-  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; maps.b2[i] = maps.b2[0]; }
+  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; }
   const int slots = (two_per_sm ? 2 : 1) * device_sm_count();
   if (raw_ok) grp.split = split_of(tiles * m_tiles, slots, min_k1);
   grp.stages = pl.nw;
   grp.estages = pl.ne;
   grp.wbox = pl.wbox;
+  if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)pl.ne * buf_bytes + (size_t)pl.nw * GBM * pl.wbox + 1024;
   dim3 grid(tiles, m_tiles, grp.split);
   cudaError_t e = cudaErrorInvalidValue;
 #define FRB_WQ(BNV) (fmt == FMT_INT8 ? launch_gemm_wq_t<BNV, FMT_INT8>(maps, grp, grid, smem, st) : launch_gemm_wq_t<BNV, FMT_INT4>(maps, grp, grid, smem, st))
-  e = bn == 32 ? FRB_WQ(32) : bn == 64 ? FRB_WQ(64) : bn == 128 ? FRB_WQ(128) : FRB_WQ(256);
+  e = bn == 32 ? FRB_WQ(32) : bn == 64 ? FRB_WQ(64) : FRB_WQ(128);
 #undef FRB_WQ
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
@@ -1999,6 +2330,21 @@ cudaError_t launch_gemm_wq(const GemmArgs *probs, int n, cudaStream_t st, int *d
   return cudaGetLastError();
 }
 
+// Costs in clocks, fitted to products of 256 and 1000 rows (2048 x 2048 up to 65536 x 2048 and 2048 x 8192) with 64 to 256 columns
+// and 1 to 9 cuts, within 10 % of the times.
+// Slabs: the next kernel reads them at about 2,500 bytes a clock; without one that does, a finishing pass is launched.
+float slab_cost(int split, int M, int sum_n, bool deferred) {
+  return split > 1 ? (deferred ? 0.f : 8000.f) + (float)split * (float)M * (float)sum_n * 4.f / 2500.f : 0.f;
+}
+// `tiles` pair tiles of nk slices: rounds of two CTAs per SM, the last one alone on its SMs where it is at most half full
+float pair_cost(int tiles, int nk, int bn, float passes, int num_pairs) {
+  const float start_end = 11000.f + 16.f * (float)bn;
+  const float shared = 2.f * (float)nk * std::max(2.3f * passes * (float)bn, 256.f + passes * (float)bn) + start_end;
+  const float alone = (float)nk * std::max(2.05f * passes * (float)bn, 420.f + 150.f * passes) + start_end;
+  const int rounds = tiles / (2 * num_pairs), rest = tiles - rounds * 2 * num_pairs;
+  return (float)rounds * shared + (rest > num_pairs ? shared : rest > 0 ? alone : 0.f);
+}
+
 // more than 128 rows of X, fp16 weights: gemm_pair_kernel
 cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
   const int M = probs[0].M, num_pairs = device_sm_count() / 2;
@@ -2007,10 +2353,11 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   memset(&grp, 0, sizeof(grp));
   grp.n = n;
   int tiles = 0, tiles128 = 0, units = 0, min_k1 = 1 << 30, sum_n = 0;
-  bool raw_ok = M <= GEMM_SMALL_M;
+  bool raw_ok = M <= GEMM_SMALL_M, any_lo = false;
   for (int i = 0; i < n; ++i) {
     const GemmArgs &g = probs[i];
-    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M || g.Bt2 || g.col_scale) return cudaErrorInvalidValue;
+    any_lo = any_lo || g.A2;
+    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M || g.col_scale) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
       return cudaErrorInvalidValue;
     grp.p[i] = g;
@@ -2031,15 +2378,11 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   grp.split = 1;
   grp.bn = 256;
   float best = 0.f;
+  const float passes = (float)units / (float)tiles;
   for (int rt = (M + 255) / 256; rt <= (M + 127) / 128; ++rt) {
     const int bn = ((M + rt - 1) / rt + 31) / 32 * 32;
     for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
-      // in clocks: a slice takes a pair 256 + bn (shared memory: 32 KB of weights and 64 bn bytes of X in, the same out
-      // to the MMAs, at 128 bytes a clock and SM), a wave of tiles about 8 slices more to start and to end, and the slabs are
-      // written and read at about 2,700 bytes a clock
-      const int waves = (units * rt * sp + num_pairs - 1) / num_pairs;
-      float cost = (float)waves * (float)((min_k1 + sp - 1) / sp + 8) * (float)(256 + bn);
-      if (sp > 1) cost += 3000.f + (float)sp * (float)M * (float)sum_n * 8.f / 2700.f;
+      const float cost = pair_cost(tiles * rt * sp, (min_k1 + sp - 1) / sp, bn, passes, num_pairs) + slab_cost(sp, M, sum_n, defer_split != nullptr);
       if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
     }
   }
@@ -2049,14 +2392,86 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
     const GemmArgs &g = probs[i < n ? i : 0];
     if (!make_map(&maps.a[i], g.A, g.M, g.K, grp.bn / 2) || !make_map(&maps.b[i], g.Bt, g.N, g.K, GBM)) return cudaErrorNotSupported;
     if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, grp.bn / 2)) return cudaErrorNotSupported;
-    maps.b2[i] = maps.b[i];
   }
-  grp.stage_bytes = G_A_BYTES + (uint32_t)grp.bn * GBK;
-  grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((110u << 10) / grp.stage_bytes));
+  grp.stage_bytes = G_A_BYTES + (grp.lo_each && any_lo ? 2u : 1u) * (uint32_t)grp.bn * GBK;
+  // tiles that have an SM each to themselves take a ring of twice the depth
+  const bool alone = tiles * grp.m_tiles * grp.split <= num_pairs;
+  grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((alone ? 200u << 10 : 110u << 10) / grp.stage_bytes));
+  if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
   cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if ((e = launch_k(gemm_pair_kernel, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
+  if (defer_split) *defer_split = grp.split;
+  if (grp.split > 1 && !defer_split) {
+    int max_n = 0;
+    for (int i = 0; i < n; ++i) max_n = std::max(max_n, probs[i].N);
+    launch_k(gemm_finish_kernel, dim3((M * (max_n / 4) + 255) / 256, n), dim3(256), 0, st, grp);
+  }
+  return cudaGetLastError();
+}
+
+// quantised weights in packed form, more than 128 rows: gemm_pair_wq_kernel
+cudaError_t launch_gemm_pair_wq(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
+  const int M = probs[0].M, fmt = probs[0].wfmt, num_pairs = device_sm_count() / 2;
+  if (fmt != FMT_INT8 && fmt != FMT_INT4) return cudaErrorInvalidValue;
+  GemmMaps maps;
+  GemmGroup grp;
+  memset(&grp, 0, sizeof(grp));
+  grp.n = n;
+  int tiles = 0, tiles128 = 0, units = 0, min_k1 = 1 << 30, sum_n = 0;
+  bool raw_ok = M <= GEMM_SMALL_M, any_lo = false;
+  for (int i = 0; i < n; ++i) {
+    const GemmArgs &g = probs[i];
+    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M || !g.Wq || g.wfmt != fmt) return cudaErrorInvalidValue;
+    if (fmt == FMT_INT4 && !g.wq_scale) return cudaErrorInvalidValue;
+    if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Wq) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
+      return cudaErrorInvalidValue;
+    grp.p[i] = g;
+    grp.tile_start[i] = tiles;
+    const int t = (g.N + 2 * GBM - 1) / (2 * GBM), passes = (fmt == FMT_INT4 ? 2 : 1) + (g.A2 ? 1 : 0);
+    tiles += t;
+    tiles128 += (g.N + GBM - 1) / GBM;
+    units += t * passes;
+    sum_n += g.N;
+    min_k1 = std::min(min_k1, g.K / GBK);
+    raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
+    any_lo = any_lo || g.A2;
+  }
+  grp.tile_start[n] = tiles;
+  const int fixed = raw_ok && probs[0].fixed_split ? keep_split(tiles128 * ((M + 255) / 256), min_k1) : 0;   // (as in launch_gemm_pair)
+  const int max_split = raw_ok ? std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 2)) : 1;
+  grp.split = 1;
+  grp.bn = 256;
+  float best = 0.f;
+  const float passes = (float)units / (float)tiles;
+  for (int rt = (M + 255) / 256; rt <= (M + 127) / 128; ++rt) {
+    const int bn = ((M + rt - 1) / rt + 31) / 32 * 32;
+    for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
+      // in clocks: a slice is bound by its MMAs or by its expansion, a wave starts and ends
+      const int waves = (tiles * rt * sp + num_pairs - 1) / num_pairs;
+      const float cost = (float)waves * ((float)((min_k1 + sp - 1) / sp) * std::max(2.05f * (float)bn * passes, 1180.f) + 11000.f + 14.f * (float)bn) +
+                         slab_cost(sp, M, sum_n, defer_split != nullptr);
+      if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
+    }
+  }
+  grp.m_tiles = (M + grp.bn - 1) / grp.bn;
+  for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
+    const GemmArgs &g = probs[i < n ? i : 0];
+    const int row_bytes = fmt == FMT_INT8 ? g.K : g.K / 2;
+    if (!make_map(&maps.a[i], g.A, g.M, g.K, grp.bn / 2) || !make_map_bytes(&maps.b[i], g.Wq, g.N, row_bytes, 128)) return cudaErrorNotSupported;
+    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, grp.bn / 2)) return cudaErrorNotSupported;
+  }
+  grp.stage_bytes = (any_lo ? 2u : 1u) * (uint32_t)grp.bn * GBK;
+  grp.stages = 4;
+  grp.estages = std::min<int>(fmt == FMT_INT4 ? 4 : 8, (int)(((220u << 10) - 4u * GBM * 128) / grp.stage_bytes));
+  if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
+  const size_t rings = (size_t)grp.estages * grp.stage_bytes + (size_t)grp.stages * GBM * 128;
+  const size_t smem = 1024 + std::max<size_t>(rings, 12 * 2 * EPI_BUF) + 1024;
+  auto kern = fmt == FMT_INT4 ? gemm_pair_wq_kernel<FMT_INT4> : gemm_pair_wq_kernel<FMT_INT8>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if ((e = launch_k(kern, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(PQ_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
     int max_n = 0;
@@ -2073,7 +2488,7 @@ cudaError_t launch_gemm_group(const GemmArgs *probs, int n, int mt, cudaStream_t
   if (n < 1 || n > GEMM_GROUP_MAX || (mt != 1 && mt != 2)) return cudaErrorInvalidValue;
   const int M = probs[0].M;
   if (defer_split) *defer_split = 1;
-  if (probs[0].Wq) return launch_gemm_wq(probs, n, st, defer_split);
+  if (probs[0].Wq) return M <= 128 ? launch_gemm_wq(probs, n, st, defer_split) : launch_gemm_pair_wq(probs, n, st, defer_split);
   return M <= 128 ? launch_gemm_wt(probs, n, st, defer_split) : launch_gemm_pair(probs, n, st, defer_split);
 }
 

@@ -45,6 +45,22 @@ def test_many_streams_match_oracle(pkg, orc, synth, name, fmt, B):
     m.close()
 
 
+@pytest.mark.parametrize("name,fmt,B", [("tiny4b", "int4", 129), ("tiny4b", "int8", 161), ("tiny4b", "fp16", 129), ("mid4", "int8", 257),
+                                        ("tiny52", "int4", 193), ("wide4", "int4", 256), ("wide4", "int8", 1030)])
+def test_streams_over_pair_tiles(pkg, orc, synth, name, fmt, B):
+    """More than 128 streams run on pairs of SMs: row tiles of 96 to 256 rows whose last one is ragged, 3 to 7 slices of K
+    (scales taken slice by slice and four at a time, weight slots that are not full), channel tiles whose second half is
+    partly or wholly outside, K cut in several pieces and, above 1024 rows, in one.  First, last and tile-edge streams."""
+    shape, m, ref = _pair(pkg, orc, synth, name, fmt, B)
+    ids = synth.token_ids(shape, 2 * B, seed=31).reshape(2, B)
+    got = [m.decode(ids[t]) for t in range(2)]
+    for b in sorted({0, 31, 95, 127, 128, B // 2, B - 1}):
+        ref.reset()
+        for t in range(2):
+            _close(got[t][b], ref.run(int(ids[t, b])), f"{name} {fmt} stream {b} of {B} step {t}")
+    m.close()
+
+
 @pytest.mark.parametrize("fmt", ["fp16", "int4"])
 def test_eight_streams_of_a_wide_model_take_the_gemm_path(pkg, orc, synth, fmt):
     """A model whose channel-mix width does not leave room for 8 streams in the persistent kernel's shared memory
