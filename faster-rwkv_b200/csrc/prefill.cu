@@ -44,16 +44,29 @@ bool pdl_enabled() {
   return on != 0;
 }
 template <typename... KArgs, typename... Args>
-cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+cudaError_t launch_cluster_k(void (*kern)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = (unsigned)cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (pdl_enabled()) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+  return launch_cluster_k(kern, 1, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -112,6 +125,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // Place in a ring of barriers.  Its slot and phase are counted: a division by a depth that only the launch knows costs 100
 // to 200 clocks of a chain that takes 300 to 1,000 per slice, and every role had two to four of them.
 struct Ring {
@@ -143,8 +166,8 @@ __device__ __forceinline__ float epi_half_op(int epi, float a) {
 struct GemmGroup {
   int n;
   int stages;                           // ring depth; packed-weight GEMM: weight slots
-  int estages;                          // packed-weight GEMM: buffers (expanded weights + X; stage_bytes = the X part)
-  uint32_t wbox;                        // packed-weight GEMM: bytes per row of a weight slot (64 or 128)
+  int estages, xstages;                 // packed-weight GEMM: expanded slices in TMEM, slots of X (stage_bytes each)
+  uint32_t acc_cols, tmem_cols;         // packed-weight GEMM: TMEM columns of the accumulator, and in all
   uint32_t stage_bytes;                 // bytes per ring slot
   int split;                            // split-K factor (grid.z); > 1: CTAs write raw partial sums to GemmArgs::raw
   int dual;                             // few-row GEMM: some problem has A2 (the slot holds an X lo tile)
@@ -269,48 +292,6 @@ __device__ __forceinline__ void slab_rows(const GemmArgs &g, int z, int ch, int 
   for (int i = 0; i < 32; ++i)
     if (row0 + i < g.M) dst[(size_t)i * g.N] = __uint_as_float(acc[i]);
 }
-// The same with few registers (72 in gemm_wq_kernel): all kinds of results that are not fp32 as they stand go back through
-// shared memory row by row.
-__device__ __forceinline__ void tile_out_lean(const GemmArgs &g, const CUtensorMap *om, bool raw, int z, int ch_w, int row0,
-                                              const uint32_t (&acc)[32], uint32_t buf) {
-  const int lane = threadIdx.x & 31, ch = ch_w + lane;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) sts_u32(buf + i * 128 + lane * 4, acc[i]);
-  if (raw || (g.tma_out && g.epi == GEMM_EPI_F32)) {
-    fence_proxy_async();
-    __syncwarp();
-    if (lane == 0) {
-      if (ch_w < g.N) tma_store_3d(om, buf, ch_w, row0, raw ? z : 0);
-      asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group.read 1;" ::: "memory");
-    }
-    __syncwarp();
-    return;
-  }
-  if (ch < g.N) {
-    const int nr = min(32, g.M - row0);
-    size_t o = (size_t)row0 * g.ldo + ch;
-#pragma unroll 8
-    for (int i = 0; i < nr; ++i, o += g.ldo) {
-      float e = lds_f32(buf + i * 128 + lane * 4);
-      if (g.epi == GEMM_EPI_F32) {
-        reinterpret_cast<float *>(g.out)[o] = e;
-      } else if (g.epi == GEMM_EPI_ADD_F32) {
-        reinterpret_cast<float *>(g.out)[o] = (reinterpret_cast<const float *>(g.aux0)[o] + e) * g.scale;
-      } else if (g.epi == GEMM_EPI_MULADD_F32) {
-        float r = __half2float(reinterpret_cast<const __half *>(g.aux1)[o]);
-        if (g.aux1_lo) r += __half2float(reinterpret_cast<const __half *>(g.aux1_lo)[o]);
-        reinterpret_cast<float *>(g.out)[o] = (reinterpret_cast<const float *>(g.aux0)[o] + r * e) * g.scale;
-      } else {
-        e = g.epi == GEMM_EPI_SILU_F16 ? epi_half_op<GEMM_EPI_SILU_F16>(e) : g.epi == GEMM_EPI_SIGMOID_F16 ? epi_half_op<GEMM_EPI_SIGMOID_F16>(e)
-            : g.epi == GEMM_EPI_RELU2_F16 ? epi_half_op<GEMM_EPI_RELU2_F16>(e) : e;
-        const __half h = __float2half_rn(e);
-        reinterpret_cast<__half *>(g.out)[o] = h;
-        if (g.out_lo) reinterpret_cast<__half *>(g.out_lo)[o] = __float2half_rn(e - __half2float(h));
-      }
-    }
-  }
-  __syncwarp();   // (the buffer is filled again two turns on)
-}
 // before the CTA may end: its stores have read shared memory
 __device__ __forceinline__ void tile_out_end() {
   if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -366,7 +347,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 constexpr int PAIR_MAX_STAGES = 8;
 constexpr uint32_t PAIR_TMEM_COLS = 256;
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 2)
+__global__ void __launch_bounds__(G_THREADS, 2)
 gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   const int STAGES = grp.stages, BN = grp.bn;
   const uint32_t X_BYTES = (uint32_t)BN * (GBK * 2 / 2);          // this CTA's half of the X tile
@@ -632,28 +613,6 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   }
 }
 
-// ------------------------------------------------------------------------------------------------
-// The few-row GEMM for quantised weights: the weight operand is read in its packed form (int8 codes [N, K], or int4
-// nibbles [N, K/2] with fp16 group scales [N, K/32]: the bytes a step has to stream) and expanded to the K-major fp16
-// tile the tensor core wants inside the kernel, by eight warps that do nothing else.  Per K slice of 64 inputs:
-//   warp 0      TMA: packed weights into a ring of slots of their own (128 rows x 32..128 bytes = 1, 2 or 4 slices
-//               per slot) and the X tile(s) into buffer kb % NE
-//   warps 6..13 expanders (two threads per row): packed slice -> 128 x 64 fp16 in the 128-byte-swizzled layout of a
-//               TMA-loaded tile, expanded buffer kb % NE
-//               (int8: the integer code, exact in fp16, the row scale is applied to the accumulator;
-//                int4: hi = fp16(q * scale) and lo = q * scale - hi, an exact pair)
-//   warp 1      MMA: acc += W_hi [X_hi | X_lo] (+ W_lo X_hi)
-//   warps 2..5  epilogue, as in gemm_wt_kernel
-// Buffer e (its X slot and its expanded weights) is free again when the MMAs that read it have retired: one commit
-// per slice.  A weight slot is free when the expanders have read its last slice.  Shared-memory writes of the
-// expanders are made visible to the tensor core's (asynchronous) reads with fence.proxy.async before the barrier
-// arrive.  The weights are constants, so their loads and their expansion do not wait for the kernels before this
-// one: under programmatic dependent launch the first slices are ready when X arrives.
-constexpr int WQ_MAX_E = 4;        // most buffers (expanded weights + X)
-constexpr int WQ_MAX_W = 8;        // deepest ring of packed weight slots
-constexpr int WQ_EXP_WARPS = 8;
-constexpr int WQ_THREADS = 192 + 32 * WQ_EXP_WARPS;
-
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -723,252 +682,34 @@ struct GroupScales {
   }
 };
 
-// 72 registers: two CTAs share an SM whenever the launcher's shared-memory plan allows it
-template <int BN, int FMT>
-__global__ void __launch_bounds__(WQ_THREADS, 2)
-gemm_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
-  constexpr uint32_t X_BYTES = BN * GBK * 2;
-  constexpr uint32_t ROW_B = FMT == FMT_INT8 ? GBK : GBK / 2;                  // packed bytes per row and K slice: 64 / 32
-  constexpr uint32_t E_BYTES = (FMT == FMT_INT4 ? 2u : 1u) * G_A_BYTES;        // expanded weights: hi (+ lo)
-  // Up to 128 rows the hi and lo halves of X sit back to back in a buffer and are one B operand of 2 BN rows: one MMA
-  // gives W X_hi in accumulator columns [0, BN) and W X_lo in [BN, 2 BN), which the epilogue adds up.  An MMA with
-  // few columns costs about as much as a wide one (it reads the whole 128-row weight operand either way), so this
-  // takes a third (int4) or half (int8) of the MMAs off the issue thread.  At 256 rows the halves are passes of their own.
-  constexpr bool FUSE_LO = BN <= 128;
-  constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GBM >> 4) << 24);
-  constexpr uint32_t IDESC2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(GBM >> 4) << 24);
-  constexpr uint32_t TMEM_COLS = FUSE_LO ? 2 * BN : BN;
-  // weight slot: 128 rows x WB bytes = KSUB consecutive K slices of the tile; WB = 128 (swizzled like every 128-byte
-  // tile: whole lines for the TMA unit and for HBM) where shared memory allows, else 64 or 32 (plain rows)
-  const uint32_t WB = grp.wbox, WS_BYTES = GBM * WB;
-  const int KSUB = (int)(WB / ROW_B), KSH = KSUB == 4 ? 2 : KSUB == 2 ? 1 : 0;
-  const int NW = grp.stages, NE = grp.estages;
-  const uint32_t XS_BYTES = grp.stage_bytes;                                   // X part of a buffer: hi (+ lo)
-  extern __shared__ uint8_t gsm_raw[];
-  uint8_t *gsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t *wfull = reinterpret_cast<uint64_t *>(gsm);
-  uint64_t *wempty = wfull + WQ_MAX_W;
-  uint64_t *xfull = wempty + WQ_MAX_W;
-  uint64_t *a_full = xfull + WQ_MAX_E;
-  uint64_t *a_empty = a_full + WQ_MAX_E;
-  uint64_t *acc_full = a_empty + WQ_MAX_E;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  const uint32_t etiles = smem_u32(gsm + 1024);                                // NE expanded buffers, 1024-byte aligned
-  const uint32_t xtiles = etiles + (uint32_t)NE * E_BYTES;                     // NE X slots
-  const uint32_t wtiles = xtiles + (uint32_t)NE * XS_BYTES;                    // NW weight slots
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int pi = 0;
-  while (pi + 1 < grp.n && (int)blockIdx.x >= grp.tile_start[pi + 1]) ++pi;
-  const GemmArgs &g = grp.p[pi];
-  const int tile_n = blockIdx.x - grp.tile_start[pi], m0 = blockIdx.y * BN;
-  const int num_k1 = g.K / GBK;
-  const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
-  const bool x_lo = g.A2 != nullptr;
-  // this CTA's slices [kz0, kz0 + nkz) touch weight slots g0 .. g0 + ng - 1 of the matrix
-  const int g0 = kz0 >> KSH, ng = nkz > 0 ? ((kz0 + nkz - 1) >> KSH) - g0 + 1 : 0;
-
-  if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (x_lo) prefetch_tmap(&maps.a2[pi]); }
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < NW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], WQ_EXP_WARPS); }
-    for (int e = 0; e < NE; ++e) { mbar_init(&xfull[e], 1); mbar_init(&a_full[e], WQ_EXP_WARPS); mbar_init(&a_empty[e], 1); }
-    mbar_init(acc_full, 1);
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
-  // What the kernels before this one wrote (X, the epilogue's inputs and outputs) is touched only after pdl_wait():
-  // by the X loads and by the epilogue warps.
-
-  if (warp == 0) {
-    if (lane == 0) {
-      // one thread feeds both rings: whichever has a free slot gets its next tile
-      int kw = 0, kx = 0, idle = 0;
-      unsigned long long t0 = 0;
-      for (; kw < ng && kw < NW; ++kw) {
-        mbar_expect_tx(&wfull[kw], WS_BYTES);
-        tma_load_2d(wtiles + (uint32_t)kw * WS_BYTES, &maps.b[pi], (g0 + kw) * (int)WB, tile_n * GBM, &wfull[kw]);
-      }
-      pdl_wait();
-      Ring wat, xat;
-      if (kw == NW) wat.phase = 1; else wat.slot = kw;
-      while (kw < ng || kx < nkz) {
-        bool moved = false;
-        if (kw < ng && mbar_try(&wempty[wat.slot], wat.phase ^ 1u)) {
-          const int s = wat.slot;
-          mbar_expect_tx(&wfull[s], WS_BYTES);
-          tma_load_2d(wtiles + (uint32_t)s * WS_BYTES, &maps.b[pi], (g0 + kw) * (int)WB, tile_n * GBM, &wfull[s]);
-          ++kw;
-          wat.next(NW);
-          moved = true;
-        }
-        if (kx < nkz && mbar_try(&a_empty[xat.slot], xat.phase ^ 1u)) {
-          const int e = xat.slot;
-          const uint32_t dst = xtiles + (uint32_t)e * XS_BYTES;
-          const int kc = (kz0 + kx) * GBK;
-          mbar_expect_tx(&xfull[e], (x_lo ? 2u : 1u) * X_BYTES);
-          tma_load_2d(dst, &maps.a[pi], kc, m0, &xfull[e]);
-          if (x_lo) tma_load_2d(dst + X_BYTES, &maps.a2[pi], kc, m0, &xfull[e]);
-          ++kx;
-          xat.next(NE);
-          moved = true;
-        }
-        if (moved) { idle = 0; continue; }
-        if (idle == 0) t0 = globaltimer_ns();
-        if ((++idle & 63) == 0) {
-          if (*abort_flag) break;
-          if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) { *abort_flag = 1; atomicCAS(g.status, 0, ST_GEMM_TIMEOUT); break; }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      Ring at;
-      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
-        const int e = at.slot;
-        if (!mbar_wait(&xfull[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        if (!mbar_wait(&a_full[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        tc_fence_after();
-        const uint32_t xb = xtiles + (uint32_t)e * XS_BYTES, eb = etiles + (uint32_t)e * E_BYTES;
-        const uint64_t wd = umma_desc_k128(eb), xd = umma_desc_k128(xb);
-        const bool wide = FUSE_LO && x_lo;
-#pragma unroll
-        for (int k4 = 0; k4 < GBK / 16; ++k4)
-          umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
-        if (x_lo && !wide) {
-          const uint64_t xl = umma_desc_k128(xb + X_BYTES);
-#pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
-        if (FMT == FMT_INT4) {
-          const uint64_t wl = umma_desc_k128(eb + G_A_BYTES);
-#pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16(tmem_base, wl + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
-        umma_commit(&a_empty[e]);   // X slot e and expanded buffer e are free once these MMAs have retired
-      }
-      umma_commit(acc_full);
-    }
-  } else if (warp >= 6) {
-    // expanders: two threads per row of the tile, each expands half of the row's 64 inputs
-    const int et = (int)threadIdx.x - 192;
-    const int row = et >> 1, part = et & 1;
-    const int ch = tile_n * GBM + row;                      // output channel of this row
-    const uint32_t swz = (uint32_t)(row & 7);
-    const uint32_t wswz = WB == 128u ? swz : 0u;
-    const uint32_t erow = (uint32_t)row * 128u;             // byte offset of the row inside an expanded tile
-    GroupScales scales;
-    if (FMT == FMT_INT4) scales.start(g, ch, kz0, nkz);
-    Ring wat, at;
-    for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
-      const int ks = kz0 + kb, sub = ks & (KSUB - 1);
-      const int s = wat.slot, e = at.slot;
-      const uint32_t sc = FMT == FMT_INT4 ? scales.at(ks) : 0u;   // the two 32-input groups of this slice
-      if (!mbar_wait(&wfull[s], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-      if (!mbar_wait(&a_empty[e], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-      // 16-byte chunk c of the row's WB bytes is at (c ^ wswz) << 4
-      const uint32_t src = wtiles + (uint32_t)s * WS_BYTES + (uint32_t)row * WB;
-      const uint32_t c0 = (uint32_t)sub * (ROW_B / 16u);
-      const uint32_t dst = etiles + (uint32_t)e * E_BYTES + erow;
-      if (FMT == FMT_INT8) {
-        // two 16-byte pieces of 16 codes per thread; neighbouring rows take theirs in opposite order, which spreads a
-        // quarter warp's stores over all eight 16-byte columns of the swizzled rows
-#pragma unroll
-        for (int pp = 0; pp < 2; ++pp) {
-          const uint32_t piece = (uint32_t)part * 2u + ((uint32_t)(pp + row) & 1u);
-          const uint4 w = lds128(src + (((c0 + piece) ^ wswz) << 4));
-          uint32_t v[8];
-          expand_int8(w.x, v); expand_int8(w.y, v + 2); expand_int8(w.z, v + 4); expand_int8(w.w, v + 6);
-          const uint4 o0 = make_uint4(v[0], v[1], v[2], v[3]), o1 = make_uint4(v[4], v[5], v[6], v[7]);
-          sts128(dst + (((piece * 2u) ^ swz) << 4), o0);        // inputs 16 piece .. +7: 16-byte chunk 2 piece
-          sts128(dst + (((piece * 2u + 1u) ^ swz) << 4), o1);
-        }
-      } else {
-        // one 16-byte piece of 32 nibbles per thread = one of the two scale groups of the slice
-        const uint4 w = lds128(src + (((c0 + (uint32_t)part) ^ wswz) << 4));
-        const uint32_t s16 = part ? (sc >> 16) : (sc & 0xffffu);
-        const uint32_t s2 = s16 | (s16 << 16);
-        const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int wi = 0; wi < 4; ++wi) {
-          // 8 nibbles = 8 consecutive inputs -> one 16-byte chunk of hi and one of lo
-          uint32_t hi[4], lo[4];
-          expand_int4(words[wi], s2, hi, lo);
-          const uint32_t chunk = ((uint32_t)part * 4u + (uint32_t)wi) ^ swz;
-          sts128(dst + (chunk << 4), make_uint4(hi[0], hi[1], hi[2], hi[3]));
-          sts128(dst + G_A_BYTES + (chunk << 4), make_uint4(lo[0], lo[1], lo[2], lo[3]));
-        }
-      }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&a_full[e]);
-        if (sub == KSUB - 1) mbar_arrive(&wempty[s]);   // (the last slot of this K range is not asked for again)
-      }
-      if (sub == KSUB - 1) wat.next(NW);
-    }
-  } else {
-    const int quad = warp & 3;
-    const int ch = tile_n * GBM + quad * 32 + lane;
-    pdl_wait();
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
-    tc_fence_after();
-    if (ok) {
-      const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
-      const uint32_t buf = etiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
-      uint32_t flip = 0;
-      for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
-        if (m0 + c0 >= g.M) break;   // warp-uniform
-        uint32_t acc[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
-        if (FUSE_LO && x_lo) {
-          uint32_t part[32];
-          tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(BN + c0), part);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
-        }
-        if (g.col_scale && grp.split == 1) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
-        }
-        if (BN == 32 && grp.split > 1) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
-        else tile_out_lean(g, &maps.o[pi], grp.split > 1, blockIdx.z, tile_n * GBM + quad * 32, m0 + c0, acc, buf + flip);
-      }
-      tile_out_end();
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
-  }
-}
-
 // ------------------------------------------------------------------------------------------------
-// Quantised weights, more than 128 rows: the pair product of gemm_pair_kernel with the weight operand in TMEM.  Eight warps
-// expand a slice of the packed codes straight into the MMA's A operand (TMEM lane = channel, a column = two inputs), so
-// shared memory carries X alone.  Expanded into shared memory instead (one CTA, 128 x 256), a slice of int4 asked it for 163 bytes a
-// clock where it gives 128, with room for two slices only.
-//   warp 0      TMA: this CTA's half of X into slot e, counted on the even CTA's barrier
-//   warp 1      TMEM; in the even CTA the MMAs: acc += W_hi X_hi, W_hi X_lo, and for int4 W_lo X_hi (int8 codes are exact in fp16)
-//   warps 6..13 expanders: warp quadrant = TMEM lane quadrant, two warps share a row's 64 inputs (one scale group each)
-//   warp 14     TMA: packed weights, 128 rows x 128 bytes = 4 (int4) or 2 (int8) slices per slot
-//   warps 2..13 epilogue, three warps per quadrant
-// One commit per slice frees X slot e and A slot e in both CTAs.  The weights do not depend on the kernels before this one.
-__device__ __forceinline__ void umma_f16_pair_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// Quantised weights, read in their packed form (int8 codes [N, K], or int4 nibbles [N, K/2] with fp16 group scales [N, K/32]: the
+// bytes a step has to stream).  Eight warps expand a slice of 64 inputs straight into the MMA's A operand in TMEM (lane =
+// channel, a column = two inputs), so shared memory carries X alone.
+//   PAIR:  more than 128 rows; out^T[256 channels, BN rows] per pair of SMs as in gemm_pair_kernel, one CTA per SM.  Expanded into
+//          shared memory instead (one CTA, 128 x 256), a slice of int4 asked it for 163 bytes a clock where it gives 128.
+//   !PAIR: up to 128 rows; out^T[128 channels, BN rows] per CTA, two CTAs per SM where 256 columns of TMEM hold the accumulator
+//          and some slices.  A step of few streams is a chain of such products of 3 to 11 slices each: every slice that has a
+//          slot is loaded and expanded before the kernels ahead have finished, and what is left behind them is X, its MMAs and the epilogue.
+//   warp 0      TMA: X into slot x, counted on the even CTA's barrier
+//   warp 1      TMEM; (in the even CTA) the MMAs: acc += W_hi X_hi, W_hi X_lo, and for int4 W_lo X_hi (int8 codes are exact in
+//               fp16, the row scale is applied to the accumulator; int4: hi = fp16(q s), lo = q s - hi, an exact pair)
+//   warps 2..9  expanders: warp quadrant = TMEM lane quadrant, two warps share a row's 64 inputs (one scale group each); then epilogue
+//   warp 10     TMA: packed weights, 128 rows x 128 bytes = 4 (int4) or 2 (int8) slices per slot
+// !PAIR: the hi and lo halves of X sit back to back in a slot and are one B operand of 2 BN rows: one MMA gives W X_hi in
+// accumulator columns [0, BN) and W X_lo in [BN, 2 BN), which the epilogue adds up (an MMA with few columns costs as much as a
+// wide one).  PAIR: the halves multiply into the same accumulator, slice by slice.
+__device__ __forceinline__ void umma_f16_ta(bool pair, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  if (pair)
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -982,39 +723,42 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-constexpr int PQ_THREADS = 32 * 15;
-constexpr int PQ_MAX = 8;                // most slots of any ring
-constexpr uint32_t PQ_ACC_COLS = 256;    // TMEM: accumulator in columns [0, 256), A slots in [256, 512)
+constexpr int GQ_EXP_WARPS = 8;
+constexpr int GQ_THREADS = 32 * (3 + GQ_EXP_WARPS);
+constexpr int GQ_MAX = 8;                // most slots of any ring
 
-template <int FMT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PQ_THREADS, 1)
-gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
+template <int FMT, bool PAIR>
+__global__ void __launch_bounds__(GQ_THREADS, PAIR ? 1 : 2)
+gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   constexpr uint32_t ROW_B = FMT == FMT_INT8 ? GBK : GBK / 2;          // packed bytes per row and slice
   constexpr int KSH = FMT == FMT_INT8 ? 1 : 2, KSUB = 1 << KSH;        // slices per weight slot
   constexpr uint32_t WS_BYTES = GBM * 128;
   constexpr uint32_t A_COLS = FMT == FMT_INT4 ? 64 : 32;               // expanded slice: hi (+ lo)
-  const int NW = grp.stages, NE = grp.estages, BN = grp.bn;
-  const uint32_t X_BYTES = (uint32_t)BN * (GBK * 2 / 2), XS_BYTES = grp.stage_bytes;
-  const uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * GBM >> 4) << 24);
+  constexpr int CH = PAIR ? 2 * GBM : GBM;
+  const int NW = grp.stages, NE = grp.estages, NX = grp.xstages, BN = grp.bn;
+  const uint32_t X_BYTES = (uint32_t)(PAIR ? BN / 2 : BN) * (GBK * 2), XS_BYTES = grp.stage_bytes;
+  const uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CH >> 4) << 24);
+  const uint32_t IDESC2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(CH >> 4) << 24);
   extern __shared__ uint8_t gsm_raw[];
   uint8_t *gsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t *wfull = reinterpret_cast<uint64_t *>(gsm);
-  uint64_t *wempty = wfull + PQ_MAX;
-  uint64_t *xfull = wempty + PQ_MAX;
-  uint64_t *a_full = xfull + PQ_MAX;
-  uint64_t *a_peer = a_full + PQ_MAX;       // (even CTA) the other CTA's expanded slice
-  uint64_t *empty = a_peer + PQ_MAX;
-  uint64_t *acc_full = empty + PQ_MAX;
+  uint64_t *wempty = wfull + GQ_MAX;
+  uint64_t *xfull = wempty + GQ_MAX;
+  uint64_t *xempty = xfull + GQ_MAX;
+  uint64_t *a_full = xempty + GQ_MAX;
+  uint64_t *a_empty = a_full + GQ_MAX;
+  uint64_t *a_peer = a_empty + GQ_MAX;      // (even CTA of a pair) the other CTA's expanded slice
+  uint64_t *acc_full = a_peer + GQ_MAX;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  const uint32_t xtiles = smem_u32(gsm + 1024), wtiles = xtiles + (uint32_t)NE * XS_BYTES;
+  const uint32_t xtiles = smem_u32(gsm + 1024), wtiles = xtiles + (uint32_t)NX * XS_BYTES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank();
-  const int pair = blockIdx.x >> 1, ct = pair / grp.m_tiles, m0 = (pair - ct * grp.m_tiles) * BN;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  const int id = PAIR ? blockIdx.x >> 1 : blockIdx.x, ct = id / grp.m_tiles, m0 = (id - ct * grp.m_tiles) * BN;
   int pi = 0;
   while (pi + 1 < grp.n && ct >= grp.tile_start[pi + 1]) ++pi;
   const GemmArgs &g = grp.p[pi];
-  const int ch0 = (ct - grp.tile_start[pi]) * (2 * GBM) + (int)rank * GBM;
+  const int ch0 = (ct - grp.tile_start[pi]) * CH + (int)rank * GBM;
   const int num_k1 = g.K / GBK;
   const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
   const bool x_lo = g.A2 != nullptr;
@@ -1022,19 +766,25 @@ gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
 
   if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (x_lo) prefetch_tmap(&maps.a2[pi]); }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 8); }
-    for (int e = 0; e < NE; ++e) { mbar_init(&xfull[e], 1); mbar_init(&a_full[e], 8); mbar_init(&a_peer[e], 1); mbar_init(&empty[e], 1); }
+    for (int s = 0; s < NW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], GQ_EXP_WARPS); }
+    for (int x = 0; x < NX; ++x) { mbar_init(&xfull[x], 1); mbar_init(&xempty[x], 1); }
+    for (int e = 0; e < NE; ++e) { mbar_init(&a_full[e], GQ_EXP_WARPS); mbar_init(&a_empty[e], 1); mbar_init(&a_peer[e], 1); }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(grp.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(grp.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync();      // the barriers of both CTAs exist before anything arrives on them from the other one
+  if (PAIR) cluster_sync();      // the barriers of both CTAs exist before anything arrives on them from the other one
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
@@ -1043,52 +793,59 @@ gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
     if (lane == 0) {
       pdl_wait();
       Ring at;
-      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
-        const int e = at.slot;
-        if (!mbar_wait(&empty[e], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        const uint32_t dst = xtiles + (uint32_t)e * XS_BYTES, bar = mapa_u32(smem_u32(&xfull[e]), 0);
-        const int kx = (kz0 + kb) * GBK, row = m0 + (int)rank * (BN / 2);
-        if (rank == 0) mbar_expect_tx(&xfull[e], (x_lo ? 4u : 2u) * X_BYTES);   // of both CTAs
-        tma_load_2d_pair(dst, &maps.a[pi], kx, row, bar);
-        if (x_lo) tma_load_2d_pair(dst + X_BYTES, &maps.a2[pi], kx, row, bar);
+      for (int kb = 0; kb < nkz; ++kb, at.next(NX)) {
+        if (!mbar_wait(&xempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        const uint32_t dst = xtiles + (uint32_t)at.slot * XS_BYTES;
+        const int kx = (kz0 + kb) * GBK;
+        if (PAIR) {
+          const uint32_t bar = mapa_u32(smem_u32(&xfull[at.slot]), 0);
+          const int row = m0 + (int)rank * (BN / 2);
+          if (rank == 0) mbar_expect_tx(&xfull[at.slot], (x_lo ? 4u : 2u) * X_BYTES);   // of both CTAs
+          tma_load_2d_pair(dst, &maps.a[pi], kx, row, bar);
+          if (x_lo) tma_load_2d_pair(dst + X_BYTES, &maps.a2[pi], kx, row, bar);
+        } else {
+          mbar_expect_tx(&xfull[at.slot], (x_lo ? 2u : 1u) * X_BYTES);
+          tma_load_2d(dst, &maps.a[pi], kx, m0, &xfull[at.slot]);
+          if (x_lo) tma_load_2d(dst + X_BYTES, &maps.a2[pi], kx, m0, &xfull[at.slot]);
+        }
       }
     }
-  } else if (warp == 14) {
+  } else if (warp == 2 + GQ_EXP_WARPS) {
     if (lane == 0) {
       Ring at;
       for (int kw = 0; kw < ng; ++kw, at.next(NW)) {
-        const int s = at.slot;
-        if (!mbar_wait(&wempty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        mbar_expect_tx(&wfull[s], WS_BYTES);
-        tma_load_2d(wtiles + (uint32_t)s * WS_BYTES, &maps.b[pi], (g0 + kw) * 128, ch0, &wfull[s]);
+        if (!mbar_wait(&wempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        mbar_expect_tx(&wfull[at.slot], WS_BYTES);
+        tma_load_2d(wtiles + (uint32_t)at.slot * WS_BYTES, &maps.b[pi], (g0 + kw) * 128, ch0, &wfull[at.slot]);
       }
     }
   } else if (warp == 1) {
     if (rank == 0 && lane == 0) {
-      Ring at;
-      for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
-        const int e = at.slot;
-        if (!mbar_wait(&a_full[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        if (!mbar_wait(&a_peer[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        if (!mbar_wait(&xfull[e], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+      Ring ea, xa;
+      for (int kb = 0; kb < nkz; ++kb, ea.next(NE), xa.next(NX)) {
+        if (!mbar_wait(&a_full[ea.slot], ea.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (PAIR && !mbar_wait(&a_peer[ea.slot], ea.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!mbar_wait(&xfull[xa.slot], xa.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         tc_fence_after();
-        const uint32_t xb = xtiles + (uint32_t)e * XS_BYTES, ta = tmem_base + PQ_ACC_COLS + (uint32_t)e * A_COLS;
+        const uint32_t xb = xtiles + (uint32_t)xa.slot * XS_BYTES, ta = tmem_base + grp.acc_cols + (uint32_t)ea.slot * A_COLS;
         const uint64_t xd = umma_desc_k128(xb), xl = umma_desc_k128(xb + X_BYTES);
+        const bool wide = !PAIR && x_lo;
 #pragma unroll
         for (int k4 = 0; k4 < GBK / 16; ++k4)       // 16 inputs = 8 columns of A
-          umma_f16_pair_ta(tmem_base, ta + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, (kb | k4) != 0);
-        if (x_lo) {
+          umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
+        if (PAIR && x_lo) {
 #pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair_ta(tmem_base, ta + (uint32_t)k4 * 8, xl + (uint64_t)(k4 * 2), IDESC, 1u);
+          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xl + (uint64_t)(k4 * 2), IDESC, 1u);
         }
         if (FMT == FMT_INT4) {
 #pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair_ta(tmem_base, ta + 32u + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, 1u);
+          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + 32u + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, 1u);
         }
-        umma_commit_pair(&empty[e]);
+        if (PAIR) { umma_commit_pair(&a_empty[ea.slot]); umma_commit_pair(&xempty[xa.slot]); }
+        else { umma_commit(&a_empty[ea.slot]); umma_commit(&xempty[xa.slot]); }
       }
-      umma_commit_pair(acc_full);
-    } else if (rank == 1 && lane == 0) {
+      if (PAIR) umma_commit_pair(acc_full); else umma_commit(acc_full);
+    } else if (PAIR && rank == 1 && lane == 0) {
       // A release across the cluster takes 500 to 900 clocks: this thread, which has no MMAs to issue, passes the slices of
       // its CTA's expanders on.
       Ring at;
@@ -1099,25 +856,24 @@ gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
         mbar_arrive_cluster(mapa_u32(smem_u32(&a_peer[at.slot]), 0));
       }
     }
-  } else if (warp >= 6) {
-    const int quad = warp & 3, part = (warp - 6) >> 2;
+  } else {
+    const int quad = warp & 3, part = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
     const uint32_t swz = (uint32_t)(row & 7);
     GroupScales scales;
     if (FMT == FMT_INT4) scales.start(g, ch0 + row, kz0, nkz);
-    const uint32_t ta = tmem_base + ((uint32_t)(quad * 32) << 16) + PQ_ACC_COLS + (uint32_t)part * 16;
+    const uint32_t ta = tmem_base + ((uint32_t)(quad * 32) << 16) + grp.acc_cols + (uint32_t)part * 16;
     Ring wat, at;
     for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
       const int ks = kz0 + kb, sub = ks & (KSUB - 1);
-      const int s = wat.slot, e = at.slot;
       uint32_t s2 = 0;
       if (FMT == FMT_INT4) {
         const uint32_t sc = scales.at(ks), s16 = part ? (sc >> 16) : (sc & 0xffffu);
         s2 = s16 | (s16 << 16);
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(&wfull[s], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&wfull[wat.slot], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
       // 16-byte chunk c of the row's 128 bytes is at (c ^ swz) << 4
-      const uint32_t src = wtiles + (uint32_t)s * WS_BYTES + (uint32_t)row * 128u, c0 = (uint32_t)sub * (ROW_B / 16u);
+      const uint32_t src = wtiles + (uint32_t)wat.slot * WS_BYTES + (uint32_t)row * 128u, c0 = (uint32_t)sub * (ROW_B / 16u);
       uint32_t hi[16], lo[16];
       if (FMT == FMT_INT4) {
         const uint4 w = lds128(src + (((c0 + (uint32_t)part) ^ swz) << 4));
@@ -1131,23 +887,21 @@ gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
           expand_int8(w.z, hi + pp * 8 + 4); expand_int8(w.w, hi + pp * 8 + 6);
         }
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(&empty[e], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
       tc_fence_after();
-      tmem_st16(ta + (uint32_t)e * A_COLS, hi);
-      if (FMT == FMT_INT4) tmem_st16(ta + (uint32_t)e * A_COLS + 32u, lo);
+      tmem_st16(ta + (uint32_t)at.slot * A_COLS, hi);
+      if (FMT == FMT_INT4) tmem_st16(ta + (uint32_t)at.slot * A_COLS + 32u, lo);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&a_full[e]);
-        if (sub == KSUB - 1) mbar_arrive(&wempty[s]);   // (the last slot of this K range is not asked for again)
+        mbar_arrive(&a_full[at.slot]);
+        if (sub == KSUB - 1) mbar_arrive(&wempty[wat.slot]);   // (the last slot of this K range is not asked for again)
       }
       if (sub == KSUB - 1) wat.next(NW);
     }
-  }
-  if (warp >= 2 && warp < 14) {
-    const int quad = warp & 3;
-    const int ch = ch0 + quad * 32 + lane;
+    // epilogue
+    const int ch = ch0 + row;
     pdl_wait();
     const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
@@ -1155,25 +909,37 @@ gemm_pair_wq_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
       const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
       const uint32_t buf = xtiles + (uint32_t)(warp - 2) * 2 * EPI_BUF;   // the rings have been read
       uint32_t flip = 0;
-      for (int c0 = ((warp - 2) >> 2) * 32; c0 < BN; c0 += 96, flip ^= EPI_BUF) {
+      for (int c0 = part * 32; c0 < BN; c0 += 64, flip ^= EPI_BUF) {
         if (m0 + c0 >= g.M) break;   // warp-uniform
+        const uint32_t at_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
         uint32_t acc[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
+        tmem_ld32(at_acc, acc);
+        if (!PAIR && x_lo) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t more[16];
+            tmem_ld16(at_acc + (uint32_t)(BN + h * 16), more);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[h * 16 + i] = __float_as_uint(__uint_as_float(acc[h * 16 + i]) + __uint_as_float(more[i]));
+          }
+        }
         if (g.col_scale && grp.split == 1) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
         }
-        tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
+        if (!PAIR && BN == 32 && grp.split > 1) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
+        else tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
       }
       tile_out_end();
     }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync();      // neither CTA leaves while the other's MMAs or commits may still reach into it
+  if (PAIR) cluster_sync();      // neither CTA leaves while the other's MMAs or commits may still reach into it
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(grp.tmem_cols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(grp.tmem_cols) : "memory");
   }
 }
 
@@ -1256,17 +1022,16 @@ bool make_map(CUtensorMap *map, const void *base, int rows, int K, int box_rows)
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// [rows, row_bytes] bytes row-major -> tensor map with a (box_bytes x 128 rows) box, zero fill outside; 128-byte boxes
-// are swizzled, narrower ones are plain rows
-bool make_map_bytes(CUtensorMap *map, const void *base, int rows, int row_bytes, int box_bytes) {
+// [rows, row_bytes] bytes row-major -> tensor map with a (128 bytes x 128 rows) box, 128-byte swizzle, zero fill outside
+bool make_map_bytes(CUtensorMap *map, const void *base, int rows, int row_bytes) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)GBM};
+  const cuuint32_t box[2] = {128, (cuuint32_t)GBM};
   const cuuint32_t estr[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -2233,103 +1998,6 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   }
   return cudaGetLastError();
 }
-template <int BN, int FMT>
-cudaError_t launch_gemm_wq_t(const GemmMaps &maps, const GemmGroup &grp, dim3 grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(gemm_wq_kernel<BN, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  launch_k(gemm_wq_kernel<BN, FMT>, dim3(grid), dim3(WQ_THREADS), smem, st, maps, grp);
-  return cudaGetLastError();
-}
-
-// shared-memory plan of the packed-weight GEMM inside `avail` bytes: ne buffers (expanded weights + X slot, released
-// together) and nw weight slots of `wbox`-byte rows; the weight ring grows first
-struct WqPlan { int ne, nw; uint32_t wbox; bool ok; };
-WqPlan wq_plan(long long avail, long long buf_bytes, uint32_t wbox, int want_ne, int want_nw) {
-  WqPlan p{2, 2, wbox, false};
-  const long long ws = (long long)GBM * wbox;
-  if (avail - 2 * buf_bytes - 2 * ws < 0) return p;
-  p.ok = true;
-  for (bool grown = true; grown;) {
-    grown = false;
-    const long long left = avail - p.ne * buf_bytes - p.nw * ws;
-    if (p.nw < want_nw && left >= ws) { ++p.nw; grown = true; continue; }
-    if (p.ne < want_ne && left >= buf_bytes) { ++p.ne; grown = true; }
-  }
-  return p;
-}
-
-// quantised weights in packed form (GemmArgs::Wq): up to 128 rows
-cudaError_t launch_gemm_wq(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
-  const int M = probs[0].M, fmt = probs[0].wfmt;
-  if (fmt != FMT_INT8 && fmt != FMT_INT4) return cudaErrorInvalidValue;
-  const int bn = M <= 32 ? 32 : M <= 64 ? 64 : 128;
-  GemmMaps maps;
-  GemmGroup grp;
-  memset(&grp, 0, sizeof(grp));
-  grp.n = n;
-  int tiles = 0, min_k1 = 1 << 30;
-  bool raw_ok = M <= GEMM_SMALL_M;
-  for (int i = 0; i < n; ++i) {
-    const GemmArgs &g = probs[i];
-    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M || !g.Wq || g.wfmt != fmt) return cudaErrorInvalidValue;
-    if (fmt == FMT_INT4 && !g.wq_scale) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Wq) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
-      return cudaErrorInvalidValue;
-    grp.p[i] = g;
-    grp.tile_start[i] = tiles;
-    tiles += (g.N + GBM - 1) / GBM;
-    min_k1 = std::min(min_k1, g.K / GBK);
-    raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
-    if (g.A2) grp.dual |= 1;
-  }
-  grp.tile_start[n] = tiles;
-  const int m_tiles = (M + bn - 1) / bn;
-  grp.split = 1;
-  grp.stage_bytes = ((grp.dual & 1) ? 2u : 1u) * (uint32_t)bn * GBK * 2;
-  const long long buf_bytes = (long long)(fmt == FMT_INT4 ? 2u : 1u) * G_A_BYTES + grp.stage_bytes;
-  const uint32_t row_b = fmt == FMT_INT8 ? GBK : GBK / 2;
-  // Two CTAs per SM where two or three buffers and a weight ring fit in half an SM's shared memory (up to 64 rows) --
-  // the step is a chain of short GEMMs, and a second CTA (of this kernel or, launched early, of the next) hides the
-  // hand-overs between the kernel's roles: a quarter of the step time at 32 rows; else one CTA with everything as
-  // deep as fits.  Weight slots are as wide as the plan allows.
-  WqPlan pl{};
-  bool two_per_sm = false;
-  for (uint32_t wb = 128; wb >= row_b && !two_per_sm; wb >>= 1) {
-    pl = wq_plan(110ll << 10, buf_bytes, wb, 3, wb == 128 ? 3 : wb == 64 ? 4 : 8);
-    two_per_sm = pl.ok;
-  }
-  if (!two_per_sm) pl = wq_plan(225ll << 10, buf_bytes, 128, WQ_MAX_E, 4);
-  if (!pl.ok) return cudaErrorInvalidValue;
-  for (int i = 0; i < n; ++i) {
-    const GemmArgs &g = probs[i];
-    const int row_bytes = fmt == FMT_INT8 ? g.K : g.K / 2;
-    if (!make_map(&maps.a[i], g.A, g.M, g.K, bn) || !make_map_bytes(&maps.b[i], g.Wq, g.N, row_bytes, (int)pl.wbox))
-      return cudaErrorNotSupported;
-    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, bn)) return cudaErrorNotSupported;
-  }
-  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; }
-  const int slots = (two_per_sm ? 2 : 1) * device_sm_count();
-  if (raw_ok) grp.split = split_of(tiles * m_tiles, slots, min_k1);
-  grp.stages = pl.nw;
-  grp.estages = pl.ne;
-  grp.wbox = pl.wbox;
-  if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
-  const size_t smem = 1024 + (size_t)pl.ne * buf_bytes + (size_t)pl.nw * GBM * pl.wbox + 1024;
-  dim3 grid(tiles, m_tiles, grp.split);
-  cudaError_t e = cudaErrorInvalidValue;
-#define FRB_WQ(BNV) (fmt == FMT_INT8 ? launch_gemm_wq_t<BNV, FMT_INT8>(maps, grp, grid, smem, st) : launch_gemm_wq_t<BNV, FMT_INT4>(maps, grp, grid, smem, st))
-  e = bn == 32 ? FRB_WQ(32) : bn == 64 ? FRB_WQ(64) : FRB_WQ(128);
-#undef FRB_WQ
-  if (e != cudaSuccess) return e;
-  if (defer_split) *defer_split = grp.split;
-  if (grp.split > 1 && !defer_split) {
-    int max_n = 0;
-    for (int i = 0; i < n; ++i) max_n = std::max(max_n, probs[i].N);
-    launch_k(gemm_finish_kernel, dim3(dim3((M * (max_n / 4) + 255) / 256, n)), dim3(256), 0, st, grp);
-  }
-  return cudaGetLastError();
-}
-
 // Costs in clocks, fitted to products of 256 and 1000 rows (2048 x 2048 up to 65536 x 2048 and 2048 x 8192) with 64 to 256 columns
 // and 1 to 9 cuts, within 10 % of the times.
 // Slabs: the next kernel reads them at about 2,500 bytes a clock; without one that does, a finishing pass is launched.
@@ -2401,7 +2069,7 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
   cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  if ((e = launch_k(gemm_pair_kernel, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
+  if ((e = launch_cluster_k(gemm_pair_kernel, 2, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
     int max_n = 0;
@@ -2411,9 +2079,10 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   return cudaGetLastError();
 }
 
-// quantised weights in packed form, more than 128 rows: gemm_pair_wq_kernel
-cudaError_t launch_gemm_pair_wq(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
-  const int M = probs[0].M, fmt = probs[0].wfmt, num_pairs = device_sm_count() / 2;
+// quantised weights in packed form (GemmArgs::Wq): gemm_q_kernel, on pairs of SMs above 128 rows
+cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
+  const int M = probs[0].M, fmt = probs[0].wfmt, sms = device_sm_count(), num_pairs = sms / 2;
+  const bool pair = M > 128;
   if (fmt != FMT_INT8 && fmt != FMT_INT4) return cudaErrorInvalidValue;
   GemmMaps maps;
   GemmGroup grp;
@@ -2429,49 +2098,67 @@ cudaError_t launch_gemm_pair_wq(const GemmArgs *probs, int n, cudaStream_t st, i
       return cudaErrorInvalidValue;
     grp.p[i] = g;
     grp.tile_start[i] = tiles;
-    const int t = (g.N + 2 * GBM - 1) / (2 * GBM), passes = (fmt == FMT_INT4 ? 2 : 1) + (g.A2 ? 1 : 0);
+    const int t128 = (g.N + GBM - 1) / GBM, t = pair ? (t128 + 1) / 2 : t128;
     tiles += t;
-    tiles128 += (g.N + GBM - 1) / GBM;
-    units += t * passes;
+    tiles128 += t128;
+    units += t * ((fmt == FMT_INT4 ? 2 : 1) + (g.A2 ? 1 : 0));
     sum_n += g.N;
     min_k1 = std::min(min_k1, g.K / GBK);
     raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
     any_lo = any_lo || g.A2;
   }
   grp.tile_start[n] = tiles;
-  const int fixed = raw_ok && probs[0].fixed_split ? keep_split(tiles128 * ((M + 255) / 256), min_k1) : 0;   // (as in launch_gemm_pair)
-  const int max_split = raw_ok ? std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 2)) : 1;
   grp.split = 1;
-  grp.bn = 256;
-  float best = 0.f;
-  const float passes = (float)units / (float)tiles;
-  for (int rt = (M + 255) / 256; rt <= (M + 127) / 128; ++rt) {
-    const int bn = ((M + rt - 1) / rt + 31) / 32 * 32;
-    for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
-      // in clocks: a slice is bound by its MMAs or by its expansion, a wave starts and ends
-      const int waves = (tiles * rt * sp + num_pairs - 1) / num_pairs;
-      const float cost = (float)waves * ((float)((min_k1 + sp - 1) / sp) * std::max(2.05f * (float)bn * passes, 1180.f) + 11000.f + 14.f * (float)bn) +
-                         slab_cost(sp, M, sum_n, defer_split != nullptr);
-      if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
+  const uint32_t a_cols = fmt == FMT_INT4 ? 64u : 32u;
+  bool two_per_sm = false;
+  if (pair) {
+    const int fixed = raw_ok && probs[0].fixed_split ? keep_split(tiles128 * ((M + 255) / 256), min_k1) : 0;   // (as in launch_gemm_pair)
+    const int max_split = raw_ok ? std::max(1, std::min(GEMM_SPLIT_MAX, min_k1 / 2)) : 1;
+    const float passes = (float)units / (float)tiles;
+    float best = 0.f;
+    for (int rt = (M + 255) / 256; rt <= (M + 127) / 128; ++rt) {
+      const int bn = ((M + rt - 1) / rt + 31) / 32 * 32;
+      for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
+        // in clocks: a slice is bound by its MMAs or by its expansion, a wave starts and ends
+        const int waves = (tiles * rt * sp + num_pairs - 1) / num_pairs;
+        const float cost = (float)waves * ((float)((min_k1 + sp - 1) / sp) * std::max(2.05f * (float)bn * passes, 1180.f) + 11000.f + 14.f * (float)bn) +
+                           slab_cost(sp, M, sum_n, defer_split != nullptr);
+        if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
+      }
     }
+    grp.acc_cols = 256;
+    grp.tmem_cols = 512;
+  } else {
+    grp.bn = M <= 32 ? 32 : M <= 64 ? 64 : 128;
+    // K is cut for two CTAs per SM where their accumulators are narrow
+    if (raw_ok) grp.split = split_of(tiles, (grp.bn <= 64 || !any_lo) ? 2 * sms : sms, min_k1);
+    grp.acc_cols = (any_lo ? 2u : 1u) * (uint32_t)grp.bn;
+    two_per_sm = grp.acc_cols <= 128;
+    grp.tmem_cols = two_per_sm ? 256 : 512;
   }
   grp.m_tiles = (M + grp.bn - 1) / grp.bn;
+  const int xrows = pair ? grp.bn / 2 : grp.bn;
   for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
-    const GemmArgs &g = probs[i < n ? i : 0];
-    const int row_bytes = fmt == FMT_INT8 ? g.K : g.K / 2;
-    if (!make_map(&maps.a[i], g.A, g.M, g.K, grp.bn / 2) || !make_map_bytes(&maps.b[i], g.Wq, g.N, row_bytes, 128)) return cudaErrorNotSupported;
-    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, grp.bn / 2)) return cudaErrorNotSupported;
+    if (i >= n) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; continue; }
+    const GemmArgs &g = probs[i];
+    if (!make_map(&maps.a[i], g.A, g.M, g.K, xrows) || !make_map_bytes(&maps.b[i], g.Wq, g.N, fmt == FMT_INT8 ? g.K : g.K / 2)) return cudaErrorNotSupported;
+    maps.a2[i] = maps.a[i];
+    if (g.A2 && !make_map(&maps.a2[i], g.A2, g.M, g.K, xrows)) return cudaErrorNotSupported;
   }
-  grp.stage_bytes = (any_lo ? 2u : 1u) * (uint32_t)grp.bn * GBK;
-  grp.stages = 4;
-  grp.estages = std::min<int>(fmt == FMT_INT4 ? 4 : 8, (int)(((220u << 10) - 4u * GBM * 128) / grp.stage_bytes));
+  grp.stage_bytes = (any_lo ? 2u : 1u) * (uint32_t)xrows * GBK * 2;
+  grp.estages = std::min<int>(GQ_MAX, (int)((grp.tmem_cols - grp.acc_cols) / a_cols));
+  const uint32_t avail = (two_per_sm ? 110u : 220u) << 10, ws = GBM * 128;
+  grp.stages = two_per_sm ? ((avail - 3 * ws) / grp.stage_bytes >= 4 ? 3 : 2) : 4;
+  grp.xstages = std::min<int>(GQ_MAX, (int)((avail - grp.stages * ws) / grp.stage_bytes));
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
-  const size_t rings = (size_t)grp.estages * grp.stage_bytes + (size_t)grp.stages * GBM * 128;
-  const size_t smem = 1024 + std::max<size_t>(rings, 12 * 2 * EPI_BUF) + 1024;
-  auto kern = fmt == FMT_INT4 ? gemm_pair_wq_kernel<FMT_INT4> : gemm_pair_wq_kernel<FMT_INT8>;
+  const size_t rings = (size_t)grp.xstages * grp.stage_bytes + (size_t)grp.stages * ws;
+  const size_t smem = 1024 + std::max<size_t>(rings, GQ_EXP_WARPS * 2 * EPI_BUF) + 1024;
+  auto kern = pair ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, true> : gemm_q_kernel<FMT_INT8, true>)
+                   : (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false> : gemm_q_kernel<FMT_INT8, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  if ((e = launch_k(kern, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(PQ_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
+  const dim3 grid((pair ? 2 : 1) * tiles * grp.m_tiles, 1, grp.split);
+  if ((e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(GQ_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
     int max_n = 0;
@@ -2488,7 +2175,7 @@ cudaError_t launch_gemm_group(const GemmArgs *probs, int n, int mt, cudaStream_t
   if (n < 1 || n > GEMM_GROUP_MAX || (mt != 1 && mt != 2)) return cudaErrorInvalidValue;
   const int M = probs[0].M;
   if (defer_split) *defer_split = 1;
-  if (probs[0].Wq) return M <= 128 ? launch_gemm_wq(probs, n, st, defer_split) : launch_gemm_pair_wq(probs, n, st, defer_split);
+  if (probs[0].Wq) return launch_gemm_q(probs, n, st, defer_split);
   return M <= 128 ? launch_gemm_wt(probs, n, st, defer_split) : launch_gemm_pair(probs, n, st, defer_split);
 }
 
