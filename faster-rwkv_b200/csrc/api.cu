@@ -691,13 +691,7 @@ int ensure_row_copies(fr_b200_model *m) {
   for (auto &kv : m->mats) {
     const MatrixSlot &s = kv.second;
     if (!s.has_plain) continue;
-    const size_t n = (size_t)s.K * s.N;
-    int rc;
-    if ((rc = ensure_scratch(m, 0, n * 4))) return rc;
-    if ((rc = ensure_scratch(m, 1, n * 2))) return rc;
-    CU(launch_unpack(FMT_FP16, m->d_weights + s.tile_off, s.item_stride, nullptr, 0, s.K, s.N, reinterpret_cast<float *>(m->d_scratch[0]), 0));
-    CU(launch_f32_to_f16(reinterpret_cast<const float *>(m->d_scratch[0]), reinterpret_cast<__half *>(m->d_scratch[1]), n, 0));
-    CU(launch_transpose_f16(reinterpret_cast<const __half *>(m->d_scratch[1]), s.K, s.N, m->d_plain + s.plain_off, 0));
+    CU(launch_tiles_to_rows_f16(m->d_weights + s.tile_off, s.item_stride, s.K, s.N, m->d_plain + s.plain_off, 0));
   }
   CU(cudaDeviceSynchronize());
   free_scratch(m);
@@ -1016,6 +1010,8 @@ int fr_b200_vocab_padded(const fr_b200_model *m) { return m ? m->Vpad : FR_B200_
 
 namespace {
 
+constexpr int PROMPT_BUILD_ROWS = 8, PROMPT_PAIR_ROWS = 32;   // see fr_b200_run_seq, rows_forward
+
 // Prompts of up to this many rows and channels have no finishing pass: 29 int4 tokens of the 1.5B shape take 1.61 ms
 // instead of 1.67, 60 fp16 ones 1.39 instead of 1.49, 100 1.61 instead of 1.64; 200 int8 ones would take 2.56 instead of 2.51,
 // and at 2,560 channels a CTA has no registers left for the slabs of two rows (29 tokens: 2.73 instead of 2.40).
@@ -1032,6 +1028,9 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   const int C = m->C, F = m->F, H = m->H, af = m->cfg.act_fp16, T = R;
   if (C > 8192) return fail(FR_B200_E_UNSUPPORTED, "the row kernels of the GEMM path hold at most n_embd = 8192");
   const size_t TC = (size_t)T * C, TF = (size_t)T * F;
+  // Every GEMM input as a hi + lo pair: streams, and the short prompts that a model without row copies would feed token by
+  // token (whose persistent kernels do the same): the result is as exact whichever way it takes.
+  const bool pairs = batch_mode || (m->fmt == FMT_FP16 && !m->v5 && T < PROMPT_PAIR_ROWS);
   const bool defer_x = batch_mode || (T <= PROMPT_DEFER_ROWS && C <= PROMPT_DEFER_C);
   // activation buffers: one blob, 256-byte aligned pieces
   size_t off = 0;
@@ -1039,8 +1038,8 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   const size_t o_ids = take((size_t)T * 4), o_x = take(TC * 4), o_r = take(TC * 4), o_k = take(TC * 4), o_v = take(TC * 4),
                o_y = take(TC * 4), o_op0 = take(TC * 2), o_op1 = take(TC * 2), o_op2 = take(TC * 2), o_op3 = take(TC * 2),
                o_g = take(TC * 2), o_yn = take(TC * 2), o_kk = take(TF * 2), o_lo0 = take(TC * 2), o_lo1 = take(TC * 2),
-               o_lo2 = take(batch_mode ? TC * 2 : 0), o_lo3 = take(batch_mode ? TC * 2 : 0), o_ynlo = take(batch_mode ? TC * 2 : 0),
-               o_kklo = take(batch_mode ? TF * 2 : 0), o_glo = take(batch_mode ? TC * 2 : 0),
+               o_lo2 = take(pairs ? TC * 2 : 0), o_lo3 = take(pairs ? TC * 2 : 0), o_ynlo = take(pairs ? TC * 2 : 0),
+               o_kklo = take(pairs ? TF * 2 : 0), o_glo = take(pairs ? TC * 2 : 0),
                o_x2 = take(!batch_mode && defer_x ? TC * 4 : 0),   // the residual rows of a short prompt alternate between two buffers
                o_raw = take(T <= GEMM_SMALL_M ? (size_t)GEMM_SPLIT_MAX * T * std::max(4 * C, F + C) * 4 : 0);   // split-K slabs
   // Long prompts are cut into pieces of rows that run on streams of their own, a layer apart: piece p's layer l needs
@@ -1076,11 +1075,10 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   __half *op_all[4] = {(__half *)(B + o_op0), (__half *)(B + o_op1), (__half *)(B + o_op2), (__half *)(B + o_op3)};
   __half *g_all = (__half *)(B + o_g), *yn_all = (__half *)(B + o_yn), *kk_all = (__half *)(B + o_kk);   // (the ffn receptance reuses g)
   __half *lo0_all = (__half *)(B + o_lo0), *lo1_all = (__half *)(B + o_lo1);
-  // batch mode keeps every GEMM input as a hi + lo pair: the steps are bound by weight bytes, not flops, and the
-  // per-stream error must not depend on how many streams share the step
-  __half *lo2_all = batch_mode ? (__half *)(B + o_lo2) : nullptr, *lo3_all = batch_mode ? (__half *)(B + o_lo3) : nullptr;
-  __half *ynlo_all = batch_mode ? (__half *)(B + o_ynlo) : nullptr, *kklo_all = batch_mode ? (__half *)(B + o_kklo) : nullptr;
-  __half *glo_all = batch_mode ? (__half *)(B + o_glo) : nullptr;
+  // (streams: the steps are bound by weight bytes, not flops, and the per-stream error must not depend on how many streams share the step)
+  __half *lo2_all = pairs ? (__half *)(B + o_lo2) : nullptr, *lo3_all = pairs ? (__half *)(B + o_lo3) : nullptr;
+  __half *ynlo_all = pairs ? (__half *)(B + o_ynlo) : nullptr, *kklo_all = pairs ? (__half *)(B + o_kklo) : nullptr;
+  __half *glo_all = pairs ? (__half *)(B + o_glo) : nullptr;
   cudaStream_t st_main = st;
   if (ids != d_ids) CU(cudaMemcpyAsync(d_ids, ids, (size_t)T * 4, cudaMemcpyDefault, st));
   CU(launch_gather_emb(m->d_emb, m->emb_dtype == FR_B200_T_F32, d_ids, T, C, x, st));
@@ -1230,7 +1228,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     la.x = x; la.ln_w = vp(b + "ln2.weight"); la.ln_b = vp(b + "ln2.bias");
     la.mix[0] = vp(f + "time_mix_k"); la.mix[1] = vp(f + "time_mix_r");
     la.op[0] = op[0]; la.op[1] = op[1];
-    la.op_lo[0] = batch_mode ? lo0 : nullptr; la.op_lo[1] = batch_mode ? lo1 : nullptr;
+    la.op_lo[0] = pairs ? lo0 : nullptr; la.op_lo[1] = pairs ? lo1 : nullptr;
     la.sx_rd = stb + off_ffn_sx(C, H, m->v5, af, par); la.sx_wr = stb + off_ffn_sx(C, H, m->v5, af, par ^ 1);
     la.T = T; la.C = C; la.nvec = 2; la.act_fp16 = af;
     la.batch_mode = batch_mode; la.state_stride = m->state_stride;
@@ -1239,8 +1237,8 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     CU(launch_ln_mix_seq(la, st));
     const bool halve = af && (l + 1) % 6 == 0;   // x / 2 every 6 layers under fp16 activations (model_forward_seq.cpp:165-167)
     {
-      GemmArgs grp[2] = {mk(T, op[0], f + "key.weight", F, C, GEMM_EPI_RELU2_F16, kk, nullptr, nullptr, 1.f, batch_mode ? lo0 : nullptr),
-                         mk(T, op[1], f + "receptance.weight", C, C, GEMM_EPI_SIGMOID_F16, rr, nullptr, nullptr, 1.f, batch_mode ? lo1 : nullptr)};
+      GemmArgs grp[2] = {mk(T, op[0], f + "key.weight", F, C, GEMM_EPI_RELU2_F16, kk, nullptr, nullptr, 1.f, pairs ? lo0 : nullptr),
+                         mk(T, op[1], f + "receptance.weight", C, C, GEMM_EPI_SIGMOID_F16, rr, nullptr, nullptr, 1.f, pairs ? lo1 : nullptr)};
       grp[0].out_lo = kk_lo; grp[1].out_lo = rr_lo;
       give_raw(grp, 2);
       CU(launch_gemm_group(grp, 2, mt, st));
@@ -1306,12 +1304,13 @@ int fr_b200_run_seq(fr_b200_model *m, int slot, const int32_t *ids, int n, float
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int seq_min = 2;   // shorter prompts take the token loop
   if (const char *e = getenv("FR_B200_SEQ_MIN")) seq_min = atoi(e);
-  // fp16 RWKV-4 models build their row copies (as many bytes as the weights) when the first prompt of 32 tokens or more
-  // arrives; until then shorter ones go token by token, which is the slower way from 3 tokens on.  1.5B shape, ms: 2 tokens 1.29
-  // by the token loop, 1.28 by rows; 3: 1.91, 1.28; 29: 18.2, 1.34; the first prompt of 32 17.9, the next 1.35.  0.1B shape: 2:
-  // 0.38, 0.43; 3: 0.56, 0.43; 29: 5.1, 0.45; the first of 32 13.4, then 0.45.
+  // fp16 RWKV-4 models build their row copies (as many bytes as the weights) when the first prompt of PROMPT_BUILD_ROWS tokens or
+  // more arrives; until then shorter ones go token by token, which is the slower way from 3 tokens on.  The line lies where the
+  // first prompt, which pays for the copies, is no slower than by the token loop at the 1.5B shape.  In ms there: a token 0.66, a prompt of
+  // 2 to 12 tokens 1.25 to 1.28 by rows, the first one 5.3 (5.3 for 8 tokens by the loop); 29 tokens 1.34 against 18.2.  0.1B shape: a token 0.21,
+  // 2 to 12 tokens 0.42 to 0.43, the first one 5; 14B shape: 5.07, 6.7, 22.
   bool by_rows = rows_path_built(m) && n >= seq_min;
-  if (!by_rows && m->fmt == FMT_FP16 && m->row_copies && m->plain_halfs && n >= std::max(seq_min, 32)) {
+  if (!by_rows && m->fmt == FMT_FP16 && m->row_copies && m->plain_halfs && n >= std::max(seq_min, PROMPT_BUILD_ROWS)) {
     CU(cudaSetDevice(m->device));
     int rc = ensure_row_copies(m);
     if (rc) return rc;

@@ -285,4 +285,7 @@ cudaError_t launch_pack(int fmt, const void *src, const __half *scales, int K, i
 cudaError_t launch_unpack(int fmt, const uint8_t *tiles, size_t item_stride, const __half *rscale,
                           size_t rscale_stride, int K, int N, float *W, cudaStream_t st);
 
+// fp16 tiles -> W^T [N, K] row-major
+cudaError_t launch_tiles_to_rows_f16(const uint8_t *tiles, size_t item_stride, int K, int N, __half *rows, cudaStream_t st);
+
 }  // namespace frb

@@ -190,6 +190,26 @@ __global__ void k_unpack(int fmt, const uint8_t *tiles, size_t item_stride, cons
   W[i] = v;
 }
 
+// fp16 tiles -> W^T [N, K]: a warp per chunk of 64 inputs x 16 rows, 16 bytes per lane and MMA = 4 consecutive inputs of rows g
+// and g + 8; four lanes make a 32-byte sector of an output row.  Memory bound: all projections of the 1.5B shape, 2 x 2.6 GB.
+__global__ void __launch_bounds__(256) k_tiles_to_rows_f16(const uint8_t *tiles, size_t item_stride, int K, int N, __half *rows) {
+  const int chunks = K / CHUNK_K, lane = threadIdx.x & 31;
+  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int rb = (int)(w / chunks), c = (int)(w - (long long)rb * chunks);
+  if (rb * ROWS >= N) return;
+  const uint4 *src = reinterpret_cast<const uint4 *>(tiles + (size_t)rb * item_stride + chunk_off(FMT_FP16, c)) + lane;
+  const int n = rb * ROWS + (lane >> 2);
+  __half *dst = rows + (size_t)n * K + c * CHUNK_K + (lane & 3) * 4;
+  uint4 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = src[j * 32];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (n < N) *reinterpret_cast<uint2 *>(dst + j * 16) = make_uint2(v[j].x, v[j].z);
+    if (n + 8 < N) *reinterpret_cast<uint2 *>(dst + (size_t)8 * K + j * 16) = make_uint2(v[j].y, v[j].w);
+  }
+}
+
 inline unsigned blocks_for(size_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 }  // namespace
@@ -251,6 +271,12 @@ cudaError_t launch_pack(int fmt, const void *src, const __half *scales, int K, i
 cudaError_t launch_unpack(int fmt, const uint8_t *tiles, size_t item_stride, const __half *rscale, size_t rscale_stride,
                           int K, int N, float *W, cudaStream_t st) {
   k_unpack<<<blocks_for((size_t)K * N, 256), 256, 0, st>>>(fmt, tiles, item_stride, rscale, rscale_stride, K, N, W);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tiles_to_rows_f16(const uint8_t *tiles, size_t item_stride, int K, int N, __half *rows, cudaStream_t st) {
+  const size_t warps = (size_t)((N + ROWS - 1) / ROWS) * (K / CHUNK_K);
+  k_tiles_to_rows_f16<<<blocks_for(warps, 8), 256, 0, st>>>(tiles, item_stride, K, N, rows);
   return cudaGetLastError();
 }
 

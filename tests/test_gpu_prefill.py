@@ -197,6 +197,23 @@ def test_long_prompts_in_pipelined_pieces(pkg, orc, synth, monkeypatch, name, st
     m.close()
 
 
+@pytest.mark.parametrize("name,T", [("tiny4b", 7), ("tiny4b", 8), ("mid4", 31), ("mid4", 32)])
+def test_short_fp16_prompts_of_rwkv4(pkg, orc, synth, name, T):
+    """fp16 RWKV-4 prompts: token by token up to 7 tokens, by rows with every operand as a pair up to 31 (the first such prompt
+    builds the row copies out of the streaming tiles, ragged in N for the 211-word head), single halves from 32 on.  With
+    pairs an operand is off by 2^-22 of itself, so what is left over 7 layers is the fp16 shift state both sides round."""
+    shape, tensors, ref = _models(pkg, orc, synth, name)
+    ids = [int(t) for t in synth.token_ids(shape, 2 * T, seed=2)]
+    m = pkg.Model(tensors, "cuda fp16", shape=shape)
+    for part in (ids[:T], ids[T:]):
+        got, want = m.run(part), ref.run_seq(part)
+        _close(got, want, f"{name} T={T}")
+        if T < 32:
+            assert np.linalg.norm(got - want) / np.linalg.norm(want) < 3e-4
+    _close(m.run(7), ref.run(7), "token after the prompts")
+    m.close()
+
+
 @pytest.mark.parametrize("T", [2, 64, 65, 257, 769, 1023, 1090])
 def test_rwkv4_prompt_scan(pkg, orc, synth, T):
     """RWKV-4 prompts are scanned in 64 chunks (of 1, 2, 5, 13, 16 and 18 tokens here; the last ones short or empty):
