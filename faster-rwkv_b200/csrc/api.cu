@@ -42,6 +42,7 @@ struct MatrixSlot {       // where a projection matrix lives inside the packed w
   size_t pscale_off = 0;  // int8: offset of the [N] output-row scales that go with the copy (the copy holds the codes)
   size_t q_off = 0;       // int8 / int4: byte offset of the row-major packed copy ([N, K] codes or [N, K/2] nibbles)
   size_t qs_off = 0;      // int4: offset (halfs) of its [N, K/32] group scales
+  WeightMap wmap;         // the copy's tensor map (encoded by the first GEMM over it)
 };
 
 struct VecSlot {
@@ -99,6 +100,10 @@ struct fr_b200_model {
   size_t scratch_bytes[4] = {0, 0, 0, 0};
   // bookkeeping
   std::map<std::string, MatrixSlot> mats;
+  // the layers' vectors and matrices by place (a forward pass of few rows enqueues 170 launches in little more than the GPU takes)
+  struct LayerMats { MatrixSlot *key, *value, *receptance, *gate, *output, *ffn_key, *ffn_receptance, *ffn_value; };
+  std::vector<LayerDev> layer_vecs;
+  std::vector<LayerMats> layer_mats;
   std::map<std::string, VecSlot> vecs;
   std::vector<char> emb_rows_set;
   bool emb_set = false;
@@ -560,6 +565,15 @@ int fr_b200_finalize(fr_b200_model *m) {
     if (m->v5) { d.lnx_w = vp(a + "ln_x.weight"); d.lnx_b = vp(a + "ln_x.bias"); }
   }
   CU(cudaMemcpy(m->d_layers, layers.data(), sizeof(LayerDev) * m->L, cudaMemcpyHostToDevice));
+  m->layer_vecs = layers;
+  m->layer_mats.clear();
+  for (int l = 0; l < m->L; ++l) {
+    const std::string b = "blocks." + std::to_string(l) + ".", a = b + "att.", f = b + "ffn.";
+    m->layer_mats.push_back({&m->mats[a + "key.weight"], &m->mats[a + "value.weight"], &m->mats[a + "receptance.weight"],
+                             m->gate ? &m->mats[a + "gate.weight"] : nullptr, &m->mats[a + "output.weight"],
+                             &m->mats[f + "key.weight"], &m->mats[f + "receptance.weight"], &m->mats[f + "value.weight"]});
+  }
+  CU(gemm_prepare(m->device));
   // kernel geometry: as many ring stages as shared memory allows (capped), one CTA per SM
   int optin = 0;
   CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device));
@@ -1084,11 +1098,13 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   CU(launch_gather_emb(m->d_emb, m->emb_dtype == FR_B200_T_F32, d_ids, T, C, x, st));
   auto vp = [&](const std::string &n) -> const float * { return m->d_vecs + m->vecs[n].off; };
   const bool quant = m->fmt != FMT_FP16;
-  auto mk = [&](int rows, const __half *A, const std::string &w, int N, int K, int epi, void *out, const void *aux0, const void *aux1,
+  GemmMapCache map_cache;
+  auto mk = [&](int rows, const __half *A, MatrixSlot *w, int N, int K, int epi, void *out, const void *aux0, const void *aux1,
                 float scale, const __half *A2 = nullptr) -> GemmArgs {
     GemmArgs ga;
     memset(&ga, 0, sizeof(ga));
-    const MatrixSlot &ms = m->mats[w];
+    MatrixSlot &ms = *w;
+    ga.wmap = &ms.wmap; ga.maps = &map_cache;
     ga.A = A; ga.A2 = A2; ga.M = rows;
     if (quant) {
       ga.Wq = m->d_qcopy + ms.q_off; ga.wfmt = m->fmt;
@@ -1101,7 +1117,6 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     ga.scale = scale; ga.status = m->out_status(); ga.fixed_split = m->v5;
     return ga;
   };
-  const int mt = Tp > 128 ? 2 : 1;   // 256-row tiles once the rows fill them
   // few rows: every GEMM of a launch gets its own run of split-K slabs
   auto give_raw = [&](GemmArgs *grp, int n) {
     if (T > GEMM_SMALL_M) return;
@@ -1140,7 +1155,8 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   };
   for (int l = 0; l < m->L; ++l)
   for (int pc = 0; pc < n_pieces; ++pc) {
-    const std::string b = "blocks." + std::to_string(l) + ".", a = b + "att.", f = b + "ffn.";
+    const LayerDev &lv = m->layer_vecs[l];
+    const fr_b200_model::LayerMats &lm = m->layer_mats[l];
     uint8_t *stb = st0 + (size_t)l * m->layer_stride;
     // this piece's rows of every activation buffer, its stream, its copy of the shift states (they alternate piece by
     // piece exactly as they alternate token by token) and its scan scratch
@@ -1165,9 +1181,8 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     // ---- time mix ----
     SeqLnArgs la;
     memset(&la, 0, sizeof(la));
-    la.x = x; la.ln_w = vp(b + "ln1.weight"); la.ln_b = vp(b + "ln1.bias");
-    la.mix[0] = vp(a + "time_mix_k"); la.mix[1] = vp(a + "time_mix_v"); la.mix[2] = vp(a + "time_mix_r");
-    if (m->gate) la.mix[3] = vp(a + "time_mix_g");
+    la.x = x; la.ln_w = lv.ln1_w; la.ln_b = lv.ln1_b;
+    for (int i = 0; i < 4; ++i) la.mix[i] = lv.att_mix[i];
     for (int i = 0; i < 4; ++i) la.op[i] = op[i];
     la.sx_rd = stb + off_sx(C, af, par); la.sx_wr = stb + off_sx(C, af, par ^ 1);
     la.T = T; la.C = C; la.nvec = nvec; la.act_fp16 = af;
@@ -1183,30 +1198,30 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     const float *kvr_raw[3] = {nullptr, nullptr, nullptr};
     {
       // the attention projections in one launch; the two with a second pass over K first
-      GemmArgs grp[4] = {mk(T, op[0], a + "key.weight", C, C, GEMM_EPI_F32, k, nullptr, nullptr, 1.f, lo0),
-                         mk(T, op[1], a + "value.weight", C, C, GEMM_EPI_F32, v, nullptr, nullptr, 1.f, lo1),
-                         mk(T, op[2], a + "receptance.weight", C, C, GEMM_EPI_F32, r, nullptr, nullptr, 1.f, lo2),
-                         mk(T, op[2], a + "receptance.weight", C, C, GEMM_EPI_F32, r, nullptr, nullptr, 1.f, lo2)};
-      if (m->gate) { grp[3] = mk(T, op[3], a + "gate.weight", C, C, GEMM_EPI_SILU_F16, g, nullptr, nullptr, 1.f, lo3); grp[3].out_lo = g_lo; }
+      GemmArgs grp[4] = {mk(T, op[0], lm.key, C, C, GEMM_EPI_F32, k, nullptr, nullptr, 1.f, lo0),
+                         mk(T, op[1], lm.value, C, C, GEMM_EPI_F32, v, nullptr, nullptr, 1.f, lo1),
+                         mk(T, op[2], lm.receptance, C, C, GEMM_EPI_F32, r, nullptr, nullptr, 1.f, lo2),
+                         mk(T, op[2], lm.receptance, C, C, GEMM_EPI_F32, r, nullptr, nullptr, 1.f, lo2)};
+      if (m->gate) { grp[3] = mk(T, op[3], lm.gate, C, C, GEMM_EPI_SILU_F16, g, nullptr, nullptr, 1.f, lo3); grp[3].out_lo = g_lo; }
       give_raw(grp, m->gate ? 4 : 3);
       const bool defer = defer_x && !m->v5 && (batch_mode || T <= PROMPT_DEFER_KVR);
-      CU(launch_gemm_group(grp, m->gate ? 4 : 3, mt, st, defer ? &kvr_split : nullptr));
+      CU(launch_gemm_group(grp, m->gate ? 4 : 3, st, defer ? &kvr_split : nullptr));
       for (int i = 0; i < 3; ++i) { kvr_cs[i] = grp[i].col_scale; kvr_raw[i] = grp[i].raw; }
     }
     if (m->v5) {
       SeqWkvArgs wa;
       memset(&wa, 0, sizeof(wa));
-      wa.r = r; wa.k = k; wa.v = v; wa.decay = vp(a + "time_decay"); wa.first = vp(a + "time_first");
+      wa.r = r; wa.k = k; wa.v = v; wa.decay = lv.decay; wa.first = lv.first;
       wa.state = reinterpret_cast<float *>(stb + off_mid(C, af)); wa.y = y; wa.T = T; wa.C = C;
       wa.per_head = m->cfg.version == FR_B200_V5_0;
       wa.n_chunks = n_chunks; wa.chunk_len = chunk_len; wa.e_out = (float *)(B + o_e + scan_bytes * pc); wa.s_in = (float *)(B + o_sin + scan_bytes * pc);
       wa.batch_mode = batch_mode; wa.state_stride = m->state_stride / 4;
       CU(launch_wkv5_seq(wa, H, st));
-      CU(launch_gn_gate_seq(y, vp(a + "ln_x.weight"), vp(a + "ln_x.bias"), m->gate ? g : nullptr, m->gate ? g_lo : nullptr, T, H, yn, yn_lo, st));
+      CU(launch_gn_gate_seq(y, lv.lnx_w, lv.lnx_b, m->gate ? g : nullptr, m->gate ? g_lo : nullptr, T, H, yn, yn_lo, st));
     } else {
       Wkv4Args wa;
       memset(&wa, 0, sizeof(wa));
-      wa.k = k; wa.v = v; wa.r = r; wa.decay = vp(a + "time_decay"); wa.first = vp(a + "time_first");
+      wa.k = k; wa.v = v; wa.r = r; wa.decay = lv.decay; wa.first = lv.first;
       wa.state = stb + off_mid(C, af); wa.state_stride = m->state_stride; wa.out = yn; wa.out_lo = yn_lo; wa.T = T; wa.C = C; wa.batch_mode = batch_mode;
       if (kvr_split > 1) {
         wa.split = kvr_split;
@@ -1216,17 +1231,16 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
       CU(launch_wkv4_rows(wa, st));
     }
     {
-      GemmArgs go = mk(T, yn, a + "output.weight", C, C, GEMM_EPI_ADD_F32, x, x, nullptr, 1.f, yn_lo);
+      GemmArgs go = mk(T, yn, lm.output, C, C, GEMM_EPI_ADD_F32, x, x, nullptr, 1.f, yn_lo);
       give_raw(&go, 1);
-      // prompts: few tiles, 128-row tiles fill the SMs better (measured); streams: one pass over the weights for all rows
       int sp = 1;
-      CU(launch_gemm_group(&go, 1, batch_mode ? mt : 1, st, defer_x ? &sp : nullptr));
+      CU(launch_gemm_group(&go, 1, st, defer_x ? &sp : nullptr));
       if (sp > 1) pend_x = {go.raw, go.col_scale, nullptr, nullptr, go.scale, sp};
     }
     // ---- channel mix ----
     memset(&la, 0, sizeof(la));
-    la.x = x; la.ln_w = vp(b + "ln2.weight"); la.ln_b = vp(b + "ln2.bias");
-    la.mix[0] = vp(f + "time_mix_k"); la.mix[1] = vp(f + "time_mix_r");
+    la.x = x; la.ln_w = lv.ln2_w; la.ln_b = lv.ln2_b;
+    la.mix[0] = lv.ffn_mix[0]; la.mix[1] = lv.ffn_mix[1];
     la.op[0] = op[0]; la.op[1] = op[1];
     la.op_lo[0] = pairs ? lo0 : nullptr; la.op_lo[1] = pairs ? lo1 : nullptr;
     la.sx_rd = stb + off_ffn_sx(C, H, m->v5, af, par); la.sx_wr = stb + off_ffn_sx(C, H, m->v5, af, par ^ 1);
@@ -1237,16 +1251,16 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     CU(launch_ln_mix_seq(la, st));
     const bool halve = af && (l + 1) % 6 == 0;   // x / 2 every 6 layers under fp16 activations (model_forward_seq.cpp:165-167)
     {
-      GemmArgs grp[2] = {mk(T, op[0], f + "key.weight", F, C, GEMM_EPI_RELU2_F16, kk, nullptr, nullptr, 1.f, pairs ? lo0 : nullptr),
-                         mk(T, op[1], f + "receptance.weight", C, C, GEMM_EPI_SIGMOID_F16, rr, nullptr, nullptr, 1.f, pairs ? lo1 : nullptr)};
+      GemmArgs grp[2] = {mk(T, op[0], lm.ffn_key, F, C, GEMM_EPI_RELU2_F16, kk, nullptr, nullptr, 1.f, pairs ? lo0 : nullptr),
+                         mk(T, op[1], lm.ffn_receptance, C, C, GEMM_EPI_SIGMOID_F16, rr, nullptr, nullptr, 1.f, pairs ? lo1 : nullptr)};
       grp[0].out_lo = kk_lo; grp[1].out_lo = rr_lo;
       give_raw(grp, 2);
-      CU(launch_gemm_group(grp, 2, mt, st));
-      GemmArgs gv = mk(T, kk, f + "value.weight", C, F, GEMM_EPI_MULADD_F32, x, x, rr, halve ? 0.5f : 1.f, kk_lo);
+      CU(launch_gemm_group(grp, 2, st));
+      GemmArgs gv = mk(T, kk, lm.ffn_value, C, F, GEMM_EPI_MULADD_F32, x, x, rr, halve ? 0.5f : 1.f, kk_lo);
       gv.aux1_lo = rr_lo;
       give_raw(&gv, 1);
       int sp = 1;
-      CU(launch_gemm_group(&gv, 1, batch_mode ? mt : 1, st, defer_x && (batch_mode || l + 1 < m->L) ? &sp : nullptr));
+      CU(launch_gemm_group(&gv, 1, st, defer_x && (batch_mode || l + 1 < m->L) ? &sp : nullptr));
       if (sp > 1) pend_x = {gv.raw, gv.col_scale, rr, rr_lo, gv.scale, sp};
     }
     m->launches += m->v5 ? 9 : 7;
@@ -1264,10 +1278,10 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     la.T = T; la.C = C; la.nvec = 0; la.act_fp16 = af; la.batch_mode = 1;
     take_pending(la, x);
     CU(launch_ln_mix_seq(la, st));
-    GemmArgs gh = mk(T, op_all[0], "head.weight", m->V, C, GEMM_EPI_F32, m->d_out, nullptr, nullptr, 1.f, lo0_all);
+    GemmArgs gh = mk(T, op_all[0], &m->mats["head.weight"], m->V, C, GEMM_EPI_F32, m->d_out, nullptr, nullptr, 1.f, lo0_all);
     gh.ldo = m->Vpad;
     // (no split-K scratch for the head: it has a thousand column tiles of its own)
-    CU(launch_gemm_group(&gh, 1, mt, st));
+    CU(launch_gemm_group(&gh, 1, st));
     m->launches += 2;
     for (int bq = 0; bq < R; ++bq) m->par[bq] ^= 1u;
     return 0;

@@ -162,6 +162,17 @@ enum GemmEpilogue {
   GEMM_EPI_MULADD_F32,      // out f32 = (aux0 + aux1 * acc) * scale         (aux1 f16 [M, N])
   GEMM_EPI_PLAIN_F16        // out f16 = acc
 };
+// Encoded tensor maps that a caller with many GEMMs keeps: one per weight matrix for good, those of the activations for the
+// length of one forward pass (every layer uses the same buffers).
+struct alignas(64) TensorMapBytes { unsigned char b[128]; };
+struct WeightMap { TensorMapBytes map; bool set = false; };
+struct GemmMapCache {
+  static constexpr int MAX = 48;
+  struct Key { const void *base; int rows, cols, box, kind; };
+  int n = 0;
+  Key key[MAX];
+  TensorMapBytes map[MAX];
+};
 struct GemmArgs {
   const __half *A;     // [M, K] row-major
   const __half *A2;    // optional [M, K]: low halves of the activations (A + A2 is the fp32 value to ~22 bits)
@@ -181,6 +192,8 @@ struct GemmArgs {
   float scale;
   int *status;         // device word: set when a bounded wait gives up
   float *raw;          // optional scratch [GEMM_SPLIT_MAX][M][N] f32: allows split-K when M <= GEMM_SMALL_M
+  WeightMap *wmap;     // host, optional: the map of Bt or Wq
+  GemmMapCache *maps;  // host, optional
   int tma_out;         // set by the launcher: out (and out_lo) are written by tensor stores
   int fixed_split;     // 1: K is cut the same way whatever kernel serves the product (RWKV-5, see launch_gemm_pair)
 };
@@ -188,9 +201,10 @@ constexpr int GEMM_GROUP_MAX = 4;
 constexpr int GEMM_SMALL_M = 1024;    // up to this many rows the GEMM puts the weights along the MMA rows (and splits K, given scratch)
 constexpr int GEMM_SPLIT_MAX = 16;
 int device_sm_count();   // SMs of the current device
-cudaError_t launch_gemm_f16(const GemmArgs &g, cudaStream_t st);   // one GEMM; 256-row tiles when M > 128
-// n <= 4 GEMMs with equal M in one launch; mt = 128-row sub-tiles per CTA (1 or 2)
-cudaError_t launch_gemm_group(const GemmArgs *probs, int n, int mt, cudaStream_t st, int *defer_split = nullptr);
+cudaError_t launch_gemm_f16(const GemmArgs &g, cudaStream_t st);   // one GEMM
+// n <= 4 GEMMs with equal M in one launch, after gemm_prepare() for the device
+cudaError_t launch_gemm_group(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split = nullptr);
+cudaError_t gemm_prepare(int device);   // kernel attributes
 // row kernels of seq mode
 struct SeqLnArgs {
   const float *x;            // [T, C] residual stream

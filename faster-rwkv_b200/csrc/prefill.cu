@@ -1009,62 +1009,89 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [rows, K] fp16 row-major -> tensor map with a (64 x box_rows) box, 128-byte swizzle, zero fill outside
-bool make_map(CUtensorMap *map, const void *base, int rows, int K, int box_rows) {
+bool encode_map(CUtensorMap *map, CUtensorMapDataType type, int rank, void *base, const cuuint64_t *dims, const cuuint64_t *strides,
+                const cuuint32_t *box, bool swizzle, bool promote) {
   EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn && fn(map, type, (cuuint32_t)rank, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  promote ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+static_assert(sizeof(CUtensorMap) == sizeof(TensorMapBytes), "tensor maps are kept as bytes");
+// An activation's map out of the forward pass's cache, or encoded.  (A map takes about 0.2 us, a launch of few rows needs up to 15.)
+template <typename Encode>
+bool cached_map(GemmMapCache *c, CUtensorMap *map, const GemmMapCache::Key &k, Encode encode) {
+  if (c)
+    for (int i = 0; i < c->n; ++i)
+      if (c->key[i].base == k.base && c->key[i].rows == k.rows && c->key[i].cols == k.cols && c->key[i].box == k.box && c->key[i].kind == k.kind) {
+        memcpy(map, &c->map[i], sizeof(*map));
+        return true;
+      }
+  if (!encode()) return false;
+  if (c && c->n < GemmMapCache::MAX) {
+    c->key[c->n] = k;
+    memcpy(&c->map[c->n++], map, sizeof(*map));
+  }
+  return true;
+}
+bool encode_rows_f16(CUtensorMap *map, const void *base, int rows, int K, int box_rows) {
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)K * 2};
   const cuuint32_t box[2] = {(cuuint32_t)GBK, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, true, true);
 }
-
-// [rows, row_bytes] bytes row-major -> tensor map with a (128 bytes x 128 rows) box, 128-byte swizzle, zero fill outside
-bool make_map_bytes(CUtensorMap *map, const void *base, int rows, int row_bytes) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t box[2] = {128, (cuuint32_t)GBM};
-  const cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+// X [rows, K] fp16 row-major -> tensor map with a (64 x box_rows) box, 128-byte swizzle, zero fill outside
+bool make_map_x(CUtensorMap *map, const GemmArgs &g, const __half *X, int box_rows) {
+  return cached_map(g.maps, map, {X, g.M, g.K, box_rows, 0}, [&] { return encode_rows_f16(map, X, g.M, g.K, box_rows); });
 }
-
+// the weights: [N, K] fp16 row-major in (64 x 128 rows) boxes, or [N, packed row] bytes in (128 bytes x 128 rows) boxes, 128-byte swizzle
+bool make_map_w(CUtensorMap *map, const GemmArgs &g) {
+  if (g.wmap && g.wmap->set) { memcpy(map, &g.wmap->map, sizeof(*map)); return true; }
+  bool ok;
+  if (g.Wq) {
+    const int row_bytes = g.wfmt == FMT_INT8 ? g.K : g.K / 2;
+    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)g.N}, strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {128, (cuuint32_t)GBM};
+    ok = encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(g.Wq), dims, strides, box, true, true);
+  } else {
+    ok = encode_rows_f16(map, g.Bt, g.N, g.K, GBM);
+  }
+  if (ok && g.wmap) { memcpy(&g.wmap->map, map, sizeof(*map)); g.wmap->set = true; }
+  return ok;
+}
 // [planes, rows, cols] of fp16 or fp32 with rows `ld` elements and planes rows x ld elements apart -> tensor map with a
 // (32 cols x 32 rows) box
-bool make_map_out(CUtensorMap *map, void *base, bool f32, int cols, int rows, int planes, int ld) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  const size_t elt = f32 ? 4 : 2;
-  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)planes};
-  const cuuint64_t strides[2] = {(cuuint64_t)ld * elt, (cuuint64_t)ld * elt * rows};
-  const cuuint32_t box[3] = {32, 32, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+bool make_map_out(CUtensorMap *map, const GemmArgs &g, void *base, bool f32, int planes, int ld) {
+  return cached_map(g.maps, map, {base, g.M, g.N, ld, (f32 ? 2 : 1) + 4 * planes}, [&] {
+    const size_t elt = f32 ? 4 : 2;
+    const cuuint64_t dims[3] = {(cuuint64_t)g.N, (cuuint64_t)g.M, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)ld * elt, (cuuint64_t)ld * elt * g.M};
+    const cuuint32_t box[3] = {32, 32, 1};
+    return encode_map(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, false, false);
+  });
 }
 // where a group's results go: slabs when K is split, else the outputs, as tensors when their rows allow it
 bool make_out_maps(GemmMaps &maps, GemmGroup &grp) {
-  for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
-    if (i >= grp.n) { maps.o[i] = maps.o[0]; maps.o_lo[i] = maps.o_lo[0]; continue; }
+  for (int i = 0; i < grp.n; ++i) {
     GemmArgs &g = grp.p[i];
     g.tma_out = 0;
-    maps.o[i] = maps.o_lo[i] = maps.a[0];
     if (grp.split > 1) {
-      if (!make_map_out(&maps.o[i], g.raw, true, g.N, g.M, grp.split, g.N)) return false;
+      if (!make_map_out(&maps.o[i], g, g.raw, true, grp.split, g.N)) return false;
       continue;
     }
     const bool f32 = g.epi == GEMM_EPI_F32 || g.epi == GEMM_EPI_ADD_F32 || g.epi == GEMM_EPI_MULADD_F32;
     if (((size_t)g.ldo * (f32 ? 4 : 2)) % 16 || (reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.out_lo)) % 16) continue;
     g.tma_out = 1;
-    if (!make_map_out(&maps.o[i], g.out, f32, g.N, g.M, 1, g.ldo)) return false;
-    if (!f32 && g.out_lo && !make_map_out(&maps.o_lo[i], g.out_lo, false, g.N, g.M, 1, g.ldo)) return false;
+    if (!make_map_out(&maps.o[i], g, g.out, f32, 1, g.ldo)) return false;
+    if (!f32 && g.out_lo && !make_map_out(&maps.o_lo[i], g, g.out_lo, false, 1, g.ldo)) return false;
+  }
+  return true;
+}
+// X and weights of a group (the maps of problems that do not exist are not read)
+bool make_in_maps(GemmMaps &maps, const GemmGroup &grp, int box_rows) {
+  for (int i = 0; i < grp.n; ++i) {
+    const GemmArgs &g = grp.p[i];
+    if (!make_map_x(&maps.a[i], g, g.A, box_rows) || !make_map_w(&maps.b[i], g)) return false;
+    if (g.A2 && !make_map_x(&maps.a2[i], g, g.A2, box_rows)) return false;
   }
   return true;
 }
@@ -1919,13 +1946,6 @@ cudaError_t launch_ln_row(const float *x, const float *w, const float *b, int C,
 }
 
 namespace {
-template <int BN>
-cudaError_t launch_gemm_wt_t(const GemmMaps &maps, const GemmGroup &grp, dim3 grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(gemm_wt_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  launch_k(gemm_wt_kernel<BN>, dim3(grid), dim3(G_THREADS), smem, st, maps, grp);
-  return cudaGetLastError();
-}
 
 // In how many pieces K is cut for `ctas` tiles of which a device holds `slots`: the cost of a split, in K slices of one CTA, is
 // waves x (slices per CTA + fill and drain) + the slabs it adds.
@@ -1958,8 +1978,6 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
     if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
       return cudaErrorInvalidValue;
-    if (!make_map(&maps.a[i], g.A, g.M, g.K, bn) || !make_map(&maps.b[i], g.Bt, g.N, g.K, GBM)) return cudaErrorNotSupported;
-    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, bn)) return cudaErrorNotSupported;
     grp.p[i] = g;
     grp.tile_start[i] = tiles;
     tiles += (g.N + GBM - 1) / GBM;
@@ -1967,7 +1985,7 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
     raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
     if (g.A2) grp.dual = 1;
   }
-  for (int i = n; i < GEMM_GROUP_MAX; ++i) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; }
+  if (!make_in_maps(maps, grp, bn)) return cudaErrorNotSupported;
   grp.tile_start[n] = tiles;
   const int m_tiles = (M + bn - 1) / bn;
   // one CTA per SM, none waiting for a second wave: split K until the tiles about cover the SMs
@@ -1986,9 +2004,8 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
   dim3 grid(tiles, m_tiles, grp.split);
-  cudaError_t e = bn == 32    ? launch_gemm_wt_t<32>(maps, grp, grid, smem, st)
-                  : bn == 64  ? launch_gemm_wt_t<64>(maps, grp, grid, smem, st)
-                              : launch_gemm_wt_t<128>(maps, grp, grid, smem, st);
+  auto kern = bn == 32 ? gemm_wt_kernel<32> : bn == 64 ? gemm_wt_kernel<64> : gemm_wt_kernel<128>;
+  cudaError_t e = launch_k(kern, grid, dim3(G_THREADS), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
@@ -2056,20 +2073,15 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   }
   grp.m_tiles = (M + grp.bn - 1) / grp.bn;
   grp.lo_each = M <= GEMM_SMALL_M;
-  for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
-    const GemmArgs &g = probs[i < n ? i : 0];
-    if (!make_map(&maps.a[i], g.A, g.M, g.K, grp.bn / 2) || !make_map(&maps.b[i], g.Bt, g.N, g.K, GBM)) return cudaErrorNotSupported;
-    if (!make_map(&maps.a2[i], g.A2 ? g.A2 : g.A, g.M, g.K, grp.bn / 2)) return cudaErrorNotSupported;
-  }
+  if (!make_in_maps(maps, grp, grp.bn / 2)) return cudaErrorNotSupported;
   grp.stage_bytes = G_A_BYTES + (grp.lo_each && any_lo ? 2u : 1u) * (uint32_t)grp.bn * GBK;
   // tiles that have an SM each to themselves take a ring of twice the depth
   const bool alone = tiles * grp.m_tiles * grp.split <= num_pairs;
   grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((alone ? 200u << 10 : 110u << 10) / grp.stage_bytes));
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
-  cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = launch_cluster_k(gemm_pair_kernel, 2, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
-  if ((e = launch_cluster_k(gemm_pair_kernel, 2, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
     int max_n = 0;
@@ -2138,13 +2150,7 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
   }
   grp.m_tiles = (M + grp.bn - 1) / grp.bn;
   const int xrows = pair ? grp.bn / 2 : grp.bn;
-  for (int i = 0; i < GEMM_GROUP_MAX; ++i) {
-    if (i >= n) { maps.a[i] = maps.a[0]; maps.a2[i] = maps.a2[0]; maps.b[i] = maps.b[0]; continue; }
-    const GemmArgs &g = probs[i];
-    if (!make_map(&maps.a[i], g.A, g.M, g.K, xrows) || !make_map_bytes(&maps.b[i], g.Wq, g.N, fmt == FMT_INT8 ? g.K : g.K / 2)) return cudaErrorNotSupported;
-    maps.a2[i] = maps.a[i];
-    if (g.A2 && !make_map(&maps.a2[i], g.A2, g.M, g.K, xrows)) return cudaErrorNotSupported;
-  }
+  if (!make_in_maps(maps, grp, xrows)) return cudaErrorNotSupported;
   grp.stage_bytes = (any_lo ? 2u : 1u) * (uint32_t)xrows * GBK * 2;
   grp.estages = std::min<int>(GQ_MAX, (int)((grp.tmem_cols - grp.acc_cols) / a_cols));
   const uint32_t avail = (two_per_sm ? 110u : 220u) << 10, ws = GBM * 128;
@@ -2155,10 +2161,9 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
   const size_t smem = 1024 + std::max<size_t>(rings, GQ_EXP_WARPS * 2 * EPI_BUF) + 1024;
   auto kern = pair ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, true> : gemm_q_kernel<FMT_INT8, true>)
                    : (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false> : gemm_q_kernel<FMT_INT8, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   const dim3 grid((pair ? 2 : 1) * tiles * grp.m_tiles, 1, grp.split);
-  if ((e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(GQ_THREADS), smem, st, maps, grp)) != cudaSuccess) return e;
+  cudaError_t e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(GQ_THREADS), smem, st, maps, grp);
+  if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
     int max_n = 0;
@@ -2171,16 +2176,30 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
 
 // defer_split (optional): the caller's next kernel sums the split-K slabs itself (ln_mix_seq_kernel, wkv4_rows_kernel);
 // it receives the split that was chosen, 1 meaning that the outputs are already complete.
-cudaError_t launch_gemm_group(const GemmArgs *probs, int n, int mt, cudaStream_t st, int *defer_split) {
-  if (n < 1 || n > GEMM_GROUP_MAX || (mt != 1 && mt != 2)) return cudaErrorInvalidValue;
+cudaError_t launch_gemm_group(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
+  if (n < 1 || n > GEMM_GROUP_MAX) return cudaErrorInvalidValue;
   const int M = probs[0].M;
   if (defer_split) *defer_split = 1;
   if (probs[0].Wq) return launch_gemm_q(probs, n, st, defer_split);
   return M <= 128 ? launch_gemm_wt(probs, n, st, defer_split) : launch_gemm_pair(probs, n, st, defer_split);
 }
 
+cudaError_t gemm_prepare(int device) {
+  int optin = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  const void *kerns[] = {(const void *)gemm_wt_kernel<32>, (const void *)gemm_wt_kernel<64>, (const void *)gemm_wt_kernel<128>,
+                         (const void *)gemm_pair_kernel, (const void *)gemm_q_kernel<FMT_INT8, false>, (const void *)gemm_q_kernel<FMT_INT8, true>,
+                         (const void *)gemm_q_kernel<FMT_INT4, false>, (const void *)gemm_q_kernel<FMT_INT4, true>};
+  for (const void *k : kerns)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  return e;
+}
+
 cudaError_t launch_gemm_f16(const GemmArgs &g, cudaStream_t st) {
-  return launch_gemm_group(&g, 1, g.M > GBM ? 2 : 1, st, nullptr);   // no raw scratch: no split-K
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = gemm_prepare(device);
+  return e != cudaSuccess ? e : launch_gemm_group(&g, 1, st, nullptr);   // no raw scratch: no split-K
 }
 
 }  // namespace frb
