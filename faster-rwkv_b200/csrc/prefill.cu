@@ -1583,11 +1583,14 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
 
 // greedy sample of every row: index of the largest logit (lowest index on ties).  ctl (optional): the id also goes
 // to row ctl->step of the history ctl->hist -- fixed kernel arguments, so that a captured graph can be replayed.
+// A cluster of CTAs per row (gridDim.x of them), each over its part of the vocabulary: one CTA has 64 KB in flight at most, and a row of
+// 65536 logits took it 29 us; eight take 5.
 __global__ void __launch_bounds__(256) argmax_rows_kernel(const float *logits, int V, int ld, int32_t *out, const GreedyCtl *ctl) {
   pdl_trigger();
   pdl_wait();
-  __shared__ unsigned long long best[8];
-  const float *row = logits + (size_t)blockIdx.x * ld;
+  __shared__ unsigned long long best[8], parts[8];
+  const int b = blockIdx.y;
+  const float *row = logits + (size_t)b * ld;
   unsigned long long m = 0;
   auto take = [&](float f, int i) {
     unsigned u = __float_as_uint(f);
@@ -1596,13 +1599,13 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(const float *logits, i
     m = w > m ? w : m;
   };
   const int V4 = ((ld & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) ? (V & ~3) : 0;
-  // 16-byte loads, eight in flight per thread: a row is read by one CTA, so the loads in flight set its speed
+  // 16-byte loads, eight in flight per thread
 #pragma unroll 8
-  for (int i = threadIdx.x * 4; i < V4; i += blockDim.x * 4) {
+  for (int i = (blockIdx.x * 256 + threadIdx.x) * 4; i < V4; i += gridDim.x * 1024) {
     const float4 f = *reinterpret_cast<const float4 *>(row + i);
     take(f.x, i); take(f.y, i + 1); take(f.z, i + 2); take(f.w, i + 3);
   }
-  for (int i = V4 + threadIdx.x; i < V; i += blockDim.x) take(row[i], i);
+  for (int i = V4 + blockIdx.x * 256 + threadIdx.x; i < V; i += gridDim.x * 256) take(row[i], i);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long other = __shfl_xor_sync(0xffffffffu, m, o);
@@ -1612,9 +1615,16 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(const float *logits, i
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w8 = 1; w8 < 8; ++w8) m = best[w8] > m ? best[w8] : m;
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(mapa_u32(smem_u32(&parts[blockIdx.x]), 0)), "l"(m) : "memory");
+  }
+  __syncwarp();
+  cluster_sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    m = parts[0];
+    for (int r = 1; r < (int)gridDim.x; ++r) m = parts[r] > m ? parts[r] : m;
     const int32_t id = (int32_t)(0xffffffffu - (unsigned)m);
-    out[blockIdx.x] = id;
-    if (ctl) ctl->hist[(size_t)ctl->step * gridDim.x + blockIdx.x] = id;
+    out[b] = id;
+    if (ctl) ctl->hist[(size_t)ctl->step * gridDim.y + b] = id;
   }
 }
 __global__ void greedy_bump_kernel(GreedyCtl *ctl) { pdl_trigger(); pdl_wait(); ctl->step += 1; }
@@ -1931,7 +1941,10 @@ cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 cudaError_t launch_argmax_rows(const float *logits, int rows, int V, int ld, int32_t *out, GreedyCtl *ctl, cudaStream_t st) {
-  launch_k(argmax_rows_kernel, dim3(rows), dim3(256), 0, st, logits, V, ld, out, ctl);
+  // as many CTAs per row as about four per SM allow
+  const int slots = 4 * device_sm_count() / std::max(rows, 1), cluster = slots >= 8 ? 8 : slots >= 4 ? 4 : slots >= 2 ? 2 : 1;
+  const cudaError_t e = launch_cluster_k(argmax_rows_kernel, cluster, dim3(cluster, rows), dim3(256), 0, st, logits, V, ld, out, (const GreedyCtl *)ctl);
+  if (e != cudaSuccess) return e;
   if (ctl) launch_k(greedy_bump_kernel, dim3(1), dim3(1), 0, st, ctl);
   return cudaGetLastError();
 }
