@@ -154,6 +154,15 @@ void free_scratch(fr_b200_model *m) {
 // (fp16 weights give the same bits in both.)
 bool wide_batch(int fmt, bool v5, int batch) { return batch > 4 || (fmt != FMT_FP16 && (v5 || batch > 2)); }
 
+// RWKV-4 batches that the row path (GEMMs over row copies) takes from both of them.  ms, persistent kernel against rows: 0.1B shape 5
+// and 8 fp16 streams 0.50 and 0.64 against 0.39, int8 0.50 and 0.60 against 0.41, int4 0.48 and 0.59 against 0.42, 4 of any format
+// 0.34 to 0.40 against the same; 1.5B shape (whose 5 to 8 streams never fitted) 3 and 4 int8 streams 1.18 and 1.31 against 1.09, int4 1.13 and
+// 1.26 against 1.23.  (4 fp16 streams would win there, too, 1.25 against 1.11, but for a second copy of the weights.)  RWKV-5 keeps its
+// kernel for its sums.
+bool rows_batch(const fr_b200_model *m, int batch) {
+  return !m->v5 && m->row_copies && (batch > 4 || (batch > 2 && m->fmt == FMT_INT8 && m->C >= 2048));
+}
+
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 // Lay out every matrix / vector of the model.  Per layer the weight blob holds the phases in the
@@ -233,12 +242,12 @@ void plan(fr_b200_model *m) {
   m->plain_halfs = 0; m->pscale_halfs = 0; m->qcopy_bytes = 0; m->qscale_halfs = 0;
   // The GEMM path (prompts, and decode of more than 8 streams at once) reads the projections row by output channel:
   // fp16 models keep W^T fp16 [N, K] (with the head when more than 8 streams can be decoded: all rows want logits;
-  // a prompt's head is a matvec over the last token), made at load for RWKV-5.x and for max_batch > 8, else on the
+  // a prompt's head is a matvec over the last token), made at load for RWKV-5.x and where rows_batch() takes max_batch streams, else on the
   // first long prompt; int8 / int4 models keep the packed codes row-major [N, K] / [N, K/2] (+ scales), the same
   // bytes as the streaming tiles, which the GEMM expands in shared memory.
   // (also when the persistent kernel cannot carry max_batch streams of a model this wide: its shared memory holds the
   // activation vectors of every stream, e.g. 8 streams x 8192 channel-mix inputs do not fit)
-  bool big = m->cfg.max_batch > MAX_B;
+  bool big = m->cfg.max_batch > MAX_B || rows_batch(m, m->cfg.max_batch);
   if (!big) {
     int optin = 0;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) == cudaSuccess)
@@ -690,9 +699,12 @@ int align_parity(fr_b200_model *m, int batch, cudaStream_t st) {
 }
 int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids, int R, cudaStream_t st);
 // more streams than the persistent kernel carries (or a model too wide for that many): the GEMM path decodes them
+bool token_kernel_fits(const fr_b200_model *m, int batch) {
+  return batch <= MAX_B && (wide_batch(m->fmt, m->v5, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) != 0;
+}
 bool decode_by_rows(const fr_b200_model *m, int batch) {
-  if (batch > MAX_B) return true;
-  return (wide_batch(m->fmt, m->v5, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) == 0;
+  if (batch > MAX_B || rows_batch(m, batch)) return true;
+  return !token_kernel_fits(m, batch);
 }
 // fp16 models that were created without the W^T copies build them from the streaming tiles (exact: the tiles hold
 // the same fp16 values) the first time the GEMM path is asked for
@@ -939,7 +951,7 @@ int fr_b200_decode_profile(fr_b200_model *m, const int32_t *ids, int batch, uint
   if (!m || !ids || !stamps) return fail(FR_B200_E_ARG, "null argument");
   if (!m->finalized) return fail(FR_B200_E_STATE, "finalize the model first");
   if (batch < 1 || batch > m->cfg.max_batch) return fail(FR_B200_E_ARG, "batch must be 1..max_batch");
-  if (decode_by_rows(m, batch)) return fail(FR_B200_E_UNSUPPORTED, "the trace exists for the persistent kernel (at most 8 streams) only");
+  if (!token_kernel_fits(m, batch)) return fail(FR_B200_E_UNSUPPORTED, "the trace exists for the persistent kernel (at most 8 streams) only");
   const int need = (int)m->phases.size() * 8 * m->grid;
   if (n_stamps < need) return fail(FR_B200_E_ARG, "stamps must hold 8 * n_phases * n_ctas entries");
   CU(cudaSetDevice(m->device));
