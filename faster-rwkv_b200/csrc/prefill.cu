@@ -163,6 +163,9 @@ __device__ __forceinline__ float epi_half_op(int epi, float a) {
 }
 // Up to four GEMMs with the same M in one launch (grid.x walks their N tiles back to back, heaviest first): the
 // attention projections of a layer, or the two channel-mix projections that read the LayerNorm output.
+// Low halves of X in the pair GEMM: in MMA columns of their own beside the high ones (up to 128 rows; the even CTA holds the high
+// half, the odd one the low half), after the high half of the same slice, or after all of K.
+enum { LO_BESIDE, LO_EACH, LO_AFTER };
 struct GemmGroup {
   int n;
   int stages;                           // ring depth; packed-weight GEMM: weight slots
@@ -172,7 +175,7 @@ struct GemmGroup {
   int split;                            // split-K factor (grid.z); > 1: CTAs write raw partial sums to GemmArgs::raw
   int dual;                             // few-row GEMM: some problem has A2 (the slot holds an X lo tile)
   int bn, m_tiles;                      // pair GEMM: rows of X per tile, row tiles
-  int lo_each;                          // pair GEMM: the low halves of X follow the high halves slice by slice
+  int lo_mode;                          // pair GEMM: where the low halves of X come in
   int tile_start[GEMM_GROUP_MAX + 1];   // first channel tile of each problem
   GemmArgs p[GEMM_GROUP_MAX];
 };
@@ -332,7 +335,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// fp16 weights, more than 128 rows: out^T[256 channels, BN rows] per pair of CTAs (BN a multiple of 32 up to 256,
+// fp16 weights, more than 128 rows (64, with low halves): out^T[256 channels, BN rows] per pair of CTAs (BN a multiple of 32 up to 256,
 // chosen at launch).  The pair is one tcgen05.mma.cta_group::2: each CTA holds the weights of its own 128 channels and
 // half of the X tile, so a slice of 64 inputs costs an SM 16 KB of weights and 16 KB of X for 512 clocks of MMA, where a CTA
 // of its own with the same 128 x 256 accumulator would fetch, and read from shared memory at every MMA, all 32 KB of X.
@@ -342,17 +345,15 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 // epilogue nothing hid, 182.  Without its epilogue 82, without its loads 100: the epilogue is what is left.
 //   warp 0: TMA into the own shared memory; the bytes of both CTAs are counted on the even CTA's barrier
 //   warp 1: TMEM, and in the even CTA the MMAs of the pair        warps 2..5: epilogue, a TMEM lane quadrant each
-// Low halves of X (A2) are ring slots of their own that meet the same weights again: after the high halves of the same
-// slice (lo_each) or after all of K.
+// Low halves of X (A2) meet the same weights beside the high ones, after them in the same slot, or in slots of their own after
+// all of K (LO_BESIDE, LO_EACH, LO_AFTER): sums in the order they always had, which RWKV-5 asks for.
 constexpr int PAIR_MAX_STAGES = 8;
 constexpr uint32_t PAIR_TMEM_COLS = 256;
 
 __global__ void __launch_bounds__(G_THREADS, 2)
 gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   const int STAGES = grp.stages, BN = grp.bn;
-  const uint32_t X_BYTES = (uint32_t)BN * (GBK * 2 / 2);          // this CTA's half of the X tile
   const uint32_t STAGE_BYTES = grp.stage_bytes;
-  const uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * GBM >> 4) << 24);
   extern __shared__ uint8_t gsm_raw[];
   // the same offsets in both CTAs: barriers in the first KB, tiles from the next 1024-byte boundary
   uint8_t *gsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
@@ -373,7 +374,10 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   const int num_k1 = g.K / GBK;
   const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
   const bool has_lo = g.A2 != nullptr;
-  const bool lo_now = has_lo && grp.lo_each, lo_pass = has_lo && !grp.lo_each;
+  const bool wide = has_lo && grp.lo_mode == LO_BESIDE, lo_now = has_lo && grp.lo_mode == LO_EACH, lo_pass = has_lo && grp.lo_mode == LO_AFTER;
+  const int cols = wide ? 2 * BN : BN;                            // MMA columns; this CTA holds half of them
+  const uint32_t X_BYTES = (uint32_t)cols * (GBK * 2 / 2);
+  const uint32_t IDESC = (1u << 4) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(2 * GBM >> 4) << 24);
   const int num_e = lo_pass ? 2 * nkz : nkz;
 
   if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (has_lo) prefetch_tmap(&maps.a2[pi]); }
@@ -405,13 +409,13 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
         const int s = at.slot;
         const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES, bar = mapa_u32(smem_u32(&full[s]), 0);
-        const int kx = (kz0 + (e < nkz ? e : e - nkz)) * GBK, row = m0 + (int)rank * (BN / 2);
+        const int kx = (kz0 + (e < nkz ? e : e - nkz)) * GBK, row = wide ? m0 : m0 + (int)rank * (BN / 2);
         if (e >= pre) {
           if (!mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
           tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
         }
         if (rank == 0) mbar_expect_tx(&full[s], 2 * (G_A_BYTES + (lo_now ? 2u : 1u) * X_BYTES));   // (bytes that arrived before are counted, too)
-        tma_load_2d_pair(dst + G_A_BYTES, e < nkz ? &maps.a[pi] : &maps.a2[pi], kx, row, bar);
+        tma_load_2d_pair(dst + G_A_BYTES, (wide ? rank == 0 : e < nkz) ? &maps.a[pi] : &maps.a2[pi], kx, row, bar);
         if (lo_now) tma_load_2d_pair(dst + G_A_BYTES + X_BYTES, &maps.a2[pi], kx, row, bar);
       }
     }
@@ -447,7 +451,14 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
         if (m0 + c0 >= g.M) break;   // warp-uniform
         uint32_t acc[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
+        const uint32_t at_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+        tmem_ld32(at_acc, acc);
+        if (wide) {
+          uint32_t part[32];
+          tmem_ld32(at_acc + (uint32_t)BN, part);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
+        }
         tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
       }
       tile_out_end();
@@ -1087,11 +1098,12 @@ bool make_out_maps(GemmMaps &maps, GemmGroup &grp) {
   return true;
 }
 // X and weights of a group (the maps of problems that do not exist are not read)
-bool make_in_maps(GemmMaps &maps, const GemmGroup &grp, int box_rows) {
+bool make_in_maps(GemmMaps &maps, const GemmGroup &grp, int box_rows, int box_rows_lo) {   // boxes of problems without and with A2
   for (int i = 0; i < grp.n; ++i) {
     const GemmArgs &g = grp.p[i];
-    if (!make_map_x(&maps.a[i], g, g.A, box_rows) || !make_map_w(&maps.b[i], g)) return false;
-    if (g.A2 && !make_map_x(&maps.a2[i], g, g.A2, box_rows)) return false;
+    const int box = g.A2 ? box_rows_lo : box_rows;
+    if (!make_map_x(&maps.a[i], g, g.A, box) || !make_map_w(&maps.b[i], g)) return false;
+    if (g.A2 && !make_map_x(&maps.a2[i], g, g.A2, box)) return false;
   }
   return true;
 }
@@ -1973,10 +1985,10 @@ int split_of(int ctas, int slots, int min_k1) {
   }
   return split;
 }
-// the cut of a product of RWKV-5 over more than 128 rows: that of one 128 x 256 tile per SM
+// the cut of a product of RWKV-5 over more than 64 (quantised: 128) rows: that of one 128 x 256 tile per SM
 int keep_split(int ctas, int min_k1) { return split_of(ctas, device_sm_count(), min_k1); }
 
-// up to 128 rows: weights along the MMA rows (gemm_wt_kernel), split-K into slabs when scratch was given
+// up to 128 rows: gemm_wt_kernel, split-K into slabs when scratch was given
 cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
   const int M = probs[0].M;
   const int bn = M <= 32 ? 32 : M <= 64 ? 64 : 128;
@@ -1998,7 +2010,7 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
     raw_ok = raw_ok && g.raw != nullptr && (g.N & 3) == 0 && (g.ldo & 3) == 0;
     if (g.A2) grp.dual = 1;
   }
-  if (!make_in_maps(maps, grp, bn)) return cudaErrorNotSupported;
+  if (!make_in_maps(maps, grp, bn, bn)) return cudaErrorNotSupported;
   grp.tile_start[n] = tiles;
   const int m_tiles = (M + bn - 1) / bn;
   // one CTA per SM, none waiting for a second wave: split K until the tiles about cover the SMs
@@ -2043,7 +2055,7 @@ float pair_cost(int tiles, int nk, int bn, float passes, int num_pairs) {
   return (float)rounds * shared + (rest > num_pairs ? shared : rest > 0 ? alone : 0.f);
 }
 
-// more than 128 rows of X, fp16 weights: gemm_pair_kernel
+// fp16 weights, more than 128 rows of X, or more than 64 with low halves: gemm_pair_kernel
 cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
   const int M = probs[0].M, num_pairs = device_sm_count() / 2;
   GemmMaps maps;
@@ -2077,17 +2089,19 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   grp.bn = 256;
   float best = 0.f;
   const float passes = (float)units / (float)tiles;
+  const bool beside = M <= 128;
   for (int rt = (M + 255) / 256; rt <= (M + 127) / 128; ++rt) {
     const int bn = ((M + rt - 1) / rt + 31) / 32 * 32;
     for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
-      const float cost = pair_cost(tiles * rt * sp, (min_k1 + sp - 1) / sp, bn, passes, num_pairs) + slab_cost(sp, M, sum_n, defer_split != nullptr);
+      const float cost = (beside ? pair_cost(tiles * sp, (min_k1 + sp - 1) / sp, any_lo ? 2 * bn : bn, 1.f, num_pairs)
+                                 : pair_cost(tiles * rt * sp, (min_k1 + sp - 1) / sp, bn, passes, num_pairs)) + slab_cost(sp, M, sum_n, defer_split != nullptr);
       if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
     }
   }
   grp.m_tiles = (M + grp.bn - 1) / grp.bn;
-  grp.lo_each = M <= GEMM_SMALL_M;
-  if (!make_in_maps(maps, grp, grp.bn / 2)) return cudaErrorNotSupported;
-  grp.stage_bytes = G_A_BYTES + (grp.lo_each && any_lo ? 2u : 1u) * (uint32_t)grp.bn * GBK;
+  grp.lo_mode = beside ? LO_BESIDE : M <= GEMM_SMALL_M ? LO_EACH : LO_AFTER;
+  if (!make_in_maps(maps, grp, grp.bn / 2, beside ? grp.bn : grp.bn / 2)) return cudaErrorNotSupported;
+  grp.stage_bytes = G_A_BYTES + (grp.lo_mode != LO_AFTER && any_lo ? 2u : 1u) * (uint32_t)grp.bn * GBK;
   // tiles that have an SM each to themselves take a ring of twice the depth
   const bool alone = tiles * grp.m_tiles * grp.split <= num_pairs;
   grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((alone ? 200u << 10 : 110u << 10) / grp.stage_bytes));
@@ -2163,7 +2177,7 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
   }
   grp.m_tiles = (M + grp.bn - 1) / grp.bn;
   const int xrows = pair ? grp.bn / 2 : grp.bn;
-  if (!make_in_maps(maps, grp, xrows)) return cudaErrorNotSupported;
+  if (!make_in_maps(maps, grp, xrows, xrows)) return cudaErrorNotSupported;
   grp.stage_bytes = (any_lo ? 2u : 1u) * (uint32_t)xrows * GBK * 2;
   grp.estages = std::min<int>(GQ_MAX, (int)((grp.tmem_cols - grp.acc_cols) / a_cols));
   const uint32_t avail = (two_per_sm ? 110u : 220u) << 10, ws = GBM * 128;
@@ -2194,7 +2208,12 @@ cudaError_t launch_gemm_group(const GemmArgs *probs, int n, cudaStream_t st, int
   const int M = probs[0].M;
   if (defer_split) *defer_split = 1;
   if (probs[0].Wq) return launch_gemm_q(probs, n, st, defer_split);
-  return M <= 128 ? launch_gemm_wt(probs, n, st, defer_split) : launch_gemm_pair(probs, n, st, defer_split);
+  // 65 to 128 rows: X as hi + lo pairs is worth a pair of SMs (every CTA reads half of it), X of single halves is not.  1.5B shape, ms:
+  // 100 streams 1.53 on pairs, 1.61 without; a prompt of 100 tokens 1.70 and 1.61, 1.65 with its key / value
+  // / receptance alone on pairs (of which two have low halves).
+  bool pairs = M > 64;
+  for (int i = 0; i < n && M <= 128; ++i) pairs = pairs && probs[i].A2;
+  return pairs ? launch_gemm_pair(probs, n, st, defer_split) : launch_gemm_wt(probs, n, st, defer_split);
 }
 
 cudaError_t gemm_prepare(int device) {
