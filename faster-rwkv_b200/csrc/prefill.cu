@@ -135,6 +135,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// One lane of a converged warp, the same one every time.  The warps that issue MMAs and copies run their loops whole and elect a lane for the
+// instruction: inside a branch that one lane took alone, descriptors and addresses move to uniform registers one by one and an MMA took
+// about 100 clocks to issue (a slice of int8 over 160 columns 0.34 us, now 0.24; of int4 0.56, now 0.38).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
+}
+
 // Place in a ring of barriers.  Its slot and phase are counted: a division by a depth that only the launch knows costs 100
 // to 200 clocks of a chain that takes 300 to 1,000 per slice, and every role had two to four of them.
 struct Ring {
@@ -399,11 +408,11 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   pdl_trigger();
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
       // the weights do not depend on the kernels before this one: the first round of them is asked for ahead of the wait
       const int pre = num_e < STAGES ? num_e : STAGES;
       for (int e = 0; e < pre; ++e)
-        tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + (e < nkz ? e : e - nkz)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
+        if (elect_one()) tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + (e < nkz ? e : e - nkz)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
       pdl_wait();
       Ring at;
       for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
@@ -411,23 +420,26 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
         const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES, bar = mapa_u32(smem_u32(&full[s]), 0);
         const int kx = (kz0 + (e < nkz ? e : e - nkz)) * GBK, row = wide ? m0 : m0 + (int)rank * (BN / 2);
         if (e >= pre) {
-          if (!mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-          tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+          if (elect_one()) tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
         }
+        if (elect_one()) {
         if (rank == 0) mbar_expect_tx(&full[s], 2 * (G_A_BYTES + (lo_now ? 2u : 1u) * X_BYTES));   // (bytes that arrived before are counted, too)
         tma_load_2d_pair(dst + G_A_BYTES, (wide ? rank == 0 : e < nkz) ? &maps.a[pi] : &maps.a2[pi], kx, row, bar);
         if (lo_now) tma_load_2d_pair(dst + G_A_BYTES + X_BYTES, &maps.a2[pi], kx, row, bar);
+        }
       }
     }
   } else if (warp == 1) {
-    if (rank == 0 && lane == 0) {
+    if (rank == 0) {
       Ring at;
       for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
         const int s = at.slot;
-        if (!mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
         tc_fence_after();
         const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
         const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + G_A_BYTES);
+        if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < GBK / 16; ++k4)
           umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, (e | k4) != 0);
@@ -437,8 +449,10 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
           for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
         }
         umma_commit_pair(&empty[s]);
+        }
+        __syncwarp();
       }
-      umma_commit_pair(acc_full);
+      if (elect_one()) umma_commit_pair(acc_full);
     }
   } else {
     const int quad = warp & 3;
@@ -539,10 +553,11 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   // the X loads and by the epilogue warps.
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
       const uint32_t w_bytes = G_A_BYTES, x_bytes = (x_lo ? 2u : 1u) * X_BYTES;
       const int pre = nkz < STAGES ? nkz : STAGES;
       for (int kb = 0; kb < pre; ++kb) {
+        if (!elect_one()) continue;
         mbar_expect_tx_only(&full[kb], w_bytes);
         const uint32_t dst = tiles + (uint32_t)kb * STAGE_BYTES;
         tma_load_2d(dst, &maps.b[pi], (kz0 + kb) * GBK, tile_n * GBM, &full[kb]);
@@ -554,7 +569,10 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES;
         const int kx = (kz0 + kb) * GBK;
         if (kb >= pre) {
-          if (!mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+        }
+        if (elect_one()) {
+        if (kb >= pre) {
           mbar_expect_tx(&full[s], w_bytes + x_bytes);
           tma_load_2d(dst, &maps.b[pi], kx, tile_n * GBM, &full[s]);
         } else {
@@ -562,18 +580,20 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         }
         tma_load_2d(dst + X_OFF, &maps.a[pi], kx, m0, &full[s]);
         if (x_lo) tma_load_2d(dst + XLO_OFF, &maps.a2[pi], kx, m0, &full[s]);
+        }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       Ring at;
       for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
         const int s = at.slot;
-        if (!mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
         tc_fence_after();
         const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
         const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + X_OFF);
         const bool wide = FUSE_LO && x_lo;
+        if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < GBK / 16; ++k4)
           umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
@@ -583,8 +603,10 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
           for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
         }
         umma_commit(&empty[s]);
+        }
+        __syncwarp();
       }
-      umma_commit(acc_full);
+      if (elect_one()) umma_commit(acc_full);
     }
   } else {
     const int quad = warp & 3;
@@ -702,11 +724,12 @@ struct GroupScales {
 //   !PAIR: up to 128 rows; out^T[128 channels, BN rows] per CTA, two CTAs per SM where 256 columns of TMEM hold the accumulator
 //          and some slices.  A step of few streams is a chain of such products of 3 to 11 slices each: every slice that has a
 //          slot is loaded and expanded before the kernels ahead have finished, and what is left behind them is X, its MMAs and the epilogue.
-//   warp 0      TMA: X into slot x, counted on the even CTA's barrier
+//   warp 0      TMA: X into slot x, counted on the even CTA's barrier (PAIR: X and expanded slices share their slots, and that barrier
+//               also counts the expanders of both CTAs: the thread that issues the MMAs has one wait and one commit per slice)
 //   warp 1      TMEM; (in the even CTA) the MMAs: acc += W_hi X_hi, W_hi X_lo, and for int4 W_lo X_hi (int8 codes are exact in
 //               fp16, the row scale is applied to the accumulator; int4: hi = fp16(q s), lo = q s - hi, an exact pair)
-//   warps 2..9  expanders: warp quadrant = TMEM lane quadrant, two warps share a row's 64 inputs (one scale group each); then epilogue
-//   warp 10     TMA: packed weights, 128 rows x 128 bytes = 4 (int4) or 2 (int8) slices per slot
+//   EW warps    expanders: warp quadrant = TMEM lane quadrant, two warps share a row's 64 inputs (one scale group each); then epilogue
+//   last warp   TMA: packed weights, 128 rows x 128 bytes = 4 (int4) or 2 (int8) slices per slot
 // !PAIR: the hi and lo halves of X sit back to back in a slot and are one B operand of 2 BN rows: one MMA gives W X_hi in
 // accumulator columns [0, BN) and W X_lo in [BN, 2 BN), which the epilogue adds up (an MMA with few columns costs as much as a
 // wide one).  PAIR: the halves multiply into the same accumulator, slice by slice.
@@ -729,17 +752,20 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
-// arrive on a barrier of either CTA of the cluster (address from mapa_u32)
+// Arrive on a barrier of either CTA of the cluster (address from mapa_u32).  Relaxed: it hands over no memory, but columns of TMEM, whose
+// writes are complete (tcgen05.wait::st) and ordered by the tcgen05 fences on both sides.  With .release it took 500 to 900 clocks, a slice of
+// int8 0.70 us instead of 0.50.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-constexpr int GQ_EXP_WARPS = 8;
-constexpr int GQ_THREADS = 32 * (3 + GQ_EXP_WARPS);
+// EW expander warps: 8 where two CTAs share an SM, else 16 in two groups of eight that take the slices in turn: a warp's way through a slice
+// (wait, load, expand, wait, store, hand over) is longer than the MMAs of most (512 clocks at 256 columns and one pass).
+constexpr int gq_threads(int ew) { return 32 * (3 + ew); }
 constexpr int GQ_MAX = 8;                // most slots of any ring
 
-template <int FMT, bool PAIR>
-__global__ void __launch_bounds__(GQ_THREADS, PAIR ? 1 : 2)
+template <int FMT, bool PAIR, int EW>
+__global__ void __launch_bounds__(gq_threads(EW), EW == 8 ? 2 : 1)
 gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   constexpr uint32_t ROW_B = FMT == FMT_INT8 ? GBK : GBK / 2;          // packed bytes per row and slice
   constexpr int KSH = FMT == FMT_INT8 ? 1 : 2, KSUB = 1 << KSH;        // slices per weight slot
@@ -758,8 +784,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
   uint64_t *xempty = xfull + GQ_MAX;
   uint64_t *a_full = xempty + GQ_MAX;
   uint64_t *a_empty = a_full + GQ_MAX;
-  uint64_t *a_peer = a_empty + GQ_MAX;      // (even CTA of a pair) the other CTA's expanded slice
-  uint64_t *acc_full = a_peer + GQ_MAX;
+  uint64_t *acc_full = a_empty + GQ_MAX;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t xtiles = smem_u32(gsm + 1024), wtiles = xtiles + (uint32_t)NX * XS_BYTES;
@@ -777,9 +802,9 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
 
   if (threadIdx.x == 64) { prefetch_tmap(&maps.b[pi]); prefetch_tmap(&maps.a[pi]); if (x_lo) prefetch_tmap(&maps.a2[pi]); }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], GQ_EXP_WARPS); }
-    for (int x = 0; x < NX; ++x) { mbar_init(&xfull[x], 1); mbar_init(&xempty[x], 1); }
-    for (int e = 0; e < NE; ++e) { mbar_init(&a_full[e], GQ_EXP_WARPS); mbar_init(&a_empty[e], 1); mbar_init(&a_peer[e], 1); }
+    for (int s = 0; s < NW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], EW); }
+    for (int x = 0; x < NX; ++x) { mbar_init(&xfull[x], PAIR ? 1 + 8 + 1 : 1); mbar_init(&xempty[x], 1); }
+    for (int e = 0; e < NE; ++e) { mbar_init(&a_full[e], 8); mbar_init(&a_empty[e], 1); }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -801,11 +826,12 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
   pdl_trigger();
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
       pdl_wait();
       Ring at;
       for (int kb = 0; kb < nkz; ++kb, at.next(NX)) {
-        if (!mbar_wait(&xempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(PAIR ? &a_empty[at.slot] : &xempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+        if (!elect_one()) continue;
         const uint32_t dst = xtiles + (uint32_t)at.slot * XS_BYTES;
         const int kx = (kz0 + kb) * GBK;
         if (PAIR) {
@@ -821,7 +847,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
         }
       }
     }
-  } else if (warp == 2 + GQ_EXP_WARPS) {
+  } else if (warp == 2 + EW) {
     if (lane == 0) {
       Ring at;
       for (int kw = 0; kw < ng; ++kw, at.next(NW)) {
@@ -831,16 +857,16 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
       }
     }
   } else if (warp == 1) {
-    if (rank == 0 && lane == 0) {
+    if (rank == 0) {
       Ring ea, xa;
       for (int kb = 0; kb < nkz; ++kb, ea.next(NE), xa.next(NX)) {
-        if (!mbar_wait(&a_full[ea.slot], ea.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        if (PAIR && !mbar_wait(&a_peer[ea.slot], ea.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
-        if (!mbar_wait(&xfull[xa.slot], xa.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
+        if (!PAIR && !__all_sync(0xffffffffu, mbar_wait(&a_full[ea.slot], ea.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&xfull[xa.slot], xa.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
         tc_fence_after();
         const uint32_t xb = xtiles + (uint32_t)xa.slot * XS_BYTES, ta = tmem_base + grp.acc_cols + (uint32_t)ea.slot * A_COLS;
         const uint64_t xd = umma_desc_k128(xb), xl = umma_desc_k128(xb + X_BYTES);
         const bool wide = !PAIR && x_lo;
+        if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < GBK / 16; ++k4)       // 16 inputs = 8 columns of A
           umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
@@ -852,23 +878,25 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
 #pragma unroll
           for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + 32u + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, 1u);
         }
-        if (PAIR) { umma_commit_pair(&a_empty[ea.slot]); umma_commit_pair(&xempty[xa.slot]); }
+        if (PAIR) { umma_commit_pair(&a_empty[ea.slot]); }
         else { umma_commit(&a_empty[ea.slot]); umma_commit(&xempty[xa.slot]); }
+        }
+        __syncwarp();
       }
-      if (PAIR) umma_commit_pair(acc_full); else umma_commit(acc_full);
+      if (elect_one()) { if (PAIR) umma_commit_pair(acc_full); else umma_commit(acc_full); }
     } else if (PAIR && rank == 1 && lane == 0) {
-      // A release across the cluster takes 500 to 900 clocks: this thread, which has no MMAs to issue, passes the slices of
-      // its CTA's expanders on.
+      // An arrive in the other CTA takes some hundred clocks: this thread, which has no MMAs to issue, passes the slices of its
+      // CTA's expanders on.
       Ring at;
       for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
         if (!mbar_wait(&a_full[at.slot], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         tc_fence_after();
         tc_fence_before();
-        mbar_arrive_cluster(mapa_u32(smem_u32(&a_peer[at.slot]), 0));
+        mbar_arrive_cluster(mapa_u32(smem_u32(&xfull[at.slot]), 0));
       }
     }
   } else {
-    const int quad = warp & 3, part = (warp - 2) >> 2;
+    const int quad = warp & 3, nth = (warp - 2) >> 2, part = nth & 1, group = nth >> 1;
     const int row = quad * 32 + lane;
     const uint32_t swz = (uint32_t)(row & 7);
     GroupScales scales;
@@ -882,6 +910,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
         const uint32_t sc = scales.at(ks), s16 = part ? (sc >> 16) : (sc & 0xffffu);
         s2 = s16 | (s16 << 16);
       }
+      if (EW == 8 || (kb & 1) == group) {
       if (!__all_sync(0xffffffffu, mbar_wait(&wfull[wat.slot], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
       // 16-byte chunk c of the row's 128 bytes is at (c ^ swz) << 4
       const uint32_t src = wtiles + (uint32_t)wat.slot * WS_BYTES + (uint32_t)row * 128u, c0 = (uint32_t)sub * (ROW_B / 16u);
@@ -905,11 +934,12 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&a_full[at.slot]);
-        if (sub == KSUB - 1) mbar_arrive(&wempty[wat.slot]);   // (the last slot of this K range is not asked for again)
+      if (lane == 0) mbar_arrive(PAIR && rank == 0 ? &xfull[at.slot] : &a_full[at.slot]);
       }
-      if (sub == KSUB - 1) wat.next(NW);
+      if (sub == KSUB - 1) {
+        if (lane == 0) mbar_arrive(&wempty[wat.slot]);   // (the last slot of this K range is not asked for again)
+        wat.next(NW);
+      }
     }
     // epilogue
     const int ch = ch0 + row;
@@ -920,7 +950,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
       const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
       const uint32_t buf = xtiles + (uint32_t)(warp - 2) * 2 * EPI_BUF;   // the rings have been read
       uint32_t flip = 0;
-      for (int c0 = part * 32; c0 < BN; c0 += 64, flip ^= EPI_BUF) {
+      for (int c0 = nth * 32; c0 < BN; c0 += 8 * EW, flip ^= EPI_BUF) {
         if (m0 + c0 >= g.M) break;   // warp-uniform
         const uint32_t at_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
         uint32_t acc[32];
@@ -2160,7 +2190,7 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
       for (int sp = fixed ? fixed : 1; sp <= (fixed ? fixed : max_split); ++sp) {
         // in clocks: a slice is bound by its MMAs or by its expansion, a wave starts and ends
         const int waves = (tiles * rt * sp + num_pairs - 1) / num_pairs;
-        const float cost = (float)waves * ((float)((min_k1 + sp - 1) / sp) * std::max(2.05f * (float)bn * passes, 1180.f) + 11000.f + 14.f * (float)bn) +
+        const float cost = (float)waves * ((float)((min_k1 + sp - 1) / sp) * std::max(2.05f * (float)bn * passes, 460.f) + 11000.f + 14.f * (float)bn) +
                            slab_cost(sp, M, sum_n, defer_split != nullptr);
         if (best == 0.f || cost < best) { best = cost; grp.split = sp; grp.bn = bn; }
       }
@@ -2183,13 +2213,16 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
   const uint32_t avail = (two_per_sm ? 110u : 220u) << 10, ws = GBM * 128;
   grp.stages = two_per_sm ? ((avail - 3 * ws) / grp.stage_bytes >= 4 ? 3 : 2) : 4;
   grp.xstages = std::min<int>(GQ_MAX, (int)((avail - grp.stages * ws) / grp.stage_bytes));
+  if (pair) grp.xstages = grp.estages = std::min(grp.xstages, grp.estages);
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t rings = (size_t)grp.xstages * grp.stage_bytes + (size_t)grp.stages * ws;
-  const size_t smem = 1024 + std::max<size_t>(rings, GQ_EXP_WARPS * 2 * EPI_BUF) + 1024;
-  auto kern = pair ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, true> : gemm_q_kernel<FMT_INT8, true>)
-                   : (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false> : gemm_q_kernel<FMT_INT8, false>);
+  const int ew = two_per_sm ? 8 : 16;
+  const size_t smem = 1024 + std::max<size_t>(rings, ew * 2 * EPI_BUF) + 1024;
+  auto kern = pair         ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, true, 16> : gemm_q_kernel<FMT_INT8, true, 16>)
+              : two_per_sm ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false, 8> : gemm_q_kernel<FMT_INT8, false, 8>)
+                           : (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false, 16> : gemm_q_kernel<FMT_INT8, false, 16>);
   const dim3 grid((pair ? 2 : 1) * tiles * grp.m_tiles, 1, grp.split);
-  cudaError_t e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(GQ_THREADS), smem, st, maps, grp);
+  cudaError_t e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(gq_threads(ew)), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
@@ -2220,8 +2253,8 @@ cudaError_t gemm_prepare(int device) {
   int optin = 0;
   cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   const void *kerns[] = {(const void *)gemm_wt_kernel<32>, (const void *)gemm_wt_kernel<64>, (const void *)gemm_wt_kernel<128>,
-                         (const void *)gemm_pair_kernel, (const void *)gemm_q_kernel<FMT_INT8, false>, (const void *)gemm_q_kernel<FMT_INT8, true>,
-                         (const void *)gemm_q_kernel<FMT_INT4, false>, (const void *)gemm_q_kernel<FMT_INT4, true>};
+                         (const void *)gemm_pair_kernel, (const void *)gemm_q_kernel<FMT_INT8, false, 8>, (const void *)gemm_q_kernel<FMT_INT8, false, 16>, (const void *)gemm_q_kernel<FMT_INT8, true, 16>,
+                         (const void *)gemm_q_kernel<FMT_INT4, false, 8>, (const void *)gemm_q_kernel<FMT_INT4, false, 16>, (const void *)gemm_q_kernel<FMT_INT4, true, 16>};
   for (const void *k : kerns)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   return e;
