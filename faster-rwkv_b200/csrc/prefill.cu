@@ -1598,6 +1598,12 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
     sh[0][ch][j] = xa; sh[1][ch][j] = xb; sh[2][ch][j] = xp;
   }
   __syncthreads();
+  constexpr int RG = LEN > 4 ? 4 : 2;
+  float rn[RG];
+  if (LEN > 1) {
+#pragma unroll
+    for (int i = 0; i < RG; ++i) rn[i] = i < NR && t0 + i < t1 ? rp[(size_t)(t0 + i) * a.C] : 0.f;
+  }
   // this chunk's start state: the stream's state followed by all chunks before
   aa = st[c]; bb = st[a.C + c]; pp = st[2 * a.C + c];
   __syncthreads();                       // every thread has read the state the last chunk overwrites
@@ -1612,10 +1618,22 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
     if (a.out_lo) a.out_lo[(size_t)t * a.C + c] = __float2half_rn(y - __half2float(oh));
     absorb(k, v);
   };
-  if (LEN > 0) {
+  if (LEN == 1) {
+    if (t0 < t1) step(t0, kr[0], vr[0], rsum);
+  } else if (LEN > 0) {
+    // r comes a group of tokens ahead of its use: asked for token by token it waits behind the stores of the one before
 #pragma unroll
-    for (int i = 0; i < NR; ++i)
-      if (t0 + i < t1) step(t0 + i, kr[i], vr[i], LEN == 1 ? rsum : rp[(size_t)(t0 + i) * a.C]);
+    for (int i0 = 0; i0 < NR; i0 += RG) {
+      float r[RG];
+#pragma unroll
+      for (int i = 0; i < RG; ++i) {
+        r[i] = rn[i];
+        if (i0 + RG + i < NR && t0 + i0 + RG + i < t1) rn[i] = rp[(size_t)(t0 + i0 + RG + i) * a.C];
+      }
+#pragma unroll
+      for (int i = 0; i < RG; ++i)
+        if (i0 + i < NR && t0 + i0 + i < t1) step(t0 + i0 + i, kr[i0 + i], vr[i0 + i], r[i]);
+    }
   } else {
 #pragma unroll 4
     for (int t = t0; t < t1; ++t) step(t, kp[(size_t)t * a.C], vp[(size_t)t * a.C], rp[(size_t)t * a.C]);
