@@ -1206,8 +1206,8 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     x = x_all + rc;
     CU(launch_ln_mix_seq(la, st));
     int kvr_split = 1;
-    const __half *kvr_cs[3] = {nullptr, nullptr, nullptr};
-    const float *kvr_raw[3] = {nullptr, nullptr, nullptr};
+    const __half *kvr_cs[4] = {nullptr, nullptr, nullptr, nullptr};
+    const float *kvr_raw[4] = {nullptr, nullptr, nullptr, nullptr};
     {
       // the attention projections in one launch; the two with a second pass over K first
       GemmArgs grp[4] = {mk(T, op[0], lm.key, C, C, GEMM_EPI_F32, k, nullptr, nullptr, 1.f, lo0),
@@ -1216,18 +1216,27 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
                          mk(T, op[2], lm.receptance, C, C, GEMM_EPI_F32, r, nullptr, nullptr, 1.f, lo2)};
       if (m->gate) { grp[3] = mk(T, op[3], lm.gate, C, C, GEMM_EPI_SILU_F16, g, nullptr, nullptr, 1.f, lo3); grp[3].out_lo = g_lo; }
       give_raw(grp, m->gate ? 4 : 3);
-      const bool defer = defer_x && !m->v5 && (batch_mode || T <= PROMPT_DEFER_KVR);
+      const bool defer = batch_mode || (defer_x && !m->v5 && T <= PROMPT_DEFER_KVR);
       CU(launch_gemm_group(grp, m->gate ? 4 : 3, st, defer ? &kvr_split : nullptr));
-      for (int i = 0; i < 3; ++i) { kvr_cs[i] = grp[i].col_scale; kvr_raw[i] = grp[i].raw; }
+      for (int i = 0; i < (m->gate ? 4 : 3); ++i) { kvr_cs[i] = grp[i].col_scale; kvr_raw[i] = grp[i].raw; }
     }
-    if (m->v5) {
+    if (m->v5 && batch_mode) {
+      Wkv5RowsArgs wa;
+      memset(&wa, 0, sizeof(wa));
+      wa.k = k; wa.v = v; wa.r = r; wa.g = g; wa.g_lo = g_lo; wa.gated = m->gate;
+      for (int i = 0; i < 4; ++i) { wa.raw[i] = kvr_raw[i]; wa.cs[i] = kvr_cs[i]; }
+      wa.split = kvr_split; wa.rows = T; wa.C = C; wa.per_head = m->cfg.version == FR_B200_V5_0;
+      wa.decay = lv.decay; wa.first = lv.first; wa.lnx_w = lv.lnx_w; wa.lnx_b = lv.lnx_b;
+      wa.state = reinterpret_cast<float *>(stb + off_mid(C, af)); wa.state_stride = m->state_stride / 4;
+      wa.out = yn; wa.out_lo = yn_lo;
+      CU(launch_wkv5_rows(wa, H, st));
+    } else if (m->v5) {
       SeqWkvArgs wa;
       memset(&wa, 0, sizeof(wa));
       wa.r = r; wa.k = k; wa.v = v; wa.decay = lv.decay; wa.first = lv.first;
       wa.state = reinterpret_cast<float *>(stb + off_mid(C, af)); wa.y = y; wa.T = T; wa.C = C;
       wa.per_head = m->cfg.version == FR_B200_V5_0;
       wa.n_chunks = n_chunks; wa.chunk_len = chunk_len; wa.e_out = (float *)(B + o_e + scan_bytes * pc); wa.s_in = (float *)(B + o_sin + scan_bytes * pc);
-      wa.batch_mode = batch_mode; wa.state_stride = m->state_stride / 4;
       CU(launch_wkv5_seq(wa, H, st));
       CU(launch_gn_gate_seq(y, lv.lnx_w, lv.lnx_b, m->gate ? g : nullptr, m->gate ? g_lo : nullptr, T, H, yn, yn_lo, st));
     } else {

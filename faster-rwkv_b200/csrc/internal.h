@@ -234,8 +234,18 @@ struct SeqWkvArgs {
   int T, C, per_head;
   int n_chunks, chunk_len;   // the sequence is scanned in n_chunks parallel pieces of chunk_len tokens
   float *e_out, *s_in;       // [H, n_chunks, 64, 64] scratch: chunk end states from zero, chunk start states
-  int batch_mode;            // rows are streams (T of them, one token each); n_chunks must be 1
+};
+struct Wkv5RowsArgs {        // rows are streams, one token each
+  const float *k, *v, *r;    // [rows, C], when split is 1
+  const __half *g, *g_lo;    // [rows, C], when split is 1: the gate (SiLU applied) as a pair
+  const float *raw[4];       // split > 1: key, value, receptance (, gate) are still split-K slabs [split][rows][C] ...
+  const __half *cs[4];       // ... with per-column scales, or null
+  int split, rows, C, per_head;
+  bool gated;
+  const float *decay, *first, *lnx_w, *lnx_b;
+  float *state;              // [H, 64 key, 64 value] of stream 0, updated in place
   size_t state_stride;       // floats between the states of consecutive streams
+  __half *out, *out_lo;      // [rows, C] the operand of the output projection; out_lo optional
 };
 struct Wkv4Args {
   const float *k, *v, *r;    // [rows, C]; r before the sigmoid
@@ -253,6 +263,7 @@ struct Wkv4Args {
 cudaError_t launch_gather_emb(const void *emb, int emb_f32, const int32_t *ids, int T, int C, float *x, cudaStream_t st);
 cudaError_t launch_ln_mix_seq(const SeqLnArgs &a, cudaStream_t st);
 cudaError_t launch_wkv5_seq(const SeqWkvArgs &a, int H, cudaStream_t st);
+cudaError_t launch_wkv5_rows(const Wkv5RowsArgs &a, int H, cudaStream_t st);
 int wkv5_scan_slots();   // resident (head, chunk) CTAs of the scan on this device
 cudaError_t launch_gn_gate_seq(const float *y, const float *lnx_w, const float *lnx_b, const __half *g, const __half *g_lo, int T,
                                int H, __half *out, __half *out_lo, cudaStream_t st);

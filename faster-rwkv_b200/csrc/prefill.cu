@@ -408,26 +408,24 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   pdl_trigger();
 
   if (warp == 0) {
-    {
-      // the weights do not depend on the kernels before this one: the first round of them is asked for ahead of the wait
-      const int pre = num_e < STAGES ? num_e : STAGES;
-      for (int e = 0; e < pre; ++e)
-        if (elect_one()) tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + (e < nkz ? e : e - nkz)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
-      pdl_wait();
-      Ring at;
-      for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
-        const int s = at.slot;
-        const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES, bar = mapa_u32(smem_u32(&full[s]), 0);
-        const int kx = (kz0 + (e < nkz ? e : e - nkz)) * GBK, row = wide ? m0 : m0 + (int)rank * (BN / 2);
-        if (e >= pre) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
-          if (elect_one()) tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
-        }
-        if (elect_one()) {
+    // the weights do not depend on the kernels before this one: the first round of them is asked for ahead of the wait
+    const int pre = num_e < STAGES ? num_e : STAGES;
+    for (int e = 0; e < pre; ++e)
+      if (elect_one()) tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + (e < nkz ? e : e - nkz)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
+    pdl_wait();
+    Ring at;
+    for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
+      const int s = at.slot;
+      const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES, bar = mapa_u32(smem_u32(&full[s]), 0);
+      const int kx = (kz0 + (e < nkz ? e : e - nkz)) * GBK, row = wide ? m0 : m0 + (int)rank * (BN / 2);
+      if (e >= pre) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+        if (elect_one()) tma_load_2d_pair(dst, &maps.b[pi], kx, ch0, bar);
+      }
+      if (elect_one()) {
         if (rank == 0) mbar_expect_tx(&full[s], 2 * (G_A_BYTES + (lo_now ? 2u : 1u) * X_BYTES));   // (bytes that arrived before are counted, too)
         tma_load_2d_pair(dst + G_A_BYTES, (wide ? rank == 0 : e < nkz) ? &maps.a[pi] : &maps.a2[pi], kx, row, bar);
         if (lo_now) tma_load_2d_pair(dst + G_A_BYTES + X_BYTES, &maps.a2[pi], kx, row, bar);
-        }
       }
     }
   } else if (warp == 1) {
@@ -441,14 +439,14 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
         const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + G_A_BYTES);
         if (elect_one()) {
 #pragma unroll
-        for (int k4 = 0; k4 < GBK / 16; ++k4)
-          umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, (e | k4) != 0);
-        if (lo_now) {
-          const uint64_t xl = umma_desc_k128(base + G_A_BYTES + X_BYTES);
+          for (int k4 = 0; k4 < GBK / 16; ++k4)
+            umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), IDESC, (e | k4) != 0);
+          if (lo_now) {
+            const uint64_t xl = umma_desc_k128(base + G_A_BYTES + X_BYTES);
 #pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
-        umma_commit_pair(&empty[s]);
+            for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_pair(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
+          }
+          umma_commit_pair(&empty[s]);
         }
         __syncwarp();
       }
@@ -492,8 +490,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 // swapped, out^T[N, M] = W^T[N, K] . X[M, K]^T.  The 128 MMA rows are 128 output channels of the weight matrix, the
 // MMA columns are the BN rows of X (32 .. 256), so a ring slot is 16 KB of weights plus a small X tile instead of a
 // 128-row X tile that is mostly zero fill plus 8 KB of weights: several times the weight bytes in flight per SM,
-// which is what a step that streams every weight once is bound by.  The low halves of X (A2) and of the weights
-// (Bt2) sit in the same slot and multiply into the same accumulator; (lo W) x (lo X) is below fp32 resolution.
+// which is what a step that streams every weight once is bound by.  The low halves of X (A2) sit in the same slot.
 // The accumulator holds out^T: TMEM lane = output channel, column = row of X; the epilogue warps write with the
 // lanes along the channels (coalesced), either the finished values or the split-K slabs gemm_finish_kernel sums.
 constexpr int WT_MAX_STAGES = 8;
@@ -504,11 +501,10 @@ __global__ void __launch_bounds__(G_THREADS, 2)
 gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   constexpr uint32_t X_BYTES = BN * GBK * 2;
   constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GBM >> 4) << 24);
-  // up to 128 rows the hi and lo tiles of X, back to back in the slot, are one B operand of 2 BN rows (accumulator
-  // columns [0, BN) and [BN, 2 BN), added up by the epilogue): an MMA with few columns costs about as much as a wide one
-  constexpr bool FUSE_LO = BN <= 128;
+  // the hi and lo tiles of X, back to back in the slot, are one B operand of 2 BN rows (accumulator columns [0, BN) and
+  // [BN, 2 BN), added up by the epilogue): an MMA with few columns costs about as much as a wide one
   constexpr uint32_t IDESC2 = (1u << 4) | ((uint32_t)((2 * BN) >> 3) << 17) | ((uint32_t)(GBM >> 4) << 24);
-  constexpr uint32_t TMEM_COLS = FUSE_LO ? 2 * BN : BN;
+  constexpr uint32_t TMEM_COLS = 2 * BN;
   const int STAGES = grp.stages;
   const uint32_t STAGE_BYTES = grp.stage_bytes;
   constexpr uint32_t X_OFF = G_A_BYTES, XLO_OFF = X_OFF + X_BYTES;
@@ -553,25 +549,24 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   // the X loads and by the epilogue warps.
 
   if (warp == 0) {
-    {
-      const uint32_t w_bytes = G_A_BYTES, x_bytes = (x_lo ? 2u : 1u) * X_BYTES;
-      const int pre = nkz < STAGES ? nkz : STAGES;
-      for (int kb = 0; kb < pre; ++kb) {
-        if (!elect_one()) continue;
-        mbar_expect_tx_only(&full[kb], w_bytes);
-        const uint32_t dst = tiles + (uint32_t)kb * STAGE_BYTES;
-        tma_load_2d(dst, &maps.b[pi], (kz0 + kb) * GBK, tile_n * GBM, &full[kb]);
+    const uint32_t w_bytes = G_A_BYTES, x_bytes = (x_lo ? 2u : 1u) * X_BYTES;
+    const int pre = nkz < STAGES ? nkz : STAGES;
+    for (int kb = 0; kb < pre; ++kb) {
+      if (!elect_one()) continue;
+      mbar_expect_tx_only(&full[kb], w_bytes);
+      const uint32_t dst = tiles + (uint32_t)kb * STAGE_BYTES;
+      tma_load_2d(dst, &maps.b[pi], (kz0 + kb) * GBK, tile_n * GBM, &full[kb]);
+    }
+    pdl_wait();
+    Ring at;
+    for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
+      const int s = at.slot;
+      const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES;
+      const int kx = (kz0 + kb) * GBK;
+      if (kb >= pre) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
       }
-      pdl_wait();
-      Ring at;
-      for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
-        const int s = at.slot;
-        const uint32_t dst = tiles + (uint32_t)s * STAGE_BYTES;
-        const int kx = (kz0 + kb) * GBK;
-        if (kb >= pre) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
-        }
-        if (elect_one()) {
+      if (elect_one()) {
         if (kb >= pre) {
           mbar_expect_tx(&full[s], w_bytes + x_bytes);
           tma_load_2d(dst, &maps.b[pi], kx, tile_n * GBM, &full[s]);
@@ -580,34 +575,25 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         }
         tma_load_2d(dst + X_OFF, &maps.a[pi], kx, m0, &full[s]);
         if (x_lo) tma_load_2d(dst + XLO_OFF, &maps.a2[pi], kx, m0, &full[s]);
-        }
       }
     }
   } else if (warp == 1) {
-    {
-      Ring at;
-      for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
-        const int s = at.slot;
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
-        tc_fence_after();
-        const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
-        const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + X_OFF);
-        const bool wide = FUSE_LO && x_lo;
-        if (elect_one()) {
+    Ring at;
+    for (int kb = 0; kb < nkz; ++kb, at.next(STAGES)) {
+      const int s = at.slot;
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[s], at.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+      tc_fence_after();
+      const uint32_t base = tiles + (uint32_t)s * STAGE_BYTES;
+      const uint64_t wd = umma_desc_k128(base), xd = umma_desc_k128(base + X_OFF);
+      if (elect_one()) {
 #pragma unroll
         for (int k4 = 0; k4 < GBK / 16; ++k4)
-          umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
-        if (x_lo && !wide) {
-          const uint64_t xl = umma_desc_k128(base + XLO_OFF);
-#pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xl + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
+          umma_f16(tmem_base, wd + (uint64_t)(k4 * 2), xd + (uint64_t)(k4 * 2), x_lo ? IDESC2 : IDESC, (kb | k4) != 0);
         umma_commit(&empty[s]);
-        }
-        __syncwarp();
       }
-      if (elect_one()) umma_commit(acc_full);
+      __syncwarp();
     }
+    if (elect_one()) umma_commit(acc_full);
   } else {
     const int quad = warp & 3;
     const int ch = tile_n * GBM + quad * 32 + lane;
@@ -622,7 +608,7 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         if (m0 + c0 >= g.M) break;   // warp-uniform
         uint32_t acc[32];
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
-        if (FUSE_LO && x_lo) {
+        if (x_lo) {
           uint32_t part[32];
           tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(BN + c0), part);
 #pragma unroll
@@ -826,25 +812,23 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
   pdl_trigger();
 
   if (warp == 0) {
-    {
-      pdl_wait();
-      Ring at;
-      for (int kb = 0; kb < nkz; ++kb, at.next(NX)) {
-        if (!__all_sync(0xffffffffu, mbar_wait(PAIR ? &a_empty[at.slot] : &xempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
-        if (!elect_one()) continue;
-        const uint32_t dst = xtiles + (uint32_t)at.slot * XS_BYTES;
-        const int kx = (kz0 + kb) * GBK;
-        if (PAIR) {
-          const uint32_t bar = mapa_u32(smem_u32(&xfull[at.slot]), 0);
-          const int row = m0 + (int)rank * (BN / 2);
-          if (rank == 0) mbar_expect_tx(&xfull[at.slot], (x_lo ? 4u : 2u) * X_BYTES);   // of both CTAs
-          tma_load_2d_pair(dst, &maps.a[pi], kx, row, bar);
-          if (x_lo) tma_load_2d_pair(dst + X_BYTES, &maps.a2[pi], kx, row, bar);
-        } else {
-          mbar_expect_tx(&xfull[at.slot], (x_lo ? 2u : 1u) * X_BYTES);
-          tma_load_2d(dst, &maps.a[pi], kx, m0, &xfull[at.slot]);
-          if (x_lo) tma_load_2d(dst + X_BYTES, &maps.a2[pi], kx, m0, &xfull[at.slot]);
-        }
+    pdl_wait();
+    Ring at;
+    for (int kb = 0; kb < nkz; ++kb, at.next(NX)) {
+      if (!__all_sync(0xffffffffu, mbar_wait(PAIR ? &a_empty[at.slot] : &xempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+      if (!elect_one()) continue;
+      const uint32_t dst = xtiles + (uint32_t)at.slot * XS_BYTES;
+      const int kx = (kz0 + kb) * GBK;
+      if (PAIR) {
+        const uint32_t bar = mapa_u32(smem_u32(&xfull[at.slot]), 0);
+        const int row = m0 + (int)rank * (BN / 2);
+        if (rank == 0) mbar_expect_tx(&xfull[at.slot], (x_lo ? 4u : 2u) * X_BYTES);   // of both CTAs
+        tma_load_2d_pair(dst, &maps.a[pi], kx, row, bar);
+        if (x_lo) tma_load_2d_pair(dst + X_BYTES, &maps.a2[pi], kx, row, bar);
+      } else {
+        mbar_expect_tx(&xfull[at.slot], (x_lo ? 2u : 1u) * X_BYTES);
+        tma_load_2d(dst, &maps.a[pi], kx, m0, &xfull[at.slot]);
+        if (x_lo) tma_load_2d(dst + X_BYTES, &maps.a2[pi], kx, m0, &xfull[at.slot]);
       }
     }
   } else if (warp == 2 + EW) {
@@ -868,18 +852,18 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
         const bool wide = !PAIR && x_lo;
         if (elect_one()) {
 #pragma unroll
-        for (int k4 = 0; k4 < GBK / 16; ++k4)       // 16 inputs = 8 columns of A
-          umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
-        if (PAIR && x_lo) {
+          for (int k4 = 0; k4 < GBK / 16; ++k4)       // 16 inputs = 8 columns of A
+            umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), wide ? IDESC2 : IDESC, (kb | k4) != 0);
+          if (PAIR && x_lo) {
 #pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xl + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
-        if (FMT == FMT_INT4) {
+            for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + (uint32_t)k4 * 8, xl + (uint64_t)(k4 * 2), IDESC, 1u);
+          }
+          if (FMT == FMT_INT4) {
 #pragma unroll
-          for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + 32u + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, 1u);
-        }
-        if (PAIR) { umma_commit_pair(&a_empty[ea.slot]); }
-        else { umma_commit(&a_empty[ea.slot]); umma_commit(&xempty[xa.slot]); }
+            for (int k4 = 0; k4 < GBK / 16; ++k4) umma_f16_ta(PAIR, tmem_base, ta + 32u + (uint32_t)k4 * 8, xd + (uint64_t)(k4 * 2), IDESC, 1u);
+          }
+          if (PAIR) { umma_commit_pair(&a_empty[ea.slot]); }
+          else { umma_commit(&a_empty[ea.slot]); umma_commit(&xempty[xa.slot]); }
         }
         __syncwarp();
       }
@@ -911,30 +895,30 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
         s2 = s16 | (s16 << 16);
       }
       if (EW == 8 || (kb & 1) == group) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&wfull[wat.slot], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
-      // 16-byte chunk c of the row's 128 bytes is at (c ^ swz) << 4
-      const uint32_t src = wtiles + (uint32_t)wat.slot * WS_BYTES + (uint32_t)row * 128u, c0 = (uint32_t)sub * (ROW_B / 16u);
-      uint32_t hi[16], lo[16];
-      if (FMT == FMT_INT4) {
-        const uint4 w = lds128(src + (((c0 + (uint32_t)part) ^ swz) << 4));
-        expand_int4(w.x, s2, hi, lo); expand_int4(w.y, s2, hi + 4, lo + 4);
-        expand_int4(w.z, s2, hi + 8, lo + 8); expand_int4(w.w, s2, hi + 12, lo + 12);
-      } else {
+        if (!__all_sync(0xffffffffu, mbar_wait(&wfull[wat.slot], wat.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+        // 16-byte chunk c of the row's 128 bytes is at (c ^ swz) << 4
+        const uint32_t src = wtiles + (uint32_t)wat.slot * WS_BYTES + (uint32_t)row * 128u, c0 = (uint32_t)sub * (ROW_B / 16u);
+        uint32_t hi[16], lo[16];
+        if (FMT == FMT_INT4) {
+          const uint4 w = lds128(src + (((c0 + (uint32_t)part) ^ swz) << 4));
+          expand_int4(w.x, s2, hi, lo); expand_int4(w.y, s2, hi + 4, lo + 4);
+          expand_int4(w.z, s2, hi + 8, lo + 8); expand_int4(w.w, s2, hi + 12, lo + 12);
+        } else {
 #pragma unroll
-        for (int pp = 0; pp < 2; ++pp) {
-          const uint4 w = lds128(src + (((c0 + (uint32_t)(part * 2 + pp)) ^ swz) << 4));
-          expand_int8(w.x, hi + pp * 8); expand_int8(w.y, hi + pp * 8 + 2);
-          expand_int8(w.z, hi + pp * 8 + 4); expand_int8(w.w, hi + pp * 8 + 6);
+          for (int pp = 0; pp < 2; ++pp) {
+            const uint4 w = lds128(src + (((c0 + (uint32_t)(part * 2 + pp)) ^ swz) << 4));
+            expand_int8(w.x, hi + pp * 8); expand_int8(w.y, hi + pp * 8 + 2);
+            expand_int8(w.z, hi + pp * 8 + 4); expand_int8(w.w, hi + pp * 8 + 6);
+          }
         }
-      }
-      if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
-      tc_fence_after();
-      tmem_st16(ta + (uint32_t)at.slot * A_COLS, hi);
-      if (FMT == FMT_INT4) tmem_st16(ta + (uint32_t)at.slot * A_COLS + 32u, lo);
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(PAIR && rank == 0 ? &xfull[at.slot] : &a_full[at.slot]);
+        if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
+        tc_fence_after();
+        tmem_st16(ta + (uint32_t)at.slot * A_COLS, hi);
+        if (FMT == FMT_INT4) tmem_st16(ta + (uint32_t)at.slot * A_COLS + 32u, lo);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(PAIR && rank == 0 ? &xfull[at.slot] : &a_full[at.slot]);
       }
       if (sub == KSUB - 1) {
         if (lane == 0) mbar_arrive(&wempty[wat.slot]);   // (the last slot of this K range is not asked for again)
@@ -1647,6 +1631,7 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
 // 65536 logits took it 29 us; eight take 5.
 __global__ void __launch_bounds__(256) argmax_rows_kernel(const float *logits, int V, int ld, int32_t *out, const GreedyCtl *ctl) {
   pdl_trigger();
+  cluster_sync();      // the first CTA is there to be written to
   pdl_wait();
   __shared__ unsigned long long best[8], parts[8];
   const int b = blockIdx.y;
@@ -1747,10 +1732,9 @@ __global__ void __launch_bounds__(WKV_THREADS) wkv5_seq_kernel(SeqWkvArgs a) {
   __shared__ __align__(16) float sr[2][WKV_TT][64], sk[2][WKV_TT][64], sv[2][WKV_TT][64];
   const int h = blockIdx.x, c = blockIdx.y, C = a.C;
   const int jg = threadIdx.x >> 2, iq = threadIdx.x & 3;
-  // batch mode: blockIdx.y is the stream, its one token is row c, its state lies state_stride floats further
-  const int t_begin = a.batch_mode ? c : c * a.chunk_len, t_end = a.batch_mode ? c + 1 : min(a.T, t_begin + a.chunk_len);
+  const int t_begin = c * a.chunk_len, t_end = min(a.T, t_begin + a.chunk_len);
   unsigned long long s2[4][8], w2[8], u2[8];   // pairs over key rows (iq*16 + 2 p, + 2 p + 1)
-  float *Sown = a.state + (a.batch_mode ? (size_t)c * a.state_stride : 0) + (size_t)h * 4096;
+  float *Sown = a.state + (size_t)h * 4096;
   const float *Sin = a.n_chunks == 1 ? Sown : a.s_in + ((size_t)h * a.n_chunks + c) * 4096;
 #pragma unroll
   for (int p = 0; p < 8; ++p) {
@@ -1865,6 +1849,128 @@ __global__ void __launch_bounds__(256) wkv5_combine_kernel(SeqWkvArgs a) {
   S[e] = s;
 }
 
+// GroupNorm over a head's 64 values and the gate: lane l of a warp has values 2 l, 2 l + 1 (group_norm.cu:322-357, att.cu:145-152).  Written as
+// what it rounds to, so that the two kernels that do it give the same bits.
+__device__ __forceinline__ float2 gn_gate_pair(const float2 &v, const float2 &w, const float2 &b, bool gated, const float2 &gg) {
+  float s = v.x + v.y;
+#pragma unroll
+  for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+  const float mean = s * (1.f / 64.f);
+  const float d0 = v.x - mean, d1 = v.y - mean;
+  float q = __fmaf_rn(d0, d0, __fmul_rn(d1, d1));
+#pragma unroll
+  for (int k = 16; k > 0; k >>= 1) q += __shfl_xor_sync(0xffffffffu, q, k);
+  const float rstd = rsqrtf(__fmaf_rn(q, 1.f / 64.f, 1e-5f));
+  float2 o = make_float2(__fmaf_rn(__fmul_rn(d0, rstd), w.x, b.x), __fmaf_rn(__fmul_rn(d1, rstd), w.y, b.y));
+  if (gated) { o.x *= gg.x; o.y *= gg.y; }
+  return o;
+}
+__device__ __forceinline__ void store_pair(__half *out, __half *out_lo, size_t o, const float2 &v) {
+  const __half2 h = __floats2half2_rn(v.x, v.y);
+  *reinterpret_cast<__half2 *>(out + o) = h;
+  if (out_lo) {
+    const float2 f = __half22float2(h);
+    *reinterpret_cast<__half2 *>(out_lo + o) = __floats2half2_rn(v.x - f.x, v.y - f.y);
+  }
+}
+
+// RWKV-5 over rows (streams, one token each): the step of wkv5_seq_kernel<2>, with the projections' split-K slabs summed ahead of it (in slab
+// order, as gemm_finish_kernel does) and GroupNorm and gate behind it.  One CTA per (head, stream); a chain of few streams has two
+// launches fewer per layer (16 fp16 streams of the 3B shape: finishing pass 4.1 us, state 9.4, GroupNorm 2.7).
+__global__ void __launch_bounds__(WKV_THREADS) wkv5_rows_kernel(Wkv5RowsArgs a) {
+  pdl_trigger();
+  __shared__ __align__(16) float sr[64], sk[64], sv[64], sg[64], sy[64];
+  const int h = blockIdx.x, row = blockIdx.y, C = a.C, tid = threadIdx.x, jg = tid >> 2, iq = tid & 3, c = h * 64 + tid;
+  unsigned long long s2[4][8], w2[8], u2[8];   // pairs over key rows (iq*16 + 2 p, + 2 p + 1)
+#pragma unroll
+  for (int p = 0; p < 8; ++p) {
+    const int ii = iq * 16 + 2 * p;
+    w2[p] = a.per_head ? pack_f2(a.decay[h], a.decay[h]) : pack_f2(a.decay[h * 64 + ii], a.decay[h * 64 + ii + 1]);
+    u2[p] = a.per_head ? pack_f2(a.first[h], a.first[h]) : pack_f2(a.first[h * 64 + ii], a.first[h * 64 + ii + 1]);
+  }
+  float cs[4] = {1.f, 1.f, 1.f, 1.f};
+  if (a.split > 1)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (a.cs[i]) cs[i] = __half2float(a.cs[i][c]);
+  pdl_wait();
+  float *S = a.state + (size_t)row * a.state_stride + (size_t)h * 4096;
+#pragma unroll
+  for (int p = 0; p < 8; ++p)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int ii = iq * 16 + 2 * p;
+      s2[q][p] = pack_f2(S[ii * 64 + jg + 16 * q], S[(ii + 1) * 64 + jg + 16 * q]);
+    }
+  const size_t o = (size_t)row * C + c;
+  if (a.split > 1) {
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+    const size_t zs = (size_t)a.rows * C;
+    for (int z = 0; z < a.split; ++z)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < 3 || a.gated) x[i] += a.raw[i][z * zs + o];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (a.cs[i]) x[i] *= cs[i];
+    sk[tid] = x[0]; sv[tid] = x[1]; sr[tid] = x[2];
+    const float e = epi_half_op<GEMM_EPI_SILU_F16>(x[3]);
+    const __half gh = __float2half_rn(e);
+    sg[tid] = __half2float(gh) + __half2float(__float2half_rn(e - __half2float(gh)));
+  } else {
+    sk[tid] = a.k[o]; sv[tid] = a.v[o]; sr[tid] = a.r[o];
+    sg[tid] = a.gated ? __half2float(a.g[o]) + __half2float(a.g_lo[o]) : 0.f;
+  }
+  __syncthreads();
+  float vj[4];
+  unsigned long long v2[4], y2[4] = {0ull, 0ull, 0ull, 0ull}, ruk2 = 0ull;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    vj[q] = sv[jg + 16 * q];
+    v2[q] = pack_f2(vj[q], vj[q]);
+  }
+#pragma unroll
+  for (int p = 0; p < 8; ++p) {
+    const unsigned long long kk = *reinterpret_cast<const unsigned long long *>(&sk[iq * 16 + 2 * p]);
+    const unsigned long long rr = *reinterpret_cast<const unsigned long long *>(&sr[iq * 16 + 2 * p]);
+    ruk2 = fma_f2(mul_f2(rr, u2[p]), kk, ruk2);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      y2[q] = fma_f2(rr, s2[q][p], y2[q]);
+      s2[q][p] = fma_f2(s2[q][p], w2[p], mul_f2(kk, v2[q]));
+    }
+  }
+  float ra, rb;
+  unpack_f2(ruk2, ra, rb);
+  const float ruk = ra + rb;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float ya, yb;
+    unpack_f2(y2[q], ya, yb);
+    float y = fmaf(vj[q], ruk, ya + yb);
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    y += __shfl_xor_sync(0xffffffffu, y, 2);
+    if (iq == 0) sy[jg + 16 * q] = y;
+  }
+#pragma unroll
+  for (int p = 0; p < 8; ++p)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float lo, hi;
+      unpack_f2(s2[q][p], lo, hi);
+      const int ii = iq * 16 + 2 * p;
+      S[ii * 64 + jg + 16 * q] = lo;
+      S[(ii + 1) * 64 + jg + 16 * q] = hi;
+    }
+  __syncthreads();
+  if (tid < 32) {
+    const int cc = h * 64 + 2 * tid;
+    const float2 w = make_float2(a.lnx_w[cc], a.lnx_w[cc + 1]), b = make_float2(a.lnx_b[cc], a.lnx_b[cc + 1]);
+    store_pair(a.out, a.out_lo, (size_t)row * C + cc,
+               gn_gate_pair(make_float2(sy[2 * tid], sy[2 * tid + 1]), w, b, a.gated, make_float2(sg[2 * tid], sg[2 * tid + 1])));
+  }
+}
+
 // GroupNorm over each head's 64 readout values (eps 1e-5, fp32 affine), times the gate where the version has one
 // (att_seq.cu:406-415): one warp per (token, head)
 __global__ void __launch_bounds__(256) gn_gate_seq_kernel(const float *y, const float *lnx_w, const float *lnx_b, const __half *g,
@@ -1875,32 +1981,17 @@ __global__ void __launch_bounds__(256) gn_gate_seq_kernel(const float *y, const 
   if (unit >= T * H) return;
   const int t = unit / H, h = unit - t * H;
   const size_t o = (size_t)t * H * 64 + h * 64 + lane * 2;
-  const float2 v = *reinterpret_cast<const float2 *>(y + o);
-  float s = v.x + v.y;
-#pragma unroll
-  for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
-  const float mean = s * (1.f / 64.f);
-  const float d0 = v.x - mean, d1 = v.y - mean;
-  float q = d0 * d0 + d1 * d1;
-#pragma unroll
-  for (int k = 16; k > 0; k >>= 1) q += __shfl_xor_sync(0xffffffffu, q, k);
-  const float rstd = rsqrtf(q * (1.f / 64.f) + 1e-5f);
   const int c = h * 64 + lane * 2;
-  float a0 = d0 * rstd * lnx_w[c] + lnx_b[c], a1 = d1 * rstd * lnx_w[c + 1] + lnx_b[c + 1];
+  float2 gg = make_float2(0.f, 0.f);
   if (g) {
-    float2 gg = __half22float2(*reinterpret_cast<const __half2 *>(g + o));
+    gg = __half22float2(*reinterpret_cast<const __half2 *>(g + o));
     if (g_lo) {
       const float2 gl = __half22float2(*reinterpret_cast<const __half2 *>(g_lo + o));
       gg.x += gl.x; gg.y += gl.y;
     }
-    a0 *= gg.x; a1 *= gg.y;
   }
-  const __half2 hh = __floats2half2_rn(a0, a1);
-  *reinterpret_cast<__half2 *>(out + o) = hh;
-  if (out_lo) {
-    const float2 hf = __half22float2(hh);
-    *reinterpret_cast<__half2 *>(out_lo + o) = __floats2half2_rn(a0 - hf.x, a1 - hf.y);
-  }
+  store_pair(out, out_lo, o, gn_gate_pair(*reinterpret_cast<const float2 *>(y + o), make_float2(lnx_w[c], lnx_w[c + 1]),
+                                          make_float2(lnx_b[c], lnx_b[c + 1]), g != nullptr, gg));
 }
 
 // plain LayerNorm of one row -> fp32 vector (ln_out before the head, model_forward_seq.cpp:171-175)
@@ -1962,10 +2053,6 @@ int wkv5_scan_slots() {
 }
 
 cudaError_t launch_wkv5_seq(const SeqWkvArgs &a, int H, cudaStream_t st) {
-  if (a.batch_mode) {
-    launch_k(wkv5_seq_kernel<2>, dim3(dim3(H, a.T)), dim3(WKV_THREADS), 0, st, a);   // n_chunks == 1: every stream reads and writes its own state
-    return cudaGetLastError();
-  }
   if (a.n_chunks <= 1) {
     launch_k(wkv5_seq_kernel<2>, dim3(dim3(H, 1)), dim3(WKV_THREADS), 0, st, a);
     return cudaGetLastError();
@@ -1974,6 +2061,9 @@ cudaError_t launch_wkv5_seq(const SeqWkvArgs &a, int H, cudaStream_t st) {
   launch_k(wkv5_combine_kernel, dim3(H * 16), dim3(256), 0, st, a);
   launch_k(wkv5_seq_kernel<2>, dim3(dim3(H, a.n_chunks)), dim3(WKV_THREADS), 0, st, a);
   return cudaGetLastError();
+}
+cudaError_t launch_wkv5_rows(const Wkv5RowsArgs &a, int H, cudaStream_t st) {
+  return launch_k(wkv5_rows_kernel, dim3(H, a.rows), dim3(WKV_THREADS), 0, st, a);
 }
 cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
   if (!a.batch_mode) {
