@@ -244,16 +244,19 @@ __device__ __forceinline__ void tile_half(uint32_t buf, bool lo, const uint32_t 
     if (lo) sts_u16(at + 2048 + i * 64, __half_as_ushort(__float2half_rn(e - __half2float(h))));
   }
 }
-// rows row0 .. row0 + 31, channels ch_w .. ch_w + 31 (lane l: ch_w + l) of one problem; z: its K range, when raw
-__device__ __forceinline__ void tile_out(const GemmArgs &g, const CUtensorMap *om, const CUtensorMap *om_lo, bool raw, int z, int ch_w,
+// rows row0 .. row0 + 31, channels ch_w .. ch_w + 31 (lane l: ch_w + l) of one problem; RAW: its slab of K range z.  (A kernel is
+// compiled for slabs and for finished results apart: with both in one, the slabs of few rows, a dozen microseconds a product, came
+// out half a microsecond later -- 10 fp16 tokens of the RWKV-5 3B shape 2.26 ms against 2.14, 16 streams of the 0.1B shape 381 us against 372.)
+template <bool RAW>
+__device__ __forceinline__ void tile_out(const GemmArgs &g, const CUtensorMap *om, const CUtensorMap *om_lo, int z, int ch_w,
                                          int row0, uint32_t (&acc)[32], uint32_t buf) {
   const int lane = threadIdx.x & 31, ch = ch_w + lane;
   const bool ok = ch < g.N;
-  const int epi = raw ? GEMM_EPI_F32 : g.epi;
+  const int epi = RAW ? GEMM_EPI_F32 : g.epi;
   if (epi == GEMM_EPI_ADD_F32) tile_add<false>(g, ch, ok, row0, acc);
   else if (epi == GEMM_EPI_MULADD_F32) tile_add<true>(g, ch, ok, row0, acc);
   const bool f32 = epi == GEMM_EPI_F32 || epi == GEMM_EPI_ADD_F32 || epi == GEMM_EPI_MULADD_F32;
-  if (raw || g.tma_out) {
+  if (RAW || g.tma_out) {
     if (f32) {
 #pragma unroll
       for (int i = 0; i < 32; ++i) sts_u32(buf + i * 128 + lane * 4, acc[i]);
@@ -268,7 +271,7 @@ __device__ __forceinline__ void tile_out(const GemmArgs &g, const CUtensorMap *o
     __syncwarp();
     if (lane == 0) {
       if (ch_w < g.N) {
-        tma_store_3d(om, buf, ch_w, row0, raw ? z : 0);
+        tma_store_3d(om, buf, ch_w, row0, RAW ? z : 0);
         if (!f32 && g.out_lo) tma_store_3d(om_lo, buf + 2048, ch_w, row0, 0);
       }
       asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group.read 1;" ::: "memory");   // the other buffer is free again
@@ -350,8 +353,9 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 // of its own with the same 128 x 256 accumulator would fetch, and read from shared memory at every MMA, all 32 KB of X.
 // Two CTAs per SM (3 slots of 32 KB and 256 TMEM columns each): the start and the end of one hide in part behind the main loop
 // of the other, and tiles are handed out by the hardware, also across the two row pieces of a long prompt.
-// [2048 x 2560] x [2560 x 11520] with the relu^2 epilogue: 107 us (1,130 TFLOP/s); 256 x 256 tiles of single CTAs, whose
-// epilogue nothing hid, 182.  Without its epilogue 82, without its loads 100: the epilogue is what is left.
+// [2048 x 2560] x [2560 x 11520] with the relu^2 epilogue: 104 us (1,160 TFLOP/s) at 256 rows a tile; 256 x 256 tiles of single CTAs,
+// whose epilogue nothing hid, 182.  Without its epilogue 82, without its loads 100 (of 107 then): the epilogue is what is left.  One
+// CTA per SM over all tiles with two accumulators: 92, but products of one wave 10 to 40 % slower, a prompt of 4,096 36.4 ms against 35.0.
 //   warp 0: TMA into the own shared memory; the bytes of both CTAs are counted on the even CTA's barrier
 //   warp 1: TMEM, and in the even CTA the MMAs of the pair        warps 2..5: epilogue, a TMEM lane quadrant each
 // Low halves of X (A2) meet the same weights beside the high ones, after them in the same slot, or in slots of their own after
@@ -359,6 +363,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 constexpr int PAIR_MAX_STAGES = 8;
 constexpr uint32_t PAIR_TMEM_COLS = 256;
 
+template <bool SLABS>
 __global__ void __launch_bounds__(G_THREADS, 2)
 gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   const int STAGES = grp.stages, BN = grp.bn;
@@ -471,7 +476,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
         }
-        tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
+        tile_out<SLABS>(g, &maps.o[pi], &maps.o_lo[pi], blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
       }
       tile_out_end();
     }
@@ -496,7 +501,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 constexpr int WT_MAX_STAGES = 8;
 
 // grp.dual here: some problem has A2 (the slot holds an X lo tile)
-template <int BN>
+template <int BN, bool SLABS>
 __global__ void __launch_bounds__(G_THREADS, 2)
 gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   constexpr uint32_t X_BYTES = BN * GBK * 2;
@@ -601,7 +606,7 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
     const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
-      const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
+      const float sc = (!SLABS && g.col_scale && ch < g.N) ? __half2float(g.col_scale[ch]) : 1.f;
       const uint32_t buf = tiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
       uint32_t flip = 0;
       for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
@@ -614,12 +619,12 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
         }
-        if (g.col_scale && grp.split == 1) {
+        if (!SLABS && g.col_scale) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
         }
-        if (BN == 32 && grp.split > 1) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
-        else tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, tile_n * GBM + quad * 32, m0 + c0, acc, buf + flip);
+        if (SLABS && BN == 32) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
+        else tile_out<SLABS>(g, &maps.o[pi], &maps.o_lo[pi], blockIdx.z, tile_n * GBM + quad * 32, m0 + c0, acc, buf + flip);
       }
       tile_out_end();
     }
@@ -750,7 +755,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
 constexpr int gq_threads(int ew) { return 32 * (3 + ew); }
 constexpr int GQ_MAX = 8;                // most slots of any ring
 
-template <int FMT, bool PAIR, int EW>
+template <int FMT, bool PAIR, int EW, bool SLABS>
 __global__ void __launch_bounds__(gq_threads(EW), EW == 8 ? 2 : 1)
 gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup grp) {
   constexpr uint32_t ROW_B = FMT == FMT_INT8 ? GBK : GBK / 2;          // packed bytes per row and slice
@@ -931,7 +936,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
     const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
-      const float sc = (g.col_scale && ch < g.N && grp.split == 1) ? __half2float(g.col_scale[ch]) : 1.f;
+      const float sc = (!SLABS && g.col_scale && ch < g.N) ? __half2float(g.col_scale[ch]) : 1.f;
       const uint32_t buf = xtiles + (uint32_t)(warp - 2) * 2 * EPI_BUF;   // the rings have been read
       uint32_t flip = 0;
       for (int c0 = nth * 32; c0 < BN; c0 += 8 * EW, flip ^= EPI_BUF) {
@@ -948,12 +953,12 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
             for (int i = 0; i < 16; ++i) acc[h * 16 + i] = __float_as_uint(__uint_as_float(acc[h * 16 + i]) + __uint_as_float(more[i]));
           }
         }
-        if (g.col_scale && grp.split == 1) {
+        if (!SLABS && g.col_scale) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
         }
-        if (!PAIR && BN == 32 && grp.split > 1) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
-        else tile_out(g, &maps.o[pi], &maps.o_lo[pi], grp.split > 1, blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
+        if (SLABS && !PAIR && BN == 32) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
+        else tile_out<SLABS>(g, &maps.o[pi], &maps.o_lo[pi], blockIdx.z, ch0 + quad * 32, m0 + c0, acc, buf + flip);
       }
       tile_out_end();
     }
@@ -1628,7 +1633,7 @@ __global__ void __launch_bounds__(W4_THREADS) wkv4_seq_kernel(Wkv4Args a) {
 // greedy sample of every row: index of the largest logit (lowest index on ties).  ctl (optional): the id also goes
 // to row ctl->step of the history ctl->hist -- fixed kernel arguments, so that a captured graph can be replayed.
 // A cluster of CTAs per row (gridDim.x of them), each over its part of the vocabulary: one CTA has 64 KB in flight at most, and a row of
-// 65536 logits took it 29 us; eight take 5.
+// 65536 logits took it 29 us.  A step of 16 streams: 410 -> 396 us (0.1B shape), 1185 -> 1154 (1.5B).
 __global__ void __launch_bounds__(256) argmax_rows_kernel(const float *logits, int V, int ld, int32_t *out, const GreedyCtl *ctl) {
   pdl_trigger();
   cluster_sync();      // the first CTA is there to be written to
@@ -2167,7 +2172,8 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
   dim3 grid(tiles, m_tiles, grp.split);
-  auto kern = bn == 32 ? gemm_wt_kernel<32> : bn == 64 ? gemm_wt_kernel<64> : gemm_wt_kernel<128>;
+  auto kern = grp.split > 1 ? (bn == 32 ? gemm_wt_kernel<32, true> : bn == 64 ? gemm_wt_kernel<64, true> : gemm_wt_kernel<128, true>)
+                            : (bn == 32 ? gemm_wt_kernel<32, false> : bn == 64 ? gemm_wt_kernel<64, false> : gemm_wt_kernel<128, false>);
   cudaError_t e = launch_k(kern, grid, dim3(G_THREADS), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
@@ -2245,7 +2251,7 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((alone ? 200u << 10 : 110u << 10) / grp.stage_bytes));
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
-  cudaError_t e = launch_cluster_k(gemm_pair_kernel, 2, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp);
+  cudaError_t e = launch_cluster_k(grp.split > 1 ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, 2, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
   if (grp.split > 1 && !defer_split) {
@@ -2254,6 +2260,14 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
     launch_k(gemm_finish_kernel, dim3((M * (max_n / 4) + 255) / 256, n), dim3(256), 0, st, grp);
   }
   return cudaGetLastError();
+}
+
+using GemmKernel = void (*)(GemmMaps, GemmGroup);
+template <bool SLABS>
+GemmKernel gemm_q_kern(int fmt, bool pair, bool two_per_sm) {
+  if (pair) return fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, true, 16, SLABS> : gemm_q_kernel<FMT_INT8, true, 16, SLABS>;
+  if (two_per_sm) return fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false, 8, SLABS> : gemm_q_kernel<FMT_INT8, false, 8, SLABS>;
+  return fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false, 16, SLABS> : gemm_q_kernel<FMT_INT8, false, 16, SLABS>;
 }
 
 // quantised weights in packed form (GemmArgs::Wq): gemm_q_kernel, on pairs of SMs above 128 rows
@@ -2326,9 +2340,7 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
   const size_t rings = (size_t)grp.xstages * grp.stage_bytes + (size_t)grp.stages * ws;
   const int ew = two_per_sm ? 8 : 16;
   const size_t smem = 1024 + std::max<size_t>(rings, ew * 2 * EPI_BUF) + 1024;
-  auto kern = pair         ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, true, 16> : gemm_q_kernel<FMT_INT8, true, 16>)
-              : two_per_sm ? (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false, 8> : gemm_q_kernel<FMT_INT8, false, 8>)
-                           : (fmt == FMT_INT4 ? gemm_q_kernel<FMT_INT4, false, 16> : gemm_q_kernel<FMT_INT8, false, 16>);
+  auto kern = grp.split > 1 ? gemm_q_kern<true>(fmt, pair, two_per_sm) : gemm_q_kern<false>(fmt, pair, two_per_sm);
   const dim3 grid((pair ? 2 : 1) * tiles * grp.m_tiles, 1, grp.split);
   cudaError_t e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(gq_threads(ew)), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
@@ -2360,11 +2372,15 @@ cudaError_t launch_gemm_group(const GemmArgs *probs, int n, cudaStream_t st, int
 cudaError_t gemm_prepare(int device) {
   int optin = 0;
   cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  const void *kerns[] = {(const void *)gemm_wt_kernel<32>, (const void *)gemm_wt_kernel<64>, (const void *)gemm_wt_kernel<128>,
-                         (const void *)gemm_pair_kernel, (const void *)gemm_q_kernel<FMT_INT8, false, 8>, (const void *)gemm_q_kernel<FMT_INT8, false, 16>, (const void *)gemm_q_kernel<FMT_INT8, true, 16>,
-                         (const void *)gemm_q_kernel<FMT_INT4, false, 8>, (const void *)gemm_q_kernel<FMT_INT4, false, 16>, (const void *)gemm_q_kernel<FMT_INT4, true, 16>};
-  for (const void *k : kerns)
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  const GemmKernel f16[] = {gemm_wt_kernel<32, false>, gemm_wt_kernel<64, false>, gemm_wt_kernel<128, false>, gemm_pair_kernel<false>,
+                            gemm_wt_kernel<32, true>, gemm_wt_kernel<64, true>, gemm_wt_kernel<128, true>, gemm_pair_kernel<true>};
+  for (GemmKernel k : f16)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  for (int fmt : {(int)FMT_INT8, (int)FMT_INT4})
+    for (int way = 0; way < 3; ++way) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)gemm_q_kern<false>(fmt, way == 0, way == 1), cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute((const void *)gemm_q_kern<true>(fmt, way == 0, way == 1), cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    }
   return e;
 }
 

@@ -115,6 +115,40 @@ def test_layernorm_rows_of_every_width(pkg, orc, synth, C):
     m.close()
 
 
+@pytest.mark.parametrize("version,fmt,B", [("5.2", "fp16", 9), ("5.1", "int8", 17), ("5", "int4", 33), ("5.2", "int8", 130)])
+def test_rwkv5_rows_add_their_slabs(pkg, orc, synth, version, fmt, B):
+    """The RWKV-5 row kernel behind products whose K is cut in several pieces (1,088 inputs: 17 slices, the last piece a short
+    one), with and without the gate, decay by head and by channel, up to 128 rows and above."""
+    shape = synth.Shape(version, 1, 1088, 1152, 96, n_head=17)
+    strat, fdt = STR[fmt]
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), fdt)
+    ref = orc.OracleModel(shape, tensors, synth.param_names(shape), rescale_every=6 if fmt == "fp16" else 0,
+                          weight_format=fmt, state_fp16=fmt == "fp16")
+    m = pkg.Model(tensors, strat, shape=shape, max_batch=B)
+    ids = synth.token_ids(shape, 3 * B, seed=8).reshape(3, B)
+    got = [m.decode(ids[t]) for t in range(3)]
+    for b in (0, B // 2, B - 1):
+        ref.reset()
+        for t in range(3):
+            _close(got[t][b], ref.run(int(ids[t, b])), f"{version} {fmt} stream {b} of {B} step {t}")
+    m.close()
+
+
+@pytest.mark.parametrize("vocab", [61, 1027, 16390, 40001])
+def test_argmax_of_rows_with_ties(pkg, synth, vocab):
+    """The arg-max of a row is found in parts: every logit turns up several times (the head repeats after 59 words), so that the
+    largest one stands in several parts, and its first place is the answer.  Ragged widths, some parts with nothing to do."""
+    shape = synth.Shape("4", 1, 128, 256, vocab)
+    tensors = synth.generate(shape, seed=3, ln_random=True)
+    tensors["head.weight"] = np.ascontiguousarray(tensors["head.weight"][:, np.arange(vocab) % 59])
+    m = pkg.Model(synth.to_file_dtypes(shape, tensors, "fp16"), "cuda fp16", shape=shape, max_batch=9)
+    ids = synth.token_ids(shape, 9, seed=6)
+    want = m.decode(ids).argmax(1)
+    m.reset_states()
+    assert np.array_equal(m.decode(ids, want_logits=False, want_argmax=True), want) and want.max() < 59
+    m.close()
+
+
 def test_small_and_large_batches_share_state(pkg, orc, synth):
     """The persistent kernel (<= 8 streams) and the GEMM path (> 8) read and write the same state slots, and streams
     that are decoded together need not have seen the same number of tokens (continuous batching: a stream joins a
