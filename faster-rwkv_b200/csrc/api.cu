@@ -77,11 +77,12 @@ struct fr_b200_model {
   __half *d_plain = nullptr;     size_t plain_halfs = 0;   // fp16 models: W^T [out, in]
   __half *d_pscale = nullptr;    size_t pscale_halfs = 0;  // int8: per output row scales, per matrix
   // int8 / int4: every projection a second time in its packed interchange form, row-major (one row per output
-  // channel): what the few-row GEMM streams for prompts and for decode of more than 8 streams
+  // channel): what the GEMM path streams for prompts and for the batches of rows_batch() and above
   uint8_t *d_qcopy = nullptr;    size_t qcopy_bytes = 0;
   __half *d_qscale = nullptr;    size_t qscale_halfs = 0;
   bool row_copies = true;        // keep the copies the GEMM path needs (FR_B200_ROW_COPIES=0: decode-only model)
-  bool rows_planned = false;     // some batch up to max_batch is decoded by the GEMM path
+  bool rows_planned = false;     // some batch up to max_batch is decoded by the GEMM path,
+  bool rows_needed = false;      // and no other kernel could
   uint8_t *d_seq = nullptr;      size_t seq_bytes = 0; int seq_T = 0;
   PhaseDev *d_head_phase = nullptr;   // the head as a stand-alone matvec phase
   // greedy runs of many streams: two decode steps captured as a CUDA graph and replayed (the step is ~170 launches)
@@ -160,7 +161,7 @@ bool wide_batch(int fmt, bool v5, int batch) { return batch > 4 || (fmt != FMT_F
 // 1.26 against 1.23.  (4 fp16 streams would win there, too, 1.25 against 1.11, but for a second copy of the weights.)  RWKV-5 keeps its
 // kernel for its sums.
 bool rows_batch(const fr_b200_model *m, int batch) {
-  return !m->v5 && m->row_copies && (batch > 4 || (batch > 2 && m->fmt == FMT_INT8 && m->C >= 2048));
+  return !m->v5 && m->row_copies && m->C <= 8192 && (batch > 4 || (batch > 2 && m->fmt == FMT_INT8 && m->C >= 2048));
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
@@ -240,20 +241,22 @@ void plan(fr_b200_model *m) {
   woff += (size_t)nbV * rbC; roff += (size_t)nbV * ROWS;
   m->weights_bytes = woff; m->rscale_n = roff; m->vecs_n = voff;
   m->plain_halfs = 0; m->pscale_halfs = 0; m->qcopy_bytes = 0; m->qscale_halfs = 0;
-  // The GEMM path (prompts, and decode of more than 8 streams at once) reads the projections row by output channel:
-  // fp16 models keep W^T fp16 [N, K] (with the head when more than 8 streams can be decoded: all rows want logits;
+  // The GEMM path (prompts, and the batches that decode_by_rows() sends there) reads the projections row by output channel:
+  // fp16 models keep W^T fp16 [N, K] (with the head when such a batch can be decoded: all rows want logits;
   // a prompt's head is a matvec over the last token), made at load for RWKV-5.x and where rows_batch() takes max_batch streams, else on the
   // first long prompt; int8 / int4 models keep the packed codes row-major [N, K] / [N, K/2] (+ scales), the same
-  // bytes as the streaming tiles, which the GEMM expands in shared memory.
+  // bytes as the streaming tiles, which the GEMM expands into tensor memory.
   // (also when the persistent kernel cannot carry max_batch streams of a model this wide: its shared memory holds the
   // activation vectors of every stream, e.g. 8 streams x 8192 channel-mix inputs do not fit)
-  bool big = m->cfg.max_batch > MAX_B || rows_batch(m, m->cfg.max_batch);
+  bool big = m->cfg.max_batch > MAX_B;
   if (!big) {
     int optin = 0;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) == cudaSuccess)
       for (int b = 2; b <= m->cfg.max_batch; ++b)
         if ((wide_batch(fmt, m->v5, b) ? decode_smem_bytes(fmt, decode_mode(b), C, F, m->v5 ? 5 : 4, 2) : step_smem_bytes(fmt, step_mode(b), C, F, m->gate ? 4 : 3, 2)) > (size_t)optin) big = true;
   }
+  m->rows_needed = big;
+  big = big || rows_batch(m, m->cfg.max_batch);
   m->rows_planned = big;
   for (auto &kv : m->mats) {
     MatrixSlot &ms = kv.second;
@@ -448,8 +451,14 @@ int fr_b200_create(const fr_b200_config *cfg, fr_b200_model **out) {
   if (!rc) rc = alloc((void **)&m->d_v5buf, (size_t)5 * B * m->C * sizeof(exch_t));
   if (!rc) rc = alloc((void **)&m->d_out, m->out_bytes());
   if (!rc) rc = alloc((void **)&m->d_amax, (size_t)B * 8);
-  // fp16 W^T copies now for RWKV-5.x (seq kernels) and for models that decode more than 8 streams; else on demand
-  if (!rc && m->plain_halfs && m->row_copies && (m->v5 || m->rows_planned)) rc = alloc((void **)&m->d_plain, m->plain_halfs * 2);
+  // fp16 W^T copies now for RWKV-5.x (seq kernels) and for models whose largest batch goes by rows; else on demand
+  if (!rc && m->plain_halfs && m->row_copies && (m->v5 || m->rows_planned)) {
+    rc = alloc((void **)&m->d_plain, m->plain_halfs * 2);
+    if (rc && !m->v5 && !m->rows_needed) {   // the persistent kernels take every batch of this model
+      cudaGetLastError();
+      m->d_plain = nullptr; m->rows_planned = false; rc = 0;
+    }
+  }
   if (!rc && m->qcopy_bytes) rc = alloc((void **)&m->d_qcopy, m->qcopy_bytes);
   if (!rc && m->qscale_halfs) rc = alloc((void **)&m->d_qscale, m->qscale_halfs * 2);
   if (!rc && m->pscale_halfs) rc = alloc((void **)&m->d_pscale, m->pscale_halfs * 2);
@@ -702,9 +711,17 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
 bool token_kernel_fits(const fr_b200_model *m, int batch) {
   return batch <= MAX_B && (wide_batch(m->fmt, m->v5, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) != 0;
 }
-bool decode_by_rows(const fr_b200_model *m, int batch) {
-  if (batch > MAX_B || rows_batch(m, batch)) return true;
-  return !token_kernel_fits(m, batch);
+bool rows_path_built(const fr_b200_model *m) { return m->d_plain || m->d_qcopy; }
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (st && cudaStreamIsCapturing(st, &s) != cudaSuccess) cudaGetLastError();
+  return s != cudaStreamCaptureStatusNone;
+}
+// A batch that the persistent kernels can take, too, stays with them where the rows would have to allocate and must not (a stream
+// that is being captured) or could not (no room for the row copies).
+bool decode_by_rows(const fr_b200_model *m, int batch, cudaStream_t st) {
+  if (!token_kernel_fits(m, batch)) return true;
+  return rows_batch(m, batch) && rows_path_built(m) && !capturing(st);
 }
 // fp16 models that were created without the W^T copies build them from the streaming tiles (exact: the tiles hold
 // the same fp16 values) the first time the GEMM path is asked for
@@ -713,7 +730,7 @@ int ensure_row_copies(fr_b200_model *m) {
   if (m->fmt != FMT_FP16 || !m->row_copies || !m->plain_halfs) return fail(FR_B200_E_UNSUPPORTED, "the model keeps no row copies for the GEMM path");
   CU(cudaDeviceSynchronize());
   cudaError_t e = cudaMalloc((void **)&m->d_plain, m->plain_halfs * 2);
-  if (e != cudaSuccess) { m->d_plain = nullptr; return fail(FR_B200_E_NOMEM, std::string("cudaMalloc(row copies): ") + cudaGetErrorString(e)); }
+  if (e != cudaSuccess) { m->d_plain = nullptr; cudaGetLastError(); return fail(FR_B200_E_NOMEM, std::string("cudaMalloc(row copies): ") + cudaGetErrorString(e)); }
   for (auto &kv : m->mats) {
     const MatrixSlot &s = kv.second;
     if (!s.has_plain) continue;
@@ -723,7 +740,6 @@ int ensure_row_copies(fr_b200_model *m) {
   free_scratch(m);
   return 0;
 }
-bool rows_path_built(const fr_b200_model *m) { return m->d_plain || m->d_qcopy; }
 int rows_decode_check(fr_b200_model *m, const int32_t *ids_host, int batch, cudaStream_t st) {
   if (m->fmt == FMT_FP16 && !m->mats["head.weight"].has_plain)
     return fail(FR_B200_E_UNSUPPORTED, "this batch size needs the GEMM path, which the model was created without");
@@ -804,9 +820,13 @@ int fr_b200_decode(fr_b200_model *m, const int32_t *ids, int batch, float *logit
   CU(cudaSetDevice(m->device));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int rc;
-  if (decode_by_rows(m, batch)) {
-    if ((rc = rows_decode_check(m, ids, batch, st))) return rc;
-    if ((rc = rows_forward(m, true, 0, ids, batch, st))) return rc;
+  bool rows = decode_by_rows(m, batch, st);
+  if (rows) {
+    if ((rc = rows_decode_check(m, ids, batch, st)) == 0) rc = rows_forward(m, true, 0, ids, batch, st);
+    if (rc == FR_B200_E_NOMEM && token_kernel_fits(m, batch)) rows = false;   // nothing has been launched
+    else if (rc) return rc;
+  }
+  if (rows) {
     if (argmax) {
       CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, m->out_argmax(), nullptr, st));
       m->launches++;
@@ -858,16 +878,21 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
     CU(cudaMalloc((void **)&m->d_hist, need * 12));
     m->hist_n = need;
   }
-  if (decode_by_rows(m, batch)) {
-    // GEMM path: ids stay on the device, row t of the history feeds step t + 1
-    int rc = rows_decode_check(m, first_ids, batch, st);
-    if (rc) return rc;
+  int rc;
+  bool rows = decode_by_rows(m, batch, st);
+  if (rows) {
+    // GEMM path, step 0 from the host ids
+    if ((rc = rows_decode_check(m, first_ids, batch, st)) == 0) rc = rows_forward(m, true, 0, first_ids, batch, st);
+    if (rc == FR_B200_E_NOMEM && token_kernel_fits(m, batch)) rows = false;   // nothing has been launched
+    else if (rc) return rc;
+  }
+  if (rows) {
+    // ids stay on the device, row t of the history feeds step t + 1: every sampled id goes to the row-id buffer of the next step
+    // and to the history
     int32_t *hist32 = reinterpret_cast<int32_t *>(m->d_hist + need);
     GreedyCtl ctl;
     ctl.hist = hist32; ctl.step = 0;
     CU(cudaMemcpyAsync(m->d_ctl, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
-    // step 0 from the host ids; every sampled id goes to the row-id buffer of the next step and to the history
-    if ((rc = rows_forward(m, true, 0, first_ids, batch, st))) return rc;
     int32_t *row_ids = reinterpret_cast<int32_t *>(m->d_seq);   // first piece of the activation blob
     CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, row_ids, m->d_ctl, st));
     m->launches += 2;
@@ -929,8 +954,8 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
   // one packed arg-max word per (token, stream), all cleared up front; token t+1 reads its ids from row t
   CU(cudaMemsetAsync(m->d_hist, 0, need * 8, st));
   for (int t = 0; t < n_tokens; ++t) {
-    int rc = decode_impl(m, t == 0 ? first_ids : nullptr, t == 0 ? nullptr : m->d_hist + (size_t)(t - 1) * batch, batch, st,
-                         m->d_hist + (size_t)t * batch);
+    rc = decode_impl(m, t == 0 ? first_ids : nullptr, t == 0 ? nullptr : m->d_hist + (size_t)(t - 1) * batch, batch, st,
+                     m->d_hist + (size_t)t * batch);
     if (rc) return rc;
   }
   int32_t *ids32 = reinterpret_cast<int32_t *>(m->d_hist + need);   // unpacked ids behind the packed words
@@ -1092,7 +1117,8 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     CU(cudaStreamSynchronize(st));
     if (m->d_seq) cudaFree(m->d_seq);
     m->d_seq = nullptr; m->seq_bytes = 0;
-    CU(cudaMalloc((void **)&m->d_seq, off));
+    const cudaError_t e = cudaMalloc((void **)&m->d_seq, off);
+    if (e != cudaSuccess) { m->d_seq = nullptr; cudaGetLastError(); return fail(FR_B200_E_NOMEM, std::string("cudaMalloc(activation rows): ") + cudaGetErrorString(e)); }
     m->seq_bytes = off;
   }
   uint8_t *B = m->d_seq;
@@ -1345,18 +1371,24 @@ int fr_b200_run_seq(fr_b200_model *m, int slot, const int32_t *ids, int n, float
   // 2 to 12 tokens 1.25 to 1.28 by rows, the first one 5.3 (5.3 for 8 tokens by the loop); 29 tokens 1.34 against 18.2.  0.1B shape: a token 0.21,
   // 2 to 12 tokens 0.42 to 0.43, the first one 5; 14B shape: 5.07, 6.7, 22.
   bool by_rows = rows_path_built(m) && n >= seq_min;
-  if (!by_rows && m->fmt == FMT_FP16 && m->row_copies && m->plain_halfs && n >= std::max(seq_min, PROMPT_BUILD_ROWS)) {
+  // (Short prompts keep the loop on a stream that is being captured, and where there is no room for the copies or the rows.)
+  const bool may_loop = m->fmt == FMT_FP16 && !m->v5 && n < PROMPT_PAIR_ROWS && slot == 0;
+  int rc = 0;
+  if (!by_rows && m->fmt == FMT_FP16 && m->row_copies && m->plain_halfs && n >= std::max(seq_min, PROMPT_BUILD_ROWS) && !(may_loop && capturing(st))) {
     CU(cudaSetDevice(m->device));
-    int rc = ensure_row_copies(m);
-    if (rc) return rc;
-    by_rows = true;
+    rc = ensure_row_copies(m);
+    if (rc && !(rc == FR_B200_E_NOMEM && may_loop)) return rc;
+    by_rows = rc == 0;
   }
   if (by_rows) {
     CU(cudaSetDevice(m->device));
     for (int i = 0; i < n; ++i)
       if (ids[i] < 0 || ids[i] >= m->V) return fail(FR_B200_E_ARG, "token id out of range");
-    int rc = rows_forward(m, false, slot, ids, n, st);
-    if (rc) return rc;
+    rc = rows_forward(m, false, slot, ids, n, st);
+    if (rc && !(rc == FR_B200_E_NOMEM && may_loop)) return rc;
+    by_rows = rc == 0;
+  }
+  if (by_rows) {
     if (last_logits) {
       if (is_host_ptr(last_logits)) {
         CU(cudaMemcpyAsync(m->h_out, m->d_out + (size_t)slot * m->Vpad, (size_t)m->V * 4, cudaMemcpyDeviceToHost, st));
@@ -1375,7 +1407,7 @@ int fr_b200_run_seq(fr_b200_model *m, int slot, const int32_t *ids, int n, float
   }
   if (slot != 0) return fail(FR_B200_E_UNSUPPORTED, "the token loop of run_seq uses stream slot 0");
   for (int i = 0; i < n; ++i) {
-    int rc = fr_b200_decode(m, ids + i, 1, i == n - 1 ? last_logits : nullptr, nullptr, stream);
+    rc = fr_b200_decode(m, ids + i, 1, i == n - 1 ? last_logits : nullptr, nullptr, stream);
     if (rc) return rc;
   }
   if (!last_logits) {

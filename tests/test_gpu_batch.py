@@ -149,6 +149,36 @@ def test_argmax_of_rows_with_ties(pkg, synth, vocab):
     m.close()
 
 
+@pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 8), ("tiny4", "int4", 5)])
+def test_a_captured_step_of_few_streams(pkg, synth, name, fmt, B):
+    """5 to 8 RWKV-4 streams on a stream that is being captured: the first such step (the row path, which would have to allocate its
+    rows, is not taken there) can be captured and replayed, and agrees with the step outside a capture."""
+    import ctypes
+    import torch
+    shape = synth.SHAPES[name]
+    strat, fdt = STR[fmt]
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), fdt)
+    m = pkg.Model(tensors, strat, shape=shape, max_batch=B)
+    ids = synth.token_ids(shape, B, seed=9).astype(np.int32)
+    m.decode(ids[:1])           # what a first launch loads is loaded
+    m.reset_states()
+    got = torch.zeros(B, shape.vocab, device="cuda")
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="thread_local")
+        rc = pkg.lib().fr_b200_decode(m.handle, ids.ctypes.data_as(ctypes.c_void_p), B, ctypes.c_void_p(got.data_ptr()), None,
+                                      ctypes.c_void_p(side.cuda_stream))
+        graph.capture_end()
+    pkg.check(rc, "captured decode")
+    graph.replay()
+    torch.cuda.synchronize()
+    m.reset_states()
+    _close(got.cpu().numpy(), m.decode(ids), f"{name} {fmt} captured")
+    m.close()
+
+
 def test_small_and_large_batches_share_state(pkg, orc, synth):
     """The persistent kernel (<= 8 streams) and the GEMM path (> 8) read and write the same state slots, and streams
     that are decoded together need not have seen the same number of tokens (continuous batching: a stream joins a
