@@ -155,13 +155,14 @@ void free_scratch(fr_b200_model *m) {
 // (fp16 weights give the same bits in both.)
 bool wide_batch(int fmt, bool v5, int batch) { return batch > 4 || (fmt != FMT_FP16 && (v5 || batch > 2)); }
 
-// RWKV-4 batches that the row path (GEMMs over row copies) takes from both of them.  ms, persistent kernel against rows: 0.1B shape 5
-// and 8 fp16 streams 0.50 and 0.64 against 0.39, int8 0.50 and 0.60 against 0.41, int4 0.48 and 0.59 against 0.42, 4 of any format
-// 0.34 to 0.40 against the same; 1.5B shape (whose 5 to 8 streams never fitted) 3 and 4 int8 streams 1.18 and 1.31 against 1.09, int4 1.13 and
-// 1.26 against 1.23.  (4 fp16 streams would win there, too, 1.25 against 1.11, but for a second copy of the weights.)  RWKV-5 keeps its
-// kernel for its sums.
+// RWKV-4 batches that the row path (GEMMs over row copies) takes from both of them.  us, persistent kernel against rows: 0.1B shape 5
+// and 8 fp16 streams 500 and 640 against 365, int8 500 and 600 against 363, int4 480 and 590 against 375; 3 and 4 int8 streams 369 and 391
+// against 360 and 362, int4 367 and 390 against 368 and 372, 2 of either 255 against 360; 1.5B shape (whose 5 to 8 streams never fitted) 3 and
+// 4 int8 streams 1180 and 1310 against 918 and 924, int4 1117 and 1254 against 1054 and 1066, 2 of either 765 to 785 against 918 and 1065.
+// (3 and 4 fp16 streams would win there, too, 1123 and 1228 against 1059 and 1067, but for a second copy of the weights; at the 0.1B shape they
+// take 297 and 326 against 363 and 365.)  RWKV-5 keeps its kernel for its sums.
 bool rows_batch(const fr_b200_model *m, int batch) {
-  return !m->v5 && m->row_copies && m->C <= 8192 && (batch > 4 || (batch > 2 && m->fmt == FMT_INT8 && m->C >= 2048));
+  return !m->v5 && m->row_copies && m->C <= 8192 && batch > (m->fmt == FMT_FP16 ? 4 : 2);
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
