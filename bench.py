@@ -73,8 +73,13 @@ def measured_peaks():
         return 6650.0, 1590.0, 1400.0, "fallback"
 
 
-# which of the two takes a batch: wide_batch() in api.cu
+# which of the two takes a batch: wide_batch() in api.cu; which batches of an RWKV-4 model go by rows: rows_batch()
 TOKEN_KERNEL = "step_kernel / decode_kernel (persistent, one launch per token)"
+ROWS_KERNEL = "batched decode step: few-row tcgen05 GEMMs + row kernels (steps replayed as a CUDA graph)"
+
+
+def kernel_of(shape, fmt, B):
+    return TOKEN_KERNEL if B <= (8 if shape.version.startswith("5") else 4 if fmt == "fp16" else 2) else ROWS_KERNEL
 
 
 def hbm_roofline(shape, fmt, ms_per_step, kernel):
@@ -92,7 +97,7 @@ def batched_roofline(shape, fmt, streams, ms_per_step):
     algo_b, algo_f = algorithmic_bytes(shape, fmt), 2.0 * projection_params(shape) * streams
     t_b, t_f = algo_b / (hbm * 1e9), algo_f / (tens * 1e12)
     s = ms_per_step * 1e-3
-    kernel = "batched decode step: few-row tcgen05 GEMMs + row kernels (steps replayed as a CUDA graph)"
+    kernel = ROWS_KERNEL
     if t_f >= t_b:
         ach = algo_f / s / 1e12
         return {"bound": "tensor", "achieved": ach, "peak": tens, "unit": "TFLOP/s", "frac": ach / tens, "traffic": None,
@@ -162,7 +167,7 @@ def prefill_leg(pkg, device_index: int, wl: str = "c3", T: int = 4096, reps: int
                "roofline": {"bound": "tensor", "achieved": tf, "peak": burst, "unit": "TFLOP/s", "frac": tf / burst,
                             "traffic": None, "peak_source": kind + " (burst: the prompt is one 30-50 ms call)",
                             "frac_of_sustained_peak": tf / sustained,
-                            "kernel": "gemm_f16_kernel (tcgen05) + state scan + row kernels"}}
+                            "kernel": "gemm_pair_kernel (tcgen05) + state scan + row kernels"}}
         drop(m)
         del m
         # 16 streams: one prompt each, slot by slot (a 4096-token prompt already fills the tensor cores), then 64
@@ -578,7 +583,7 @@ def main():
         clocks = cs.summary()
         ms_max = max_over_ranks(ms)
         value = world * B * K / (ms_max * 1e-3)
-        roofline = hbm_roofline(shape, fmt, ms_max / K, TOKEN_KERNEL) if B <= 8 else \
+        roofline = hbm_roofline(shape, fmt, ms_max / K, kernel_of(shape, fmt, B)) if B <= 8 else \
             batched_roofline(shape, fmt, B, ms_max / K)
         # end to end: host ids in, host logits out, every step, through the public API
         model.reset_states()
@@ -620,7 +625,7 @@ def main():
                 steps_v = 256
                 vms, _, _ = timed_greedy(torch, barrier, mv, synth.token_ids(c1, vb, seed=0), steps_v, W)
                 variants[f"c1_{vf}_b{vb}"] = {"tok_s": vb * steps_v / (vms * 1e-3), "ms_per_step": vms / steps_v,
-                                             "roofline": hbm_roofline(c1, vf, vms / steps_v, TOKEN_KERNEL)}
+                                             "roofline": hbm_roofline(c1, vf, vms / steps_v, kernel_of(c1, vf, vb))}
                 drop(mv)
                 del mv
             except Exception as ex:  # a variant must not lose the headline
