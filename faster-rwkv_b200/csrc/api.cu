@@ -561,6 +561,8 @@ int fr_b200_set_tensor(fr_b200_model *m, const char *name, const void *data, int
   return fail(FR_B200_E_ARG, "unknown tensor name " + nm);
 }
 
+namespace { int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids, int R, cudaStream_t st); }
+
 int fr_b200_finalize(fr_b200_model *m) {
   if (!m) return fail(FR_B200_E_ARG, "null model");
   if (m->finalized) return FR_B200_OK;
@@ -683,6 +685,12 @@ int fr_b200_finalize(fr_b200_model *m) {
     hp.rscale = m->fmt == FMT_INT8 ? m->d_rscale + reinterpret_cast<size_t>(hp.rscale) : nullptr;
     hp.kind = PH_MATVEC; hp.rot = 0;
     CU(cudaMemcpy(m->d_head_phase, &hp, sizeof(hp), cudaMemcpyHostToDevice));
+  }
+  // a few streams that go by rows find their buffers, as those of the persistent kernels do (3 int4 streams of the 1.5B shape: the first
+  // step took 1.5 ms, 0.3 of them for this; larger batches and prompts size theirs when they come)
+  if (m->rows_planned && !m->rows_needed && (m->d_plain || m->d_qcopy)) {
+    const int rc = rows_forward(m, true, 0, nullptr, m->cfg.max_batch, nullptr);
+    if (rc && rc != FR_B200_E_NOMEM) return rc;
   }
   m->finalized = true;
   return fr_b200_state_reset(m, -1);
@@ -1075,7 +1083,7 @@ constexpr int PROMPT_DEFER_ROWS = 128, PROMPT_DEFER_C = 2048, PROMPT_DEFER_KVR =
 //              (def::ModelForwardSeq, kernels/default/model_forward_seq.cpp:48-184); logits of the last row only.
 //   batch mode (batch_mode = true):  row b is the next token of stream b, b < R (the batched decode the reference
 //              lacks); logits of every row into d_out.
-// ids: host or device.  The residual stream stays fp32 between the layers; GEMM inputs are fp16.
+// ids: host or device (null: only the buffers for R rows).  The residual stream stays fp32 between the layers; GEMM inputs are fp16.
 int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids, int R, cudaStream_t st) {
   const int C = m->C, F = m->F, H = m->H, af = m->cfg.act_fp16, T = R;
   if (C > 8192) return fail(FR_B200_E_UNSUPPORTED, "the row kernels of the GEMM path hold at most n_embd = 8192");
@@ -1122,6 +1130,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     if (e != cudaSuccess) { m->d_seq = nullptr; cudaGetLastError(); return fail(FR_B200_E_NOMEM, std::string("cudaMalloc(activation rows): ") + cudaGetErrorString(e)); }
     m->seq_bytes = off;
   }
+  if (!ids) return FR_B200_OK;
   uint8_t *B = m->d_seq;
   int32_t *d_ids = (int32_t *)(B + o_ids);
   float *x = (float *)(B + o_x), *r_all = (float *)(B + o_r), *k_all = (float *)(B + o_k), *v_all = (float *)(B + o_v), *y_all = (float *)(B + o_y);
