@@ -64,7 +64,8 @@ struct fr_b200_model {
   float *d_vecs = nullptr;       size_t vecs_n = 0;
   uint8_t *d_emb = nullptr;      int emb_dtype = -1;   // rows kept in the dtype they arrive in
   uint8_t *d_state = nullptr;    size_t state_stride = 0, layer_stride = 0;
-  exch_t *d_x = nullptr, *d_xa = nullptr, *d_rwkv = nullptr, *d_kk = nullptr, *d_rr = nullptr;   // tagged exchange vectors
+  uint8_t *d_exch = nullptr;     size_t exch_bytes = 0;   // tagged exchange vectors, cleared as one:
+  exch_t *d_x = nullptr, *d_xa = nullptr, *d_rwkv = nullptr, *d_kk = nullptr, *d_rr = nullptr;
   exch_t *d_v5buf = nullptr;     // k5, v5, r5, g5, o5
   int exch_batch = 0;            // streams the last launch wrote into the exchange vectors (0: clear them first)
   unsigned seq = 0;              // phases launched so far (tags continue across launches)
@@ -444,12 +445,13 @@ int fr_b200_create(const fr_b200_config *cfg, fr_b200_model **out) {
       cudaGetLastError();   // the advice is an optimisation: a platform that refuses it still works
     }
   } else if (!rc) rc = alloc((void **)&m->d_state, m->state_stride * B);
-  if (!rc) rc = alloc((void **)&m->d_x, (size_t)B * m->C * sizeof(exch_t));
-  if (!rc) rc = alloc((void **)&m->d_xa, (size_t)B * m->C * sizeof(exch_t));
-  if (!rc) rc = alloc((void **)&m->d_rwkv, (size_t)B * m->C * sizeof(exch_t));
-  if (!rc) rc = alloc((void **)&m->d_kk, (size_t)B * m->F * sizeof(exch_t));
-  if (!rc) rc = alloc((void **)&m->d_rr, (size_t)B * m->C * sizeof(exch_t));
-  if (!rc) rc = alloc((void **)&m->d_v5buf, (size_t)5 * B * m->C * sizeof(exch_t));
+  {
+    const size_t bc = align256((size_t)B * m->C * sizeof(exch_t)), bf = align256((size_t)B * m->F * sizeof(exch_t));
+    m->exch_bytes = 4 * bc + bf + align256((size_t)5 * B * m->C * sizeof(exch_t));
+    if (!rc) rc = alloc((void **)&m->d_exch, m->exch_bytes);
+    auto at = [&](size_t off) { return reinterpret_cast<exch_t *>(m->d_exch + off); };
+    if (!rc) { m->d_x = at(0); m->d_xa = at(bc); m->d_rwkv = at(2 * bc); m->d_rr = at(3 * bc); m->d_kk = at(4 * bc); m->d_v5buf = at(4 * bc + bf); }
+  }
   if (!rc) rc = alloc((void **)&m->d_out, m->out_bytes());
   if (!rc) rc = alloc((void **)&m->d_amax, (size_t)B * 8);
   // fp16 W^T copies now for RWKV-5.x (seq kernels) and for models whose largest batch goes by rows; else on demand
@@ -484,8 +486,7 @@ void fr_b200_destroy(fr_b200_model *m) {
   if (!m) return;
   cudaSetDevice(m->device);
   free_scratch(m);
-  void *ptrs[] = {m->d_weights, m->d_rscale, m->d_vecs, m->d_emb, m->d_state, m->d_x, m->d_xa, m->d_rwkv, m->d_kk, m->d_rr,
-                  m->d_v5buf, m->d_out, m->d_layers, m->d_phases, m->d_amax, m->d_plain, m->d_pscale, m->d_qcopy, m->d_qscale, m->d_seq, m->d_head_phase, m->d_lnvec};
+  void *ptrs[] = {m->d_weights, m->d_rscale, m->d_vecs, m->d_emb, m->d_state, m->d_exch, m->d_out, m->d_layers, m->d_phases, m->d_amax, m->d_plain, m->d_pscale, m->d_qcopy, m->d_qscale, m->d_seq, m->d_head_phase, m->d_lnvec};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (m->h_out) cudaFreeHost(m->h_out);
@@ -778,16 +779,11 @@ static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned
   p.amax = amax;
   // Exchange words carry 8-bit tags: unambiguous only against the write just before them in the same slot.  Slots of
   // streams the previous launch did not write, or words a failed launch left half written, could alias: start clean.
-  if (m->exch_batch != batch) {
-    const size_t B = m->cfg.max_batch;
-    CU(cudaMemsetAsync(m->d_x, 0, B * m->C * sizeof(exch_t), st));
-    CU(cudaMemsetAsync(m->d_xa, 0, B * m->C * sizeof(exch_t), st));
-    CU(cudaMemsetAsync(m->d_rwkv, 0, B * m->C * sizeof(exch_t), st));
-    CU(cudaMemsetAsync(m->d_kk, 0, B * m->F * sizeof(exch_t), st));
-    CU(cudaMemsetAsync(m->d_rr, 0, B * m->C * sizeof(exch_t), st));
-    CU(cudaMemsetAsync(m->d_v5buf, 0, 5 * B * m->C * sizeof(exch_t), st));
-    m->exch_batch = batch;
-  }
+  // A captured launch keeps its tags at every replay, whatever ran before and whatever runs next: it clears the words on both
+  // sides (with one layer every word of the replay before would pass for this one's).
+  const bool replayed = capturing(st);
+  if (m->exch_batch != batch || replayed) CU(cudaMemsetAsync(m->d_exch, 0, m->exch_bytes, st));
+  m->exch_batch = replayed ? 0 : batch;   // (nothing has run yet: the next launch starts clean)
   p.seq_base = 255u + m->seq;
   {
     int rc = align_parity(m, batch, st);
@@ -815,6 +811,7 @@ static int decode_impl(fr_b200_model *m, const int32_t *ids_host, const unsigned
   } else {
     CU(launch_step(p, m->fmt, mode, m->grid, m->smem[mode], st));
   }
+  if (replayed) CU(cudaMemsetAsync(m->d_exch, 0, m->exch_bytes, st));
   m->launches++;
   // a phase count that is a multiple of 255 would give consecutive tokens identical tags: skip one tag per token then
   m->seq = (m->seq + (unsigned)m->phases.size() + (m->phases.size() % 255u == 0 ? 1u : 0u)) % 255u;

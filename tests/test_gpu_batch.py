@@ -2,6 +2,8 @@
 through the tensor-core GEMM path, every weight format and model version, against the CPU oracle run stream by
 stream.  fp16 models created for such batches keep W^T copies, quantised models a row-major copy of their packed
 codes (expanded inside the GEMM); their prompts use the same path."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -176,6 +178,51 @@ def test_a_captured_step_of_few_streams(pkg, synth, name, fmt, B):
     torch.cuda.synchronize()
     m.reset_states()
     _close(got.cpu().numpy(), m.decode(ids), f"{name} {fmt} captured")
+    m.close()
+
+
+def _capture(pkg, calls):
+    """The C calls of `calls(stream)`, which return their status, as one CUDA graph; nothing runs."""
+    import torch
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="thread_local")
+        rcs = calls(ctypes.c_void_p(side.cuda_stream))
+        graph.capture_end()
+    for rc in rcs:
+        pkg.check(rc, "captured call")
+    return graph
+
+
+@pytest.mark.parametrize("version,L,fmt,B", [("4", 1, "fp16", 1), ("4", 1, "int8", 2), ("4", 3, "fp16", 4), ("5.2", 1, "fp16", 5)])
+def test_replays_of_captured_steps(pkg, synth, version, L, fmt, B):
+    """Two captured steps of the persistent kernels, replayed three times with steps outside the graph in between: the bits of the
+    same steps one by one.  A replay writes its exchange words with the tags of the replay before; with one layer a word is
+    written once a token, so that nothing but a clear tells the two apart."""
+    import torch
+    shape = synth.Shape(version, L, 128, 512, 96, n_head=2 if version != "4" else 0)
+    strat, fdt = STR[fmt]
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), fdt)
+    m = pkg.Model(tensors, strat, shape=shape, max_batch=B)
+    ids = synth.token_ids(shape, 3 * B, seed=9).reshape(3, B).astype(np.int32)
+    want = [m.decode(ids[t]) for t in (0, 1, 0, 1, 2, 2, 0, 1, 2)]
+    state = [m.export_state(b) for b in range(B)]
+    m.reset_states()
+    got = torch.zeros(2, B, shape.vocab, device="cuda")
+    graph = _capture(pkg, lambda st: [pkg.lib().fr_b200_decode(m.handle, ids[t].ctypes.data_as(ctypes.c_void_p), B,
+                                                               ctypes.c_void_p(got[t].data_ptr()), None, st) for t in (0, 1)])
+    have = []
+    for what in ("graph", "graph", 2, 2, "graph", 2):
+        if what == "graph":
+            graph.replay()
+            torch.cuda.synchronize()
+            have.extend(got.cpu().numpy())
+        else:
+            have.append(m.decode(ids[what]))
+    assert np.array_equal(np.stack(have), np.stack(want))
+    assert all(np.array_equal(m.export_state(b), state[b]) for b in range(B))
     m.close()
 
 
