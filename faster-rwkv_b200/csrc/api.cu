@@ -896,14 +896,13 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
     // ids stay on the device, row t of the history feeds step t + 1: every sampled id goes to the row-id buffer of the next step
     // and to the history
     int32_t *hist32 = reinterpret_cast<int32_t *>(m->d_hist + need);
-    GreedyCtl ctl;
-    ctl.hist = hist32; ctl.step = 0;
-    CU(cudaMemcpyAsync(m->d_ctl, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
+    // (the cursor is set by a kernel: a copy from here would be made again, from a stack long gone, when a captured run is replayed)
+    CU(launch_greedy_start(m->d_ctl, hist32, st));
     int32_t *row_ids = reinterpret_cast<int32_t *>(m->d_seq);   // first piece of the activation blob
     CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, row_ids, m->d_ctl, st));
-    m->launches += 2;
+    m->launches += 3;
     int left = n_tokens - 1;
-    bool graphs = left >= 4;
+    bool graphs = left >= 4 && !capturing(st);
     if (const char *e = getenv("FR_B200_GRAPH")) graphs = graphs && atoi(e) != 0;
     if (graphs) {
       // two steps (the shift-state copies alternate) as one graph on an internal stream: capture is not allowed on the
@@ -1139,8 +1138,13 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   __half *ynlo_all = pairs ? (__half *)(B + o_ynlo) : nullptr, *kklo_all = pairs ? (__half *)(B + o_kklo) : nullptr;
   __half *glo_all = pairs ? (__half *)(B + o_glo) : nullptr;
   cudaStream_t st_main = st;
-  if (ids != d_ids) CU(cudaMemcpyAsync(d_ids, ids, (size_t)T * 4, cudaMemcpyDefault, st));
-  CU(launch_gather_emb(m->d_emb, m->emb_dtype == FR_B200_T_F32, d_ids, T, C, x, st));
+  if (ids != d_ids && capturing(st)) {
+    // (a copy from the caller's array would be made again at each replay)
+    CU(launch_gather_emb_host(m->d_emb, m->emb_dtype == FR_B200_T_F32, ids, T, C, x, st));
+  } else {
+    if (ids != d_ids) CU(cudaMemcpyAsync(d_ids, ids, (size_t)T * 4, cudaMemcpyDefault, st));
+    CU(launch_gather_emb(m->d_emb, m->emb_dtype == FR_B200_T_F32, d_ids, T, C, x, st));
+  }
   auto vp = [&](const std::string &n) -> const float * { return m->d_vecs + m->vecs[n].off; };
   const bool quant = m->fmt != FMT_FP16;
   GemmMapCache map_cache;

@@ -261,6 +261,7 @@ struct Wkv4Args {
   int split;
 };
 cudaError_t launch_gather_emb(const void *emb, int emb_f32, const int32_t *ids, int T, int C, float *x, cudaStream_t st);
+cudaError_t launch_gather_emb_host(const void *emb, int emb_f32, const int32_t *ids, int T, int C, float *x, cudaStream_t st);   // ids go with the launches
 cudaError_t launch_ln_mix_seq(const SeqLnArgs &a, cudaStream_t st);
 cudaError_t launch_wkv5_seq(const SeqWkvArgs &a, int H, cudaStream_t st);
 cudaError_t launch_wkv5_rows(const Wkv5RowsArgs &a, int H, cudaStream_t st);
@@ -277,6 +278,7 @@ struct GreedyCtl {           // device-side cursor of a greedy run through the G
   int32_t *hist;             // [n_tokens][rows] sampled ids
   int step;                  // next row of hist
 };
+cudaError_t launch_greedy_start(GreedyCtl *ctl, int32_t *hist, cudaStream_t st);
 cudaError_t launch_argmax_rows(const float *logits, int rows, int V, int ld, int32_t *out, GreedyCtl *ctl, cudaStream_t st);
 cudaError_t launch_ln_row(const float *x, const float *w, const float *b, int C, float *out, cudaStream_t st);
 cudaError_t launch_transpose_f16(const __half *src, int K, int N, __half *dst, cudaStream_t st);   // [K,N] -> [N,K]

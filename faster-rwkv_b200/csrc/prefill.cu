@@ -1187,14 +1187,23 @@ __device__ __forceinline__ float2 row_stats(const float *x, int C, float *red) {
 }
 
 // x[t, :] = embedding row of ids[t]
+__device__ __forceinline__ void gather_row(const void *emb, int emb_f32, int id, int C, float *x) {
+  const size_t row = (size_t)id * C;
+  for (int i = threadIdx.x; i < C; i += blockDim.x)
+    x[i] = emb_f32 ? reinterpret_cast<const float *>(emb)[row + i] : __half2float(reinterpret_cast<const __half *>(emb)[row + i]);
+}
 __global__ void gather_emb_kernel(const void *emb, int emb_f32, const int32_t *ids, int C, float *x) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.x;
-  const size_t row = (size_t)ids[t] * C;
-  for (int i = threadIdx.x; i < C; i += blockDim.x)
-    x[(size_t)t * C + i] = emb_f32 ? reinterpret_cast<const float *>(emb)[row + i]
-                                   : __half2float(reinterpret_cast<const __half *>(emb)[row + i]);
+  gather_row(emb, emb_f32, ids[blockIdx.x], C, x + (size_t)blockIdx.x * C);
+}
+// the same for ids that travel with the launch (captured steps: a graph holds them by value)
+constexpr int INLINE_IDS = 512;
+struct InlineIds { int32_t id[INLINE_IDS]; };
+__global__ void gather_emb_inline_kernel(const void *emb, int emb_f32, const __grid_constant__ InlineIds ids, int C, float *x) {
+  pdl_trigger();
+  pdl_wait();
+  gather_row(emb, emb_f32, ids.id[blockIdx.x], C, x + (size_t)blockIdx.x * C);
 }
 
 // LayerNorm + token shift + mix for every token row (LN of att_seq.cu:375, the shifted cat of :377-381 and the
@@ -1678,6 +1687,7 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(const float *logits, i
   }
 }
 __global__ void greedy_bump_kernel(GreedyCtl *ctl) { pdl_trigger(); pdl_wait(); ctl->step += 1; }
+__global__ void greedy_start_kernel(GreedyCtl *ctl, int32_t *hist) { pdl_trigger(); pdl_wait(); ctl->hist = hist; ctl->step = 0; }
 
 
 // RWKV-5 state scan over the tokens of one head (rwkv5_2_kernel_forward, att_seq.cu:258-322; per-head decay for 5.0):
@@ -2014,6 +2024,16 @@ cudaError_t launch_gather_emb(const void *emb, int emb_f32, const int32_t *ids, 
   launch_k(gather_emb_kernel, dim3(T), dim3(256), 0, st, emb, emb_f32, ids, C, x);
   return cudaGetLastError();
 }
+cudaError_t launch_gather_emb_host(const void *emb, int emb_f32, const int32_t *ids, int T, int C, float *x, cudaStream_t st) {
+  for (int t0 = 0; t0 < T; t0 += INLINE_IDS) {
+    const int n = std::min(T - t0, INLINE_IDS);
+    InlineIds in = {};
+    memcpy(in.id, ids + t0, (size_t)n * 4);
+    const cudaError_t e = launch_k(gather_emb_inline_kernel, dim3(n), dim3(256), 0, st, emb, emb_f32, in, C, x + (size_t)t0 * C);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
 namespace {
 template <LnKind KIND>
 void launch_ln_mix_t(const SeqLnArgs &a, bool few, cudaStream_t st) {
@@ -2094,6 +2114,9 @@ cudaError_t launch_wkv4_rows(const Wkv4Args &a, cudaStream_t st) {
   if ((long long)a.T * a.C <= 64 * 2048) launch_k(wkv4_rows_kernel<8>, dim3(grid), dim3(256), 0, st, a);
   else launch_k(wkv4_rows_kernel<4>, dim3(grid), dim3(256), 0, st, a);
   return cudaGetLastError();
+}
+cudaError_t launch_greedy_start(GreedyCtl *ctl, int32_t *hist, cudaStream_t st) {
+  return launch_k(greedy_start_kernel, dim3(1), dim3(1), 0, st, ctl, hist);
 }
 cudaError_t launch_argmax_rows(const float *logits, int rows, int V, int ld, int32_t *out, GreedyCtl *ctl, cudaStream_t st) {
   // as many CTAs per row as about four per SM allow

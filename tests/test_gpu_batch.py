@@ -226,6 +226,41 @@ def test_replays_of_captured_steps(pkg, synth, version, L, fmt, B):
     m.close()
 
 
+@pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 9), ("tiny52", "int8", 9), ("tiny4", "int4", 520)])
+def test_replays_of_captured_row_steps(pkg, synth, name, fmt, B):
+    """Captured steps and greedy runs of the GEMM path hold their ids: replays give the bits of the same calls one by one when the
+    caller's array has other ids in it by then."""
+    import torch
+    shape = synth.SHAPES[name]
+    strat, fdt = STR[fmt]
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), fdt)
+    m = pkg.Model(tensors, strat, shape=shape, max_batch=B)
+    lib, n_greedy = pkg.lib(), 6
+    ids = synth.token_ids(shape, 3 * B, seed=9).reshape(3, B).astype(np.int32)
+    want = [m.decode(ids[t]) for t in (0, 1, 0, 1)]
+    want_ids = [m.decode_greedy(ids[2], n_greedy), m.decode_greedy(ids[2], n_greedy)]
+    m.reset_states()
+    got = torch.zeros(2, B, shape.vocab, device="cuda")
+    picked = torch.zeros(n_greedy, B, dtype=torch.int32, device="cuda")
+    own = ids.copy()
+
+    def at(t):
+        return own[t].ctypes.data_as(ctypes.c_void_p)
+    steps = _capture(pkg, lambda st: [lib.fr_b200_decode(m.handle, at(t), B, ctypes.c_void_p(got[t].data_ptr()), None, st) for t in (0, 1)])
+    greedy = _capture(pkg, lambda st: [lib.fr_b200_decode_greedy(m.handle, at(2), B, n_greedy, ctypes.c_void_p(picked.data_ptr()), st)])
+    own[:] = 1
+
+    def replay(graph, out):
+        graph.replay()
+        torch.cuda.synchronize()
+        return out.cpu().numpy()
+    have = list(replay(steps, got))
+    have += list(replay(steps, got))
+    assert np.array_equal(np.stack(have), np.stack(want))
+    assert np.array_equal(replay(greedy, picked), want_ids[0]) and np.array_equal(replay(greedy, picked), want_ids[1])
+    m.close()
+
+
 def test_small_and_large_batches_share_state(pkg, orc, synth):
     """The persistent kernel (<= 8 streams) and the GEMM path (> 8) read and write the same state slots, and streams
     that are decoded together need not have seen the same number of tokens (continuous batching: a stream joins a
