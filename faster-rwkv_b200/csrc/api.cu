@@ -72,7 +72,7 @@ struct fr_b200_model {
   std::vector<unsigned> par;     // per stream slot: which copy of the token-shift states it reads next
   float *d_out = nullptr;        // [B][Vpad] logits, then [B] argmax ints, then status int
   uint8_t *h_out = nullptr;      // pinned mirror of d_out
-  unsigned long long *d_hist = nullptr; size_t hist_n = 0;   // packed arg-max words of decode_greedy, [tokens][batch]
+  uint8_t *d_hist = nullptr;     size_t hist_bytes = 0;   // decode_greedy: packed arg-max words [tokens][batch], then as many ids
   unsigned long long *d_amax = nullptr;   // packed arg-max words of a single decode, [max_batch]
   // GEMM path: row copies of the projection matrices, activation buffers for seq_T rows
   __half *d_plain = nullptr;     size_t plain_halfs = 0;   // fp16 models: W^T [out, in]
@@ -97,6 +97,9 @@ struct fr_b200_model {
   float *d_lnvec = nullptr;           // ln_out of the last prompt token
   cudaStream_t seq_streams[4] = {nullptr, nullptr, nullptr, nullptr};   // long prompts: one stream per piece of rows
   std::vector<cudaEvent_t> seq_events;                                  // [piece][layer] + one start event
+  // buffers that were outgrown after a call on a capturing stream: its graph goes on using them (see grow())
+  bool captured = false;
+  std::vector<void *> outgrown;
   // scratch for uploads
   void *d_scratch[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t scratch_bytes[4] = {0, 0, 0, 0};
@@ -137,6 +140,30 @@ int ensure_scratch(fr_b200_model *m, int idx, size_t bytes) {
   CU(cudaMalloc(&m->d_scratch[idx], bytes));
   m->scratch_bytes[idx] = bytes;
   return 0;
+}
+
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (st && cudaStreamIsCapturing(st, &s) != cudaSuccess) cudaGetLastError();
+  return s != cudaStreamCaptureStatusNone;
+}
+
+// Working buffers that grow with the calls.  A captured graph keeps the addresses it was captured with, so from the first call on a
+// capturing stream on what is outgrown stays until the model goes (it is the smaller one each time).  A captured call itself cannot
+// allocate: the same call has to have run once before.
+int grow(fr_b200_model *m, uint8_t **p, size_t *have, size_t need, const char *what, cudaStream_t st) {
+  const bool cap = st != m->gstream && capturing(st);   // (the graph of decode_greedy knows its buffers)
+  m->captured = m->captured || cap;
+  if (*have >= need) return FR_B200_OK;
+  if (cap) return fail(FR_B200_E_STATE, std::string(what) + ": no buffer of this size yet, and none can be made while the stream is captured; run the call once before");
+  CU(cudaStreamSynchronize(st));
+  if (*p && m->captured) m->outgrown.push_back(*p);
+  else if (*p) cudaFree(*p);
+  *p = nullptr; *have = 0;
+  const cudaError_t e = cudaMalloc((void **)p, need);
+  if (e != cudaSuccess) { *p = nullptr; cudaGetLastError(); return fail(FR_B200_E_NOMEM, std::string("cudaMalloc(") + what + "): " + cudaGetErrorString(e)); }
+  *have = need;
+  return FR_B200_OK;
 }
 
 void free_scratch(fr_b200_model *m) {
@@ -499,6 +526,7 @@ void fr_b200_destroy(fr_b200_model *m) {
   if (m->d_sample) cudaFree(m->d_sample);
   if (m->d_adj) cudaFree(m->d_adj);
   if (m->d_hist) cudaFree(m->d_hist);
+  for (void *p : m->outgrown) cudaFree(p);
   delete m;
 }
 
@@ -722,11 +750,6 @@ bool token_kernel_fits(const fr_b200_model *m, int batch) {
   return batch <= MAX_B && (wide_batch(m->fmt, m->v5, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) != 0;
 }
 bool rows_path_built(const fr_b200_model *m) { return m->d_plain || m->d_qcopy; }
-bool capturing(cudaStream_t st) {
-  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-  if (st && cudaStreamIsCapturing(st, &s) != cudaSuccess) cudaGetLastError();
-  return s != cudaStreamCaptureStatusNone;
-}
 // A batch that the persistent kernels can take, too, stays with them where the rows would have to allocate and must not (a stream
 // that is being captured) or could not (no room for the row copies).
 bool decode_by_rows(const fr_b200_model *m, int batch, cudaStream_t st) {
@@ -877,14 +900,10 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
   CU(cudaSetDevice(m->device));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const size_t need = (size_t)n_tokens * batch;
-  if (m->hist_n < need) {
-    CU(cudaStreamSynchronize(st));
-    if (m->d_hist) cudaFree(m->d_hist);
-    m->d_hist = nullptr; m->hist_n = 0;
-    CU(cudaMalloc((void **)&m->d_hist, need * 12));
-    m->hist_n = need;
-  }
   int rc;
+  if ((rc = grow(m, &m->d_hist, &m->hist_bytes, need * 12, "sampled ids", st))) return rc;
+  unsigned long long *words = reinterpret_cast<unsigned long long *>(m->d_hist);
+  int32_t *ids32 = reinterpret_cast<int32_t *>(words + need);   // ids behind the packed words
   bool rows = decode_by_rows(m, batch, st);
   if (rows) {
     // GEMM path, step 0 from the host ids
@@ -895,9 +914,8 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
   if (rows) {
     // ids stay on the device, row t of the history feeds step t + 1: every sampled id goes to the row-id buffer of the next step
     // and to the history
-    int32_t *hist32 = reinterpret_cast<int32_t *>(m->d_hist + need);
     // (the cursor is set by a kernel: a copy from here would be made again, from a stack long gone, when a captured run is replayed)
-    CU(launch_greedy_start(m->d_ctl, hist32, st));
+    CU(launch_greedy_start(m->d_ctl, ids32, st));
     int32_t *row_ids = reinterpret_cast<int32_t *>(m->d_seq);   // first piece of the activation blob
     CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, row_ids, m->d_ctl, st));
     m->launches += 3;
@@ -947,7 +965,7 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
       CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, row_ids, m->d_ctl, st));
       m->launches += 2;
     }
-    CU(cudaMemcpyAsync(out_ids, hist32, need * 4, cudaMemcpyDefault, st));
+    CU(cudaMemcpyAsync(out_ids, ids32, need * 4, cudaMemcpyDefault, st));
     if (is_host_ptr(out_ids)) {
       int status = 0;
       CU(cudaMemcpyAsync(&status, m->out_status(), 4, cudaMemcpyDeviceToHost, st));
@@ -957,14 +975,13 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
     return FR_B200_OK;
   }
   // one packed arg-max word per (token, stream), all cleared up front; token t+1 reads its ids from row t
-  CU(cudaMemsetAsync(m->d_hist, 0, need * 8, st));
+  CU(cudaMemsetAsync(words, 0, need * 8, st));
   for (int t = 0; t < n_tokens; ++t) {
-    rc = decode_impl(m, t == 0 ? first_ids : nullptr, t == 0 ? nullptr : m->d_hist + (size_t)(t - 1) * batch, batch, st,
-                     m->d_hist + (size_t)t * batch);
+    rc = decode_impl(m, t == 0 ? first_ids : nullptr, t == 0 ? nullptr : words + (size_t)(t - 1) * batch, batch, st,
+                     words + (size_t)t * batch);
     if (rc) return rc;
   }
-  int32_t *ids32 = reinterpret_cast<int32_t *>(m->d_hist + need);   // unpacked ids behind the packed words
-  CU(launch_unpack_ids(m->d_hist, (int)need, ids32, st));
+  CU(launch_unpack_ids(words, (int)need, ids32, st));
   m->launches++;
   if (is_host_ptr(out_ids)) {
     CU(cudaMemcpyAsync(out_ids, ids32, need * 4, cudaMemcpyDeviceToHost, st));
@@ -1011,13 +1028,7 @@ int fr_b200_sample(fr_b200_model *m, int batch, float temperature, int top_k, fl
   const float *u = uniform;
   if (!u_inline) {
     const size_t need = (size_t)batch * 4;
-    if (m->sample_bytes < need) {
-      CU(cudaStreamSynchronize(st));
-      if (m->d_sample) cudaFree(m->d_sample);
-      m->d_sample = nullptr; m->sample_bytes = 0;
-      CU(cudaMalloc((void **)&m->d_sample, need));
-      m->sample_bytes = need;
-    }
+    if (const int rc = grow(m, &m->d_sample, &m->sample_bytes, need, "draws", st)) return rc;
     CU(cudaMemcpyAsync(m->d_sample, uniform, need, cudaMemcpyDefault, st));
     u = reinterpret_cast<const float *>(m->d_sample);
   }
@@ -1118,14 +1129,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   if (!batch_mode && m->v5) max_chunks = std::max(1, std::min(Tp / 32, std::max(1, wkv5_scan_slots() / H)));
   const size_t scan_bytes = max_chunks > 1 ? (size_t)H * max_chunks * 4096 * 4 : 0;
   const size_t o_e = take(scan_bytes * n_pieces), o_sin = take(scan_bytes * n_pieces);
-  if (m->seq_bytes < off) {
-    CU(cudaStreamSynchronize(st));
-    if (m->d_seq) cudaFree(m->d_seq);
-    m->d_seq = nullptr; m->seq_bytes = 0;
-    const cudaError_t e = cudaMalloc((void **)&m->d_seq, off);
-    if (e != cudaSuccess) { m->d_seq = nullptr; cudaGetLastError(); return fail(FR_B200_E_NOMEM, std::string("cudaMalloc(activation rows): ") + cudaGetErrorString(e)); }
-    m->seq_bytes = off;
-  }
+  if (const int rc = grow(m, &m->d_seq, &m->seq_bytes, off, "activation rows", st)) return rc;
   if (!ids) return FR_B200_OK;
   uint8_t *B = m->d_seq;
   int32_t *d_ids = (int32_t *)(B + o_ids);

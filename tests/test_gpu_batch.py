@@ -228,8 +228,8 @@ def test_replays_of_captured_steps(pkg, synth, version, L, fmt, B):
 
 @pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 9), ("tiny52", "int8", 9), ("tiny4", "int4", 520)])
 def test_replays_of_captured_row_steps(pkg, synth, name, fmt, B):
-    """Captured steps and greedy runs of the GEMM path hold their ids: replays give the bits of the same calls one by one when the
-    caller's array has other ids in it by then."""
+    """Captured steps and greedy runs of the GEMM path hold their ids and their buffers: replays give the bits of the same calls one
+    by one when the caller's array has other ids in it by then, and after a prompt and a greedy run have asked for larger buffers."""
     import torch
     shape = synth.SHAPES[name]
     strat, fdt = STR[fmt]
@@ -255,6 +255,11 @@ def test_replays_of_captured_row_steps(pkg, synth, name, fmt, B):
         torch.cuda.synchronize()
         return out.cpu().numpy()
     have = list(replay(steps, got))
+    now = [m.export_state(b) for b in range(B)]
+    m.run([int(t) for t in ids[0]] * (4000 // B))           # more rows than any call before
+    m.decode_greedy(ids[0], 8)                               # and more ids
+    for b in range(B):
+        m.import_state(now[b], b)
     have += list(replay(steps, got))
     assert np.array_equal(np.stack(have), np.stack(want))
     assert np.array_equal(replay(greedy, picked), want_ids[0]) and np.array_equal(replay(greedy, picked), want_ids[1])
