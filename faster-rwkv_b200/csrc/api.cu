@@ -750,11 +750,13 @@ bool token_kernel_fits(const fr_b200_model *m, int batch) {
   return batch <= MAX_B && (wide_batch(m->fmt, m->v5, batch) ? m->wide_stages[decode_mode(batch)] : m->n_stages[step_mode(batch)]) != 0;
 }
 bool rows_path_built(const fr_b200_model *m) { return m->d_plain || m->d_qcopy; }
-// A batch that the persistent kernels can take, too, stays with them where the rows would have to allocate and must not (a stream
-// that is being captured) or could not (no room for the row copies).
-bool decode_by_rows(const fr_b200_model *m, int batch, cudaStream_t st) {
-  if (!token_kernel_fits(m, batch)) return true;
-  return rows_batch(m, batch) && rows_path_built(m) && !capturing(st);
+bool decode_by_rows(const fr_b200_model *m, int batch) {
+  return !token_kernel_fits(m, batch) || (rows_batch(m, batch) && rows_path_built(m));
+}
+// A batch that the persistent kernels can take, too, goes to them where the row path would have to allocate and could not (no room) or
+// must not (a captured stream, before the rows are there).  Nothing has been launched then.
+bool back_to_token_kernel(const fr_b200_model *m, int batch, int rc) {
+  return (rc == FR_B200_E_NOMEM || rc == FR_B200_E_STATE) && token_kernel_fits(m, batch);
 }
 // fp16 models that were created without the W^T copies build them from the streaming tiles (exact: the tiles hold
 // the same fp16 values) the first time the GEMM path is asked for
@@ -849,10 +851,10 @@ int fr_b200_decode(fr_b200_model *m, const int32_t *ids, int batch, float *logit
   CU(cudaSetDevice(m->device));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int rc;
-  bool rows = decode_by_rows(m, batch, st);
+  bool rows = decode_by_rows(m, batch);
   if (rows) {
     if ((rc = rows_decode_check(m, ids, batch, st)) == 0) rc = rows_forward(m, true, 0, ids, batch, st);
-    if (rc == FR_B200_E_NOMEM && token_kernel_fits(m, batch)) rows = false;   // nothing has been launched
+    if (back_to_token_kernel(m, batch, rc)) rows = false;
     else if (rc) return rc;
   }
   if (rows) {
@@ -904,11 +906,11 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
   if ((rc = grow(m, &m->d_hist, &m->hist_bytes, need * 12, "sampled ids", st))) return rc;
   unsigned long long *words = reinterpret_cast<unsigned long long *>(m->d_hist);
   int32_t *ids32 = reinterpret_cast<int32_t *>(words + need);   // ids behind the packed words
-  bool rows = decode_by_rows(m, batch, st);
+  bool rows = decode_by_rows(m, batch);
   if (rows) {
     // GEMM path, step 0 from the host ids
     if ((rc = rows_decode_check(m, first_ids, batch, st)) == 0) rc = rows_forward(m, true, 0, first_ids, batch, st);
-    if (rc == FR_B200_E_NOMEM && token_kernel_fits(m, batch)) rows = false;   // nothing has been launched
+    if (back_to_token_kernel(m, batch, rc)) rows = false;
     else if (rc) return rc;
   }
   if (rows) {

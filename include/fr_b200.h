@@ -110,9 +110,8 @@ int fr_b200_get_config(const fr_b200_model *m, fr_b200_config *cfg);
  * Synchronous with respect to the host when logits or argmax is a host pointer.
  *
  * On a capturing stream (also fr_b200_decode_greedy): results to device memory only.  The graph holds the ids by value and stays
- * valid as long as the model.  A batch that takes the GEMM path has to have run once before (FR_B200_E_STATE otherwise); batches that
- * both kernels can take are captured with the persistent one, whose buffers are there from the start, and differ from the
- * same step outside a capture in their last digits.  Every token reads one copy of the token-shift states and writes the other:
+ * valid as long as the model.  A batch that takes the GEMM path and is not captured with the buffers of an earlier call (or of the
+ * model: few streams) goes to the persistent kernel where that can take it, else FR_B200_E_STATE.  Every token reads one copy of the token-shift states and writes the other:
  * a graph that is replayed more than once captures an even number of tokens, with an even number between replays. */
 int fr_b200_decode(fr_b200_model *m, const int32_t *ids, int batch, float *logits, int32_t *argmax,
                    void *stream);

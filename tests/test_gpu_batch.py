@@ -153,8 +153,8 @@ def test_argmax_of_rows_with_ties(pkg, synth, vocab):
 
 @pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 8), ("tiny4", "int4", 5)])
 def test_a_captured_step_of_few_streams(pkg, synth, name, fmt, B):
-    """5 to 8 RWKV-4 streams on a stream that is being captured: the first such step (the row path, which would have to allocate its
-    rows, is not taken there) can be captured and replayed, and agrees with the step outside a capture."""
+    """5 to 8 RWKV-4 streams on a stream that is being captured: the first such step (by rows, whose buffers came with the model) can be
+    captured and replayed, and agrees with the step outside a capture."""
     import ctypes
     import torch
     shape = synth.SHAPES[name]
@@ -224,6 +224,35 @@ def test_replays_of_captured_steps(pkg, synth, version, L, fmt, B):
     assert np.array_equal(np.stack(have), np.stack(want))
     assert all(np.array_equal(m.export_state(b), state[b]) for b in range(B))
     m.close()
+
+
+def test_captured_batches_take_the_kernel_of_the_same_step_outside(pkg, synth):
+    """5 streams of RWKV-4 have the bits of the row path inside a capture, too; in a model made for more streams, whose rows are not
+    there before the first step, the capture falls back to the persistent kernel, and 9 streams are refused and break no capture."""
+    import torch
+    shape = synth.SHAPES["tiny4b"]
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), "fp16")
+    ids = synth.token_ids(shape, 9, seed=9).astype(np.int32)
+    p = ids.ctypes.data_as(ctypes.c_void_p)
+    got = torch.zeros(9, shape.vocab, device="cuda")
+    for max_batch in (5, 9):
+        m = pkg.Model(tensors, "cuda fp16", shape=shape, max_batch=max_batch)
+        refused = []
+
+        def calls(st):
+            if max_batch == 9:
+                refused.append(pkg.lib().fr_b200_decode(m.handle, p, 9, ctypes.c_void_p(got.data_ptr()), None, st))
+            return [pkg.lib().fr_b200_decode(m.handle, p, 5, ctypes.c_void_p(got.data_ptr()), None, st)]
+        graph = _capture(pkg, calls)
+        assert refused == ([-4] if max_batch == 9 else [])
+        graph.replay()
+        torch.cuda.synchronize()
+        have = got[:5].cpu().numpy()
+        m.reset_states()
+        want = m.decode(ids[:5])
+        assert np.array_equal(have, want) == (max_batch == 5)
+        _close(have, want, f"captured, max_batch {max_batch}")
+        m.close()
 
 
 @pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 9), ("tiny52", "int8", 9), ("tiny4", "int4", 520)])
