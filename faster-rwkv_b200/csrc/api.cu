@@ -94,6 +94,7 @@ struct fr_b200_model {
   cudaEvent_t gev = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int g_batch = 0; unsigned g_par = 0; const void *g_seq = nullptr;   // what the captured graph was built for
+  long long g_launches = 0;                                           // and how many kernels it holds
   float *d_lnvec = nullptr;           // ln_out of the last prompt token
   cudaStream_t seq_streams[4] = {nullptr, nullptr, nullptr, nullptr};   // long prompts: one stream per piece of rows
   std::vector<cudaEvent_t> seq_events;                                  // [piece][layer] + one start event
@@ -141,6 +142,14 @@ int ensure_scratch(fr_b200_model *m, int idx, size_t bytes) {
   m->scratch_bytes[idx] = bytes;
   return 0;
 }
+
+// adds the kernels that a call launches through prefill.cu to the model's count
+struct RowLaunches {
+  fr_b200_model *m;
+  long long before = row_launches;
+  explicit RowLaunches(fr_b200_model *model) : m(model) {}
+  ~RowLaunches() { m->launches += row_launches - before; }
+};
 
 bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
@@ -850,6 +859,7 @@ int fr_b200_decode(fr_b200_model *m, const int32_t *ids, int batch, float *logit
   if (batch < 1 || batch > m->cfg.max_batch) return fail(FR_B200_E_ARG, "batch must be 1..max_batch");
   CU(cudaSetDevice(m->device));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  RowLaunches count(m);
   int rc;
   bool rows = decode_by_rows(m, batch);
   if (rows) {
@@ -858,10 +868,7 @@ int fr_b200_decode(fr_b200_model *m, const int32_t *ids, int batch, float *logit
     else if (rc) return rc;
   }
   if (rows) {
-    if (argmax) {
-      CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, m->out_argmax(), nullptr, st));
-      m->launches++;
-    }
+    if (argmax) CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, m->out_argmax(), nullptr, st));
   } else {
     if (argmax) CU(cudaMemsetAsync(m->d_amax, 0, (size_t)batch * 8, st));
     rc = decode_impl(m, ids, nullptr, batch, st, argmax ? m->d_amax : nullptr);
@@ -902,6 +909,7 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
   CU(cudaSetDevice(m->device));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const size_t need = (size_t)n_tokens * batch;
+  RowLaunches count(m);
   int rc;
   if ((rc = grow(m, &m->d_hist, &m->hist_bytes, need * 12, "sampled ids", st))) return rc;
   unsigned long long *words = reinterpret_cast<unsigned long long *>(m->d_hist);
@@ -920,7 +928,6 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
     CU(launch_greedy_start(m->d_ctl, ids32, st));
     int32_t *row_ids = reinterpret_cast<int32_t *>(m->d_seq);   // first piece of the activation blob
     CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, row_ids, m->d_ctl, st));
-    m->launches += 3;
     int left = n_tokens - 1;
     bool graphs = left >= 4 && !capturing(st);
     if (const char *e = getenv("FR_B200_GRAPH")) graphs = graphs && atoi(e) != 0;
@@ -933,7 +940,7 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
       }
       if (!m->gexec || m->g_batch != batch || m->g_par != m->par[0] || m->g_seq != m->d_seq) {
         if (m->gexec) { cudaGraphExecDestroy(m->gexec); m->gexec = nullptr; }
-        const long long l0 = m->launches;
+        const long long l0 = row_launches;
         cudaGraph_t graph = nullptr;
         bool ok = cudaStreamBeginCapture(m->gstream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         for (int i = 0; i < 2 && ok; ++i) {
@@ -943,7 +950,8 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
         cudaError_t ce = cudaStreamEndCapture(m->gstream, &graph);
         ok = ok && ce == cudaSuccess && graph && cudaGraphInstantiate(&m->gexec, graph, 0) == cudaSuccess;
         if (graph) cudaGraphDestroy(graph);
-        m->launches = l0;
+        m->g_launches = row_launches - l0;
+        row_launches = l0;   // (nothing has run)
         if (!ok) {
           if (getenv("FR_B200_DEBUG")) fprintf(stderr, "fr_b200: graph capture failed (%s): running the steps one by one\n", cudaGetErrorString(ce));
           cudaGetLastError(); m->gexec = nullptr; graphs = false;
@@ -952,12 +960,11 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
       }
     }
     if (graphs && m->gexec) {
-      const long long per_step = (m->v5 ? 9 : 7) * (long long)m->L + 4;
       CU(cudaEventRecord(m->gev, st));
       CU(cudaStreamWaitEvent(m->gstream, m->gev, 0));
       for (; left >= 2; left -= 2) {
         CU(cudaGraphLaunch(m->gexec, m->gstream));
-        m->launches += 2 * per_step;
+        m->launches += m->g_launches;
       }
       CU(cudaEventRecord(m->gev, m->gstream));
       CU(cudaStreamWaitEvent(st, m->gev, 0));
@@ -965,7 +972,6 @@ int fr_b200_decode_greedy(fr_b200_model *m, const int32_t *first_ids, int batch,
     for (; left > 0; --left) {
       if ((rc = rows_forward(m, true, 0, row_ids, batch, st))) return rc;
       CU(launch_argmax_rows(m->d_out, batch, m->V, m->Vpad, row_ids, m->d_ctl, st));
-      m->launches += 2;
     }
     CU(cudaMemcpyAsync(out_ids, ids32, need * 4, cudaMemcpyDefault, st));
     if (is_host_ptr(out_ids)) {
@@ -1327,7 +1333,6 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
       CU(launch_gemm_group(&gv, 1, st, defer_x && (batch_mode || l + 1 < m->L) ? &sp : nullptr));
       if (sp > 1) pend_x = {gv.raw, gv.col_scale, rr, rr_lo, gv.scale, sp};
     }
-    m->launches += m->v5 ? 9 : 7;
     if (n_pieces > 1) CU(cudaEventRecord(m->seq_events[pc * m->L + l], st));
   }
   if (n_pieces > 1) {
@@ -1346,7 +1351,6 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
     gh.ldo = m->Vpad;
     // (no split-K scratch for the head: it has a thousand column tiles of its own)
     CU(launch_gemm_group(&gh, 1, st));
-    m->launches += 2;
     for (int bq = 0; bq < R; ++bq) m->par[bq] ^= 1u;
     return 0;
   }
@@ -1368,7 +1372,7 @@ int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids
   CU(decode_max_grid(m->fmt, 0, smem, m->device, &grid));
   if (!grid) return fail(FR_B200_E_UNSUPPORTED, "kernel does not fit");
   CU(launch_decode(p, 0, grid, smem, st));
-  m->launches += 3;
+  m->launches++;
   if (n_pieces & 1) m->par[slot] ^= 1u;   // every piece flipped the shift-state copies once
   return 0;
 }
@@ -1401,6 +1405,7 @@ int fr_b200_run_seq(fr_b200_model *m, int slot, const int32_t *ids, int n, float
     CU(cudaSetDevice(m->device));
     for (int i = 0; i < n; ++i)
       if (ids[i] < 0 || ids[i] >= m->V) return fail(FR_B200_E_ARG, "token id out of range");
+    RowLaunches count(m);
     rc = rows_forward(m, false, slot, ids, n, st);
     if (rc && !(rc == FR_B200_E_NOMEM && may_loop)) return rc;
     by_rows = rc == 0;

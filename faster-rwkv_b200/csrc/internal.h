@@ -274,6 +274,7 @@ constexpr int SAMPLE_INLINE_U = 512;   // draws of up to this many rows travel a
 cudaError_t launch_sample_rows(const float *logits, int rows, int V, int ld, float temperature, int top_k, float top_p,
                                const float *u, bool u_on_host, int32_t *out, cudaStream_t st);
 cudaError_t launch_logits_add(float *logits, int ld, const int32_t *stream, const int32_t *token, const float *delta, int n, cudaStream_t st);
+extern thread_local long long row_launches;   // kernels of prefill.cu that this thread has launched
 struct GreedyCtl {           // device-side cursor of a greedy run through the GEMM path
   int32_t *hist;             // [n_tokens][rows] sampled ids
   int step;                  // next row of hist

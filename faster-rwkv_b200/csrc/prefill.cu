@@ -33,6 +33,8 @@ int device_sm_count() {
   return cached[dev];
 }
 
+thread_local long long row_launches = 0;
+
 namespace {
 
 // Every kernel of the seq / batch chain goes through here.  With FR_B200_PDL != 0 (the default) the launch carries
@@ -62,7 +64,9 @@ cudaError_t launch_cluster_k(void (*kern)(KArgs...), int cluster, dim3 grid, dim
   }
   cfg.attrs = at;
   cfg.numAttrs = n;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+  if (e == cudaSuccess) ++row_launches;
+  return e;
 }
 template <typename... KArgs, typename... Args>
 cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {

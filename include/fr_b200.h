@@ -273,7 +273,7 @@ int fr_b200_gemm_f16(const float *A, const float *W, int M, int N, int K, int ep
 typedef struct fr_b200_info {
   int n_ctas, n_threads, smem_bytes, n_stages, stage_bytes, n_phases;
   long long weight_stream_bytes;   /* bytes of packed weights one token streams (algorithmic bytes) */
-  long long launches;              /* kernels launched by this model so far */
+  long long launches;              /* kernels that this model's forward and sampling calls have launched so far */
 } fr_b200_info;
 int fr_b200_get_info(const fr_b200_model *m, fr_b200_info *info);
 

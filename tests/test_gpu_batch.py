@@ -181,11 +181,11 @@ def test_a_captured_step_of_few_streams(pkg, synth, name, fmt, B):
     m.close()
 
 
-def _capture(pkg, calls):
+def _capture(pkg, calls, keep=False):
     """The C calls of `calls(stream)`, which return their status, as one CUDA graph; nothing runs."""
     import torch
     side = torch.cuda.Stream()
-    graph = torch.cuda.CUDAGraph()
+    graph = torch.cuda.CUDAGraph(keep_graph=keep)
     torch.cuda.synchronize()
     with torch.cuda.stream(side):
         graph.capture_begin(capture_error_mode="thread_local")
@@ -223,6 +223,43 @@ def test_replays_of_captured_steps(pkg, synth, version, L, fmt, B):
             have.append(m.decode(ids[what]))
     assert np.array_equal(np.stack(have), np.stack(want))
     assert all(np.array_equal(m.export_state(b), state[b]) for b in range(B))
+    m.close()
+
+
+@pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 12), ("tiny4", "int4", 1), ("tiny52", "int8", 9), ("mid4", "int8", 200)])
+def test_launch_counts(pkg, synth, name, fmt, B):
+    """info()["launches"] counts the kernels of a call: the kernel nodes of the same call as a CUDA graph, for a step and for a greedy
+    run (whose steps the model replays from a graph of its own outside a capture)."""
+    import torch
+    cu = ctypes.CDLL("libcuda.so.1")
+    shape = synth.SHAPES[name]
+    strat, fdt = STR[fmt]
+    m = pkg.Model(synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), fdt), strat, shape=shape, max_batch=B)
+    ids = synth.token_ids(shape, B, seed=9).astype(np.int32)
+    p = ids.ctypes.data_as(ctypes.c_void_p)
+    out = torch.zeros(8, B, dtype=torch.int32, device="cuda")
+
+    def kernels(calls):
+        graph = _capture(pkg, calls, keep=True)
+        h, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t()
+        assert cu.cuGraphGetNodes(h, None, ctypes.byref(n)) == 0
+        nodes = (ctypes.c_void_p * n.value)()
+        assert cu.cuGraphGetNodes(h, nodes, ctypes.byref(n)) == 0
+        kinds = []
+        for node in nodes:
+            kind = ctypes.c_int(-1)
+            assert cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+            kinds.append(kind.value)
+        return kinds.count(0)               # CU_GRAPH_NODE_TYPE_KERNEL
+
+    def counted(call):
+        l0 = m.info()["launches"]
+        call()
+        return m.info()["launches"] - l0
+    step = counted(lambda: m.decode(ids, want_logits=False, want_argmax=True))
+    run = counted(lambda: m.decode_greedy(ids, 8))
+    assert step == kernels(lambda st: [pkg.lib().fr_b200_decode(m.handle, p, B, None, ctypes.c_void_p(out.data_ptr()), st)])
+    assert run == kernels(lambda st: [pkg.lib().fr_b200_decode_greedy(m.handle, p, B, 8, ctypes.c_void_p(out.data_ptr()), st)])
     m.close()
 
 
