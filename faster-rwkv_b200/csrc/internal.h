@@ -177,10 +177,10 @@ struct GemmArgs {
   const __half *A;     // [M, K] row-major
   const __half *A2;    // optional [M, K]: low halves of the activations (A + A2 is the fp32 value to ~22 bits)
   const __half *Bt;    // [N, K] row-major (the weight matrix transposed: one row per output channel)
-  const __half *col_scale;   // optional [N]: acc *= col_scale[n] before the epilogue (int8: Bt holds the integer codes)
+  const __half *col_scale;   // int8 weights: [N] row scales, acc *= col_scale[n] before the epilogue
   // quantised weights in packed form instead of Bt (the GEMM expands them into tensor memory):
   const uint8_t *Wq;         // wfmt FMT_INT8: codes [N, K] int8;  FMT_INT4: [N, K/2], nibble = q + 8, even k low
-  const __half *wq_scale;    // FMT_INT4: group scales [N, K/32] (int8 row scales go in col_scale)
+  const __half *wq_scale;    // FMT_INT4: group scales [N, K/32] (int8 row scales: col_scale)
   int wfmt;
   int M, N, K;         // K a multiple of 64
   int epi;

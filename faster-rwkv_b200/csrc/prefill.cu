@@ -78,8 +78,9 @@ cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
 // accumulate.  A2 (optional) holds what rounding the activations to fp16 lost.
 // All of them put the weights along the MMA rows, so that an accumulator holds out^T (TMEM lane = output channel, column = row
 // of X) and the epilogue's lanes run along the channels; K is walked in 64-wide slices through a TMA ring.
-//   warp 0 (one lane): TMA producer          warp 1 (one lane): MMA issue; the warp owns the TMEM allocation
+//   warp 0: TMA producer          warp 1: MMA issue; it owns the TMEM allocation
 //   warps 2..5: epilogue, one TMEM lane quadrant (32 channels) each
+// Warps 0 and 1 run their loops whole and elect a lane for each copy or MMA: in a branch of one lane an MMA took 100 clocks to issue.
 constexpr int GBM = 128, GBK = 64;
 constexpr int G_THREADS = 192;
 constexpr uint32_t G_A_BYTES = GBM * GBK * 2;
@@ -497,7 +498,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
 // ------------------------------------------------------------------------------------------------
 // Few rows (batched decode: one row per stream, or a short prompt): the same product with the operands' roles
 // swapped, out^T[N, M] = W^T[N, K] . X[M, K]^T.  The 128 MMA rows are 128 output channels of the weight matrix, the
-// MMA columns are the BN rows of X (32 .. 256), so a ring slot is 16 KB of weights plus a small X tile instead of a
+// MMA columns are the up to BN = 32, 64 or 128 rows of X, so a ring slot is 16 KB of weights plus a small X tile instead of a
 // 128-row X tile that is mostly zero fill plus 8 KB of weights: several times the weight bytes in flight per SM,
 // which is what a step that streams every weight once is bound by.  The low halves of X (A2) sit in the same slot.
 // The accumulator holds out^T: TMEM lane = output channel, column = row of X; the epilogue warps write with the
@@ -529,7 +530,7 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
   int pi = 0;
   while (pi + 1 < grp.n && (int)blockIdx.x >= grp.tile_start[pi + 1]) ++pi;
   const GemmArgs &g = grp.p[pi];
-  const int tile_n = blockIdx.x - grp.tile_start[pi], m0 = blockIdx.y * BN;
+  const int tile_n = blockIdx.x - grp.tile_start[pi];
   const int num_k1 = g.K / GBK;
   const int kz0 = (int)((long long)blockIdx.z * num_k1 / grp.split), nkz = (int)((long long)(blockIdx.z + 1) * num_k1 / grp.split) - kz0;
   const bool x_lo = g.A2 != nullptr;
@@ -582,8 +583,8 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
         } else {
           mbar_expect_tx(&full[s], x_bytes);
         }
-        tma_load_2d(dst + X_OFF, &maps.a[pi], kx, m0, &full[s]);
-        if (x_lo) tma_load_2d(dst + XLO_OFF, &maps.a2[pi], kx, m0, &full[s]);
+        tma_load_2d(dst + X_OFF, &maps.a[pi], kx, 0, &full[s]);
+        if (x_lo) tma_load_2d(dst + XLO_OFF, &maps.a2[pi], kx, 0, &full[s]);
       }
     }
   } else if (warp == 1) {
@@ -605,16 +606,15 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
     if (elect_one()) umma_commit(acc_full);
   } else {
     const int quad = warp & 3;
-    const int ch = tile_n * GBM + quad * 32 + lane;
+    const int ch_w = tile_n * GBM + quad * 32;
     pdl_wait();
     const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
-      const float sc = (!SLABS && g.col_scale && ch < g.N) ? __half2float(g.col_scale[ch]) : 1.f;
       const uint32_t buf = tiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
       uint32_t flip = 0;
       for (int c0 = 0; c0 < BN; c0 += 32, flip ^= EPI_BUF) {
-        if (m0 + c0 >= g.M) break;   // warp-uniform
+        if (c0 >= g.M) break;   // warp-uniform
         uint32_t acc[32];
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, acc);
         if (x_lo) {
@@ -623,12 +623,8 @@ gemm_wt_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Ge
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(part[i]));
         }
-        if (!SLABS && g.col_scale) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * sc);
-        }
-        if (SLABS && BN == 32) slab_rows(g, blockIdx.z, ch, m0 + c0, acc);
-        else tile_out<SLABS>(g, &maps.o[pi], &maps.o_lo[pi], blockIdx.z, tile_n * GBM + quad * 32, m0 + c0, acc, buf + flip);
+        if (SLABS && BN == 32) slab_rows(g, blockIdx.z, ch_w + lane, c0, acc);
+        else tile_out<SLABS>(g, &maps.o[pi], &maps.o_lo[pi], blockIdx.z, ch_w, c0, acc, buf + flip);
       }
       tile_out_end();
     }
@@ -2170,7 +2166,7 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   bool raw_ok = true;
   for (int i = 0; i < n; ++i) {
     const GemmArgs &g = probs[i];
-    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M) return cudaErrorInvalidValue;
+    if (g.K % GBK != 0 || g.M < 1 || g.N < 1 || g.M != M || M > 128 || g.col_scale) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.Bt) & 15) || (reinterpret_cast<uintptr_t>(g.A2) & 15))
       return cudaErrorInvalidValue;
     grp.p[i] = g;
@@ -2182,14 +2178,13 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   }
   if (!make_in_maps(maps, grp, bn, bn)) return cudaErrorNotSupported;
   grp.tile_start[n] = tiles;
-  const int m_tiles = (M + bn - 1) / bn;
   // one CTA per SM, none waiting for a second wave: split K until the tiles about cover the SMs
   // (up to 64 rows the slabs are small next to the weights and two CTAs fit an SM: twice the slots, so that every SM
   // streams even when the group has few tiles)
   grp.split = 1;
   const int sms = device_sm_count();
   const int slots = bn <= 64 ? 2 * sms : sms;
-  if (raw_ok) grp.split = split_of(tiles * m_tiles, slots, min_k1);
+  if (raw_ok) grp.split = split_of(tiles, slots, min_k1);
   grp.stage_bytes = G_A_BYTES + (grp.dual ? 2u : 1u) * (uint32_t)bn * GBK * 2;
   // two CTAs per SM with rings of >= 3 slots where they fit (shorter tail when there are more tiles than SMs),
   // else one CTA with as deep a ring as fits
@@ -2198,7 +2193,7 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   grp.stages = std::max(2, std::min(stages, WT_MAX_STAGES));
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
-  dim3 grid(tiles, m_tiles, grp.split);
+  dim3 grid(tiles, 1, grp.split);
   auto kern = grp.split > 1 ? (bn == 32 ? gemm_wt_kernel<32, true> : bn == 64 ? gemm_wt_kernel<64, true> : gemm_wt_kernel<128, true>)
                             : (bn == 32 ? gemm_wt_kernel<32, false> : bn == 64 ? gemm_wt_kernel<64, false> : gemm_wt_kernel<128, false>);
   cudaError_t e = launch_k(kern, grid, dim3(G_THREADS), smem, st, maps, grp);
@@ -2381,7 +2376,7 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
 }
 }  // namespace
 
-// defer_split (optional): the caller's next kernel sums the split-K slabs itself (ln_mix_seq_kernel, wkv4_rows_kernel);
+// defer_split (optional): the caller's next kernel sums the split-K slabs itself (ln_mix_seq_kernel, wkv4_rows_kernel, wkv4_seq_kernel, wkv5_rows_kernel);
 // it receives the split that was chosen, 1 meaning that the outputs are already complete.
 cudaError_t launch_gemm_group(const GemmArgs *probs, int n, cudaStream_t st, int *defer_split) {
   if (n < 1 || n > GEMM_GROUP_MAX) return cudaErrorInvalidValue;
