@@ -74,7 +74,7 @@ struct fr_b200_model {
   uint8_t *h_out = nullptr;      // pinned mirror of d_out
   uint8_t *d_hist = nullptr;     size_t hist_bytes = 0;   // decode_greedy: packed arg-max words [tokens][batch], then as many ids
   unsigned long long *d_amax = nullptr;   // packed arg-max words of a single decode, [max_batch]
-  // GEMM path: row copies of the projection matrices, activation buffers for seq_T rows
+  // GEMM path: row copies of the projection matrices, activation rows
   __half *d_plain = nullptr;     size_t plain_halfs = 0;   // fp16 models: W^T [out, in]
   __half *d_pscale = nullptr;    size_t pscale_halfs = 0;  // int8: per output row scales, per matrix
   // int8 / int4: every projection a second time in its packed interchange form, row-major (one row per output
@@ -84,7 +84,8 @@ struct fr_b200_model {
   bool row_copies = true;        // keep the copies the GEMM path needs (FR_B200_ROW_COPIES=0: decode-only model)
   bool rows_planned = false;     // some batch up to max_batch is decoded by the GEMM path,
   bool rows_needed = false;      // and no other kernel could
-  uint8_t *d_seq = nullptr;      size_t seq_bytes = 0; int seq_T = 0;
+  uint8_t *d_seq = nullptr;      size_t seq_bytes = 0;
+  int looped_tokens = 0;         // of prompts that went token by token for want of row copies (prompt_build_tokens())
   PhaseDev *d_head_phase = nullptr;   // the head as a stand-alone matvec phase
   // greedy runs of many streams: two decode steps captured as a CUDA graph and replayed (the step is ~170 launches)
   GreedyCtl *d_ctl = nullptr;
@@ -1085,7 +1086,18 @@ int fr_b200_vocab_padded(const fr_b200_model *m) { return m ? m->Vpad : FR_B200_
 
 namespace {
 
-constexpr int PROMPT_BUILD_ROWS = 8, PROMPT_PAIR_ROWS = 32;   // see fr_b200_run_seq, rows_forward
+constexpr int PROMPT_BUILD_ROWS = 8, PROMPT_PAIR_ROWS = 32;   // see prompt_build_tokens, rows_forward
+
+// fp16 RWKV-4 models build their row copies (as many bytes as the weights) when their prompts have gone token by token for about as long as
+// the prompt that builds them takes: a first prompt is never slower than by the loop, and a program that sends one short
+// prompt keeps the memory.  Until then a prompt of 3 tokens and more is slower than it could be; those of up to 7 never build, those of 32 and
+// more always do.  us, weights of W bytes: a token 130 + W / 5.76e6 (0.1B shape 178, 1.5B 632, 14B 5,050), the building prompt in a process whose
+// first it is 5,000 (most of it kernels that are loaded) + W / 1.82e6 (4,800 to 6,200, 6,400 to 6,800, 19,500; the same prompt afterwards 440, 1,250,
+// 6,600).  That makes 28, 10 and 4 tokens.
+int prompt_build_tokens(const fr_b200_model *m) {
+  const double W = (double)m->weights_bytes;
+  return std::max(PROMPT_BUILD_ROWS, std::min((int)((5000. + W / 1.82e6) / (130. + W / 5.76e6)), PROMPT_PAIR_ROWS));
+}
 
 // Prompts of up to this many rows and channels have no finishing pass: 29 int4 tokens of the 1.5B shape take 1.61 ms
 // instead of 1.67, 60 fp16 ones 1.39 instead of 1.49, 100 1.61 instead of 1.64; 200 int8 ones would take 2.56 instead of 2.51,
@@ -1386,20 +1398,19 @@ int fr_b200_run_seq(fr_b200_model *m, int slot, const int32_t *ids, int n, float
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int seq_min = 2;   // shorter prompts take the token loop
   if (const char *e = getenv("FR_B200_SEQ_MIN")) seq_min = atoi(e);
-  // fp16 RWKV-4 models build their row copies (as many bytes as the weights) when the first prompt of PROMPT_BUILD_ROWS tokens or
-  // more arrives; until then shorter ones go token by token, which is the slower way from 3 tokens on.  The line lies where the
-  // first prompt, which pays for the copies, is no slower than by the token loop at the 1.5B shape.  In ms there: a token 0.66, a prompt of
-  // 2 to 12 tokens 1.25 to 1.28 by rows, the first one 5.3 (5.3 for 8 tokens by the loop); 29 tokens 1.34 against 18.2.  0.1B shape: a token 0.21,
-  // 2 to 12 tokens 0.42 to 0.43, the first one 5; 14B shape: 5.07, 6.7, 22.
   bool by_rows = rows_path_built(m) && n >= seq_min;
   // (Short prompts keep the loop on a stream that is being captured, and where there is no room for the copies or the rows.)
   const bool may_loop = m->fmt == FMT_FP16 && !m->v5 && n < PROMPT_PAIR_ROWS && slot == 0;
   int rc = 0;
   if (!by_rows && m->fmt == FMT_FP16 && m->row_copies && m->plain_halfs && n >= std::max(seq_min, PROMPT_BUILD_ROWS) && !(may_loop && capturing(st))) {
-    CU(cudaSetDevice(m->device));
-    rc = ensure_row_copies(m);
-    if (rc && !(rc == FR_B200_E_NOMEM && may_loop)) return rc;
-    by_rows = rc == 0;
+    if (may_loop && m->looped_tokens + n < prompt_build_tokens(m)) {
+      m->looped_tokens += n;
+    } else {
+      CU(cudaSetDevice(m->device));
+      rc = ensure_row_copies(m);
+      if (rc && !(rc == FR_B200_E_NOMEM && may_loop)) return rc;
+      by_rows = rc == 0;
+    }
   }
   if (by_rows) {
     CU(cudaSetDevice(m->device));

@@ -199,8 +199,8 @@ def test_long_prompts_in_pipelined_pieces(pkg, orc, synth, monkeypatch, name, st
 
 @pytest.mark.parametrize("name,T", [("tiny4b", 7), ("tiny4b", 8), ("mid4", 31), ("mid4", 32)])
 def test_short_fp16_prompts_of_rwkv4(pkg, orc, synth, name, T):
-    """fp16 RWKV-4 prompts: token by token up to 7 tokens, by rows with every operand as a pair up to 31 (the first such prompt
-    builds the row copies out of the streaming tiles, ragged in N for the 211-word head), single halves from 32 on.  With
+    """fp16 RWKV-4 prompts: token by token up to 7 tokens and until 32 tokens have come that way, then by rows with every operand as a
+    pair up to 31 (the row copies are built out of the streaming tiles, ragged in N for the 211-word head), single halves from 32 on.  With
     pairs an operand is off by 2^-22 of itself, so what is left over 7 layers is the fp16 shift state both sides round."""
     shape, tensors, ref = _models(pkg, orc, synth, name)
     ids = [int(t) for t in synth.token_ids(shape, 2 * T, seed=2)]
@@ -211,6 +211,25 @@ def test_short_fp16_prompts_of_rwkv4(pkg, orc, synth, name, T):
         if T < 32:
             assert np.linalg.norm(got - want) / np.linalg.norm(want) < 3e-4
     _close(m.run(7), ref.run(7), "token after the prompts")
+    m.close()
+
+
+@pytest.mark.parametrize("T,by_rows", [(7, []), (8, [3, 4]), (15, [2, 3]), (16, [1, 2]), (31, [1, 2]), (32, [0, 1])])
+def test_row_copies_come_when_the_loop_has_cost_as_much(pkg, orc, synth, T, by_rows):
+    """Prompts of an fp16 RWKV-4 model this small: a first one of 8 to 31 tokens is no slower than by the token loop, because it is the
+    token loop; the copies are built by the prompt that makes it 32 tokens.  Logits are within the bound of pairs either way."""
+    shape, tensors, ref = _models(pkg, orc, synth, "tiny4b")
+    m = pkg.Model(tensors, "cuda fp16", shape=shape)
+    m.run([3, 4, 5]), ref.run_seq([3, 4, 5])                 # neither counts nor builds
+    rows = []
+    for i in range(5):
+        ids = [int(t) for t in synth.token_ids(shape, T, seed=i)]
+        before = m.info()["launches"]
+        got, want = m.run(ids), ref.run_seq(ids)
+        if m.info()["launches"] - before != T:               # the loop: one launch per token
+            rows.append(i)
+        assert np.linalg.norm(got - want) / np.linalg.norm(want) < (3e-4 if T < 32 else REL_TOL)
+    assert rows[:2] == by_rows
     m.close()
 
 
