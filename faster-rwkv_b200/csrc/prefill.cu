@@ -344,6 +344,97 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, u
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Arrive on a barrier of either CTA of the cluster (address from mapa_u32).  Relaxed: it hands over no memory, but columns of TMEM, whose
+// writes are complete (tcgen05.wait::st) and ordered by the tcgen05 fences on both sides.  With .release it took 500 to 900 clocks, a slice of
+// int8 0.70 us instead of 0.50.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// ---- TMEM of a pair of CTAs ----
+// tcgen05.alloc / dealloc with cta_group::2 are one operation of a warp of each CTA, and ask that the other CTA has been launched and has not
+// left: they stand between cluster barriers.  An SM lets one CTA at a time allocate, from its allocation until it gives the permit back, so two
+// pairs that start on the same two SMs at once could each hold the permit of one SM and wait for that of the other for good (a chain of
+// products of 300 and 500 rows with a busy row kernel between them stood still, once in some million launches).  Pairs therefore take turns: the
+// even CTA takes the lock of its SM pair, tells the odd one, and gives it back when both have their columns.  The first weights are under way meanwhile.
+// Every wait is bounded: the lock's for half of what the odd CTA waits, so that one never allocates without the other.  The kernels
+// behind may start (pdl_trigger) only then: one that took the columns first would wait for this kernel with them.
+struct PairTmem {
+  uint64_t go, there;        // the odd CTA may allocate; it has
+  uint32_t sm, slot;         // this CTA's SM; address of its columns
+  int held, ready;           // they are allocated; in both CTAs
+};
+constexpr int PAIR_LOCKS = 1024;
+__device__ int pair_lock[PAIR_LOCKS];
+
+__device__ __forceinline__ void pair_tmem_init(PairTmem *t) {   // one thread, ahead of the fence and the cluster barrier
+  mbar_init(&t->go, 1);
+  mbar_init(&t->there, 1);
+  uint32_t sm;
+  asm volatile("mov.u32 %0, %smid;" : "=r"(sm));
+  t->sm = sm;
+}
+__device__ __forceinline__ void pair_tmem_get(PairTmem *t, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&t->slot)), "r"(cols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+// one warp of each CTA, after the cluster barrier
+__device__ __forceinline__ void pair_tmem_alloc(PairTmem *t, uint32_t rank, uint32_t cols, volatile int *abort_flag, int *status) {
+  const int lane = threadIdx.x & 31;
+  bool ok = true, ready = true;
+  if (rank == 0) {
+    int *lock = nullptr;
+    if (lane == 0) {
+      uint32_t other;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other) : "r"(mapa_u32(smem_u32(&t->sm), 1)) : "memory");
+      lock = &pair_lock[min(t->sm, other) % PAIR_LOCKS];
+      const unsigned long long t0 = globaltimer_ns();
+      while (atomicCAS(lock, 0, 1) != 0) {
+        if (globaltimer_ns() - t0 > WAIT_LIMIT_NS / 2) {
+          *abort_flag = 1;
+          atomicCAS(status, 0, ST_GEMM_TIMEOUT);
+          ok = false;
+          break;
+        }
+      }
+      if (ok) mbar_arrive_cluster(mapa_u32(smem_u32(&t->go), 1));
+    }
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    if (ok) {
+      pair_tmem_get(t, cols);
+      ready = __all_sync(0xffffffffu, mbar_wait(&t->there, 0, abort_flag, status, ST_GEMM_TIMEOUT));
+      if (lane == 0) atomicExch(lock, 0);
+    }
+  } else {
+    ok = __all_sync(0xffffffffu, mbar_wait(&t->go, 0, abort_flag, status, ST_GEMM_TIMEOUT));
+    if (ok) {
+      pair_tmem_get(t, cols);
+      if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&t->there), 0));
+    }
+  }
+  if (lane == 0) { t->held = ok; t->ready = ok && ready; }
+  tc_fence_before();
+  __syncwarp();
+}
+// all threads of the CTA, each role's warps at a place of their own
+__device__ __forceinline__ bool pair_tmem_ready(const PairTmem *t) {
+  asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x) : "memory");
+  tc_fence_after();
+  pdl_trigger();
+  return t->ready != 0;
+}
+// all threads of both CTAs; neither leaves while the other's MMAs, commits or deallocation may still reach into it
+__device__ __forceinline__ void pair_tmem_end(const PairTmem *t, int warp, uint32_t cols) {
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  if (warp == 1 && t->held) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(t->slot), "r"(cols) : "memory");
+  }
+  __syncwarp();
+  cluster_sync();
+}
 // arrives on the barrier at this offset in both CTAs of the pair
 __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -379,10 +470,10 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   uint64_t *full = reinterpret_cast<uint64_t *>(gsm);
   uint64_t *empty = full + PAIR_MAX_STAGES;
   uint64_t *acc_full = empty + PAIR_MAX_STAGES;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  PairTmem *tmem = reinterpret_cast<PairTmem *>(acc_full + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem + 1);
   const uint32_t tiles = smem_u32(gsm + 1024);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
   const uint32_t rank = cluster_rank();
   // pairs walk the row tiles of one channel tile before the next channel tile
   const int pair = blockIdx.x >> 1, ct = pair / grp.m_tiles, m0 = (pair - ct * grp.m_tiles) * BN;
@@ -403,25 +494,19 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
+    pair_tmem_init(tmem);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(PAIR_TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
   __syncthreads();
-  cluster_sync();      // the barriers of both CTAs exist before either one's copies arrive on them
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
+  cluster_sync();      // both CTAs are there, and their barriers exist before either one's copies arrive on them
 
   if (warp == 0) {
     // the weights do not depend on the kernels before this one: the first round of them is asked for ahead of the wait
     const int pre = num_e < STAGES ? num_e : STAGES;
     for (int e = 0; e < pre; ++e)
       if (elect_one()) tma_load_2d_pair(tiles + (uint32_t)e * STAGE_BYTES, &maps.b[pi], (kz0 + (e < nkz ? e : e - nkz)) * GBK, ch0, mapa_u32(smem_u32(&full[e]), 0));
+    pair_tmem_ready(tmem);
     pdl_wait();
     Ring at;
     for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
@@ -439,7 +524,10 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (rank == 0) {
+    pair_tmem_alloc(tmem, rank, PAIR_TMEM_COLS, abort_flag, g.status);
+    const bool there = pair_tmem_ready(tmem);
+    const uint32_t tmem_base = tmem->slot;
+    if (rank == 0 && there) {
       Ring at;
       for (int e = 0; e < num_e; ++e, at.next(STAGES)) {
         const int s = at.slot;
@@ -464,8 +552,10 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
     }
   } else {
     const int quad = warp & 3;
+    const bool there = pair_tmem_ready(tmem);
+    const uint32_t tmem_base = tmem->slot;
     pdl_wait();
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
+    const bool ok = there && __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
       const uint32_t buf = tiles + (uint32_t)quad * 2 * EPI_BUF;   // the ring has been read
@@ -486,13 +576,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       tile_out_end();
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync();      // neither CTA leaves while the other's MMAs or commits may still reach into it
-  if (warp == 1) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PAIR_TMEM_COLS) : "memory");
-  }
+  pair_tmem_end(tmem, warp, PAIR_TMEM_COLS);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -743,12 +827,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
-// Arrive on a barrier of either CTA of the cluster (address from mapa_u32).  Relaxed: it hands over no memory, but columns of TMEM, whose
-// writes are complete (tcgen05.wait::st) and ordered by the tcgen05 fences on both sides.  With .release it took 500 to 900 clocks, a slice of
-// int8 0.70 us instead of 0.50.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 // EW expander warps: 8 where two CTAs share an SM, else 16 in two groups of eight that take the slices in turn: a warp's way through a slice
 // (wait, load, expand, wait, store, hand over) is longer than the MMAs of most (512 clocks at 256 columns and one pass).
@@ -776,8 +854,8 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
   uint64_t *a_full = xempty + GQ_MAX;
   uint64_t *a_empty = a_full + GQ_MAX;
   uint64_t *acc_full = a_empty + GQ_MAX;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  PairTmem *tmem = reinterpret_cast<PairTmem *>(acc_full + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem + 1);
   const uint32_t xtiles = smem_u32(gsm + 1024), wtiles = xtiles + (uint32_t)NX * XS_BYTES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
@@ -797,26 +875,26 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
     for (int x = 0; x < NX; ++x) { mbar_init(&xfull[x], PAIR ? 1 + 8 + 1 : 1); mbar_init(&xempty[x], 1); }
     for (int e = 0; e < NE; ++e) { mbar_init(&a_full[e], 8); mbar_init(&a_empty[e], 1); }
     mbar_init(acc_full, 1);
+    if (PAIR) pair_tmem_init(tmem);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) {
-    if (PAIR) {
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(grp.tmem_cols) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(grp.tmem_cols) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+  if (!PAIR && warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem->slot)), "r"(grp.tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync();      // the barriers of both CTAs exist before anything arrives on them from the other one
+  if (PAIR) cluster_sync();      // both CTAs are there, and their barriers exist before anything arrives on them from the other one
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  pdl_trigger();
+  uint32_t tmem_base = 0;
+  if (!PAIR) {
+    tmem_base = tmem->slot;
+    pdl_trigger();
+  }
 
   if (warp == 0) {
+    if (PAIR) pair_tmem_ready(tmem);
     pdl_wait();
     Ring at;
     for (int kb = 0; kb < nkz; ++kb, at.next(NX)) {
@@ -837,16 +915,30 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
       }
     }
   } else if (warp == 2 + EW) {
+    // PAIR: the slots are filled once before the CTA's warps meet for their columns
+    const int pre = PAIR ? min(ng, NW) : 0;
+    if (PAIR) {
+      for (int kw = 0; kw < pre && lane == 0; ++kw) {
+        mbar_expect_tx(&wfull[kw], WS_BYTES);
+        tma_load_2d(wtiles + (uint32_t)kw * WS_BYTES, &maps.b[pi], (g0 + kw) * 128, ch0, &wfull[kw]);
+      }
+      __syncwarp();
+      pair_tmem_ready(tmem);
+    }
     if (lane == 0) {
       Ring at;
       for (int kw = 0; kw < ng; ++kw, at.next(NW)) {
+        if (kw < pre) continue;
         if (!mbar_wait(&wempty[at.slot], at.phase ^ 1u, abort_flag, g.status, ST_GEMM_TIMEOUT)) break;
         mbar_expect_tx(&wfull[at.slot], WS_BYTES);
         tma_load_2d(wtiles + (uint32_t)at.slot * WS_BYTES, &maps.b[pi], (g0 + kw) * 128, ch0, &wfull[at.slot]);
       }
     }
   } else if (warp == 1) {
-    if (rank == 0) {
+    if (PAIR) pair_tmem_alloc(tmem, rank, grp.tmem_cols, abort_flag, g.status);
+    const bool there = !PAIR || pair_tmem_ready(tmem);
+    if (PAIR) tmem_base = tmem->slot;
+    if (rank == 0 && there) {
       Ring ea, xa;
       for (int kb = 0; kb < nkz; ++kb, ea.next(NE), xa.next(NX)) {
         if (!PAIR && !__all_sync(0xffffffffu, mbar_wait(&a_full[ea.slot], ea.phase, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
@@ -873,7 +965,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
         __syncwarp();
       }
       if (elect_one()) { if (PAIR) umma_commit_pair(acc_full); else umma_commit(acc_full); }
-    } else if (PAIR && rank == 1 && lane == 0) {
+    } else if (PAIR && rank == 1 && there && lane == 0) {
       // An arrive in the other CTA takes some hundred clocks: this thread, which has no MMAs to issue, passes the slices of its
       // CTA's expanders on.
       Ring at;
@@ -890,9 +982,11 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
     const uint32_t swz = (uint32_t)(row & 7);
     GroupScales scales;
     if (FMT == FMT_INT4) scales.start(g, ch0 + row, kz0, nkz);
+    const bool there = !PAIR || pair_tmem_ready(tmem);
+    if (PAIR) tmem_base = tmem->slot;
     const uint32_t ta = tmem_base + ((uint32_t)(quad * 32) << 16) + grp.acc_cols + (uint32_t)part * 16;
     Ring wat, at;
-    for (int kb = 0; kb < nkz; ++kb, at.next(NE)) {
+    for (int kb = 0; there && kb < nkz; ++kb, at.next(NE)) {
       const int ks = kz0 + kb, sub = ks & (KSUB - 1);
       uint32_t s2 = 0;
       if (FMT == FMT_INT4) {
@@ -933,7 +1027,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
     // epilogue
     const int ch = ch0 + row;
     pdl_wait();
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
+    const bool ok = there && __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, g.status, ST_GEMM_TIMEOUT));
     tc_fence_after();
     if (ok) {
       const float sc = (!SLABS && g.col_scale && ch < g.N) ? __half2float(g.col_scale[ch]) : 1.f;
@@ -963,13 +1057,15 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
       tile_out_end();
     }
   }
+  if (PAIR) {
+    pair_tmem_end(tmem, warp, grp.tmem_cols);
+    return;
+  }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync();      // neither CTA leaves while the other's MMAs or commits may still reach into it
   if (warp == 1) {
     tc_fence_after();
-    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(grp.tmem_cols) : "memory");
-    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(grp.tmem_cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(grp.tmem_cols) : "memory");
   }
 }
 
