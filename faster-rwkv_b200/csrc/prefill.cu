@@ -189,6 +189,7 @@ struct GemmGroup {
   int split;                            // split-K factor (grid.z); > 1: CTAs write raw partial sums to GemmArgs::raw
   int dual;                             // few-row GEMM: some problem has A2 (the slot holds an X lo tile)
   int bn, m_tiles;                      // pair GEMM: rows of X per tile, row tiles
+  bool lock;                            // pair GEMM: two pairs fit the same SMs
   int lo_mode;                          // pair GEMM: where the low halves of X come in
   int tile_start[GEMM_GROUP_MAX + 1];   // first channel tile of each problem
   GemmArgs p[GEMM_GROUP_MAX];
@@ -355,41 +356,55 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
 // tcgen05.alloc / dealloc with cta_group::2 are one operation of a warp of each CTA, and ask that the other CTA has been launched and has not
 // left: they stand between cluster barriers.  An SM lets one CTA at a time allocate, from its allocation until it gives the permit back, so two
 // pairs that start on the same two SMs at once could each hold the permit of one SM and wait for that of the other for good (a chain of
-// products of 300 and 500 rows with a busy row kernel between them stood still, once in some million launches).  Pairs therefore take turns: the
-// even CTA takes the lock of its SM pair, tells the odd one, and gives it back when both have their columns.  The first weights are under way meanwhile.
+// products of 300 and 500 rows with a busy row kernel between them stood still, once in some million launches).  Where two pairs fit the same
+// SMs (`lock`) they take turns: the even CTA takes the lock of its SM pair, asked for while the CTA sets up, tells the odd one, and gives
+// it back when both have their columns.  The first weights are under way meanwhile.
 // Every wait is bounded: the lock's for half of what the odd CTA waits, so that one never allocates without the other.  The kernels
-// behind may start (pdl_trigger) only then: one that took the columns first would wait for this kernel with them.
+// behind may start (pdl_trigger, by every thread) only then: one that took the columns first would wait for this kernel with them.
 struct PairTmem {
   uint64_t go, there;        // the odd CTA may allocate; it has
   uint32_t sm, slot;         // this CTA's SM; address of its columns
   int held, ready;           // they are allocated; in both CTAs
 };
 constexpr int PAIR_LOCKS = 1024;
+constexpr uint32_t PAIR_ALONE_SMEM = 150u << 10;   // of 227 KB: a pair kernel without the lock asks for this much at least, one with it for 80 KB
 __device__ int pair_lock[PAIR_LOCKS];
 
+__device__ __forceinline__ uint32_t sm_id() {
+  uint32_t sm;
+  asm volatile("mov.u32 %0, %smid;" : "=r"(sm));
+  return sm;
+}
 __device__ __forceinline__ void pair_tmem_init(PairTmem *t) {   // one thread, ahead of the fence and the cluster barrier
   mbar_init(&t->go, 1);
   mbar_init(&t->there, 1);
-  uint32_t sm;
-  asm volatile("mov.u32 %0, %smid;" : "=r"(sm));
-  t->sm = sm;
+  t->sm = sm_id();
+}
+// Warp 1, ahead of the cluster barrier.  The lock is that of half the smaller SM id, which is half of this one's where a pair has SMs 2 i and 2 i + 1.
+__device__ __forceinline__ int pair_tmem_ask(uint32_t rank, bool lock) {
+  return lock && rank == 0 && (threadIdx.x & 31) == 0 ? atomicCAS(&pair_lock[sm_id() / 2 % PAIR_LOCKS], 0, 1) : 0;
 }
 __device__ __forceinline__ void pair_tmem_get(PairTmem *t, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&t->slot)), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
 // one warp of each CTA, after the cluster barrier
-__device__ __forceinline__ void pair_tmem_alloc(PairTmem *t, uint32_t rank, uint32_t cols, volatile int *abort_flag, int *status) {
+__device__ __forceinline__ void pair_tmem_alloc(PairTmem *t, uint32_t rank, bool locked, int asked, uint32_t cols, volatile int *abort_flag, int *status) {
   const int lane = threadIdx.x & 31;
   bool ok = true, ready = true;
   if (rank == 0) {
     int *lock = nullptr;
-    if (lane == 0) {
+    if (locked && lane == 0) {
       uint32_t other;
       asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other) : "r"(mapa_u32(smem_u32(&t->sm), 1)) : "memory");
-      lock = &pair_lock[min(t->sm, other) % PAIR_LOCKS];
+      int *guess = &pair_lock[sm_id() / 2 % PAIR_LOCKS];
+      lock = &pair_lock[min(t->sm, other) / 2 % PAIR_LOCKS];
+      if (lock != guess) {
+        if (asked == 0) atomicExch(guess, 0);
+        asked = atomicCAS(lock, 0, 1);
+      }
       const unsigned long long t0 = globaltimer_ns();
-      while (atomicCAS(lock, 0, 1) != 0) {
+      for (; asked != 0; asked = atomicCAS(lock, 0, 1)) {
         if (globaltimer_ns() - t0 > WAIT_LIMIT_NS / 2) {
           *abort_flag = 1;
           atomicCAS(status, 0, ST_GEMM_TIMEOUT);
@@ -403,10 +418,10 @@ __device__ __forceinline__ void pair_tmem_alloc(PairTmem *t, uint32_t rank, uint
     if (ok) {
       pair_tmem_get(t, cols);
       ready = __all_sync(0xffffffffu, mbar_wait(&t->there, 0, abort_flag, status, ST_GEMM_TIMEOUT));
-      if (lane == 0) atomicExch(lock, 0);
+      if (locked && lane == 0) atomicExch(lock, 0);
     }
   } else {
-    ok = __all_sync(0xffffffffu, mbar_wait(&t->go, 0, abort_flag, status, ST_GEMM_TIMEOUT));
+    ok = !locked || __all_sync(0xffffffffu, mbar_wait(&t->go, 0, abort_flag, status, ST_GEMM_TIMEOUT));
     if (ok) {
       pair_tmem_get(t, cols);
       if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&t->there), 0));
@@ -498,6 +513,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
     *abort_flag = 0;
     mbar_fence_init();
   }
+  const int asked = warp == 1 ? pair_tmem_ask(rank, grp.lock) : 0;
   __syncthreads();
   cluster_sync();      // both CTAs are there, and their barriers exist before either one's copies arrive on them
 
@@ -524,7 +540,7 @@ gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    pair_tmem_alloc(tmem, rank, PAIR_TMEM_COLS, abort_flag, g.status);
+    pair_tmem_alloc(tmem, rank, grp.lock, asked, PAIR_TMEM_COLS, abort_flag, g.status);
     const bool there = pair_tmem_ready(tmem);
     const uint32_t tmem_base = tmem->slot;
     if (rank == 0 && there) {
@@ -935,7 +951,7 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
       }
     }
   } else if (warp == 1) {
-    if (PAIR) pair_tmem_alloc(tmem, rank, grp.tmem_cols, abort_flag, g.status);
+    if (PAIR) pair_tmem_alloc(tmem, rank, false, 0, grp.tmem_cols, abort_flag, g.status);   // (no other pair fits the SMs: launch_gemm_q)
     const bool there = !PAIR || pair_tmem_ready(tmem);
     if (PAIR) tmem_base = tmem->slot;
     if (rank == 0 && there) {
@@ -2368,7 +2384,8 @@ cudaError_t launch_gemm_pair(const GemmArgs *probs, int n, cudaStream_t st, int 
   const bool alone = tiles * grp.m_tiles * grp.split <= num_pairs;
   grp.stages = std::min<int>(PAIR_MAX_STAGES, (int)((alone ? 200u << 10 : 110u << 10) / grp.stage_bytes));
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
-  const size_t smem = 1024 + (size_t)grp.stages * grp.stage_bytes + 1024;
+  const size_t smem = std::max<size_t>(1024 + (size_t)grp.stages * grp.stage_bytes + 1024, alone ? PAIR_ALONE_SMEM : 0);
+  grp.lock = smem < PAIR_ALONE_SMEM;
   cudaError_t e = launch_cluster_k(grp.split > 1 ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, 2, dim3(2 * tiles * grp.m_tiles, 1, grp.split), dim3(G_THREADS), smem, st, maps, grp);
   if (e != cudaSuccess) return e;
   if (defer_split) *defer_split = grp.split;
@@ -2457,7 +2474,10 @@ cudaError_t launch_gemm_q(const GemmArgs *probs, int n, cudaStream_t st, int *de
   if (!make_out_maps(maps, grp)) return cudaErrorNotSupported;
   const size_t rings = (size_t)grp.xstages * grp.stage_bytes + (size_t)grp.stages * ws;
   const int ew = two_per_sm ? 8 : 16;
-  const size_t smem = 1024 + std::max<size_t>(rings, ew * 2 * EPI_BUF) + 1024;
+  size_t smem = 1024 + std::max<size_t>(rings, ew * 2 * EPI_BUF) + 1024;
+  // No CTA of another pair kernel shares an SM with one of these (gemm_pair_kernel's take 82 KB at least), which therefore need no lock for
+  // their allocation.
+  if (pair) smem = std::max(smem, (size_t)PAIR_ALONE_SMEM);
   auto kern = grp.split > 1 ? gemm_q_kern<true>(fmt, pair, two_per_sm) : gemm_q_kern<false>(fmt, pair, two_per_sm);
   const dim3 grid((pair ? 2 : 1) * tiles * grp.m_tiles, 1, grp.split);
   cudaError_t e = launch_cluster_k(kern, pair ? 2 : 1, grid, dim3(gq_threads(ew)), smem, st, maps, grp);
