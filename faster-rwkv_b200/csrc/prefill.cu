@@ -1034,6 +1034,10 @@ gemm_q_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ Gem
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(PAIR && rank == 0 ? &xfull[at.slot] : &a_full[at.slot]);
+      } else if (kb == 0 && sub == KSUB - 1) {
+        // The first weight slot of a K range may hold one slice, the other group's.  This group waits for it all the same: where it is
+        // back at this slot before the slot's first load is there, its wait for the second one would pass on the phase before both.
+        if (!__all_sync(0xffffffffu, mbar_wait(&wfull[0], 0, abort_flag, g.status, ST_GEMM_TIMEOUT))) break;
       }
       if (sub == KSUB - 1) {
         if (lane == 0) mbar_arrive(&wempty[wat.slot]);   // (the last slot of this K range is not asked for again)

@@ -63,6 +63,30 @@ def test_streams_over_pair_tiles(pkg, orc, synth, name, fmt, B):
     m.close()
 
 
+def test_int8_weight_slots_of_which_one_group_has_nothing(pkg, orc, synth):
+    """int8 products whose expanders work in two groups (65 to 128 streams; more than 128 tokens, on pairs of SMs) over a range of K that
+    starts at an odd slice and is long enough for the ring of weight slots to come round: its first slot holds one slice alone, the other
+    group's.  Attention projections of 100 streams: three ranges of 32 slices on 148 SMs; ffn value of 200 tokens: nine of 124."""
+    shape = synth.Shape("4", 1, 2048, 7936, 96)
+    k1 = shape.n_embd // 64
+    cuts = [z * k1 // 3 for z in range(4)]
+    assert any(a % 2 == 1 and b - a >= 8 for a, b in zip(cuts, cuts[1:])), cuts
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), "fp32")
+    ref = orc.OracleModel(shape, tensors, synth.param_names(shape), rescale_every=0, weight_format="int8", state_fp16=False)
+    m = pkg.Model(tensors, "cuda int8", shape=shape, max_batch=100)
+    ids = synth.token_ids(shape, 2 * 100, seed=9).reshape(2, 100)
+    got = [m.decode(ids[t]) for t in range(2)]
+    for b in (0, 64, 99):
+        ref.reset()
+        for t in range(2):
+            _close(got[t][b], ref.run(int(ids[t, b])), f"int8 stream {b} step {t}")
+    m.reset_states()
+    ref.reset()
+    prompt = [int(t) for t in ids.reshape(-1)]
+    _close(m.run(prompt), ref.run_seq(prompt), "int8 prompt of 200 tokens")
+    m.close()
+
+
 @pytest.mark.parametrize("fmt", ["fp16", "int4"])
 def test_eight_streams_of_a_wide_model_take_the_gemm_path(pkg, orc, synth, fmt):
     """A model whose channel-mix width does not leave room for 8 streams in the persistent kernel's shared memory
