@@ -491,14 +491,8 @@ int fr_b200_create(const fr_b200_config *cfg, fr_b200_model **out) {
   }
   if (!rc) rc = alloc((void **)&m->d_out, m->out_bytes());
   if (!rc) rc = alloc((void **)&m->d_amax, (size_t)B * 8);
-  // fp16 W^T copies now for RWKV-5.x (seq kernels) and for models whose largest batch goes by rows; else on demand
-  if (!rc && m->plain_halfs && m->row_copies && (m->v5 || m->rows_planned)) {
-    rc = alloc((void **)&m->d_plain, m->plain_halfs * 2);
-    if (rc && !m->v5 && !m->rows_needed) {   // the persistent kernels take every batch of this model
-      cudaGetLastError();
-      m->d_plain = nullptr; m->rows_planned = false; rc = 0;
-    }
-  }
+  // fp16 W^T copies now where the model cannot do without (RWKV-5.x prompts, batches that no other kernel takes); else in finalize or on demand
+  if (!rc && m->plain_halfs && m->row_copies && (m->v5 || m->rows_needed)) rc = alloc((void **)&m->d_plain, m->plain_halfs * 2);
   if (!rc && m->qcopy_bytes) rc = alloc((void **)&m->d_qcopy, m->qcopy_bytes);
   if (!rc && m->qscale_halfs) rc = alloc((void **)&m->d_qscale, m->qscale_halfs * 2);
   if (!rc && m->pscale_halfs) rc = alloc((void **)&m->d_pscale, m->pscale_halfs * 2);
@@ -600,7 +594,10 @@ int fr_b200_set_tensor(fr_b200_model *m, const char *name, const void *data, int
   return fail(FR_B200_E_ARG, "unknown tensor name " + nm);
 }
 
-namespace { int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids, int R, cudaStream_t st); }
+namespace {
+int ensure_row_copies(fr_b200_model *m);
+int rows_forward(fr_b200_model *m, bool batch_mode, int slot, const int32_t *ids, int R, cudaStream_t st);
+}
 
 int fr_b200_finalize(fr_b200_model *m) {
   if (!m) return fail(FR_B200_E_ARG, "null model");
@@ -725,10 +722,12 @@ int fr_b200_finalize(fr_b200_model *m) {
     hp.kind = PH_MATVEC; hp.rot = 0;
     CU(cudaMemcpy(m->d_head_phase, &hp, sizeof(hp), cudaMemcpyHostToDevice));
   }
-  // a few streams that go by rows find their buffers, as those of the persistent kernels do (3 int4 streams of the 1.5B shape: the first
-  // step took 1.5 ms, 0.3 of them for this; larger batches and prompts size theirs when they come)
-  if (m->rows_planned && !m->rows_needed && (m->d_plain || m->d_qcopy)) {
-    const int rc = rows_forward(m, true, 0, nullptr, m->cfg.max_batch, nullptr);
+  // Batches that go by rows although the persistent kernels take them, too, find their copies and their buffers, as those kernels do (3 int4
+  // streams of the 1.5B shape: the first step took 1.5 ms, 0.3 of them for the buffers; larger batches and prompts size theirs when they
+  // come).  They come last: what the model cannot do without has its memory by now, and without room for them it loads all the same.
+  if (m->rows_planned && !m->rows_needed) {
+    int rc = ensure_row_copies(m);
+    if (!rc) rc = rows_forward(m, true, 0, nullptr, m->cfg.max_batch, nullptr);
     if (rc && rc != FR_B200_E_NOMEM) return rc;
   }
   m->finalized = true;

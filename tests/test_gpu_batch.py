@@ -356,6 +356,40 @@ def test_replays_of_captured_row_steps(pkg, synth, name, fmt, B):
     m.close()
 
 
+def test_loading_with_room_for_one_copy_of_the_weights(pkg, synth, monkeypatch):
+    """Eight streams of an fp16 RWKV-4 model go by rows, from a second copy of the weights, though the persistent kernel takes them as well:
+    that copy must not take the memory of a model that loads without it.  272 MiB of weights, 64 of embedding and 64 to upload the largest
+    matrix: 400 MiB.  A copy of 272 made between the first two fits and leaves too little (from 544 on, below 672); made last it
+    does not fit below 608, and need not."""
+    import gc
+    import torch
+    shape = synth.Shape("4", 8, 1024, 4096, 32768)
+    tensors = synth.to_file_dtypes(shape, synth.generate(shape, seed=11, ln_random=True), "fp16")
+    ids = synth.token_ids(shape, 8, seed=9)
+
+    def logits():
+        m = pkg.Model(tensors, "cuda fp16", shape=shape, max_batch=8)
+        got = m.decode(ids)
+        m.close()
+        return got
+
+    want = logits()                      # what a first load leaves on the device is there
+    monkeypatch.setenv("FR_B200_ROW_COPIES", "0")
+    alone = logits()                     # the persistent kernel takes eight such streams
+    monkeypatch.delenv("FR_B200_ROW_COPIES")
+    gc.collect()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    taken = torch.empty(free - (576 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = logits()
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+    assert np.array_equal(got, alone)
+    _close(got, want, "persistent kernel against rows")
+
+
 def test_small_and_large_batches_share_state(pkg, orc, synth):
     """The persistent kernel (<= 8 streams) and the GEMM path (> 8) read and write the same state slots, and streams
     that are decoded together need not have seen the same number of tokens (continuous batching: a stream joins a
