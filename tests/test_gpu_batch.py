@@ -175,6 +175,25 @@ def test_argmax_of_rows_with_ties(pkg, synth, vocab):
     m.close()
 
 
+@pytest.mark.parametrize("rows", [9, 100, 200, 300])
+def test_argmax_of_rows_with_infinities_and_nan(pkg, synth, rows):
+    """8, 4, 2 and 1 CTAs per row; head entries of +inf, -inf and NaN, so that rows hold infinities of either sign and NaN.  The order is
+    that of the bit patterns, sign and magnitude (as in the persistent kernels): the logits of the same step say which id that is."""
+    shape = synth.Shape("4", 1, 128, 256, 5001)
+    tensors = synth.generate(shape, seed=3, ln_random=True)
+    ids = synth.token_ids(shape, rows, seed=6)
+    for cols in ({77: np.inf, 78: -np.inf}, {4990: np.nan}, {c: -np.inf for c in range(0, 5001, 2)}):
+        head = tensors["head.weight"].copy()
+        for c, v in cols.items():
+            head[0, c] = v
+        m = pkg.Model(synth.to_file_dtypes(shape, {**tensors, "head.weight": head}, "fp16"), "cuda fp16", shape=shape, max_batch=rows)
+        bits = m.decode(ids).view(np.uint32)
+        want = np.where(bits >> 31, ~bits, bits | 0x80000000).argmax(1)
+        m.reset_states()
+        assert np.array_equal(m.decode(ids, want_logits=False, want_argmax=True), want), sorted(cols)[:2]
+        m.close()
+
+
 @pytest.mark.parametrize("name,fmt,B", [("tiny4b", "fp16", 8), ("tiny4", "int4", 5)])
 def test_a_captured_step_of_few_streams(pkg, synth, name, fmt, B):
     """5 to 8 RWKV-4 streams on a stream that is being captured: the first such step (by rows, whose buffers came with the model) can be
