@@ -159,7 +159,9 @@ struct Ring {
   }
 };
 
-// the result is rounded to fp16: the fast exponential and division are exact enough
+// By the fast exponential (2 + 1.17 |v| ulp by CUDA's bounds) and division (2 ulp): a relative error of up to 5e-7 for v > 0 and 1.7e-6 at
+// v = -8, where the value is 3e-4.  The fp16 rounding of a single result (4.9e-4) hides it; where the low half is stored as well (streams, short
+// fp16 prompts: 2.4e-7) it is the larger part of the error.
 __device__ __forceinline__ float sigmoid_g(float v) { return __fdividef(1.f, 1.f + __expf(-v)); }
 
 template <int EPI>
@@ -464,7 +466,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
 // of its own with the same 128 x 256 accumulator would fetch, and read from shared memory at every MMA, all 32 KB of X.
 // Two CTAs per SM (3 slots of 32 KB and 256 TMEM columns each): the start and the end of one hide in part behind the main loop
 // of the other, and tiles are handed out by the hardware, also across the two row pieces of a long prompt.
-// [2048 x 2560] x [2560 x 11520] with the relu^2 epilogue: 104 us (1,160 TFLOP/s) at 256 rows a tile; 256 x 256 tiles of single CTAs,
+// [2048 x 2560] x [2560 x 11520] with the relu^2 epilogue: 104 us back to back (1,160 TFLOP/s; a single launch 94 to 95) at 256 rows a tile; 256 x 256 tiles of single CTAs,
 // whose epilogue nothing hid, 182.  Without its epilogue 82, without its loads 100 (of 107 then): the epilogue is what is left.  One
 // CTA per SM over all tiles with two accumulators: 92, but products of one wave 10 to 40 % slower, a prompt of 4,096 36.4 ms against 35.0.
 //   warp 0: TMA into the own shared memory; the bytes of both CTAs are counted on the even CTA's barrier
@@ -2323,7 +2325,8 @@ cudaError_t launch_gemm_wt(const GemmArgs *probs, int n, cudaStream_t st, int *d
   return cudaGetLastError();
 }
 // Costs in clocks, fitted to products of 256 and 1000 rows (2048 x 2048 up to 65536 x 2048 and 2048 x 8192) with 64 to 256 columns
-// and 1 to 9 cuts, within 10 % of the times.
+// and 1 to 9 cuts, within 10 % of the times of these.  Products of other widths are cut by the same constants; whether another cut would
+// be faster there has not been looked at.
 // Slabs: the next kernel reads them at about 2,500 bytes a clock; without one that does, a finishing pass is launched.
 float slab_cost(int split, int M, int sum_n, bool deferred) {
   return split > 1 ? (deferred ? 0.f : 8000.f) + (float)split * (float)M * (float)sum_n * 4.f / 2500.f : 0.f;
